@@ -63,7 +63,12 @@ extern "C" {
  * heuristic; the autotuner (mg_autotune, driven by meshes_gb300/autotune.py) measures better choices. */
 typedef struct mg_config {
   int M, V, W, CL, S;
-  int split;   /* 0: automatic, 1: two CTA kinds per SM (V and V-1 vectors per lane group), 2: uniform CTAs */
+  int split;   /* 0: automatic, 1: two CTA kinds per SM (V and V-1 vectors per lane group), 2: uniform CTAs,
+                * 3: warp pairs, 4: two CTAs per SM, 5: framed (crossings with a unit diagonal; CL and S are those of
+                * its pipeline), 6: framed, the warps of a CTA holding V and V-1 vectors in turn.  Without a
+                * configuration a nearest-neighbour MZI mesh of 64 < N takes a framed launch where that is faster; it
+                * computes with fields scaled by up to 2^22 either way, so magnitudes beyond about 1e30 (1e25 for a
+                * product of field and gradient) overflow in it */
 } mg_config;
 
 /* ---- library ---------------------------------------------------------------------------- */

@@ -21,6 +21,7 @@
 #include "mg_reduce.cuh"
 #include "mg_inst_table.h"
 #include "mg_launch.h"
+#include "mg_framed_args.cuh"
 
 using namespace mg;
 
@@ -113,6 +114,9 @@ struct Plan {
   unsigned lb, dlb;
   size_t smem;
   size_t off_kinds, off_tiles, off_dtiles, off_partial, total;
+  bool framed;      // unit-diagonal crossings on the frame pass's tiles (mg_framed.cuh)
+  size_t off_main, off_resc, off_gam, off_wts, off_dfin, off_fkinds, off_tdiag, off_toff, off_tmag, off_tcs, off_count;
+  int fcl, fs;      // layers per stage and stages of the framed pipeline (CL, S: of the unframed body in the same kernel)
   bool perm;        // MG_GEO_PERM: permutation tables at off_perm, gather scratch after the smem layout
   size_t off_perm;
 };
@@ -124,8 +128,12 @@ size_t perm_table_bytes(int N, int L) { return 4 * (2 * (size_t)(L + 1) * N + 2 
 // Shared memory of a launch of plan P over L layers, with the permutation scratch when P has one.
 size_t launch_smem(const Plan& P, int op, int gslot, int L) {
   const size_t b = prop_smem_bytes(op, gslot, P.M, P.G, P.W, P.CL, P.S, P.lb, P.dlb, L);
+  if (P.framed) return std::max(b, framed_smem_bytes(op, P.np2, P.W, P.fcl, P.fs, L));
   return P.perm ? perm_scratch_offset(b) + perm_scratch_bytes(P.W, P.M, P.real) : b;
 }
+
+// Layers without their partner from which on a mesh takes the unframed body: each costs the framed one a layer of zeros
+int framed_refuse(int L) { return std::max(4, L / 2); }
 
 // (M, V) instantiated for the stored-activation kernels (GR 4), by op (FWD writes, BWD reads)
 bool instantiated_stored(int op, int M, int V) {
@@ -172,6 +180,12 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   p.gr = stored ? 4 : (op != OP_BWD) ? 0 : (crossing == CR_MZI ? 1 : (crossing == CR_ORTH ? 2 : 0));
   const bool wide = N > 512;
   const int Np = wide ? 32 * kWideM : pow2ceil(N);
+  // framed launch: nearest-neighbour complex meshes whose vector fills the warp at M >= 4, forward and MZI
+  // back-propagation with direct gradients
+  const bool may_frame = !stored && !perm && geometry == GEO_NN && N > 64 && L > 0 && L <= kMaxSmemKinds &&
+                         (crossing == CR_MZI ? op != OP_FWDDIFF : crossing == CR_SYM && op == OP_FWD);
+  mg_config fc;
+  if (!cfg && may_frame && framed_pays(op, Np / 32, L, Np / 2, B, di.sms) && framed_pick(op, Np / 32, B, di.sms, &fc)) cfg = &fc;
   int M = (cfg && cfg->M) ? cfg->M : (wide ? kWideM : std::max(std::min(8, Np), Np / 32));
   if (wide ? M != kWideM : (M < 2 || M > 16 || (M & (M - 1))))
     return fail(MG_E_CONFIG, "modes per lane M=%d not in %s", M, wide ? "{20} for N > 512" : "{2,4,8,16}");
@@ -187,6 +201,10 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   if (perm && stored) return fail(MG_E_ARG, "stored-activation back-propagation takes no permutations");
   // warp-pair launch (split 3): back-propagation of a nearest-neighbour complex mesh with a full-warp M = 8 plan
   const int split_mode = cfg ? cfg->split : 0;
+  p.framed = split_mode == 5 || split_mode == 6;
+  if (p.framed && !(may_frame && framed_instantiated(op, M, V, G == 32, split_mode == 6)))
+    return fail(MG_E_CONFIG, "no framed kernel for op=%d crossing=%d geometry=%d M=%d G=%d V=%d", op, crossing, geometry,
+                M, G, V);
   p.pair = split_mode == 3;
   p.occ2 = split_mode == 4;
   if (p.occ2 && (stored || perm || geometry != GEO_NN || G != 32 || !nn2_instantiated(op, crossing == CR_ORTH, M, V, p.gr)))
@@ -197,7 +215,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
     if (stored || perm || geometry != GEO_NN || G != 32 || !pair_instantiated(op, crossing == CR_ORTH, M, V, p.gr, true))
       return fail(MG_E_CONFIG, "no warp-pair kernel for op=%d crossing=%d geometry=%d M=%d G=%d V=%d", op, crossing,
                   geometry, M, G, V);
-  } else if (p.occ2) {
+  } else if (p.occ2 || p.framed) {
   } else if (wide ? (perm || stored || !wide_instantiated(op, crossing == CR_ORTH, V, p.gr))
            : perm ? !perm_instantiated(op, crossing == CR_ORTH, M, V, p.gr)
                   : (stored ? !instantiated_stored(OP_BWD, M, V)
@@ -214,7 +232,9 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   // 17x those of the uniform launch).
   p.split = false;
   p.nA = 0;
-  if (split_mode != 2 && !p.pair && !p.occ2 && (op == OP_FWD || op == OP_BWD) && V >= 2 && !stored && !perm &&
+  if (p.framed) {
+    p.split = split_mode == 6;   // mixed warps (V and V - 1 vectors) in every CTA
+  } else if (split_mode != 2 && !p.pair && !p.occ2 && (op == OP_FWD || op == OP_BWD) && V >= 2 && !stored && !perm &&
       split_instantiated(op, crossing == CR_ORTH, M, V, G == 32, p.gr)) {
     const long ws = (cfg && cfg->W) ? cfg->W : 4;
     const long capA = ws * p.R * V, capB = ws * p.R * (V - 1);
@@ -227,8 +247,9 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   p.dlb = (op == OP_BWD && p.gr == 0) ? (unsigned)(p.np2 * (p.real ? 16 : 64)) : 0;
   const int gslot = (op != OP_BWD) ? 0 : ((p.gr == 1 || p.gr == 2) ? 8 : (p.real ? 16 : 32));
   const size_t gstl = (size_t)p.np2 * gslot;
-  const int maxw = p.occ2 ? 8 : prop_max_threads(op, M, V) / 32;
-  int W = (cfg && cfg->W) ? cfg->W : (p.split ? 4 : (p.pair || p.occ2) ? 8 : 0);
+  const int maxw = p.framed ? framed_max_threads(M, V) / 32 : p.occ2 ? 8 : prop_max_threads(op, M, V) / 32;
+  int W = (cfg && cfg->W) ? cfg->W : p.framed ? 8 : (p.split ? 4 : (p.pair || p.occ2) ? 8 : 0);
+  if (p.framed && p.split && W % 8) return fail(MG_E_CONFIG, "mixed warps need W a multiple of 8, got %d", W);
   if (p.pair && (W & 1)) return fail(MG_E_CONFIG, "a warp-pair launch needs an even W, got %d", W);
   if (!W) {
     // enough warps to cover the batch in one wave, rounded up to a multiple of 4 so the four
@@ -243,14 +264,23 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   int S = (cfg && cfg->S) ? cfg->S : ((op == OP_FWD || p.split) ? 2 : 3);
   if (S < 1 || S > 8) return fail(MG_E_CONFIG, "S=%d stages outside [1, 8]", S);
   // a split launch keeps two CTAs resident per SM (each also pays the 1 KB the SM reserves per CTA)
-  const size_t budget = (p.split || p.occ2) ? (size_t)di.smem_per_sm / 2 - 1024 : (size_t)di.smem_optin - 1024;
+  const size_t budget = ((p.split && !p.framed) || p.occ2) ? (size_t)di.smem_per_sm / 2 - 1024 : (size_t)di.smem_optin - 1024;
   int CL = (cfg && cfg->CL) ? cfg->CL : 0;
   const size_t per_layer = (size_t)S * p.lb + p.dlb + W * gstl;
   const size_t fixed = 8 * (size_t)(S + 1) + (L <= kMaxSmemKinds ? 4 * (size_t)L : 0) +
                        (perm ? 16 + perm_scratch_bytes(W, M, p.real) : 0);
+  if (p.framed) {
+    // the configuration's CL and S are the framed pipeline's: as many layers per stage as fit, whole pairs
+    p.fs = (cfg && cfg->S) ? S : 2;
+    p.fcl = CL ? CL : std::max(1, std::min(L, 64));
+    while (p.fcl > 1 && framed_smem_bytes(op, p.np2, W, p.fcl, p.fs, L) > budget) --p.fcl;
+    if (!CL && p.fcl > 4) p.fcl &= ~3;
+    S = 2;
+    CL = 0;
+  }
   if (!CL) {
     // forward: deep enough to hide the copies, shallow enough to start soon (split CTAs: about 68 KB measured best)
-    const size_t target = (op == OP_BWD) ? budget : std::min<size_t>(budget, (p.split ? 68 : 160) * 1024);
+    const size_t target = (op == OP_BWD) ? budget : std::min<size_t>(budget, (p.split && !p.framed ? 68 : 160) * 1024);
     CL = (int)std::max<size_t>(1, std::min<size_t>(16, (target > fixed ? target - fixed : 0) / per_layer));
     if (L > 0) CL = std::min(CL, L);
     // a uniform forward launch whose tiles all fit the target takes them in one copy and one stage: no chunk
@@ -267,11 +297,14 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
     return fail(MG_E_CONFIG, "shared memory %zu B above the %zu B available (M=%d W=%d CL=%d S=%d)", p.smem, budget, M,
                 W, CL, S);
   if (p.lb % 16 || p.dlb % 16) return fail(MG_E_CONFIG, "tile sizes %u/%u not multiples of 16 bytes", p.lb, p.dlb);
-  if ((size_t)CL * p.lb >= (1u << 20) || (size_t)CL * p.dlb >= (1u << 20))
+  if ((size_t)CL * std::max<size_t>(p.lb, 40 * (size_t)p.np2) >= (1u << 20) || (size_t)CL * p.dlb >= (1u << 20))
     return fail(MG_E_CONFIG, "one pipeline stage exceeds the 1 MB bulk-copy limit");
   const long per_cta = p.pair ? (long)(W / 2) * V : (long)W * p.R * V;
   p.grid = (int)((B + per_cta - 1) / per_cta);
-  if (p.split) {
+  if (p.framed) {
+    const long cap = framed_cta_vectors(W, p.R, V, p.split);
+    p.grid = (int)((B + cap - 1) / cap);
+  } else if (p.split) {
     const long capB = (long)W * p.R * (V - 1);
     const long nA = std::min<long>(di.sms, (B + per_cta - 1) / per_cta);
     const long rem = std::max<long>(0, (long)B - nA * per_cta);
@@ -284,6 +317,22 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   p.off_perm = p.off_dtiles + align256((size_t)L * p.dlb);
   p.off_partial = p.off_perm + (perm ? align256(perm_table_bytes(N, L)) : 0);
   p.total = p.off_partial + ((op == OP_BWD) ? align256((size_t)p.grid * L * p.np2 * (p.gr == 4 ? 32 : 8)) : 0);
+  if (p.framed) {
+    const size_t n = (size_t)L * p.np2;
+    const bool bwd = op == OP_BWD;
+    p.off_main = p.total;
+    p.off_resc = p.off_main + align256(16 * n);
+    p.off_gam = p.off_resc + align256(16 * n);
+    p.off_wts = p.off_gam + (bwd ? align256(8 * n) : 0);
+    p.off_dfin = p.off_wts + (bwd ? align256(8 * n) : 0);
+    p.off_fkinds = p.off_dfin + align256(16 * (size_t)p.np2);
+    p.off_tdiag = p.off_fkinds + align256(4 * (size_t)L);
+    p.off_toff = p.off_tdiag + align256(32 * n);
+    p.off_tmag = p.off_toff + align256(32 * n);
+    p.off_tcs = p.off_tmag + align256(8 * n);
+    p.off_count = p.off_tcs + (bwd ? align256(8 * n) : 0);
+    p.total = p.off_count + 256;
+  }
   return MG_OK;
 }
 
@@ -329,6 +378,17 @@ CoefArgs coef_args(const Plan& P, const int* lens, const int* shifts, const int*
   a.dtiles = ws + P.off_dtiles; a.dlayer_bytes = P.dlb;
   a.kinds = reinterpret_cast<int*>(ws + P.off_kinds);
   a.status = reinterpret_cast<int*>(ws);
+  a.tdiag = a.toff = nullptr;
+  a.tmag = nullptr;
+  a.tcs = nullptr;
+  a.fcount = nullptr;
+  if (P.framed) {
+    a.tdiag = reinterpret_cast<float4*>(ws + P.off_tdiag);
+    a.toff = reinterpret_cast<float4*>(ws + P.off_toff);
+    a.tmag = reinterpret_cast<float*>(ws + P.off_tmag);
+    a.fcount = reinterpret_cast<int*>(ws + P.off_count);
+    if (P.op == OP_BWD) a.tcs = reinterpret_cast<float2*>(ws + P.off_tcs);
+  }
   return a;
 }
 
@@ -351,9 +411,28 @@ int build_tiles(const Plan& P, const int* lens, const int* shifts, const int* st
   const int sms = dev_info().sms;
   int bt = 256;
   if (n < 256 * sms) bt = std::max(32, std::min(256, ((n + sms - 1) / sms + 31) / 32 * 32));
-  if (quad) coef_kernel<true><<<(n + bt - 1) / bt, bt, 0, st>>>(a);
-  else coef_kernel<false><<<(n + bt - 1) / bt, bt, 0, st>>>(a);
+  const int blocks = (n + bt - 1) / bt;
+  if (quad) P.framed ? coef_kernel<true, true><<<blocks, bt, 0, st>>>(a) : coef_kernel<true, false><<<blocks, bt, 0, st>>>(a);
+  else P.framed ? coef_kernel<false, true><<<blocks, bt, 0, st>>>(a) : coef_kernel<false, false><<<blocks, bt, 0, st>>>(a);
   cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && P.framed) {
+    FrameArgs f{};
+    f.L = P.L; f.M = P.M; f.G = P.G;
+    f.bwd = P.op == OP_BWD;
+    f.tdiag = a.tdiag;
+    f.toff = a.toff;
+    f.tmag = a.tmag;
+    f.tcs = a.tcs;
+    f.kinds = a.kinds;
+    f.main = reinterpret_cast<float4*>(ws + P.off_main);
+    f.count = a.fcount;
+    f.resc = reinterpret_cast<float4*>(ws + P.off_resc);
+    f.gam = reinterpret_cast<float4*>(ws + P.off_gam);
+    f.wts = reinterpret_cast<float4*>(ws + P.off_wts);
+    f.dfin = reinterpret_cast<float2*>(ws + P.off_dfin);
+    f.fkinds = reinterpret_cast<int*>(ws + P.off_fkinds);
+    e = launch_frames(f, sms, st);
+  }
   return e == cudaSuccess ? MG_OK : cuda_fail(e, "coef_kernel launch");
 }
 
@@ -410,7 +489,21 @@ int run_prop(const Plan& P, const void* in0, const void* in1, void* out0, void* 
   lc.smem = P.smem;
   lc.stream = st;
   cudaError_t e;
-  if (P.pair)
+  if (P.framed) {
+    FramedArgs f;
+    static_cast<PropArgs&>(f) = a;
+    f.main = reinterpret_cast<const float4*>(ws + P.off_main);
+    f.resc = reinterpret_cast<const float4*>(ws + P.off_resc);
+    f.gam = reinterpret_cast<const float4*>(ws + P.off_gam);
+    f.dfin = reinterpret_cast<const float2*>(ws + P.off_dfin);
+    f.fkinds = reinterpret_cast<const int*>(ws + P.off_fkinds);
+    f.count = reinterpret_cast<const int*>(ws + P.off_count);
+    f.fcl = P.fcl;
+    f.fs = P.fs;
+    f.xr = framed_resc_rows(P.fcl);
+    f.refuse = framed_refuse(P.L);
+    e = launch_prop_framed(P.op, P.M, P.V, P.split, lc, f);
+  } else if (P.pair)
     e = launch_prop_pair(P.V, lc, a);
   else if (P.occ2)
     e = launch_prop_nn2(P.op, P.real, P.M, P.V, P.gr, lc, a);
@@ -424,10 +517,15 @@ int run_prop(const Plan& P, const void* in0, const void* in1, void* out0, void* 
   if (e != cudaSuccess) return cuda_fail(e, "prop_kernel launch");
   if (P.op == OP_BWD && dp && P.L > 0) {
     const int n = P.L * P.np2;
+    const int* geo = reinterpret_cast<const int*>(ws + P.off_kinds) + P.L;
+    if (P.framed) {
+      e = launch_framed_reduce(a.partial, P.grid, P.L, P.np2, P.M, P.G, P.N, dp, ldp, accumulate, geo,
+                               reinterpret_cast<const float2*>(ws + P.off_wts),
+                               reinterpret_cast<const int*>(ws + P.off_count), framed_refuse(P.L), st);
+      return e == cudaSuccess ? MG_OK : cuda_fail(e, "framed_reduce_kernel launch");
+    }
     dp_reduce_kernel<<<(n + kReduceCols - 1) / kReduceCols, kReduceCols * kReduceRows, 0, st>>>(
-        a.partial, P.grid, P.L, P.np2, P.M, P.G, P.N, dp, ldp,
-                                                        crossing_np(P.crossing), accumulate,
-                                                        reinterpret_cast<const int*>(ws + P.off_kinds) + P.L);
+        a.partial, P.grid, P.L, P.np2, P.M, P.G, P.N, dp, ldp, crossing_np(P.crossing), accumulate, geo);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "dp_reduce_kernel launch");
   }
@@ -741,13 +839,22 @@ int mg_propagate(int op, int N, int L, int B, int crossing, int geometry, const 
     mg_config cf = {Pb.M, 0, 0, 0, 0, (cfg && cfg->split != 3 && cfg->split != 4) ? cfg->split : 0};
     mg_config tf;   // a measured forward configuration of this shape applies if its M matches the tiles'
     if (!cfg && !Pb.perm && lookup_tuned(OP_FWD, crossing, Pb.geometry, N, B, &tf) && tf.M == Pb.M) cf = tf;
+    if (Pb.framed) framed_pick(OP_FWD, Pb.M, B, dev_info().sms, &cf);
+    else if (cf.split >= 5) cf = {Pb.M, 0, 0, 0, 0, 2};
     TRY(make_plan(OP_FWD, N, L, B, crossing, geometry, &cf, &Pf));
+    if (Pb.framed) {
+      Pf.off_main = Pb.off_main;
+      Pf.off_resc = Pb.off_resc;
+      Pf.off_dfin = Pb.off_dfin;
+      Pf.off_fkinds = Pb.off_fkinds;
+      Pf.off_count = Pb.off_count;
+    }
     Pf.lb = Pb.lb;
     Pf.off_kinds = Pb.off_kinds;
     Pf.off_tiles = Pb.off_tiles;
     Pf.off_perm = Pb.off_perm;   // the forward rows of the tables mg_build_perms wrote for this workspace
     const DevInfo di = dev_info();
-    const size_t budget = Pf.split ? (size_t)di.smem_per_sm / 2 - 1024 : (size_t)di.smem_optin - 1024;
+    const size_t budget = Pf.split && !Pf.framed ? (size_t)di.smem_per_sm / 2 - 1024 : (size_t)di.smem_optin - 1024;
     for (;;) {
       Pf.smem = launch_smem(Pf, OP_FWD, 0, L);
       if (Pf.smem <= budget && (size_t)Pf.CL * Pf.lb < (1u << 20)) break;
@@ -788,7 +895,7 @@ int mg_propagate_wait_test(int op, int N, int L, int B, int crossing, const void
   TRY(check_field(in1, "in1", P.real, op == OP_BWD && B > 0));
   TRY(check_field(out0, "out0", P.real, op != OP_BWD && B > 0));
   TRY(check_field(out1, "out1", P.real, op != OP_FWD && B > 0));
-  const int nch = (L + P.CL - 1) / P.CL;
+  const int cl = P.framed ? P.fcl : P.CL, nch = (L + cl - 1) / cl;
   if (unarmed_chunk < 0 || unarmed_chunk >= nch)
     return fail(MG_E_ARG, "unarmed_chunk=%d outside the launch's %d pipeline chunks", unarmed_chunk, nch);
   return run_prop(P, in0, in1, out0, out1, ldu, nullptr, 0, 0, static_cast<unsigned char*>(ws),
@@ -846,7 +953,7 @@ int mg_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_co
   Plan P;
   TRY(make_plan(op, N, L, B, crossing, geometry, cfg, &P));
   if (out) {
-    out->M = P.M; out->V = P.V; out->W = P.W; out->CL = P.CL; out->S = P.S; out->G = P.G; out->grid = P.grid;
+    out->M = P.M; out->V = P.V; out->W = P.W; out->CL = P.framed ? P.fcl : P.CL; out->S = P.framed ? P.fs : P.S; out->G = P.G; out->grid = P.grid;
     out->nA = P.split ? P.nA : 0;
     out->layer_bytes = P.lb; out->dlayer_bytes = P.dlb; out->smem = P.smem;
     out->off_kinds = P.off_kinds; out->off_tiles = P.off_tiles; out->off_dtiles = P.off_dtiles;

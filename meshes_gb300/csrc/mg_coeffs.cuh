@@ -38,6 +38,14 @@ struct CoefArgs {
   unsigned dlayer_bytes;
   int* kinds;            // [L] layer kinds, followed by [L][2] (shift, len) of the active slot range
   int* status;
+  // for the frame pass (mg_frame.cuh; all null without one), [L][2*np2] in mode order, a slot's first and second
+  // mode holding (t00, t01) and (t11, t10): diagonal and off-diagonal entries in float-float (x.h, x.l, y.h, y.l),
+  // |diagonal|^2, and [L][np2] in slot order the splitter pair
+  float4* tdiag;
+  float4* toff;
+  float* tmag;
+  float2* tcs;
+  int* fcount;           // set to 0
 };
 
 __host__ __device__ inline int crossing_np(int c) { return c == CR_ORTH ? 1 : 2; }
@@ -48,14 +56,16 @@ __host__ __device__ inline int crossing_ns(int c) { return c == CR_MZI ? 2 : (c 
 // without derivative tiles, which the host guarantees when it launches the quad form.
 template <bool QUAD = false>
 __device__ __forceinline__ void slot_T(const CoefArgs& a, int l, int q, bool active, C2x2& T, C2x2& D0, C2x2& D1,
-                                       float2* csb = nullptr) {
+                                       float2* csb, Tff& F) {
   if (!active) {
     T = c2x2_identity(); D0 = c2x2_zero(); D1 = c2x2_zero();
+    tff_from(T, &F);
     return;
   }
   if (a.crossing == CR_GENERIC) {
     const float2* t = a.Tgen + ((size_t)l * (a.N / 2) + q) * 4;
     T.t00 = t[0]; T.t01 = t[1]; T.t10 = t[2]; T.t11 = t[3];
+    tff_from(T, &F);
     if (a.Dgen) {
       const float2* d = a.Dgen + ((size_t)l * (a.N / 2) + q) * 8;
       D0.t00 = d[0]; D0.t01 = d[1]; D0.t10 = d[2]; D0.t11 = d[3];
@@ -80,10 +90,15 @@ __device__ __forceinline__ void slot_T(const CoefArgs& a, int l, int q, bool act
     // tiles, or angles beyond the float-float range, the double-precision form
     const float al = ss ? ss[0] : 0.f, be = ss ? ss[1] : 0.f;
     if (need_d ||
-        !(QUAD ? mzi_T_ff_quad(pp[0], pp[1], al, be, ss == nullptr, &T, csb) : mzi_T_ff(pp[0], pp[1], al, be, &T, csb)))
+        !(QUAD ? mzi_T_ff_quad(pp[0], pp[1], al, be, ss == nullptr, &F, csb) : mzi_T_ff(pp[0], pp[1], al, be, &F, csb))) {
       mzi_T(pp[0], pp[1], al, be, &T, need_d ? &D0 : nullptr, need_d ? &D1 : nullptr, csb);
+      tff_from(T, &F);
+    } else {
+      tff_round(F, &T);
+    }
   } else {   // CR_SYM
     sym_T(pp[0], pp[1], ss ? ss[0] : 0.f, &T, need_d ? &D0 : nullptr, need_d ? &D1 : nullptr);
+    tff_from(T, &F);
   }
 }
 
@@ -115,9 +130,45 @@ __device__ __forceinline__ int layer_kind(const CoefArgs& a, int l, int q, bool*
   return (2 * st <= a.M) ? (ok ? e : 0) : KIND_XL + e;
 }
 
+// The frame pass's inputs of slot q (layer kinds 0 and odd-shift): in the quad form lane k of the quad writes entry k.
+template <bool QUAD>
+__device__ __forceinline__ void frame_inputs(const CoefArgs& a, int l, int q, int t, int sh, const Tff& F, float2 cs) {
+  const int modes = a.G * a.M, m0 = sh + 2 * q;
+  const size_t o = (size_t)l * modes;
+  // the framed gradient divides by cos(pi/4 + beta): NaN marks a slot that all but lacks it
+  const bool flat = a.tcs && !(fabsf(cs.x) >= 0x1p-6f * fabsf(cs.y));
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (QUAD && (t & 3) != k) continue;
+    ffz z = F.t[k];
+    const int m = m0 + (k >> 1);             // row of the entry
+    if (m >= modes) continue;                // (the last odd-shift slot has no second mode)
+    if (k == 0 || k == 3) {
+      float w = z.x.h * z.x.h + z.y.h * z.y.h;
+      if (w < 0x1p-60f) {                    // a diagonal entry below 2^-30 counts as 2^-30
+        z = {ff{0x1p-30f, 0.f}, ff{0.f, 0.f}};
+        w = 0x1p-60f;
+      }
+      a.tdiag[o + m] = make_float4(z.x.h, z.x.l, z.y.h, z.y.l);
+      a.tmag[o + m] = flat ? __int_as_float(0x7fc00000) : w;
+    } else {
+      a.toff[o + m] = make_float4(z.x.h, z.x.l, z.y.h, z.y.l);
+    }
+  }
+  if (t == 0) *a.fcount = 0;
+  if (QUAD ? (t & 3) == 0 : true) {
+    if (a.tcs) a.tcs[(size_t)l * (modes / 2) + q] = cs;
+    if (sh && q == 0) {                      // mode 0 lies in no slot
+      a.tdiag[o] = make_float4(1.f, 0.f, 0.f, 0.f);
+      a.toff[o] = make_float4(0.f, 0.f, 0.f, 0.f);
+      a.tmag[o] = 1.f;
+    }
+  }
+}
+
 // Thread t of the coefficient pass: one thread per slot, or (QUAD) one quad of lanes per slot - a quad shares its
 // slot, so quads leave at the bounds check whole, and its first lane writes.
-template <bool QUAD>
+template <bool QUAD, bool FRAME>
 __device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
   const int np2 = a.G * a.M / 2;
   const int idx = QUAD ? (t >> 2) : t;
@@ -155,7 +206,9 @@ __device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
   if (!real) {
     C2x2 T, D0, D1;
     float2 csv = make_float2(0.f, 0.f);   // (cos, sin)(pi/4 + beta) for the direct MZI gradient; 0 if inactive
-    slot_T<QUAD>(a, l, q, active, T, D0, D1, (a.op == OP_BWD && a.gr == 1) ? &csv : nullptr);
+    Tff F;
+    slot_T<QUAD>(a, l, q, active, T, D0, D1, (a.op == OP_BWD && a.gr == 1) ? &csv : nullptr, F);
+    if constexpr (FRAME) frame_inputs<QUAD>(a, l, q, t, kind == KIND_MIS ? 1 : 0, F, csv);
     if (!writer) return;
     if (a.op == OP_BWD && a.gr == 1) {
       float2* cs = reinterpret_cast<float2*>(tl + M * G);
@@ -239,9 +292,9 @@ __device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
   }
 }
 
-template <bool QUAD>
+template <bool QUAD, bool FRAME>
 __global__ void coef_kernel(const CoefArgs a) {
-  coef_body<QUAD>(a, blockIdx.x * blockDim.x + threadIdx.x);
+  coef_body<QUAD, FRAME>(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 }  // namespace mg

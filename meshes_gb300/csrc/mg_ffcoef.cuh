@@ -101,9 +101,25 @@ __device__ __forceinline__ bool ff_sincos(float x, ff* s, ff* c) {
   return true;
 }
 
+// T in float-float, entries 00, 01, 10, 11 (for the frame pass, which needs it before its rounding to float32)
+struct Tff {
+  ffz t[4];
+};
+__device__ __forceinline__ void tff_round(const Tff& f, C2x2* T) {
+  T->t00 = ffz_round(f.t[0]);
+  T->t01 = ffz_round(f.t[1]);
+  T->t10 = ffz_round(f.t[2]);
+  T->t11 = ffz_round(f.t[3]);
+}
+__device__ __forceinline__ void tff_from(const C2x2& T, Tff* f) {
+  const float2 t[4] = {T.t00, T.t01, T.t10, T.t11};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) f->t[k] = {ff{t[k].x, 0.f}, ff{t[k].y, 0.f}};
+}
+
 // The standard MZI T (mzi_T in mg_device.cuh, reference crossing.py:216-221) from the float-float sin/cos of
 // th/2, ph, alpha and beta, and, when given, the (cos, sin)(pi/4 + beta) pair of the direct gradient.
-__device__ __forceinline__ void mzi_T_ff_from(ff S, ff C, ff Sph, ff Cph, ff sa, ff ca, ff sb, ff cb, C2x2* T,
+__device__ __forceinline__ void mzi_T_ff_from(ff S, ff C, ff Sph, ff Cph, ff sa, ff ca, ff sb, ff cb, Tff* T,
                                               float2* csb) {
   const ff Cp = ff_sub(ff_mul(ca, cb), ff_mul(sa, sb)), Sp = ff_add(ff_mul(sa, cb), ff_mul(ca, sb));
   const ff Cm = ff_add(ff_mul(ca, cb), ff_mul(sa, sb)), Sm = ff_sub(ff_mul(sa, cb), ff_mul(ca, sb));
@@ -116,16 +132,16 @@ __device__ __forceinline__ void mzi_T_ff_from(ff S, ff C, ff Sph, ff Cph, ff sa,
   const ff CSp = ff_mul(C, Sp), SCm = ff_mul(S, Cm), SSm = ff_mul(S, Sm), CCp = ff_mul(C, Cp);
   const ffz A00 = {ff_neg(CSp), SCm}, A01 = {ff_neg(SSm), CCp};
   const ffz A10 = {SSm, CCp}, A11 = {ff_neg(CSp), ff_neg(SCm)};
-  T->t00 = ffz_round(ffz_mul(E1, A00));
-  T->t01 = ffz_round(ffz_mul(E0, A01));
-  T->t10 = ffz_round(ffz_mul(E1, A10));
-  T->t11 = ffz_round(ffz_mul(E0, A11));
+  T->t[0] = ffz_mul(E1, A00);
+  T->t[1] = ffz_mul(E0, A01);
+  T->t[2] = ffz_mul(E1, A10);
+  T->t[3] = ffz_mul(E0, A11);
 }
 
 // The same for ideal splitters (alpha = beta = 0: cos = 1, sin = 0), without the splitter products.  Each entry is
 // the value mzi_T_ff_from computes for those angles, its operations reduced to the ones that are not exact
 // multiplications by 1 or additions of 0.
-__device__ __forceinline__ void mzi_T_ff_ideal(ff S, ff C, ff Sph, ff Cph, C2x2* T, float2* csb) {
+__device__ __forceinline__ void mzi_T_ff_ideal(ff S, ff C, ff Sph, ff Cph, Tff* T, float2* csb) {
   if (csb) {
     const float r = 0.707106769f;   // (1/sqrt 2)(cos 0 -+ sin 0), rounded
     *csb = make_float2(r, r);
@@ -133,15 +149,15 @@ __device__ __forceinline__ void mzi_T_ff_ideal(ff S, ff C, ff Sph, ff Cph, C2x2*
   const ffz E1 = ffz_mul(ffz{C, S}, ffz{Cph, Sph});        // e^{i(th/2 + ph)}
   const ff E1yS = ff_mul(E1.y, S), E1xS = ff_mul(E1.x, S), E1yC = ff_mul(E1.y, C), E1xC = ff_mul(E1.x, C);
   const ff SC = ff_mul(S, C), CC = ff_mul(C, C), SS = ff_mul(S, S), CS = ff_mul(C, S);
-  T->t00 = make_float2(ff_round(ff_neg(E1yS)), ff_round(E1xS));   // e^{i(th/2+ph)} (i S)
-  T->t01 = make_float2(ff_round(ff_neg(SC)), ff_round(CC));       // e^{i th/2} (i C)
-  T->t10 = make_float2(ff_round(ff_neg(E1yC)), ff_round(E1xC));   // e^{i(th/2+ph)} (i C)
-  T->t11 = make_float2(ff_round(SS), ff_round(ff_neg(CS)));       // e^{i th/2} (-i S)
+  T->t[0] = {ff_neg(E1yS), E1xS};   // e^{i(th/2+ph)} (i S)
+  T->t[1] = {ff_neg(SC), CC};       // e^{i th/2} (i C)
+  T->t[2] = {ff_neg(E1yC), E1xC};   // e^{i(th/2+ph)} (i C)
+  T->t[3] = {SS, ff_neg(CS)};       // e^{i th/2} (-i S)
 }
 
 // mzi_T_ff_from on the angles of one thread; false (nothing written) when an angle is outside the float-float
 // range, and the caller takes the double path.
-__device__ __forceinline__ bool mzi_T_ff(float th, float ph, float al, float be, C2x2* T, float2* csb) {
+__device__ __forceinline__ bool mzi_T_ff(float th, float ph, float al, float be, Tff* T, float2* csb) {
   ff S, C, Sph, Cph, sa, ca, sb, cb;
   if (!ff_sincos(0.5f * th, &S, &C) || !ff_sincos(ph, &Sph, &Cph) || !ff_sincos(al, &sa, &ca) ||
       !ff_sincos(be, &sb, &cb))
@@ -155,7 +171,7 @@ __device__ __forceinline__ bool mzi_T_ff(float th, float ph, float al, float be,
 // shuffles, and every lane combines all four.  The four sin/cos chains, the longest part, then run side by side,
 // and the results are bitwise those of mzi_T_ff.  false on every lane of the quad when any angle is out of range.
 // ideal (uniform over the launch): no splitter array, alpha = beta = 0, and the lanes 2 and 3 of the quad idle.
-__device__ __forceinline__ bool mzi_T_ff_quad(float th, float ph, float al, float be, bool ideal, C2x2* T,
+__device__ __forceinline__ bool mzi_T_ff_quad(float th, float ph, float al, float be, bool ideal, Tff* T,
                                               float2* csb) {
   const int lane = threadIdx.x & 31, base = lane & ~3, sub = lane & 3;
   const unsigned qmask = 0xFu << base;

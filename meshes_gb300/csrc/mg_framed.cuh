@@ -1,0 +1,636 @@
+// Framed propagation of nearest-neighbour complex meshes (forward, and back-propagation with direct MZI
+// gradients) on the tiles of the frame pass (mg_frame.cuh): crossings with a unit diagonal, 8 FMAs per vector
+// forward instead of 16 and 28 instead of 44 in back-propagation.
+//
+// Fields enter in the frames of the first boundary they meet (forward: scaled by 2^-kFrameExp; back-propagation:
+// times conj(D(L))) and leave by the inverse of the last one's; a RESCALE multiplies them by a factor per mode.
+//
+// Packing: one packed f32x2 FMA serves two vectors (the same crossing, its coefficients used twice) or, for the last
+// vector of an odd number, the lane's modes m and m + M/2 (the crossings e and e + M/4, whose coefficients lie side by
+// side in the tile).  By modes, the odd-shift layer's last pair mixes the halves, (M/2 - 1, M/2) and (M - 1, the next
+// lane's 0), which costs moves: 640 instructions per pair of layers in back-propagation at M = 8, V = 4, against 568.
+//
+// What bounds it: the FMA pipe and, with two warps per scheduler, the latency of each warp's chain (ncu, N = 256, B = 4096,
+// back-propagation: FMA pipe 52%, issue 44%, stalls for fixed latency and a busy pipe).  Measured on GB300 at N = 256,
+// L = 256, B = 4096 against the unframed kernels: forward 94 -> 63 us, back-propagation 249 -> 199 us; N = 600, L = 600,
+// B = 2048: forward 314 -> 200 us, back-propagation 1412 -> 900 us.
+//
+// Work decomposition, pipeline, bounded waits and the gradient partials are those of mg_prop.cuh; a stage holds
+// three planes (main, the rows of resc that its layers have, gamma).
+#pragma once
+#include "mg_frame.cuh"
+
+namespace mg {
+
+// A layer's planes and its gradient staging as seen by one lane: shared-memory addresses
+struct FTile {
+  uint32_t main, gam, grad;
+};
+// 16 bytes of shared memory (volatile keeps them behind the barriers and waits)
+__device__ __forceinline__ ulonglong2 lds16(uint32_t addr) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ ulonglong2 ld16(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("ld.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void sts16(uint32_t addr, unsigned long long x, unsigned long long y) {
+  asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(x), "l"(y) : "memory");
+}
+
+// A packed pair of floats as one 64-bit register pair from load to store: held as two floats, the compiler splits and
+// rebuilds the pairs with moves around loops and branches.
+using p64 = unsigned long long;
+__device__ __forceinline__ p64 p_pack(float x, float y) {
+  p64 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 p_split(p64 a) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(a));
+  return d;
+}
+__device__ __forceinline__ p64 pfma(p64 a, p64 b, p64 c) {
+  p64 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ p64 pmul(p64 a, p64 b) {
+  p64 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ p64 psub(p64 a, p64 b) {
+  p64 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ p64 padd(p64 a, p64 b) {
+  p64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ p64 pneg(p64 a) { return a ^ 0x8000000080000000ull; }
+
+// two modes of a vector, or two coefficients
+struct P2 {
+  p64 r, i;
+};
+struct PK {
+  p64 r, i, n;   // n = -i
+};
+__device__ __forceinline__ PK pk(ulonglong2 q) { return PK{q.x, q.y, pneg(q.y)}; }
+
+// a + c b, a + conj(c) b
+__device__ __forceinline__ P2 p2_axpy(const PK& c, const P2& a, const P2& b) {
+  return P2{pfma(c.r, b.r, pfma(c.n, b.i, a.r)), pfma(c.r, b.i, pfma(c.i, b.r, a.i))};
+}
+__device__ __forceinline__ P2 p2_caxpy(const PK& c, const P2& a, const P2& b) {
+  return P2{pfma(c.r, b.r, pfma(c.i, b.i, a.r)), pfma(c.r, b.i, pfma(c.n, b.r, a.i))};
+}
+// The fields of one lane: its first 2 (V / 2) vectors in pairs v[p][mode], the last one of an odd V by modes
+// m[0][k] = modes (k, k + M/2)
+template <int M, int V>
+struct Fields {
+  static constexpr int kPairs = V / 2, kOdd = V & 1;
+  P2 v[kPairs ? kPairs : 1][M];
+  P2 m[1][M / 2];
+};
+
+__device__ __forceinline__ PK pk_dup(float re, float im) { return PK{p_pack(re, re), p_pack(im, im), p_pack(-im, -im)}; }
+
+// ---- one crossing per packed half, NP register pairs (ua, ub: the fields' two modes; wa, wb: the gradients'): forward, or
+// back-propagation, which returns the packed (dJ/dth, dJ/dph) sums
+template <int OP, int NP, typename UA, typename UB, typename WA, typename WB>
+__device__ __forceinline__ P2 f_crossing(const PK& al, const PK& be, const PK& ga, UA ua, UB ub, WA wa, WB wb) {
+  if constexpr (OP == OP_FWD) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const P2 a = ua(p), b = ub(p);
+      ua(p) = p2_axpy(al, a, b);
+      ub(p) = p2_axpy(be, b, a);
+    }
+    return P2{0, 0};
+  } else {
+    // dJ/dth = Im(h conj(m)) with m, h = y, g behind S(beta)^H (mode a), dJ/dph = Im(g conj(x)) of mode a at the input;
+    // each difference's two products are summed apart
+    p64 thp = 0, thq = 0, php = 0, phq = 0;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const P2 a = ua(p), b = ub(p), g = wa(p), h = wb(p);
+      const P2 m = p2_axpy(ga, a, b), mg = p2_axpy(ga, g, h);
+      thp = pfma(mg.i, m.r, thp);
+      thq = pfma(mg.r, m.i, thq);
+      const P2 x = p2_caxpy(be, a, b), gx = p2_caxpy(be, g, h);
+      ub(p) = p2_caxpy(al, b, a);
+      wb(p) = p2_caxpy(al, h, g);
+      ua(p) = x;
+      wa(p) = gx;
+      php = pfma(gx.i, x.r, php);
+      phq = pfma(gx.r, x.i, phq);
+    }
+    return P2{psub(thp, thq), psub(php, phq)};
+  }
+}
+
+// ---- one layer on the lane's vectors: KIND 0 (pairs (2e, 2e+1) in the lane) or KIND_MIS (pairs (2e+1, 2e+2), the last
+// one with the next lane's first mode, computed by this lane)
+template <int OP, int M, int V, int KIND>
+__device__ __forceinline__ void f_layer(const FTile& t, int G, int j, int r, Fields<M, V>& u, Fields<M, V>& w) {
+  constexpr int H = M / 2, sh = KIND == 0 ? 0 : 1, NV = V / 2;
+  constexpr bool odd = V & 1;
+  P2 nu[NV + 1], nw[NV + 1];   // second modes of the boundary pairs (last: of the vector packed by modes)
+  auto next_v = [&](const P2& p) {
+    const float2 x = shfl_down(p_split(p.r), 1, G), y = shfl_down(p_split(p.i), 1, G);
+    return P2{p_pack(x.x, x.y), p_pack(y.x, y.y)};
+  };
+  auto back_v = [&](P2& p, const P2& q) {
+    const float2 x = shfl_up(p_split(q.r), 1, G), y = shfl_up(p_split(q.i), 1, G), pr = p_split(p.r), pi = p_split(p.i);
+    p.r = p_pack(j != 0 ? x.x : pr.x, j != 0 ? x.y : pr.y);
+    p.i = p_pack(j != 0 ? y.x : pi.x, j != 0 ? y.y : pi.y);
+  };
+  auto next_m = [&](const P2& p) {   // modes M/2 and the next lane's 0
+    const float2 pr = p_split(p.r), pi = p_split(p.i);
+    const float2 s = shfl_down(make_float2(pr.x, pi.x), 1, G);
+    return P2{p_pack(pr.y, s.x), p_pack(pi.y, s.y)};
+  };
+  auto back_m = [&](P2& p, const P2& q) {
+    const float2 pr = p_split(p.r), pi = p_split(p.i), qr = p_split(q.r), qi = p_split(q.i);
+    const float2 s = shfl_up(make_float2(qr.y, qi.y), 1, G);
+    p.r = p_pack(j != 0 ? s.x : pr.x, qr.x);
+    p.i = p_pack(j != 0 ? s.y : pi.x, qi.x);
+  };
+  if constexpr (KIND != 0) {
+#pragma unroll
+    for (int p = 0; p < NV; ++p) {
+      nu[p] = next_v(u.v[p][0]);
+      if constexpr (OP != OP_FWD) nw[p] = next_v(w.v[p][0]);
+    }
+    if constexpr (odd) {
+      nu[NV] = next_m(u.m[0][0]);
+      if constexpr (OP != OP_FWD) nw[NV] = next_m(w.m[0][0]);
+    }
+  }
+#pragma unroll
+  for (int e = H / 2 - 1; e >= 0; --e) {   // (the boundary pair first: its results travel back while the others run)
+    const uint32_t o = (uint32_t)(2 * e * G) * 16u;
+    const ulonglong2 qa = lds16(t.main + o), qb = lds16(t.main + o + (uint32_t)G * 16u);
+    const ulonglong2 qg = OP == OP_BWD ? lds16(t.gam + o / 2) : make_ulonglong2(0, 0);
+    float2 dth = make_float2(0.f, 0.f), dph = dth;
+    const bool last = KIND != 0 && e == H / 2 - 1;
+    if constexpr (NV > 0) {
+      const float2 ar = p_split(qa.x), ai = p_split(qa.y), br = p_split(qb.x), bi = p_split(qb.y);
+      const float2 gr = p_split(qg.x), gi = p_split(qg.y);
+#pragma unroll
+      for (int c = 1; c >= 0; --c) {
+        const int ma = 2 * (e + c * (M / 4)) + sh;
+        const bool edge = last && c == 1;
+        const P2 d = f_crossing<OP, NV>(
+            c ? pk_dup(ar.y, ai.y) : pk_dup(ar.x, ai.x), c ? pk_dup(br.y, bi.y) : pk_dup(br.x, bi.x),
+            c ? pk_dup(gr.y, gi.y) : pk_dup(gr.x, gi.x), [&](int p) -> P2& { return u.v[p][ma]; },
+            [&](int p) -> P2& { return edge ? nu[p] : u.v[p][edge ? 0 : ma + 1]; }, [&](int p) -> P2& { return w.v[p][ma]; },
+            [&](int p) -> P2& { return edge ? nw[p] : w.v[p][edge ? 0 : ma + 1]; });
+        if constexpr (OP == OP_BWD) {
+          const float2 th = p_split(d.r), ph = p_split(d.i);
+          (c ? dth.y : dth.x) = th.x + th.y;
+          (c ? dph.y : dph.x) = ph.x + ph.y;
+        }
+        if (edge) {
+#pragma unroll
+          for (int p = 0; p < NV; ++p) {
+            back_v(u.v[p][0], nu[p]);
+            if constexpr (OP != OP_FWD) back_v(w.v[p][0], nw[p]);
+          }
+        }
+      }
+    }
+    p64 th = p_pack(dth.x, dth.y), ph = p_pack(dph.x, dph.y);
+    if constexpr (odd) {
+      const int k = 2 * e + sh;
+      const P2 d = f_crossing<OP, 1>(
+          pk(qa), pk(qb), pk(qg), [&](int) -> P2& { return u.m[0][k]; },
+          [&](int) -> P2& { return last ? nu[NV] : u.m[0][last ? 0 : k + 1]; }, [&](int) -> P2& { return w.m[0][k]; },
+          [&](int) -> P2& { return last ? nw[NV] : w.m[0][last ? 0 : k + 1]; });
+      if constexpr (OP == OP_BWD) {
+        th = NV ? padd(th, d.r) : d.r;
+        ph = NV ? padd(ph, d.i) : d.i;
+      }
+      if (last) {
+        back_m(u.m[0][0], nu[NV]);
+        if constexpr (OP != OP_FWD) back_m(w.m[0][0], nw[NV]);
+      }
+    }
+    if constexpr (OP == OP_BWD) {
+      if (G < 32) {
+        float2 t2 = p_split(th), p2 = p_split(ph);
+        for (int off = G; off < 32; off <<= 1) {
+          t2 = cadd(t2, shfl_xor(t2, off, 32));
+          p2 = cadd(p2, shfl_xor(p2, off, 32));
+        }
+        th = p_pack(t2.x, t2.y);
+        ph = p_pack(p2.x, p2.y);
+      }
+      if (r == 0) sts16(t.grad + o / 2, th, ph);
+    }
+  }
+}
+
+// u <- d u (CONJ: conj(d) u) with a factor for each of the lane's modes: d(k) is that of modes k and k + M/2
+template <int M, int V, bool CONJ, typename D>
+__device__ __forceinline__ void f_diag(D d, Fields<M, V>& u) {
+  auto times = [](const PK& c0, P2& p) {
+    const P2 a = p;
+    const PK c = CONJ ? PK{c0.r, c0.n, c0.i} : c0;
+    p = P2{pfma(c.r, a.r, pmul(c.n, a.i)), pfma(c.r, a.i, pmul(c.i, a.r))};
+  };
+#pragma unroll
+  for (int k = 0; k < M / 2; ++k) {
+    const ulonglong2 q = d(k);
+    if constexpr (V > 1) {
+      const float2 re = p_split(q.x), im = p_split(q.y);
+      const PK lo = pk_dup(re.x, im.x), hi = pk_dup(re.y, im.y);
+#pragma unroll
+      for (int p = 0; p < V / 2; ++p) {
+        times(lo, u.v[p][k]);
+        times(hi, u.v[p][k + M / 2]);
+      }
+    }
+    if constexpr (V & 1) times(pk(q), u.m[0][k]);
+  }
+}
+// f(a, b) on the register pairs of two lanes' fields
+template <int M, int V, typename F>
+__device__ __forceinline__ void f_each(Fields<M, V>& u, Fields<M, V>& w, F f) {
+#pragma unroll
+  for (int p = 0; p < V / 2; ++p)
+#pragma unroll
+    for (int k = 0; k < M; ++k) f(u.v[p][k], w.v[p][k]);
+  if constexpr (V & 1)
+#pragma unroll
+    for (int k = 0; k < M / 2; ++k) f(u.m[0][k], w.m[0][k]);
+}
+template <int M, int V>
+__device__ __forceinline__ void f_scale(float s, Fields<M, V>& u) {
+  f_each<M, V>(u, u, [&](P2& a, P2&) { a = P2{pmul(p_pack(s, s), a.r), pmul(p_pack(s, s), a.i)}; });
+}
+
+// Steps: the walk goes by pairs of layers, (aligned, odd-shift) forward and (odd-shift, aligned) in back-propagation, as
+// one straight-line body; a layer whose partner is not there goes with a layer of zeros (alpha = beta = 0: identity)
+// in its place.  One body for everything: with a second one in the kernel's loop the compiler moves every field register
+// where they join (300 moves per pair of layers in back-propagation, half again its arithmetic).
+// The code of the step that starts at a layer: which of the two positions are layers of the mesh, and whether a RESCALE
+// follows (back-propagation: goes before).
+constexpr int STEP_0 = 1, STEP_1 = 2, STEP_RESCALE = 4;
+constexpr int kCodePad = 4;   // codes readable before and after the layers
+template <int OP>
+__device__ __forceinline__ int step_code(const int* kinds, int L, int l) {
+  auto at = [&](int i) { return i >= 0 && i < L ? __ldg(kinds + i) : -1; };
+  const int k = at(l);
+  if (k < 0) return 0;
+  const bool mis = k & KIND_MIS, resc = k & KIND_RESCALE;
+  if (OP == OP_FWD) {
+    if (mis || resc) return (mis ? STEP_1 : STEP_0) | (resc ? STEP_RESCALE : 0);
+    const int n = at(l + 1);
+    return n < 0 || !(n & KIND_MIS) ? STEP_0 : STEP_0 | STEP_1 | (n & KIND_RESCALE ? STEP_RESCALE : 0);
+  }
+  const int c = resc ? STEP_RESCALE : 0;
+  return mis ? c | STEP_0 | (at(l - 1) == 0 ? STEP_1 : 0) : c | STEP_1;
+}
+
+// Layers [lo, hi) of a chunk in the stage's planes; resc: the stage's rows for this lane
+template <int OP, int M, int V>
+__device__ __forceinline__ void f_chunk(const FramedArgs& a, const int* codes, const FTile& st, const ulonglong2* resc,
+                                        uint32_t zero, uint32_t dump, int np2, int lo, int hi, int G, int j, int r,
+                                        Fields<M, V>& u, Fields<M, V>& w) {
+  constexpr int kDir = OP == OP_BWD ? -1 : 1;
+  const uint32_t row = (uint32_t)np2 * 16u;
+  int l = OP == OP_BWD ? hi - 1 : lo, left = hi - lo, rows = 0;
+  auto tile = [&](bool there, int at) {
+    const uint32_t i = (uint32_t)(at - lo);
+    return there ? FTile{st.main + i * row, st.gam + i * (row / 2), st.grad + i * (row / 2)} : FTile{zero, zero, dump};
+  };
+  auto rescale = [&](int at) {
+    const ulonglong2* p = rows < a.xr ? resc + (size_t)rows * np2
+                                      : reinterpret_cast<const ulonglong2*>(a.resc + (size_t)at * np2) + j;
+    ++rows;
+    f_diag<M, V, OP == OP_BWD>([&](int k) { return ld16(p + k * G); }, u);
+    if constexpr (OP == OP_BWD) f_diag<M, V, true>([&](int k) { return ld16(p + k * G); }, w);
+  };
+  int c = codes[l];
+#pragma unroll 1
+  while (left > 0) {
+    if (OP == OP_BWD && (c & STEP_RESCALE)) rescale(l);
+    bool due;
+#pragma unroll 1
+    do {
+      if (left == 1 && (c & STEP_0) && (c & STEP_1)) c &= OP == OP_BWD ? ~STEP_1 : ~(STEP_1 | STEP_RESCALE);
+      const int n = (c & 1) + ((c >> 1) & 1);
+      const FTile t0 = tile(c & STEP_0, l), t1 = tile(c & STEP_1, l + (c & STEP_0 ? kDir : 0));
+      due = OP == OP_FWD && (c & STEP_RESCALE);
+      l += n * kDir;
+      left -= n;
+      c = codes[l];
+      f_layer<OP, M, V, OP == OP_BWD ? KIND_MIS : 0>(t0, G, j, r, u, w);
+      f_layer<OP, M, V, OP == OP_BWD ? 0 : KIND_MIS>(t1, G, j, r, u, w);
+      if (OP == OP_BWD) due = c & STEP_RESCALE;
+    } while (left > 0 && !due);
+    if (OP == OP_FWD && due) rescale(l - 1);
+  }
+}
+
+// ---- field I/O: lane j's modes [j*M, j*M+M) of V vectors; vectors from vend on and modes from N on read 0
+template <int M, int V>
+__device__ __forceinline__ void f_load(Fields<M, V>& u, const void* src, int vb0, int vend, int N, int ldu, int j) {
+  auto at = [&](int v, int m) {   // modes m, m + 1
+    const float4* p = reinterpret_cast<const float4*>(static_cast<const float2*>(src) + (size_t)(vb0 + v) * ldu + j * M);
+    return vb0 + v < vend && j * M + m < N ? p[m / 2] : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto two = [](float4 x, float4 y, P2* p) {
+    p[0] = P2{p_pack(x.x, y.x), p_pack(x.y, y.y)};
+    p[1] = P2{p_pack(x.z, y.z), p_pack(x.w, y.w)};
+  };
+#pragma unroll
+  for (int p = 0; p < V / 2; ++p)
+#pragma unroll
+    for (int k = 0; k < M; k += 2) two(at(2 * p, k), at(2 * p + 1, k), &u.v[p][k]);
+  if constexpr (V & 1)
+#pragma unroll
+    for (int k = 0; k < M / 2; k += 2) two(at(V - 1, k), at(V - 1, M / 2 + k), &u.m[0][k]);
+}
+template <int M, int V>
+__device__ __forceinline__ void f_store(const Fields<M, V>& u, void* dst, int vb0, int vend, int N, int ldu, int j) {
+  auto put = [&](int v, int m, float4 x) {
+    float4* p = reinterpret_cast<float4*>(static_cast<float2*>(dst) + (size_t)(vb0 + v) * ldu + j * M);
+    if (vb0 + v < vend && j * M + m < N) p[m / 2] = x;
+  };
+  auto two = [&](const P2* p, int v0, int m0, int v1, int m1) {
+    const float2 ar = p_split(p[0].r), ai = p_split(p[0].i), br = p_split(p[1].r), bi = p_split(p[1].i);
+    put(v0, m0, make_float4(ar.x, ai.x, br.x, bi.x));
+    put(v1, m1, make_float4(ar.y, ai.y, br.y, bi.y));
+  };
+#pragma unroll
+  for (int p = 0; p < V / 2; ++p)
+#pragma unroll
+    for (int k = 0; k < M; k += 2) two(&u.v[p][k], 2 * p, k, 2 * p + 1, k);
+  if constexpr (V & 1)
+#pragma unroll
+    for (int k = 0; k < M / 2; k += 2) two(&u.m[0][k], V - 1, k, V - 1, M / 2 + k);
+}
+// the frames d of the lane's modes as f_diag's factors
+template <int M>
+__device__ __forceinline__ ulonglong2 frame_pair(const float2* __restrict__ d, int j, int k) {
+  const float2 d0 = __ldg(d + j * M + k), d1 = __ldg(d + j * M + M / 2 + k);
+  return make_ulonglong2(p_pack(d0.x, d1.x), p_pack(d0.y, d1.y));
+}
+// CTA barriers by number: with MIX, warps of both kinds meet at them from their own copies of the body
+__device__ __forceinline__ void cta_sync() { asm volatile("barrier.cta.sync.aligned 0;" ::: "memory"); }
+__device__ __forceinline__ bool cta_sync_or(bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.or.pred.aligned p, 0, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)p)
+      : "memory");
+  return r != 0;
+}
+
+// Chunk-end sum of the W warps' staged gradients (W a multiple of 4), in warp order, into this CTA's partials of the
+// layers from lo on: n float4 of consecutive layers
+__device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int W, int n, ulonglong2* out) {
+#pragma unroll 1
+  for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+    uint32_t p = gst + (uint32_t)idx * 16u;
+    ulonglong2 t = make_ulonglong2(0, 0);
+#pragma unroll 1
+    for (int w = 0; w < W; w += 4, p += 4 * warp_bytes) {
+      const ulonglong2 a = lds16(p), b = lds16(p + warp_bytes), c = lds16(p + 2 * warp_bytes), d = lds16(p + 3 * warp_bytes);
+      t.x = padd(padd(padd(padd(t.x, a.x), b.x), c.x), d.x);
+      t.y = padd(padd(padd(padd(t.y, a.y), b.y), c.y), d.y);
+    }
+    out[idx] = t;
+  }
+}
+
+// The warp's vectors [vb0, vb0 + V) (per lane group) through all layers.  The pipeline's barriers are initialised, the
+// step codes and the layer of zeros are in shared memory.
+struct FramedSmem {
+  unsigned char* base;
+  uint32_t zero, gst;
+  uint64_t* bars;
+  const int* codes;
+};
+template <int OP, int M, int V, int GT>
+__device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSmem& sm, int vb0) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const Lanes<GT> ln(a.G, a.logG);
+  const int G = ln.G, j = ln.j, r = ln.r;
+  const int np2 = (G * M) >> 1, CL = a.fcl, S = a.fs;
+  const uint32_t row = (uint32_t)np2 * 16u, warp_bytes = (uint32_t)CL * (row / 2), j16 = (uint32_t)j * 16u;
+  const uint32_t stage = (uint32_t)framed_stage_bytes(OP, np2, CL, a.xr), ring = smem_u32(sm.base);
+  Fields<M, V> u, w;
+  f_load<M, V>(u, a.in0, vb0, a.vend, a.N, a.ldu, j);
+  if constexpr (OP == OP_BWD) f_load<M, V>(w, a.target ? a.target : a.in1, vb0, a.vend, a.N, a.ldu, j);
+
+  // chunks of CL layers in the order of the walk; the first is one shorter where that keeps pairs of layers whole
+  const int first = __ldg(a.fkinds + (OP == OP_BWD ? a.L - 1 : 0));
+  const int cut = (OP == OP_BWD ? !(first & KIND_MIS) : (first & KIND_MIS) != 0) && CL > 1 ? 1 : 0;
+  const int nch = (a.L + cut + CL - 1) / CL;
+  auto walked = [&](int c) { return min(a.L, max(0, c * CL - cut)); };   // layers before chunk c
+  auto chunk_lo = [&](int c) { return OP == OP_BWD ? a.L - walked(c + 1) : walked(c); };
+  auto chunk_hi = [&](int c) { return OP == OP_BWD ? a.L - walked(c) : walked(c + 1); };
+  const uint64_t wlim = a.wait_ns ? a.wait_ns : kWaitLimitNs;
+  // warp 0: the copies of chunk c into stage s - the main plane (and gamma's) whole, and the rows of resc
+  auto issue = [&](int c, int s) {
+    if (c + 1 == a.unarmed) return;
+    const int lo = chunk_lo(c), n = chunk_hi(c) - lo;
+    const uint32_t bar = smem_u32(sm.bars + s), at = ring + (uint32_t)s * stage;
+    auto has = [&](int i) {   // the walk's i-th layer
+      return i < n && (__ldg(a.fkinds + (OP == OP_BWD ? lo + n - 1 - i : lo + i)) & KIND_RESCALE);
+    };
+    int rows = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) rows += __popc(__ballot_sync(0xffffffffu, has(i0 + lane)));
+    if (lane == 0) {
+      mbar_arrive_expect_tx(bar, (n + min(rows, a.xr)) * row + (OP == OP_BWD ? n * (row >> 1) : 0u));
+      tma_load_1d(at, a.main + (size_t)lo * np2, n * row, bar);
+      if constexpr (OP == OP_BWD)
+        tma_load_1d(at + (uint32_t)(CL + a.xr) * row, a.gam + (size_t)lo * (np2 / 2), n * (row >> 1), bar);
+    }
+    if (rows == 0) return;
+    __syncwarp();
+    rows = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + lane;
+      const bool is = has(i);
+      const unsigned b = __ballot_sync(0xffffffffu, is);
+      const int k = rows + __popc(b & ((1u << lane) - 1u));
+      if (is && k < a.xr)
+        tma_load_1d(at + (uint32_t)(CL + k) * row, a.resc + (size_t)(OP == OP_BWD ? lo + n - 1 - i : lo + i) * np2, row, bar);
+      rows += __popc(b);
+    }
+  };
+  int issued = min(S, nch);
+  if (warp == 0)
+    for (int c = 0; c < issued; ++c) issue(c, c);
+  if constexpr (OP == OP_FWD) {
+    f_scale<M, V>(1.f / (1ull << kFrameTop), u);
+  } else {
+    if (a.target)   // fused L2 loss to a target: g = 2 (y - t)
+      f_each<M, V>(u, w, [](P2& y, P2& t) {
+        const p64 two = p_pack(2.f, 2.f);
+        t = P2{pmul(two, psub(y.r, t.r)), pmul(two, psub(y.i, t.i))};
+      });
+    f_diag<M, V, true>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, u);
+    f_diag<M, V, true>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, w);
+  }
+
+  int s = 0;
+  uint32_t phase = 0;
+#pragma unroll 1
+  for (int c = 0; c < nch; ++c) {
+    const int lo = chunk_lo(c), hi = chunk_hi(c);
+    const bool ok = mbar_wait_bounded(smem_u32(sm.bars + s), phase, wlim);
+    if (ok) {
+      const uint32_t at = (uint32_t)s * stage;
+      const FTile st{ring + at + j16, ring + at + (uint32_t)(CL + a.xr) * row + j16, sm.gst + (uint32_t)warp * warp_bytes + j16};
+      f_chunk<OP, M, V>(a, sm.codes, st, reinterpret_cast<const ulonglong2*>(sm.base + at + (uint32_t)CL * row) + j,
+                        sm.zero + j16, sm.gst + (uint32_t)a.W * warp_bytes + j16, np2, lo, hi, G, j, r, u, w);
+    }
+    // every warp is done with the stage, and (back-propagation) every warp's gradients of the chunk are staged
+    if (cta_sync_or(!ok)) {
+      // give up: record, wait (bounded) for the copies still in flight, release the barriers, leave
+      if (tid == 0) {
+        set_status(a.status, ST_TIMEOUT);
+        for (int cc = c; cc < issued; ++cc)
+          if (cc + 1 != a.unarmed) mbar_wait_bounded(smem_u32(sm.bars + (cc % S)), (uint32_t)((cc / S) & 1), wlim);
+        for (int k = 0; k < S; ++k) mbar_inval(smem_u32(sm.bars + k));
+      }
+      return;
+    }
+    if (issued < nch) {
+      if (warp == 0) issue(issued, s);
+      ++issued;
+    }
+    if constexpr (OP == OP_BWD) {
+      f_reduce(sm.gst, warp_bytes, a.W, (hi - lo) * (np2 / 2),
+               reinterpret_cast<ulonglong2*>(a.partial + ((size_t)blockIdx.x * a.L + lo) * np2));
+      cta_sync();
+    }
+    if (++s == S) {
+      s = 0;
+      phase ^= 1;
+    }
+  }
+  if (tid == 0)
+    for (int k = 0; k < S; ++k) mbar_inval(smem_u32(sm.bars + k));
+  if constexpr (OP == OP_FWD) {
+    f_diag<M, V, false>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, u);
+    f_store<M, V>(u, a.out0, vb0, a.vend, a.N, a.ldu, j);
+  } else {
+    if (a.out0 != nullptr) {
+      f_scale<M, V>(1.f / (1ull << kFrameTop), u);
+      f_store<M, V>(u, a.out0, vb0, a.vend, a.N, a.ldu, j);
+    }
+    f_scale<M, V>(1.f / (1ull << kFrameTop), w);
+    f_store<M, V>(w, a.out1, vb0, a.vend, a.N, a.ldu, j);
+  }
+}
+
+// One CTA: W warps of V vectors per lane group; MIX: warps 4-7 (12-15) take V - 1, so that every scheduler carries
+// 2V - 1.  The two kinds have a body each, chosen once per warp.  A mesh that the frames do not suit (a.refuse) takes
+// the unframed body of mg_prop.cuh on the same vectors.
+template <int OP, int M, int V, int GT, bool MIX>
+__global__ void __launch_bounds__(framed_max_threads(M, V), 1) framed_kernel(const FramedArgs a0) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int G = GT ? GT : a0.G, R = 32 / G, np2 = (G * M) >> 1, r = lane / G;
+  const int v0 = blockIdx.x * framed_cta_vectors(a0.W, R, V, MIX);
+  FramedArgs a = a0;
+  a.vend = min(a.B, v0 + framed_cta_vectors(a0.W, R, V, MIX));
+  if (__ldg(a.count) >= a.refuse) {
+    a.v0 = v0;
+    if (OP == OP_BWD) a.partial = a0.partial + (size_t)blockIdx.x * a.L * np2;
+    prop_body<OP, M, V, false, GT, OP == OP_BWD ? 1 : 0, false, true>(a, smem);
+    return;
+  }
+  const size_t zero = a.fs * framed_stage_bytes(OP, np2, a.fcl, a.xr);
+  FramedSmem sm;
+  sm.base = smem;
+  sm.zero = smem_u32(smem + zero);
+  sm.gst = sm.zero + (uint32_t)np2 * 16u;
+  sm.bars = reinterpret_cast<uint64_t*>(smem + framed_bars_offset(OP, np2, a.W, a.fcl, a.fs, a.xr));
+  int* codes = reinterpret_cast<int*>(sm.bars + a.fs + (a.fs & 1)) + kCodePad;
+  sm.codes = codes;
+  for (int l = tid - kCodePad; l < a.L + kCodePad; l += blockDim.x) codes[l] = step_code<OP>(a.fkinds, a.L, l);
+  for (int i = tid; i < np2; i += blockDim.x) sts16(sm.zero + (uint32_t)i * 16u, 0, 0);
+  if (tid == 0) {
+    for (int s = 0; s < a.fs; ++s) mbar_init(smem_u32(sm.bars + s), 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  if constexpr (MIX) {
+    // warps of four alternate between V and V - 1 vectors
+    const int base = v0 + (warp >> 3) * R * 4 * (2 * V - 1), in = (warp & 3) * R + r;
+    if (warp & 4) framed_body<OP, M, V - 1, GT>(a, sm, base + R * 4 * V + in * (V - 1));
+    else framed_body<OP, M, V, GT>(a, sm, base + in * V);
+  } else {
+    framed_body<OP, M, V, GT>(a, sm, v0 + (warp * R + r) * V);
+  }
+}
+
+// dp[l][q][k] (= or +=) the sum over the nC per-CTA partials times the frames' weights, in the CTAs' order (as
+// dp_reduce_kernel, whose layout of threads it shares); a float2 holds gradient k of the crossings e and e + M/4
+static __global__ void __launch_bounds__(256) framed_reduce_kernel(const float2* __restrict__ partial, int nC, int L, int np2,
+                                                            int M, int G, int N, float* dp, int ldp, int accumulate,
+                                                            const int* __restrict__ geo, const float2* __restrict__ wts,
+                                                            const int* __restrict__ count, int refuse) {
+  constexpr int kCols = 32, kRows = 8;
+  __shared__ float2 acc[kRows][kCols];
+  const int col = threadIdx.x % kCols, row = threadIdx.x / kCols;
+  const int idx = blockIdx.x * kCols + col;
+  const bool valid = idx < L * np2;
+  const size_t stride = (size_t)L * np2;
+  float2 s = make_float2(0.f, 0.f);
+  if (valid) {
+    const float2* p = partial + idx;
+    int c = row;
+    for (; c + 3 * kRows < nC; c += 4 * kRows) {
+      const float2 a0 = __ldg(p + (size_t)c * stride), a1 = __ldg(p + (size_t)(c + kRows) * stride);
+      const float2 a2 = __ldg(p + (size_t)(c + 2 * kRows) * stride), a3 = __ldg(p + (size_t)(c + 3 * kRows) * stride);
+      s = cadd(cadd(cadd(cadd(s, a0), a1), a2), a3);
+    }
+    for (; c < nC; c += kRows) s = cadd(s, __ldg(p + (size_t)c * stride));
+  }
+  acc[row][col] = s;
+  __syncthreads();
+  if (row != 0 || !valid) return;
+  for (int k = 1; k < kRows; ++k) s = cadd(s, acc[k][col]);
+  const int l = idx / np2, rem = idx - l * np2;
+  if (__ldg(count) >= refuse) {   // partials of the unframed body: (dJ/dth, dJ/dph) of one slot
+    const int q = pos_slot(rem, M, G);
+    if (q >= N / 2) return;
+    const bool active = q >= geo[2 * l] / 2 && q < geo[2 * l] / 2 + geo[2 * l + 1];
+    float* o = dp + (size_t)l * ldp + 2 * (size_t)q;
+    o[0] = (accumulate ? o[0] : 0.f) + (active ? s.x : 0.f);
+    o[1] = (accumulate ? o[1] : 0.f) + (active ? s.y : 0.f);
+    return;
+  }
+  const int k = rem & 1, pos = rem >> 1;
+  const int j = pos % G, q0 = j * (M / 2) + pos / G;
+  const int sh = geo[2 * l] / 2, ln = geo[2 * l + 1];
+  const float2 w = __ldg(wts + idx);
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int q = q0 + c * (M / 4);
+    if (q >= N / 2) continue;
+    const float v = q >= sh && q < sh + ln ? (c ? s.y * w.y : s.x * w.x) : 0.f;
+    float* o = dp + (size_t)l * ldp + 2 * (size_t)q + k;
+    *o = accumulate ? *o + v : v;
+  }
+}
+
+}  // namespace mg

@@ -1,0 +1,78 @@
+// Arguments and sizes of the frame pass (mg_frame.cuh) and the framed kernels (mg_framed.cuh), for the host side.
+#pragma once
+#include "mg_coeffs.cuh"
+
+namespace mg {
+
+// Frames start at 2^22, are due to start again below 2^-8 and do so at once below 2^-18: the products of two framed
+// fields stay within 2^44 and 2^-16 of the fields' own, the middle of the float range (2^-76 behind a cross state)
+constexpr int kFrameTop = 22, kFrameDue = -8, kFrameNow = -18;
+constexpr int kFrameSeg = 16;              // layers per segment, about
+constexpr int kFrameBatch = 16;            // layers whose frames are held in shared memory at a time
+constexpr int kFrameThreads = 512;
+constexpr int KIND_RESCALE = 1 << 14;      // OR-ed into a layer's kind: the frames start again behind it
+
+// Tile planes of one layer, lane j, pair e < M/4 of the lane's crossings (e, e + M/4), values of the two side by side:
+//   main [(2e + h) G + j] = (re, re', im, im') of alpha (h = 0), beta (h = 1)
+//   gam  [e G + j]          gamma
+//   resc [k G + j], k < M/2 RESCALE layers: the factors of the lane's modes k and k + M/2
+// Gradient partials and their weights: float4 (th, th', ph, ph') at [e G + j].
+struct FrameArgs {
+  int L, M, G;
+  int bwd;                       // 1: gam and wts are wanted
+  const float4* tdiag;           // [L][modes], CoefArgs
+  const float4* toff;
+  const float* tmag;
+  const float2* tcs;
+  const int* kinds;              // [L]
+  float4* main;                  // [L][np2]
+  float4* resc;                  // [L][np2]
+  float4* gam;                   // [L][np2/2]
+  float4* wts;                   // [L][np2/2]
+  float2* dfin;                  // [modes]: frames after the last layer
+  int* fkinds;                   // [L] kinds with KIND_RESCALE
+  int* count;                    // layers that break a pair of layers up, plus 2^30 for an entry that is NaN (set to 0
+                                 // by the coefficient pass)
+};
+// A CTA of the frame pass takes rows * 32 modes of one segment
+constexpr int kFrameMaxRows = 5;
+inline size_t frame_smem_bytes(int modes, int rows) {
+  return (size_t)(kFrameBatch + 1) * (32 * rows + 2) * 16 + (size_t)(kFrameBatch + 1) * modes * 4;
+}
+
+// The PropArgs part describes the unframed launch on the same tiles (tiles, kinds, CL, S), which a mesh that the
+// frames do not suit takes inside the same kernel.
+struct FramedArgs : PropArgs {
+  const float4* main;
+  const float4* resc;
+  const float4* gam;
+  const float2* dfin;
+  const int* fkinds;
+  const int* count;
+  int fcl, fs;                   // layers per stage, stages
+  int xr;                        // rows of resc in a pipeline stage
+  int refuse;                    // count from which on the mesh takes the unframed body
+};
+// threads per CTA the kernels are compiled for
+__host__ __device__ constexpr int framed_max_threads(int M, int V) { return M * V <= 16 ? 512 : 256; }
+// vectors of one CTA: W warps of V per lane group (R groups per warp), mix: every second four warps V - 1
+__host__ __device__ constexpr int framed_cta_vectors(int W, int R, int V, bool mix) {
+  return R * (W * V - (mix ? W / 8 * 4 : 0));
+}
+// one pipeline stage: CL layers of the main plane, xr rows of resc, (back-propagation) CL layers of gamma
+__host__ __device__ inline size_t framed_stage_bytes(int op, int np2, int CL, int xr) {
+  return (size_t)np2 * (16 * (size_t)(CL + xr) + (op == OP_BWD ? 8 * (size_t)CL : 0));
+}
+// rows of resc in a stage of CL layers: few layers have one (each segment's last, and those that bound the frames);
+// the rows beyond are read from global memory
+inline int framed_resc_rows(int CL) { return CL / 8 + 1 < CL ? CL / 8 + 1 : CL; }
+// shared memory of a launch: [S stages][a layer of zeros][BWD: per-warp gradients, one layer beyond the last warp's]
+// [S mbarriers][step codes]
+__host__ __device__ inline size_t framed_bars_offset(int op, int np2, int W, int CL, int S, int xr) {
+  return S * framed_stage_bytes(op, np2, CL, xr) + (size_t)np2 * 16 + (op == OP_BWD ? ((size_t)W * CL + 1) * np2 * 8 : 0);
+}
+inline size_t framed_smem_bytes(int op, int np2, int W, int CL, int S, int L) {
+  return framed_bars_offset(op, np2, W, CL, S, framed_resc_rows(CL)) + 8 * (size_t)(S + (S & 1)) + 4 * (size_t)(L + 8);
+}
+
+}  // namespace mg

@@ -3,6 +3,7 @@
 #include <atomic>
 #include <cuda_runtime.h>
 
+#include "../../include/meshes_gb300.h"
 #include "mg_prop.cuh"
 
 namespace mg {
@@ -97,6 +98,18 @@ cudaError_t launch_prop_nn2(int op, bool real, int M, int V, int gr, const Launc
 // the tiles of an M = 8, G = 32 plan; V counts vectors per pair
 bool pair_instantiated(int op, bool real, int M, int V, int gr, bool full);
 cudaError_t launch_prop_pair(int V, const LaunchCfg& lc, const PropArgs& a);
+// framed propagation (mg_framed.cuh, instantiated in mg_prop_framed_*.cu): forward and back-propagation of
+// nearest-neighbour MZI meshes on the frame pass's tiles
+struct FramedArgs;
+struct FrameArgs;
+bool framed_instantiated(int op, int M, int V, bool full, bool mix);
+bool framed_pick(int op, int M, int B, int sms, mg_config* out);
+bool framed_pays(int op, int M, int L, int np2, int B, int sms);
+cudaError_t launch_prop_framed(int op, int M, int V, bool mix, const LaunchCfg& lc, const FramedArgs& a);
+cudaError_t launch_frames(const FrameArgs& a, int sms, cudaStream_t stream);
+cudaError_t launch_framed_reduce(const float2* partial, int nC, int L, int np2, int M, int G, int N, float* dp, int ldp,
+                                 int accumulate, const int* geo, const float2* wts, const int* count, int refuse,
+                                 cudaStream_t stream);
 // split launches (two CTA kinds per SM); instantiated only for the full-warp configurations in
 // split_instantiated()
 bool split_instantiated(int op, bool real, int M, int V, bool full, int gr);

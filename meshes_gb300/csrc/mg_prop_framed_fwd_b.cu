@@ -1,0 +1,5 @@
+// Framed propagation kernels of list MG_FRAMED_FWD_B.
+#include "mg_framed_launch.cuh"
+#include "mg_framed_list.h"
+
+MG_FRAMED_UNIT(framed_fwd_b, OP_FWD, MG_FRAMED_FWD_B)
