@@ -114,6 +114,7 @@ struct Plan {
   unsigned lb, dlb;
   size_t smem;
   size_t off_kinds, off_tiles, off_dtiles, off_partial, total;
+  int tree;         // stored activations: warps whose gradients are added pairwise before the others (1: none)
   bool framed;      // unit-diagonal crossings on the frame pass's tiles (mg_framed.cuh)
   size_t off_main, off_resc, off_gam, off_wts, off_dfin, off_fkinds, off_tdiag, off_toff, off_tmag, off_tcs, off_count;
   int fcl, fs;      // layers per stage and stages of the framed pipeline (CL, S: of the unframed body in the same kernel)
@@ -132,20 +133,41 @@ size_t launch_smem(const Plan& P, int op, int gslot, int L) {
   return P.perm ? perm_scratch_offset(b) + perm_scratch_bytes(P.W, P.M, P.real) : b;
 }
 
+// Warps per CTA for B vectors, per_warp of them to a warp: enough to cover the batch in one wave, rounded up to a multiple
+// of 4 so the four schedulers of an SM carry equal work (measured: 8 warps on 128 SMs beat 7 warps on 147)
+int default_warps(int B, int per_warp, int sms) {
+  const long warps = ((long)B + per_warp - 1) / per_warp;
+  long w = std::max<long>((warps + sms - 1) / sms, 1);
+  if (w > 2) w = (w + 3) / 4 * 4;
+  return (int)std::min<long>(w, 8);
+}
+
 // Layers without their partner from which on a mesh takes the unframed body: each costs the framed one a layer of zeros
 int framed_refuse(int L) { return std::max(4, L / 2); }
 
-// (M, V) instantiated for the stored-activation kernels (GR 4), by op (FWD writes, BWD reads)
-bool instantiated_stored(int op, int M, int V) {
+// (M, V) instantiated for the stored-activation kernels (GR 4), by op (FWD writes, BWD reads); the tiles of few vectors
+// per lane are nearest-neighbour and full-warp only (stored_nn_instantiated)
+bool instantiated_stored(int op, int M, int V, bool nn_full) {
   static const int fwd[][2] = {{2, 8}, {4, 8}, {8, 4}, {16, 2}};
   static const int bwd[][2] = {{2, 4}, {4, 4}, {8, 4}, {16, 2}};
   for (int i = 0; i < 4; ++i) {
     const int* t = (op == OP_FWD) ? fwd[i] : bwd[i];
     if (t[0] == M && t[1] == V) return true;
   }
-  return false;
+  return nn_full && stored_nn_instantiated(op, M, V);
 }
 int stored_default_v(int op, int M) { return op == OP_FWD ? (M <= 4 ? 8 : (M == 8 ? 4 : 2)) : (M <= 8 ? 4 : 2); }
+
+// Tile of a nearest-neighbour complex mesh whose batch would leave schedulers without a warp at the default tile (8 modes
+// and 4 vectors per lane: at N = 100 and B = 777, 98 warps for 608 schedulers): a vector over all 32 lanes, and as few
+// vectors per lane as fill the schedulers.  Measured on GB300 at B = 608: N = 128 forward 31 -> 13 us, back-propagation
+// 132 -> 35 us; N = 100 (Reck), B = 777 forward 52 -> 21 us.  From n vectors per scheduler on the default tile's reuse of
+// coefficients wins.  0: the default.
+int small_batch_v(int op, int M, int B, int sms) {
+  const long n = ((long)B + 4 * sms - 1) / (4 * sms);
+  if (op == OP_FWD) return M == 2 ? (n <= 1 ? 1 : n <= 4 ? 2 : n <= 8 ? 4 : 0) : M == 4 ? (n <= 2 ? 1 : n <= 8 ? 2 : 0) : 0;
+  return M > 4 ? 0 : n <= 2 ? 1 : n <= 8 ? 2 : 0;
+}
 
 // op MG_OP_BWD_STORED plans the back-propagation kernel in its stored-activation mode (GR 4): T tiles
 // only, 32-byte dJ/dT staging per slot, raw partials of 4 complex per slot.
@@ -186,13 +208,30 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
                          (crossing == CR_MZI ? op != OP_FWDDIFF : crossing == CR_SYM && op == OP_FWD);
   mg_config fc;
   if (!cfg && may_frame && framed_pays(op, Np / 32, L, Np / 2, B, di.sms) && framed_pick(op, Np / 32, B, di.sms, &fc)) cfg = &fc;
-  int M = (cfg && cfg->M) ? cfg->M : (wide ? kWideM : std::max(std::min(8, Np), Np / 32));
+  int small_v = 0;
+  if (!(cfg && (cfg->M || cfg->V)) && geometry == GEO_NN && !perm && !wide && N > 32 && crossing != CR_ORTH &&
+      (op == OP_FWD || (op == OP_BWD && p.gr == 1)))
+    small_v = small_batch_v(op, Np / 32, B, di.sms);
+  // stored activations, N <= 128: the default tile's lane groups (R = 32 / G per warp) as a warp each, a vector over all
+  // 32 lanes.  The CTA's vectors and the order of every gradient sum stay those of the default tile (chunk_reduce_raw
+  // adds the R warps of a former warp pairwise first), so dJ/dT keeps its bits.  Measured on GB300 at N = 128, B = 1024:
+  // the stored kernels of a step 352 -> 144 us, with one segment instead of eleven.
+  p.tree = 1;
+  if (stored && !(cfg && (cfg->M || cfg->V || cfg->W)) && geometry == GEO_NN && !wide && N > 32 && N <= 128) {
+    const int R = 256 / Np, w = default_warps(B, R * 4, di.sms);
+    if (R * w <= 8) {
+      small_v = 4;
+      p.tree = R;
+    }
+  }
+  int M = (cfg && cfg->M) ? cfg->M : small_v ? Np / 32 : (wide ? kWideM : std::max(std::min(8, Np), Np / 32));
   if (wide ? M != kWideM : (M < 2 || M > 16 || (M & (M - 1))))
     return fail(MG_E_CONFIG, "modes per lane M=%d not in %s", M, wide ? "{20} for N > 512" : "{2,4,8,16}");
   if (M > Np) M = Np;
   const int G = Np / M;
   if (G > 32) return fail(MG_E_CONFIG, "N=%d needs more than 32 lanes at M=%d", N, M);
   int V = (cfg && cfg->V) ? cfg->V : 0;
+  if (small_v) V = small_v;
   if (!V) {
     static const int vd[3][5] = {{8, 8, 4, 2, 0}, {4, 4, 2, 1, 0}, {4, 4, 4, 2, 0}};   // by ilog2(M)-1
     static const int vw[3] = {2, 1, 1};                                                // M = kWideM
@@ -218,7 +257,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   } else if (p.occ2 || p.framed) {
   } else if (wide ? (perm || stored || !wide_instantiated(op, crossing == CR_ORTH, V, p.gr))
            : perm ? !perm_instantiated(op, crossing == CR_ORTH, M, V, p.gr)
-                  : (stored ? !instantiated_stored(OP_BWD, M, V)
+                  : (stored ? !instantiated_stored(OP_BWD, M, V, geometry == GEO_NN && G == 32)
                             : !(instantiated(op, M, V) ||
                                 (geometry == GEO_NN && nn_small_instantiated(op, p.real, M, V, p.gr, G == 32)))))
     return fail(MG_E_CONFIG, "no %skernel instantiated for op=%d M=%d V=%d",
@@ -251,14 +290,10 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   int W = (cfg && cfg->W) ? cfg->W : p.framed ? 8 : (p.split ? 4 : (p.pair || p.occ2) ? 8 : 0);
   if (p.framed && p.split && W % 8) return fail(MG_E_CONFIG, "mixed warps need W a multiple of 8, got %d", W);
   if (p.pair && (W & 1)) return fail(MG_E_CONFIG, "a warp-pair launch needs an even W, got %d", W);
+  if (p.tree > 1) W = p.tree * default_warps(B, p.tree * 4, di.sms);
   if (!W) {
-    // enough warps to cover the batch in one wave, rounded up to a multiple of 4 so the four
-    // schedulers of an SM carry equal work (measured: 8 warps on 128 SMs beat 7 warps on 147)
-    const long per_warp = (long)p.R * V;
-    const long warps = (B + per_warp - 1) / per_warp;
-    long w = std::max<long>((warps + di.sms - 1) / di.sms, 1);
-    if (w > 2) w = (w + 3) / 4 * 4;
-    W = (int)std::min<long>(w, std::min(8, maxw));
+    W = std::min(default_warps(B, p.R * V, di.sms), maxw);
+    if (small_v && op == OP_BWD && W < 4) W = 4;   // fewer CTAs leave fewer partials
   }
   if (W < 1 || W > maxw) return fail(MG_E_CONFIG, "W=%d warps outside [1, %d]", W, maxw);
   int S = (cfg && cfg->S) ? cfg->S : ((op == OP_FWD || p.split) ? 2 : 3);
@@ -1011,8 +1046,9 @@ int range_impl(int op, int N, int L, int l0, int l1, int B, int crossing, int ge
   if (bwd && !dT && B > 0 && l1 > l0 && !keep_partials) return fail(MG_E_ARG, "dT is NULL");
   if (dT && (reinterpret_cast<uintptr_t>(dT) & 7)) return fail(MG_E_ARG, "dT not 8-byte aligned");
   if (act && !bwd) {   // the forward kernel's store mode has its own (M, V) instantiations
-    if (!(cfg && cfg->V)) P.V = stored_default_v(OP_FWD, P.M);
-    if (!instantiated_stored(OP_FWD, P.M, P.V))
+    const bool nn_full = geometry == GEO_NN && P.G == 32;
+    if (!(cfg && cfg->V) && !(nn_full && stored_nn_instantiated(OP_FWD, P.M, P.V))) P.V = stored_default_v(OP_FWD, P.M);
+    if (!instantiated_stored(OP_FWD, P.M, P.V, nn_full))
       return fail(MG_E_CONFIG, "no activation-storing forward kernel for M=%d V=%d", P.M, P.V);
     const long per_cta = (long)P.W * P.R * P.V;
     P.grid = (int)((B + per_cta - 1) / per_cta);
@@ -1054,6 +1090,7 @@ int range_impl(int op, int N, int L, int l0, int l1, int B, int crossing, int ge
   a.out1 = bwd ? out1 : nullptr;
   a.partial = reinterpret_cast<float2*>(w + P.off_partial) + (keep_partials ? (size_t)l0 * 4 * P.np2 : 0);
   a.pstride = keep_partials ? L : 0;
+  a.tree = P.tree;
   a.status = reinterpret_cast<int*>(w);
   a.act = act;
   a.act_plane = (size_t)B * ldu;
@@ -1064,7 +1101,11 @@ int range_impl(int op, int N, int L, int l0, int l1, int B, int crossing, int ge
   lc.block = dim3(32 * P.W);
   lc.smem = P.smem;
   lc.stream = static_cast<cudaStream_t>(stream);
-  cudaError_t e = launch_prop(P.op, P.real, P.M, P.V, P.G == 32, act ? 4 : 0, lc, a);
+  cudaError_t e = act && geometry == GEO_NN && P.G == 32 && stored_nn_instantiated(P.op, P.M, P.V)
+                      ? launch_prop_stored_nn(P.op, P.M, P.V, lc, a)
+                  : !act && geometry == GEO_NN && nn_instantiated(P.op, P.real, P.M, P.V, 0, P.G == 32, false)
+                      ? launch_prop_nn(P.op, P.real, P.M, P.V, 0, P.G == 32, false, lc, a)
+                      : launch_prop(P.op, P.real, P.M, P.V, P.G == 32, act ? 4 : 0, lc, a);
   if (e != cudaSuccess) return cuda_fail(e, "prop_kernel launch");
   if (bwd && !keep_partials) {
     const int n = nl * P.np2;
@@ -1131,9 +1172,12 @@ int mg_lossy_forward(int N, int L, int B, int geometry, int seg, const void* x, 
   TRY(check_field(x, "x", false, B > 0));
   TRY(check_field(y, "y", false, B > 0));
   TRY(check_field(ckpt, "ckpt", false, false));
-  int cl = std::min(P.CL, seg);
-  while (seg % cl) --cl;
-  P.CL = cl;
+  if (L > seg) {
+    int cl = std::min(P.CL, seg);
+    while (seg % cl) --cl;
+    if (cl < P.CL && P.S == 1) P.S = 2;   // (one stage was to hold every layer)
+    P.CL = cl;
+  }
   P.smem = launch_smem(P, OP_FWD, 0, L);
   return run_prop(P, x, nullptr, y, nullptr, ldu, nullptr, 0, 0, static_cast<unsigned char*>(ws),
                   static_cast<cudaStream_t>(stream), nullptr, L > seg ? ckpt : nullptr, seg);

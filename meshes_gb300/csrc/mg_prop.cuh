@@ -73,6 +73,8 @@ struct PropArgs {
   void* ckpt;
   size_t ckpt_plane;
   int ckpt_every;
+  // stored-activation back-propagation: this many consecutive warps are added as a tree (0, 1: none), a power of two
+  int tree;
   // layers per CTA block of the partial buffer (0: L); lets layer ranges keep every range's partials
   int pstride;
   // time limit of each pipeline wait (0: kWaitLimitNs)
@@ -776,11 +778,39 @@ __device__ __forceinline__ void chunk_reduce_raw(const PropArgs& a, const int* k
       ia = ma % M; ib = mb % M;
     }
     float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb = ra;
-    for (int w = 0; w < a.W; ++w) {
-      const float4* gl = reinterpret_cast<const float4*>(gst + ((size_t)w * a.CL + li) * gst_layer);
-      const float4 x = gl[ia * G + la], y = gl[ib * G + lb];
-      ra.x += x.x; ra.y += x.y; ra.z += x.z; ra.w += x.w;
-      rb.x += y.x; rb.y += y.y; rb.z += y.z; rb.w += y.w;
+    auto add = [](float4& s, const float4& v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; };
+    auto row = [&](int w, int i, int l2) {
+      return reinterpret_cast<const float4*>(gst + ((size_t)w * a.CL + li) * gst_layer)[i * G + l2];
+    };
+    if (a.tree > 1) {
+      for (int w = 0; w < a.W; w += a.tree) {
+        float4 xa[4], xb[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k < a.tree / 2) {
+            xa[k] = row(w + 2 * k, ia, la);
+            add(xa[k], row(w + 2 * k + 1, ia, la));
+            xb[k] = row(w + 2 * k, ib, lb);
+            add(xb[k], row(w + 2 * k + 1, ib, lb));
+          }
+        if (a.tree >= 4) {
+          add(xa[0], xa[1]);
+          add(xb[0], xb[1]);
+        }
+        if (a.tree >= 8) {
+          add(xa[2], xa[3]);
+          add(xb[2], xb[3]);
+          add(xa[0], xa[2]);
+          add(xb[0], xb[2]);
+        }
+        add(ra, xa[0]);
+        add(rb, xb[0]);
+      }
+    } else {
+      for (int w = 0; w < a.W; ++w) {
+        add(ra, row(w, ia, la));
+        add(rb, row(w, ib, lb));
+      }
     }
     float2* o = a.partial + (size_t)l * 4 * np2 + pos;
     o[0] = make_float2(ra.x, ra.y);                                        // G00 (XL: G_aa)
@@ -814,7 +844,7 @@ __device__ __forceinline__ void run_chunk(const PropArgs& pa, int vb0, const int
       F* plane = static_cast<F*>(pa.act) + (size_t)l * pa.act_plane;
       if constexpr (OP == OP_BWD) load_fields<M, V, REAL>(u, plane, vb0, pa.vend, pa.N, pa.ldu, j);
       else store_fields<M, V, REAL>(u, plane, vb0, pa.vend, pa.N, pa.ldu, j);
-      layer_any<OP, M, V, REAL, GR, false, PK>(kinds[l], reinterpret_cast<const float4*>(st + (size_t)(l - lo) * layer_bytes), G,
+      layer_any<OP, M, V, REAL, GR, NN, PK>(kinds[l], reinterpret_cast<const float4*>(st + (size_t)(l - lo) * layer_bytes), G,
                                     j, r, u, w, reinterpret_cast<float4*>(gst_warp + (size_t)(l - lo) * gst_layer));
     }
     return;

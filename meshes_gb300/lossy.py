@@ -3,13 +3,12 @@
 The lossless path back-propagates by inverting each layer with T^H (the reference's c/dot.cpp:75-80 and
 gpu/backprop.cu do the same), which needs no stored activations but is exact only for unitary crossings.
 A lossy crossing - the generic MZI of crossing.py:444-488, with phase errors and gains g_ij - breaks it.
-Here the adjoint keeps the mesh input of every segment of ceil(sqrt(L)) layers during the forward pass;
-back-propagation then walks the
-segments in reverse, recomputes each segment's layer inputs from its checkpoint (one forward launch
-that writes them to a (segment, B, N) buffer) and back-propagates
-through the segment from those stored inputs (one launch plus a deterministic reduction).  Each
-direction is one library call (mg_lossy_forward / mg_lossy_backward) that runs all its segments.  Memory is
-about 2 sqrt(L) fields instead of L; work is one extra forward pass.
+Here the adjoint keeps the mesh input of every segment of layers during the forward pass; back-propagation then walks
+the segments in reverse, recomputes each segment's layer inputs from its checkpoint (one forward launch that writes them
+to a (segment, B, N) buffer) and back-propagates through the segment from those stored inputs (one launch plus a
+deterministic reduction).  Each direction is one library call (mg_lossy_forward / mg_lossy_backward) that runs all its
+segments.  A segment is at least ceil(sqrt(L)) layers (about 2 sqrt(L) fields of memory instead of L) and as long as its
+stored inputs stay within SEGMENT_BYTES; work is one extra forward pass.
 
 The crossing is given as its transfer matrices ``T`` (L, N/2, 2, 2), complex, in the reference's slot
 grid (gpu/mesh.py:77-81); ``mzi_generic_T`` builds them from (theta, phi) and the 14 error parameters
@@ -28,6 +27,9 @@ import torch
 from . import geometry as geom
 from ._lib import GENERIC, GEO_FFT, GEO_NN, OP_BWD_STORED, OP_FWD, check, load
 from .mesh import _stream
+
+
+SEGMENT_BYTES = 1 << 30   # stored layer inputs of one segment of the adjoint
 
 
 def mzi_generic_T(p: torch.Tensor, s: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -122,13 +124,19 @@ class LossyMesh:
         self._ws = {}
 
     def segment_for(self, B: int) -> int:
-        """Checkpoint spacing used for a batch of B vectors: ceil(sqrt(L)) layers, whatever B.  Keeping a
-        segment's stored inputs inside the 129 MB L2 (8 layers at N=256, B=4096) measured slower on GB300: the
-        step took 2.07 ms with 8-layer segments, 1.93 ms with 16 (sqrt L) and 1.80 ms with 32, the gradient
-        bitwise the same; the fewer launches outweigh the inputs read back from HBM."""
+        """Checkpoint spacing used for a batch of B vectors: as many layers as keep a segment's stored inputs within
+        ``SEGMENT_BYTES``, ceil(sqrt(L)) at least, in segments of about equal length.  Each segment costs a recompute and
+        a back-propagation launch with nearly empty last waves: measured on GB300 at N=256, L=256, B=4096 a step takes
+        1.75 ms with 16-layer segments (sqrt L), 1.64 ms with 32, 1.56 ms with 64 and 1.51 ms with one segment of 2.1
+        GB, the gradient bitwise the same; at N=128, B=1024 eleven segments are 22 launches of 5 to 9 us."""
         if self._segment:
             return self._segment
-        return max(1, math.ceil(math.sqrt(max(self.L, 1))))
+        L, base = max(self.L, 1), max(1, math.ceil(math.sqrt(max(self.L, 1))))
+        seg = max(base, min(L, SEGMENT_BYTES // max(8 * B * self.N, 1)))
+        if seg >= L:
+            return L
+        seg = math.ceil(L / math.ceil(L / seg))
+        return -(-seg // 8) * 8                 # whole pipeline chunks between checkpoints
 
     @property
     def segment(self) -> int:
