@@ -21,26 +21,20 @@ import torch
 
 from . import _lib
 from ._lib import GEO_NN, OP_BWD, OP_FWD, OP_FWD_BWDTILES, check, load
-from .mesh import MeshNetworkGPU, _stream
+from .mesh import MeshNetworkGPU, Workspace, _stream
 
 
-class _Plan:
-    """Workspace cache of one (mesh, op, batch) combination."""
+class _Plan(Workspace):
+    """Workspace cache of one (mesh, op), with the version of the tiles in it."""
 
     def __init__(self, mesh: MeshNetworkGPU, op: int):
-        self.mesh, self.op = mesh, op
-        self.buf: Optional[torch.Tensor] = None
+        super().__init__(mesh.device)
+        self.mesh, self.op, self.version = mesh, op, 0
 
-    def workspace(self, B: int):
+    def size(self, B: int):
         m = self.mesh
-        nb = load().mg_workspace_bytes(self.op, m.N, m.L, B, m.crossing, m.geo_code,
-                                       _lib.cfg_ptr(m.config.get(self.op)))
-        if nb == 0:
-            check(-1, "mg_workspace_bytes")
-        if self.buf is None or self.buf.numel() < nb:
-            self.buf = torch.empty(nb, dtype=torch.uint8, device=m.device)
-            check(load().mg_workspace_init(self.buf.data_ptr(), nb, _stream(m.device)), "mg_workspace_init")
-        return self.buf.data_ptr(), self.buf.numel()
+        return lambda: load().mg_workspace_bytes(self.op, m.N, m.L, B, m.crossing, m.geo_code,
+                                                 _lib.cfg_ptr(m.config.get(self.op)))
 
 
 def _plans(mesh: MeshNetworkGPU):
@@ -55,18 +49,19 @@ def _build(mesh: MeshNetworkGPU, op: int, p: torch.Tensor, B: int):
     """Build op's tiles for phases p into the mesh's cached workspace; returns (ws, bytes, version)."""
     lib = load()
     plan_ = _plans(mesh)[op]
-    ws, nb = plan_.workspace(B)
-    plan_.version = getattr(plan_, "version", 0) + 1
     s = mesh.p_splitter
     geo = ((None, None, mesh.strides.data_ptr()) if mesh.strides is not None
            else (mesh.lens.data_ptr(), mesh.shifts.data_ptr(), None))
-    check(lib.mg_build_tiles(op, mesh.N, mesh.L, mesh.geo_code, *geo, mesh.crossing, p.data_ptr(),
-                             mesh.N // 2 * mesh.X_np, s.data_ptr() if s.numel() else None, mesh.N // 2 * mesh.X_ns,
-                             None, None, None, B, _lib.cfg_ptr(mesh.config.get(op)), ws, nb, _stream(mesh.device)),
-          "mg_build_tiles")
+    cfg, stream = _lib.cfg_ptr(mesh.config.get(op)), _stream(mesh.device)
+    plan_.version += 1                       # whatever happens below, the tiles of earlier calls are gone
+    check(plan_.call(plan_.size(B), lambda ws, nb: lib.mg_build_tiles(
+        op, mesh.N, mesh.L, mesh.geo_code, *geo, mesh.crossing, p.data_ptr(), mesh.N // 2 * mesh.X_np,
+        s.data_ptr() if s.numel() else None, mesh.N // 2 * mesh.X_ns, None, None, None, B, cfg, ws, nb, stream)),
+        "mg_build_tiles")
+    ws, nb = plan_.buf.data_ptr(), plan_.buf.numel()
     if mesh.perm_table is not None:
-        check(lib.mg_build_perms(op, mesh.N, mesh.L, B, mesh.crossing, mesh.geo_code, mesh.perm_table.data_ptr(),
-                                 _lib.cfg_ptr(mesh.config.get(op)), ws, nb, _stream(mesh.device)), "mg_build_perms")
+        check(lib.mg_build_perms(op, mesh.N, mesh.L, B, mesh.crossing, mesh.geo_code, mesh.perm_table.data_ptr(), cfg, ws,
+                                 nb, stream), "mg_build_perms")
     return ws, nb, plan_.version
 
 
@@ -92,8 +87,8 @@ class MeshFunction(torch.autograd.Function):
         B, N = y.shape
         gy = gy.resolve_conj().resolve_neg().contiguous()
         plan_ = _plans(mesh)[OP_BWD]
-        if ctx.tiles_version is not None and getattr(plan_, "version", None) == ctx.tiles_version:
-            ws, nb = plan_.workspace(B)               # tiles of this forward are still in place
+        if ctx.tiles_version is not None and plan_.version == ctx.tiles_version:
+            ws, nb = plan_.buf.data_ptr(), plan_.buf.numel()               # tiles of this forward are still in place
         else:
             ws, nb, _ = _build(mesh, OP_BWD, p, B)
         gx = torch.empty_like(gy)
@@ -147,8 +142,8 @@ class MeshL2Function(torch.autograd.Function):
         mesh = ctx.mesh
         B, N = y.shape
         plan_ = _plans(mesh)[OP_BWD]
-        if ctx.tiles_version is not None and getattr(plan_, "version", None) == ctx.tiles_version:
-            ws, nb = plan_.workspace(B)
+        if ctx.tiles_version is not None and plan_.version == ctx.tiles_version:
+            ws, nb = plan_.buf.data_ptr(), plan_.buf.numel()
         else:
             ws, nb, _ = _build(mesh, OP_BWD, p, B)
         gx = torch.empty_like(y)

@@ -26,7 +26,7 @@ import torch
 
 from . import geometry as geom
 from ._lib import GENERIC, GEO_FFT, GEO_NN, OP_BWD_STORED, OP_FWD, check, load
-from .mesh import _stream
+from .mesh import Workspace, _stream
 
 
 SEGMENT_BYTES = 1 << 30   # stored layer inputs of one segment of the adjoint
@@ -148,23 +148,16 @@ class LossyMesh:
             return None, None, self.strides.data_ptr()
         return self.lens.data_ptr(), self.shifts.data_ptr(), None
 
-    def _workspace(self, op: int, B: int):
-        lib = load()
-        nb = lib.mg_workspace_bytes(op, self.N, self.L, B, GENERIC, self.geometry, None)
-        if nb == 0:
-            check(-1, "mg_workspace_bytes")
-        buf = self._ws.get(op)
-        if buf is None or buf.numel() < nb:
-            buf = torch.empty(nb, dtype=torch.uint8, device=self.device)
-            check(lib.mg_workspace_init(buf.data_ptr(), nb, _stream(self.device)), "mg_workspace_init")
-            self._ws[op] = buf
-        return buf.data_ptr(), buf.numel()
-
     def _build(self, op: int, Tc: torch.Tensor, B: int):
-        ws, nb = self._workspace(op, B)
-        check(load().mg_build_tiles(op, self.N, self.L, self.geometry, *self._geo(), GENERIC, None, 0, None, 0, None,
-                                    Tc.data_ptr(), None, B, None, ws, nb, _stream(self.device)), "mg_build_tiles")
-        return ws, nb
+        w = self._ws.get(op)
+        if w is None:
+            w = self._ws[op] = Workspace(self.device)
+        stream = _stream(self.device)
+        check(w.call(lambda: load().mg_workspace_bytes(op, self.N, self.L, B, GENERIC, self.geometry, None),
+                     lambda ws, nb: load().mg_build_tiles(op, self.N, self.L, self.geometry, *self._geo(), GENERIC, None, 0,
+                                                          None, 0, None, Tc.data_ptr(), None, B, None, ws, nb, stream)),
+              "mg_build_tiles")
+        return w.buf.data_ptr(), w.buf.numel()
 
     def _range(self, op, l0, l1, B, in0, in1, out0, out1, act, dT, ws, nb):
         ptr = (lambda t: None if t is None else t.data_ptr())
@@ -174,13 +167,9 @@ class LossyMesh:
 
     def status(self, clear: bool = True) -> int:
         """Kernel status word of the last launches (0 = ok); reads both workspaces."""
-        lib = load()
         st = 0
-        for buf in self._ws.values():
-            r = lib.mg_read_status(buf.data_ptr(), int(clear), _stream(self.device))
-            if r < 0:
-                check(r, "mg_read_status")
-            st = st or r
+        for w in self._ws.values():
+            st = st or w.status(clear)
         return st
 
     # ---- user API

@@ -27,7 +27,10 @@ _NP_NS = {"mzi": (2, 2), "sym": (2, 1), "orth": (1, 0)}   # gpu/mesh.py:72-73
 
 
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Raw handle of the device's current stream (without a torch.cuda.Stream object around it, 11 us per call on the
+    GB300 host: a third of a small forward call)."""
+    i = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 class Workspace:
@@ -36,6 +39,20 @@ class Workspace:
     def __init__(self, device):
         self.device = device
         self.buf: Optional[torch.Tensor] = None
+
+    def call(self, size, fn) -> int:
+        """rc of fn(ws, ws_bytes) on the buffer as it is; grown to size() bytes first where the library says it is too small
+        (which it does before anything else happens), so that a call does not ask for the size each time."""
+        rc = _lib.E_WORKSPACE
+        if self.buf is not None:
+            rc = fn(self.buf.data_ptr(), self.buf.numel())
+        if rc == _lib.E_WORKSPACE:
+            nb = size()
+            if nb == 0:
+                check(-1, "mg_workspace_bytes")
+            if self.buf is None or self.buf.numel() < nb:
+                rc = fn(*self.get(nb))
+        return rc
 
     def get(self, nbytes: int) -> Tuple[int, int]:
         if self.buf is None or self.buf.numel() < nbytes:
@@ -154,7 +171,8 @@ class MeshNetworkGPU:
             v = torch.as_tensor(np.asarray(v))
         # a lazily conjugated or negated view (torch's conj/neg bits, e.g. U.t().conj()) is materialised: the
         # kernels read the memory behind data_ptr, which holds the unconjugated values
-        v = v.to(device=self.device, dtype=self.dtype).resolve_conj().resolve_neg()
+        if v.dtype != self.dtype or v.device != self.device or v.is_conj() or v.is_neg():
+            v = v.to(device=self.device, dtype=self.dtype).resolve_conj().resolve_neg()
         assert v.dim() == 2 and v.shape[0] == self.N, "v must be (N, B) with N=%d" % self.N
         align = 8 if self.X == "orth" else 16
         if (v.stride(0) == 1 and (v.shape[1] == 1 or (v.stride(1) >= self.N and v.stride(1) % 2 == 0))
@@ -179,6 +197,9 @@ class MeshNetworkGPU:
         lds = self.N // 2 * self.X_ns
         sp = s.data_ptr() if s.numel() else None
         return p.data_ptr(), ldp, sp, lds
+
+    def _ws_bytes(self, op, B):
+        return lambda: load().mg_workspace_bytes(op, self._N, self._L, B, self.crossing, self.geometry, None)
 
     def _programmed(self, op, p, s, B, dp=None) -> Tuple[int, int]:
         """Tiles of op for phases p (and direction dp) plus the permutation tables, in op's workspace."""
@@ -227,11 +248,10 @@ class MeshNetworkGPU:
                                            out.data_ptr(), None, ldu_out, None, 0, 0, None, ws, wsn, stream),
                           "mg_propagate")
                 return out
-            wsb = lib.mg_workspace_bytes(OP_FWD, self.N, self.L, B, self.crossing, self.geometry, None)
-            ws, wsn = self._ws[OP_FWD].get(wsb)
             fn = lib.mg_fwdprop_ft if self.geometry == GEO_FFT else lib.mg_fwdprop
-            check(fn(self.N, self.L, B, *self._geo_args(), pptr, ldp, sptr, lds, v.data_ptr(), out.data_ptr(), ldu_out,
-                     self.crossing, ws, wsn, stream), fn.__name__)
+            check(self._ws[OP_FWD].call(self._ws_bytes(OP_FWD, B), lambda ws, wsn: fn(
+                self._N, self._L, B, *self._geo_args(), pptr, ldp, sptr, lds, v.data_ptr(), out.data_ptr(), ldu_out,
+                self.crossing, ws, wsn, stream)), fn.__name__)
             return out
         dout, ldu_dout = self._out(dout, B)
         dpp = None if dp is None else self._param(dp).reshape(-1)
@@ -259,12 +279,11 @@ class MeshNetworkGPU:
                                        None if dv is None else dv.data_ptr(), out.data_ptr(), dout.data_ptr(), ldu_out,
                                        None, 0, 0, None, ws, wsn, stream), "mg_propagate")
             return out, dout
-        wsb = lib.mg_workspace_bytes(OP_FWDDIFF, self.N, self.L, B, self.crossing, self.geometry, None)
-        ws, wsn = self._ws[OP_FWDDIFF].get(wsb)
         fn = lib.mg_fwddiff_ft if self.geometry == GEO_FFT else lib.mg_fwddiff
-        check(fn(self.N, self.L, B, *self._geo_args(), pptr, None if dpp is None else dpp.data_ptr(), ldp, sptr, lds,
-                 v.data_ptr(), None if dv is None else dv.data_ptr(), out.data_ptr(), dout.data_ptr(), ldu_out,
-                 self.crossing, ws, wsn, stream), fn.__name__)
+        check(self._ws[OP_FWDDIFF].call(self._ws_bytes(OP_FWDDIFF, B), lambda ws, wsn: fn(
+            self._N, self._L, B, *self._geo_args(), pptr, None if dpp is None else dpp.data_ptr(), ldp, sptr, lds,
+            v.data_ptr(), None if dv is None else dv.data_ptr(), out.data_ptr(), dout.data_ptr(), ldu_out,
+            self.crossing, ws, wsn, stream)), fn.__name__)
         return out, dout
 
     # ---- objective helpers (gpu/mesh.py:176-206)
@@ -345,12 +364,12 @@ class MeshNetworkGPU:
                                    out_dp.data_ptr(), ldp, accumulate, None, ws, wsn, _stream(self.device)),
                   "mg_propagate")
             return out_dp, out_dJdv
-        wsb = lib.mg_workspace_bytes(OP_BWD, self.N, self.L, B, self.crossing, self.geometry, None)
-        ws, wsn = self._ws[OP_BWD].get(wsb)
         fn = lib.mg_backdiff_ft if self.geometry == GEO_FFT else lib.mg_backdiff
-        check(fn(self.N, self.L, B, *self._geo_args(), pptr, out_dp.data_ptr(), ldp, sptr, lds, v2.data_ptr(),
-                 g.data_ptr(), None if out_vin is None else out_vin.data_ptr(), out_dJdv.data_ptr(), ldu,
-                 self.crossing, accumulate, ws, wsn, _stream(self.device)), fn.__name__)
+        stream = _stream(self.device)
+        check(self._ws[OP_BWD].call(self._ws_bytes(OP_BWD, B), lambda ws, wsn: fn(
+            self._N, self._L, B, *self._geo_args(), pptr, out_dp.data_ptr(), ldp, sptr, lds, v2.data_ptr(),
+            g.data_ptr(), None if out_vin is None else out_vin.data_ptr(), out_dJdv.data_ptr(), ldu,
+            self.crossing, accumulate, ws, wsn, stream)), fn.__name__)
         return out_dp, out_dJdv
 
     # ---- phase screen: is_phase with phi_pos 'in' (y = U D v) or 'out' (y = D U v), D = diag(exp(i ph)),
