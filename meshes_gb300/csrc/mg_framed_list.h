@@ -9,4 +9,4 @@
 #define MG_FRAMED_BWD_B1(X) X(8, 1, false) X(8, 2, false) X(8, 2, true)
 #define MG_FRAMED_BWD_B2(X) X(8, 3, false) X(8, 4, false) X(8, 4, true)
 #define MG_FRAMED_BWD_C(X) X(16, 1, false) X(16, 2, false) X(16, 2, true)
-#define MG_FRAMED_BWD_D(X) X(20, 1, false)
+#define MG_FRAMED_BWD_D(X) X(20, 1, false) X(20, 2, false) X(20, 2, true)

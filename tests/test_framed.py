@@ -17,7 +17,7 @@ FWD = [(4, 1, 0, 4), (4, 1, 0, 8), (4, 2, 0, 16), (4, 2, 1, 8), (4, 4, 0, 8), (4
        (16, 4, 0, 8), (20, 1, 0, 8), (20, 2, 0, 8), (20, 2, 1, 8), (20, 3, 0, 8)]
 BWD = [(4, 1, 0, 4), (4, 1, 0, 8), (4, 2, 0, 16), (4, 2, 1, 8), (4, 4, 0, 8), (4, 4, 1, 16), (8, 1, 0, 4), (8, 2, 0, 8),
        (8, 2, 1, 8), (8, 3, 0, 8), (8, 4, 0, 8), (8, 4, 1, 8), (16, 1, 0, 4), (16, 1, 0, 8), (16, 2, 0, 8),
-       (16, 2, 1, 8), (20, 1, 0, 4), (20, 1, 0, 8)]
+       (16, 2, 1, 8), (20, 1, 0, 4), (20, 1, 0, 8), (20, 2, 0, 8), (20, 2, 1, 8)]
 SIZES = {4: (66, 128), 8: (130, 256), 16: (258, 400), 20: (514, 640)}
 
 
