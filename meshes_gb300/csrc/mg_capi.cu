@@ -116,8 +116,9 @@ struct Plan {
   size_t off_kinds, off_tiles, off_dtiles, off_partial, total;
   int tree;         // stored activations: warps whose gradients are added pairwise before the others (1: none)
   bool framed;      // unit-diagonal crossings on the frame pass's tiles (mg_framed.cuh)
-  size_t off_main, off_resc, off_gam, off_wts, off_dfin, off_fkinds, off_tdiag, off_toff, off_tmag, off_tcs, off_count;
-  int fcl, fs;      // layers per stage and stages of the framed pipeline (CL, S: of the unframed body in the same kernel)
+  size_t off_main, off_resc, off_wts, off_dfin, off_fkinds, off_tdiag, off_toff, off_tmag, off_tcs, off_count;
+  unsigned flb;     // bytes of a layer's framed tile
+  int fcl;          // layers per stage of the framed pipeline (CL, S: of the unframed body in the same kernel)
   bool perm;        // MG_GEO_PERM: permutation tables at off_perm, gather scratch after the smem layout
   size_t off_perm;
 };
@@ -129,7 +130,7 @@ size_t perm_table_bytes(int N, int L) { return 4 * (2 * (size_t)(L + 1) * N + 2 
 // Shared memory of a launch of plan P over L layers, with the permutation scratch when P has one.
 size_t launch_smem(const Plan& P, int op, int gslot, int L) {
   const size_t b = prop_smem_bytes(op, gslot, P.M, P.G, P.W, P.CL, P.S, P.lb, P.dlb, L);
-  if (P.framed) return std::max(b, framed_smem_bytes(op, P.np2, P.W, P.fcl, P.fs, L));
+  if (P.framed) return std::max(b, framed_smem_bytes(op, P.flb, P.np2, P.W, P.fcl, L));
   return P.perm ? perm_scratch_offset(b) + perm_scratch_bytes(P.W, P.M, P.real) : b;
 }
 
@@ -305,11 +306,11 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   const size_t fixed = 8 * (size_t)(S + 1) + (L <= kMaxSmemKinds ? 4 * (size_t)L : 0) +
                        (perm ? 16 + perm_scratch_bytes(W, M, p.real) : 0);
   if (p.framed) {
-    // the configuration's CL and S are the framed pipeline's: as many layers per stage as fit, whole pairs
-    p.fs = (cfg && cfg->S) ? S : 2;
-    p.fcl = CL ? CL : std::max(1, std::min(L, 64));
-    while (p.fcl > 1 && framed_smem_bytes(op, p.np2, W, p.fcl, p.fs, L) > budget) --p.fcl;
-    if (!CL && p.fcl > 4) p.fcl &= ~3;
+    // the configuration's CL is the framed pipeline's, of kFrameStages stages: as many layers per stage as fit, whole pairs
+    p.flb = framed_layer_bytes(op, p.np2);
+    p.fcl = CL ? CL : std::max(1, std::min(L, 32));
+    while (p.fcl > 1 && framed_smem_bytes(op, p.flb, p.np2, W, p.fcl, L) > budget) --p.fcl;
+    if (!CL && p.fcl > 1) p.fcl &= ~1;
     S = 2;
     CL = 0;
   }
@@ -356,9 +357,8 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
     const size_t n = (size_t)L * p.np2;
     const bool bwd = op == OP_BWD;
     p.off_main = p.total;
-    p.off_resc = p.off_main + align256(16 * n);
-    p.off_gam = p.off_resc + align256(16 * n);
-    p.off_wts = p.off_gam + (bwd ? align256(8 * n) : 0);
+    p.off_resc = p.off_main + align256(n * (bwd ? 24 : 16));
+    p.off_wts = p.off_resc + align256(16 * n);
     p.off_dfin = p.off_wts + (bwd ? align256(8 * n) : 0);
     p.off_fkinds = p.off_dfin + align256(16 * (size_t)p.np2);
     p.off_tdiag = p.off_fkinds + align256(4 * (size_t)L);
@@ -462,13 +462,38 @@ int build_tiles(const Plan& P, const int* lens, const int* shifts, const int* st
     f.main = reinterpret_cast<float4*>(ws + P.off_main);
     f.count = a.fcount;
     f.resc = reinterpret_cast<float4*>(ws + P.off_resc);
-    f.gam = reinterpret_cast<float4*>(ws + P.off_gam);
     f.wts = reinterpret_cast<float4*>(ws + P.off_wts);
     f.dfin = reinterpret_cast<float2*>(ws + P.off_dfin);
     f.fkinds = reinterpret_cast<int*>(ws + P.off_fkinds);
     e = launch_frames(f, sms, st);
   }
   return e == cudaSuccess ? MG_OK : cuda_fail(e, "coef_kernel launch");
+}
+
+// Forward plan Pf reads the tiles in back-propagation plan Pb's workspace: their layer strides, a stage that still fits
+int use_bwd_tiles(const Plan& Pb, Plan* Pf) {
+  if (Pb.framed) {
+    Pf->off_main = Pb.off_main;
+    Pf->off_resc = Pb.off_resc;
+    Pf->off_dfin = Pb.off_dfin;
+    Pf->off_fkinds = Pb.off_fkinds;
+    Pf->off_count = Pb.off_count;
+    Pf->flb = Pb.flb;   // (tiles with gamma)
+  }
+  Pf->lb = Pb.lb;
+  Pf->off_kinds = Pb.off_kinds;
+  Pf->off_tiles = Pb.off_tiles;
+  Pf->off_perm = Pb.off_perm;   // the forward rows of the tables mg_build_perms wrote for this workspace
+  const DevInfo di = dev_info();
+  const size_t budget = Pf->split && !Pf->framed ? (size_t)di.smem_per_sm / 2 - 1024 : (size_t)di.smem_optin - 1024;
+  for (;;) {
+    Pf->smem = launch_smem(*Pf, OP_FWD, 0, Pf->L);
+    if (Pf->smem <= budget && (size_t)Pf->CL * Pf->lb < (1u << 20)) break;
+    if (Pf->CL == 1 && !(Pf->framed && Pf->fcl > 1)) return fail(MG_E_CONFIG, "no pipeline depth fits shared memory");
+    if (Pf->CL > 1) Pf->CL -= 1;   // the back-propagation tiles are larger than the forward ones the plan was sized for
+    if (Pf->framed && Pf->fcl > 1) Pf->fcl -= Pf->fcl & 1 ? 1 : 2 - (Pf->fcl == 2);
+  }
+  return MG_OK;
 }
 
 // Permutation arguments of a launch over layers [l0, l1) of plan P (the launch's layer i is layer l0 + i):
@@ -529,13 +554,11 @@ int run_prop(const Plan& P, const void* in0, const void* in1, void* out0, void* 
     static_cast<PropArgs&>(f) = a;
     f.main = reinterpret_cast<const float4*>(ws + P.off_main);
     f.resc = reinterpret_cast<const float4*>(ws + P.off_resc);
-    f.gam = reinterpret_cast<const float4*>(ws + P.off_gam);
     f.dfin = reinterpret_cast<const float2*>(ws + P.off_dfin);
     f.fkinds = reinterpret_cast<const int*>(ws + P.off_fkinds);
     f.count = reinterpret_cast<const int*>(ws + P.off_count);
     f.fcl = P.fcl;
-    f.fs = P.fs;
-    f.xr = framed_resc_rows(P.fcl);
+    f.flb = P.flb;
     f.refuse = framed_refuse(P.L);
     e = launch_prop_framed(P.op, P.M, P.V, P.split, lc, f);
   } else if (P.pair)
@@ -877,25 +900,7 @@ int mg_propagate(int op, int N, int L, int B, int crossing, int geometry, const 
     if (Pb.framed) framed_pick(OP_FWD, Pb.M, B, dev_info().sms, &cf);
     else if (cf.split >= 5) cf = {Pb.M, 0, 0, 0, 0, 2};
     TRY(make_plan(OP_FWD, N, L, B, crossing, geometry, &cf, &Pf));
-    if (Pb.framed) {
-      Pf.off_main = Pb.off_main;
-      Pf.off_resc = Pb.off_resc;
-      Pf.off_dfin = Pb.off_dfin;
-      Pf.off_fkinds = Pb.off_fkinds;
-      Pf.off_count = Pb.off_count;
-    }
-    Pf.lb = Pb.lb;
-    Pf.off_kinds = Pb.off_kinds;
-    Pf.off_tiles = Pb.off_tiles;
-    Pf.off_perm = Pb.off_perm;   // the forward rows of the tables mg_build_perms wrote for this workspace
-    const DevInfo di = dev_info();
-    const size_t budget = Pf.split && !Pf.framed ? (size_t)di.smem_per_sm / 2 - 1024 : (size_t)di.smem_optin - 1024;
-    for (;;) {
-      Pf.smem = launch_smem(Pf, OP_FWD, 0, L);
-      if (Pf.smem <= budget && (size_t)Pf.CL * Pf.lb < (1u << 20)) break;
-      if (Pf.CL == 1) return fail(MG_E_CONFIG, "no pipeline depth fits shared memory");
-      Pf.CL -= 1;   // the back-propagation tiles are larger than the forward ones the plan was sized for
-    }
+    TRY(use_bwd_tiles(Pb, &Pf));
     TRY(check_ldu(Pf, ldu));
     TRY(check_field(in0, "in0", Pf.real, B > 0));
     TRY(check_field(out0, "out0", Pf.real, B > 0));
@@ -988,7 +993,7 @@ int mg_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_co
   Plan P;
   TRY(make_plan(op, N, L, B, crossing, geometry, cfg, &P));
   if (out) {
-    out->M = P.M; out->V = P.V; out->W = P.W; out->CL = P.framed ? P.fcl : P.CL; out->S = P.framed ? P.fs : P.S; out->G = P.G; out->grid = P.grid;
+    out->M = P.M; out->V = P.V; out->W = P.W; out->CL = P.framed ? P.fcl : P.CL; out->S = P.framed ? kFrameStages : P.S; out->G = P.G; out->grid = P.grid;
     out->nA = P.split ? P.nA : 0;
     out->layer_bytes = P.lb; out->dlayer_bytes = P.dlb; out->smem = P.smem;
     out->off_kinds = P.off_kinds; out->off_tiles = P.off_tiles; out->off_dtiles = P.off_dtiles;

@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kFrameThreads) frame_kernel(const FrameArgs a)
       if (m < sh) continue;
       const int j = q / M2, e = q - j * M2, c = e >= a.M / 4 ? 1 : 0, ep = e - c * (a.M / 4);
       const bool pair = m + 1 - 2 * h < modes;                                // the last odd-shift slot has one mode
-      const size_t o16 = (size_t)l * np2 + (size_t)(2 * ep) * a.G + j;        // h = 0; h = 1 lies G further
+      const size_t o16 = (size_t)l * (a.bwd ? 3 * np2 / 2 : np2) + (size_t)(2 * ep) * a.G + j;   // h = 0; h = 1 lies G further
       float2 kk = make_float2(0.f, 0.f);
       if (pair) kk = ffz_quot(ffz_mul(before(k2), ffz_of(to[kr])), after);
       else put(a.main + o16 + a.G, c, kk);   // its second row: nothing from outside reaches it
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kFrameThreads) frame_kernel(const FrameArgs a)
         const float t = cs[kr].x != 0.f ? cs[kr].y / cs[kr].x : 0.f;
         const ffz own = before(k);
         const size_t o8 = (size_t)l * (np2 / 2) + (size_t)ep * a.G + j;
-        put(a.gam + o8, c, make_float2(-t * ratio.y, -t * ratio.x));
+        put(a.main + (size_t)l * (3 * np2 / 2) + np2 + (size_t)ep * a.G + j, c, make_float2(-t * ratio.y, -t * ratio.x));
         reinterpret_cast<float*>(a.wts + o8)[c] = cs[kr].x * cs[kr].x / (after.x.h * after.x.h + after.y.h * after.y.h);
         reinterpret_cast<float*>(a.wts + o8)[2 + c] = 1.f / (own.x.h * own.x.h + own.y.h * own.y.h);
       }

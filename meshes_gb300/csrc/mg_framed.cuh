@@ -10,26 +10,33 @@
 // side in the tile).  By modes, the odd-shift layer's last pair mixes the halves, (M/2 - 1, M/2) and (M - 1, the next
 // lane's 0), which costs moves: 640 instructions per pair of layers in back-propagation at M = 8, V = 4, against 568.
 //
-// What bounds it: the FMA pipe and, with two warps per scheduler, the latency of each warp's chain (ncu, N = 256, B = 4096,
-// back-propagation: FMA pipe 52%, issue 44%, stalls for fixed latency and a busy pipe).  Measured on GB300 at N = 256,
-// L = 256, B = 4096 against the unframed kernels: forward 94 -> 63 us, back-propagation 249 -> 199 us; N = 600, L = 600,
-// B = 2048: forward 314 -> 200 us, back-propagation 1412 -> 900 us.
+// What bounds it: the register operands of the packed FMAs.  One with three register pairs of its own takes 3 cycles of a
+// scheduler, one that shares a pair with the FMA before it 2.3 to 2.5 (a loop of independent ones, GB300); at N = 256,
+// B = 4096 back-propagation's 458 per layer and scheduler are 1050 to 1370 of its 1500 cycles.  Three or four warps per
+// scheduler with fewer vectors each do not raise that (257 us for 12 warps of 3, 201 for 8 of 4).  Measured on GB300 at
+// N = 256, L = 256, B = 4096 against the unframed kernels: forward 94 -> 63 us, back-propagation 249 -> 197 us; N = 600,
+// L = 600, B = 2048: forward 314 -> 200 us, back-propagation 1412 -> 717 us.
 //
 // Work decomposition, pipeline, bounded waits and the gradient partials are those of mg_prop.cuh; a stage holds
-// three planes (main, the rows of resc that its layers have, gamma).
+// its layers' tiles and the factors of their first RESCALEs.
 #pragma once
 #include "mg_frame.cuh"
 
 namespace mg {
 
-// A layer's planes and its gradient staging as seen by one lane: shared-memory addresses
+// A layer's tile (main plane, gamma's behind it) and its gradient staging as seen by one lane: shared-memory addresses
 struct FTile {
-  uint32_t main, gam, grad;
+  uint32_t main, grad;
 };
 // 16 bytes of shared memory (volatile keeps them behind the barriers and waits)
 __device__ __forceinline__ ulonglong2 lds16(uint32_t addr) {
   ulonglong2 v;
   asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ int lds4(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
 __device__ __forceinline__ ulonglong2 ld16(const ulonglong2* p) {
@@ -179,7 +186,7 @@ __device__ __forceinline__ void f_layer(const FTile& t, int G, int j, int r, Fie
   for (int e = H / 2 - 1; e >= 0; --e) {   // (the boundary pair first: its results travel back while the others run)
     const uint32_t o = (uint32_t)(2 * e * G) * 16u;
     const ulonglong2 qa = lds16(t.main + o), qb = lds16(t.main + o + (uint32_t)G * 16u);
-    const ulonglong2 qg = OP == OP_BWD ? lds16(t.gam + o / 2) : make_ulonglong2(0, 0);
+    const ulonglong2 qg = OP == OP_BWD ? lds16(t.main + (uint32_t)(G * M) * 8u + o / 2) : make_ulonglong2(0, 0);
     float2 dth = make_float2(0.f, 0.f), dph = dth;
     const bool last = KIND != 0 && e == H / 2 - 1;
     if constexpr (NV > 0) {
@@ -292,35 +299,43 @@ __device__ __forceinline__ int step_code(const int* kinds, int L, int l) {
   const int k = at(l);
   if (k < 0) return 0;
   const bool mis = k & KIND_MIS, resc = k & KIND_RESCALE;
+  const int c = resc ? STEP_RESCALE : 0;
   if (OP == OP_FWD) {
-    if (mis || resc) return (mis ? STEP_1 : STEP_0) | (resc ? STEP_RESCALE : 0);
+    if (mis || resc) return c | (mis ? STEP_1 : STEP_0);
     const int n = at(l + 1);
     return n < 0 || !(n & KIND_MIS) ? STEP_0 : STEP_0 | STEP_1 | (n & KIND_RESCALE ? STEP_RESCALE : 0);
   }
-  const int c = resc ? STEP_RESCALE : 0;
   return mis ? c | STEP_0 | (at(l - 1) == 0 ? STEP_1 : 0) : c | STEP_1;
 }
 
-// Layers [lo, hi) of a chunk in the stage's planes; resc: the stage's rows for this lane
+// bytes of a layer's tile: forward launches read back-propagation's tiles too
+template <int OP>
+__device__ __forceinline__ uint32_t framed_layer(const FramedArgs& a, int np2) {
+  return OP == OP_BWD ? (uint32_t)np2 * 24u : a.flb;
+}
+
+// Layers [lo, hi) of a chunk in the stage at st; resc: the factors of its first framed_resc_rows RESCALE (more are
+// read from global memory); codes: layer 0's step code
 template <int OP, int M, int V>
-__device__ __forceinline__ void f_chunk(const FramedArgs& a, const int* codes, const FTile& st, const ulonglong2* resc,
-                                        uint32_t zero, uint32_t dump, int np2, int lo, int hi, int G, int j, int r,
-                                        Fields<M, V>& u, Fields<M, V>& w) {
+__device__ __forceinline__ void f_chunk(const FramedArgs& a, uint32_t codes, const FTile& st, uint32_t resc, const FTile& none,
+                                        int np2, int lo, int hi, int G, int j, int r, Fields<M, V>& u, Fields<M, V>& w) {
   constexpr int kDir = OP == OP_BWD ? -1 : 1;
-  const uint32_t row = (uint32_t)np2 * 16u;
-  int l = OP == OP_BWD ? hi - 1 : lo, left = hi - lo, rows = 0;
+  const uint32_t layer = framed_layer<OP>(a, np2), grad = (uint32_t)np2 * 8u;
+  int l = OP == OP_BWD ? hi - 1 : lo, left = hi - lo;
+  int rows = framed_resc_rows(a.fcl);
   auto tile = [&](bool there, int at) {
     const uint32_t i = (uint32_t)(at - lo);
-    return there ? FTile{st.main + i * row, st.gam + i * (row / 2), st.grad + i * (row / 2)} : FTile{zero, zero, dump};
+    return there ? FTile{st.main + i * layer, st.grad + i * grad} : none;
   };
   auto rescale = [&](int at) {
-    const ulonglong2* p = rows < a.xr ? resc + (size_t)rows * np2
-                                      : reinterpret_cast<const ulonglong2*>(a.resc + (size_t)at * np2) + j;
-    ++rows;
+    const ulonglong2* p = rows > 0 ? static_cast<const ulonglong2*>(__cvta_shared_to_generic(resc))
+                                   : reinterpret_cast<const ulonglong2*>(a.resc + (size_t)at * np2) + j;
+    --rows;
+    resc += (uint32_t)np2 * 16u;
     f_diag<M, V, OP == OP_BWD>([&](int k) { return ld16(p + k * G); }, u);
     if constexpr (OP == OP_BWD) f_diag<M, V, true>([&](int k) { return ld16(p + k * G); }, w);
   };
-  int c = codes[l];
+  int c = lds4(codes + 4 * l);
 #pragma unroll 1
   while (left > 0) {
     if (OP == OP_BWD && (c & STEP_RESCALE)) rescale(l);
@@ -333,7 +348,7 @@ __device__ __forceinline__ void f_chunk(const FramedArgs& a, const int* codes, c
       due = OP == OP_FWD && (c & STEP_RESCALE);
       l += n * kDir;
       left -= n;
-      c = codes[l];
+      c = lds4(codes + 4 * l);
       f_layer<OP, M, V, OP == OP_BWD ? KIND_MIS : 0>(t0, G, j, r, u, w);
       f_layer<OP, M, V, OP == OP_BWD ? 0 : KIND_MIS>(t1, G, j, r, u, w);
       if (OP == OP_BWD) due = c & STEP_RESCALE;
@@ -386,20 +401,10 @@ __device__ __forceinline__ ulonglong2 frame_pair(const float2* __restrict__ d, i
   const float2 d0 = __ldg(d + j * M + k), d1 = __ldg(d + j * M + M / 2 + k);
   return make_ulonglong2(p_pack(d0.x, d1.x), p_pack(d0.y, d1.y));
 }
-// CTA barriers by number: with MIX, warps of both kinds meet at them from their own copies of the body
+// CTA barrier by number: with MIX, warps of both kinds meet at it from their own copies of the body
 __device__ __forceinline__ void cta_sync() { asm volatile("barrier.cta.sync.aligned 0;" ::: "memory"); }
-__device__ __forceinline__ bool cta_sync_or(bool p) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
-      "barrier.cta.red.or.pred.aligned p, 0, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)p)
-      : "memory");
-  return r != 0;
-}
 
-// Chunk-end sum of the W warps' staged gradients (W a multiple of 4), in warp order, into this CTA's partials of the
+// Sum of the W warps' staged gradients of a chunk (W a multiple of 4), in warp order, into this CTA's partials of the
 // layers from lo on: n float4 of consecutive layers
 __device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int W, int n, ulonglong2* out) {
 #pragma unroll 1
@@ -418,64 +423,68 @@ __device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int 
 
 // The warp's vectors [vb0, vb0 + V) (per lane group) through all layers.  The pipeline's barriers are initialised, the
 // step codes and the layer of zeros are in shared memory.
+//
+// No CTA barrier between the first chunk and the last: a warp that has its chunk's stage goes through the chunk, sums
+// its share of the chunk before (kGradSlots of them are staged) and arrives; the only wait is for the others to have
+// finished that earlier chunk, so the warps of a scheduler may drift apart by up to a chunk and keep each other's
+// latency covered.  The copies are issued by one thread, of another warp for every chunk (those of V - 1 vectors where
+// there are some): what a warp does beyond its layers holds all the others up.  Measured on GB300 against two CTA barriers
+// and the sum at every chunk's end, copies issued by warp 0: N = 600, L = 600, B = 2048 803 -> 717 us, N = 400, B = 2432
+// 432 -> 368 us, N = 128, B = 4000 68 -> 63 us.
 struct FramedSmem {
   unsigned char* base;
   uint32_t zero, gst;
-  uint64_t* bars;
-  const int* codes;
+  uint32_t bars;        // [kFrameStages] the stage has its copies, [kFrameStages] every warp is done with the stage
+  uint32_t codes;       // of layer 0
+  uint32_t resc;        // per chunk: the layers of its first framed_resc_rows RESCALE, -1 behind the last
+  volatile int* state;  // [0] a wait ran out, [1] chunks whose copies were issued
+};
+// Layers of the walk in chunks of CL; the first chunk is one shorter where that keeps pairs of layers whole
+template <int OP>
+struct Chunks {
+  int L, CL, cut, n;
+  __device__ __forceinline__ Chunks(const FramedArgs& a) : L(a.L), CL(a.fcl) {
+    const int first = __ldg(a.fkinds + (OP == OP_BWD ? L - 1 : 0));
+    cut = (OP == OP_BWD ? !(first & KIND_MIS) : (first & KIND_MIS) != 0) && CL > 1 ? 1 : 0;
+    n = (L + cut + CL - 1) / CL;
+  }
+  __device__ __forceinline__ int walked(int c) const { return min(L, max(0, c * CL - cut)); }   // layers before chunk c
+  __device__ __forceinline__ int lo(int c) const { return OP == OP_BWD ? L - walked(c + 1) : walked(c); }
+  __device__ __forceinline__ int hi(int c) const { return OP == OP_BWD ? L - walked(c) : walked(c + 1); }
 };
 template <int OP, int M, int V, int GT>
-__device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSmem& sm, int vb0) {
+__device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSmem& sm, const Chunks<OP>& ch, int vb0, int issuer) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Lanes<GT> ln(a.G, a.logG);
   const int G = ln.G, j = ln.j, r = ln.r;
-  const int np2 = (G * M) >> 1, CL = a.fcl, S = a.fs;
-  const uint32_t row = (uint32_t)np2 * 16u, warp_bytes = (uint32_t)CL * (row / 2), j16 = (uint32_t)j * 16u;
-  const uint32_t stage = (uint32_t)framed_stage_bytes(OP, np2, CL, a.xr), ring = smem_u32(sm.base);
+  const int np2 = (G * M) >> 1, CL = a.fcl;
+  constexpr int S = kFrameStages;
+  const uint32_t layer = framed_layer<OP>(a, np2), row = (uint32_t)np2 * 16u, warp_bytes = (uint32_t)CL * (row / 2), j16 = (uint32_t)j * 16u;
+  const uint32_t stage = (uint32_t)framed_stage_bytes(layer, np2, CL), ring = smem_u32(sm.base);
+  const uint32_t slot_bytes = (uint32_t)a.W * warp_bytes;
   Fields<M, V> u, w;
   f_load<M, V>(u, a.in0, vb0, a.vend, a.N, a.ldu, j);
   if constexpr (OP == OP_BWD) f_load<M, V>(w, a.target ? a.target : a.in1, vb0, a.vend, a.N, a.ldu, j);
 
-  // chunks of CL layers in the order of the walk; the first is one shorter where that keeps pairs of layers whole
-  const int first = __ldg(a.fkinds + (OP == OP_BWD ? a.L - 1 : 0));
-  const int cut = (OP == OP_BWD ? !(first & KIND_MIS) : (first & KIND_MIS) != 0) && CL > 1 ? 1 : 0;
-  const int nch = (a.L + cut + CL - 1) / CL;
-  auto walked = [&](int c) { return min(a.L, max(0, c * CL - cut)); };   // layers before chunk c
-  auto chunk_lo = [&](int c) { return OP == OP_BWD ? a.L - walked(c + 1) : walked(c); };
-  auto chunk_hi = [&](int c) { return OP == OP_BWD ? a.L - walked(c) : walked(c + 1); };
-  const uint64_t wlim = a.wait_ns ? a.wait_ns : kWaitLimitNs;
-  // warp 0: the copies of chunk c into stage s - the main plane (and gamma's) whole, and the rows of resc
-  auto issue = [&](int c, int s) {
-    if (c + 1 == a.unarmed) return;
-    const int lo = chunk_lo(c), n = chunk_hi(c) - lo;
-    const uint32_t bar = smem_u32(sm.bars + s), at = ring + (uint32_t)s * stage;
-    auto has = [&](int i) {   // the walk's i-th layer
-      return i < n && (__ldg(a.fkinds + (OP == OP_BWD ? lo + n - 1 - i : lo + i)) & KIND_RESCALE);
-    };
-    int rows = 0;
-    for (int i0 = 0; i0 < n; i0 += 32) rows += __popc(__ballot_sync(0xffffffffu, has(i0 + lane)));
-    if (lane == 0) {
-      mbar_arrive_expect_tx(bar, (n + min(rows, a.xr)) * row + (OP == OP_BWD ? n * (row >> 1) : 0u));
-      tma_load_1d(at, a.main + (size_t)lo * np2, n * row, bar);
-      if constexpr (OP == OP_BWD)
-        tma_load_1d(at + (uint32_t)(CL + a.xr) * row, a.gam + (size_t)lo * (np2 / 2), n * (row >> 1), bar);
-    }
-    if (rows == 0) return;
-    __syncwarp();
-    rows = 0;
-    for (int i0 = 0; i0 < n; i0 += 32) {
-      const int i = i0 + lane;
-      const bool is = has(i);
-      const unsigned b = __ballot_sync(0xffffffffu, is);
-      const int k = rows + __popc(b & ((1u << lane) - 1u));
-      if (is && k < a.xr)
-        tma_load_1d(at + (uint32_t)(CL + k) * row, a.resc + (size_t)(OP == OP_BWD ? lo + n - 1 - i : lo + i) * np2, row, bar);
-      rows += __popc(b);
-    }
+  const int nch = ch.n;
+  auto wait = [&](uint32_t bar, uint32_t phase) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, a.wait_ns ? a.wait_ns : kWaitLimitNs));
   };
-  int issued = min(S, nch);
-  if (warp == 0)
-    for (int c = 0; c < issued; ++c) issue(c, c);
+  // one thread: the copies of chunk c into stage s
+  auto issue = [&](int c, int s) {
+    sm.state[1] = c + 1;
+    if (c + 1 == a.unarmed) return;
+    const int lo = ch.lo(c), n = ch.hi(c) - lo, xr = framed_resc_rows(CL);
+    int rows = 0;
+    while (rows < xr && lds4(sm.resc + 4u * (c * xr + rows)) >= 0) ++rows;
+    const uint32_t bar = sm.bars + 8u * s, at = ring + (uint32_t)s * stage;
+    mbar_arrive_expect_tx(bar, n * layer + rows * row);
+    tma_load_1d(at, reinterpret_cast<const unsigned char*>(a.main) + (size_t)lo * layer, n * layer, bar);
+    for (int k = 0; k < rows; ++k)
+      tma_load_1d(at + (uint32_t)CL * layer + (uint32_t)k * row, a.resc + (size_t)lds4(sm.resc + 4u * (c * xr + k)) * np2, row, bar);
+  };
+  if (tid == 0)
+    for (int c = 0; c < min(S, nch); ++c) issue(c, c);
   if constexpr (OP == OP_FWD) {
     f_scale<M, V>(1.f / (1ull << kFrameTop), u);
   } else {
@@ -488,45 +497,57 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
     f_diag<M, V, true>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, w);
   }
 
-  int s = 0;
-  uint32_t phase = 0;
+  // chunk c: stage and gradient slot s = c % S, of whose barriers it is phase ph = (c / S) & 1
+  auto reduce = [&](int c, int s) {
+    const int lo = ch.lo(c);
+    f_reduce(sm.gst + (uint32_t)s * slot_bytes, warp_bytes, a.W, (ch.hi(c) - lo) * (np2 / 2),
+             reinterpret_cast<ulonglong2*>(a.partial + (size_t)lo * np2));
+  };
+  const FTile none{sm.zero + j16, sm.gst + (uint32_t)S * slot_bytes + j16};
+  int c = 0, s = 0;
+  uint32_t ph = 0;
+  bool ok = true;
 #pragma unroll 1
-  for (int c = 0; c < nch; ++c) {
-    const int lo = chunk_lo(c), hi = chunk_hi(c);
-    const bool ok = mbar_wait_bounded(smem_u32(sm.bars + s), phase, wlim);
-    if (ok) {
-      const uint32_t at = (uint32_t)s * stage;
-      const FTile st{ring + at + j16, ring + at + (uint32_t)(CL + a.xr) * row + j16, sm.gst + (uint32_t)warp * warp_bytes + j16};
-      f_chunk<OP, M, V>(a, sm.codes, st, reinterpret_cast<const ulonglong2*>(sm.base + at + (uint32_t)CL * row) + j,
-                        sm.zero + j16, sm.gst + (uint32_t)a.W * warp_bytes + j16, np2, lo, hi, G, j, r, u, w);
+  for (; c < nch; ++c) {
+    ok = wait(sm.bars + 8u * s, ph);
+    if (!ok) break;
+    const uint32_t at = ring + (uint32_t)s * stage + j16;
+    f_chunk<OP, M, V>(a, sm.codes, FTile{at, sm.gst + (uint32_t)s * slot_bytes + (uint32_t)warp * warp_bytes + j16},
+                      at + (uint32_t)CL * layer, none, np2, ch.lo(c), ch.hi(c), G, j, r, u, w);
+    const bool mine = warp == issuer + (c & 3);
+    if (c > 0 && (OP == OP_BWD || mine)) {
+      // every warp is done with chunk c - 1 (and, having waited as this one does, with the sum of chunk c - 2, whose slot
+      // is the next chunk's)
+      const int prev = s ? s - 1 : S - 1;
+      ok = wait(sm.bars + 8u * (S + prev), s ? ph : ph ^ 1);
+      if (!ok) break;
+      if (mine && lane == 0 && c + S - 1 < nch) issue(c + S - 1, prev);
+      if constexpr (OP == OP_BWD) reduce(c - 1, prev);
     }
-    // every warp is done with the stage, and (back-propagation) every warp's gradients of the chunk are staged
-    if (cta_sync_or(!ok)) {
-      // give up: record, wait (bounded) for the copies still in flight, release the barriers, leave
-      if (tid == 0) {
-        set_status(a.status, ST_TIMEOUT);
-        for (int cc = c; cc < issued; ++cc)
-          if (cc + 1 != a.unarmed) mbar_wait_bounded(smem_u32(sm.bars + (cc % S)), (uint32_t)((cc / S) & 1), wlim);
-        for (int k = 0; k < S; ++k) mbar_inval(smem_u32(sm.bars + k));
-      }
-      return;
-    }
-    if (issued < nch) {
-      if (warp == 0) issue(issued, s);
-      ++issued;
-    }
-    if constexpr (OP == OP_BWD) {
-      f_reduce(sm.gst, warp_bytes, a.W, (hi - lo) * (np2 / 2),
-               reinterpret_cast<ulonglong2*>(a.partial + ((size_t)blockIdx.x * a.L + lo) * np2));
-      cta_sync();
-    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(sm.bars + 8u * (S + s));
     if (++s == S) {
       s = 0;
-      phase ^= 1;
+      ph ^= 1;
     }
   }
+  if (!ok && lane == 0) sm.state[0] = 1;
+  cta_sync();
+  if (sm.state[0]) {
+    // a wait ran out: record, wait (bounded) for the copies still in flight, release the barriers, leave
+    if (tid == 0) {
+      set_status(a.status, ST_TIMEOUT);
+      for (int cc = c; cc < sm.state[1]; ++cc)
+        if (cc + 1 != a.unarmed)
+          mbar_wait_bounded(sm.bars + 8u * (cc % S), (uint32_t)((cc / S) & 1), a.wait_ns ? a.wait_ns : kWaitLimitNs);
+      for (int k = 0; k < 2 * S; ++k) mbar_inval(sm.bars + 8u * k);
+    }
+    return;
+  }
   if (tid == 0)
-    for (int k = 0; k < S; ++k) mbar_inval(smem_u32(sm.bars + k));
+    for (int k = 0; k < 2 * S; ++k) mbar_inval(sm.bars + 8u * k);
+  if constexpr (OP == OP_BWD)
+    if (nch > 0) reduce(nch - 1, (nch - 1) % S);
   if constexpr (OP == OP_FWD) {
     f_diag<M, V, false>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, u);
     f_store<M, V>(u, a.out0, vb0, a.vend, a.N, a.ldu, j);
@@ -540,58 +561,93 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
   }
 }
 
-// One CTA: W warps of V vectors per lane group; MIX: warps 4-7 (12-15) take V - 1, so that every scheduler carries
-// 2V - 1.  The two kinds have a body each, chosen once per warp.  A mesh that the frames do not suit (a.refuse) takes
-// the unframed body of mg_prop.cuh on the same vectors.
+// The vectors [v0, vend) of a by one CTA: W warps of V vectors per lane group; MIX: warps 4-7 (12-15) take V - 1, so that
+// every scheduler carries 2V - 1.  The two kinds have a body each, chosen once per warp.  A mesh that the frames do not
+// suit (a.refuse) takes the unframed body of mg_prop.cuh on the same vectors.
 template <int OP, int M, int V, int GT, bool MIX>
-__global__ void __launch_bounds__(framed_max_threads(M, V), 1) framed_kernel(const FramedArgs a0) {
-  extern __shared__ __align__(128) unsigned char smem[];
+__device__ __forceinline__ void framed_run(const FramedArgs& a, unsigned char* smem) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = GT ? GT : a0.G, R = 32 / G, np2 = (G * M) >> 1, r = lane / G;
-  const int v0 = blockIdx.x * framed_cta_vectors(a0.W, R, V, MIX);
-  FramedArgs a = a0;
-  a.vend = min(a.B, v0 + framed_cta_vectors(a0.W, R, V, MIX));
+  const int G = GT ? GT : a.G, R = 32 / G, np2 = (G * M) >> 1, r = lane / G, v0 = a.v0;
   if (__ldg(a.count) >= a.refuse) {
-    a.v0 = v0;
-    if (OP == OP_BWD) a.partial = a0.partial + (size_t)blockIdx.x * a.L * np2;
     prop_body<OP, M, V, false, GT, OP == OP_BWD ? 1 : 0, false, true>(a, smem);
     return;
   }
-  const size_t zero = a.fs * framed_stage_bytes(OP, np2, a.fcl, a.xr);
+  const uint32_t layer = framed_layer<OP>(a, np2);
+  const size_t bars = framed_bars_offset(OP, layer, np2, a.W, a.fcl);
+  const Chunks<OP> ch(a);
   FramedSmem sm;
   sm.base = smem;
-  sm.zero = smem_u32(smem + zero);
-  sm.gst = sm.zero + (uint32_t)np2 * 16u;
-  sm.bars = reinterpret_cast<uint64_t*>(smem + framed_bars_offset(OP, np2, a.W, a.fcl, a.fs, a.xr));
-  int* codes = reinterpret_cast<int*>(sm.bars + a.fs + (a.fs & 1)) + kCodePad;
-  sm.codes = codes;
+  sm.zero = smem_u32(smem + kFrameStages * framed_stage_bytes(layer, np2, a.fcl));
+  sm.gst = sm.zero + layer;
+  sm.bars = smem_u32(smem + bars);
+  sm.state = reinterpret_cast<volatile int*>(smem + bars + 16 * kFrameStages);
+  int* codes = reinterpret_cast<int*>(smem + bars + 16 * kFrameStages + 16) + kCodePad;
+  int* resc = codes + a.L + kCodePad;
+  sm.codes = smem_u32(codes);
+  sm.resc = smem_u32(resc);
+  for (int c = tid; c < ch.n; c += blockDim.x) {
+    const int lo = ch.lo(c), n = ch.hi(c) - lo, xr = framed_resc_rows(a.fcl);
+    int rows = 0;
+    for (int i = 0; i < n && rows < xr; ++i) {
+      const int l = OP == OP_BWD ? lo + n - 1 - i : lo + i;
+      if (__ldg(a.fkinds + l) & KIND_RESCALE) resc[c * xr + rows++] = l;
+    }
+    if (rows < xr) resc[c * xr + rows] = -1;
+  }
   for (int l = tid - kCodePad; l < a.L + kCodePad; l += blockDim.x) codes[l] = step_code<OP>(a.fkinds, a.L, l);
-  for (int i = tid; i < np2; i += blockDim.x) sts16(sm.zero + (uint32_t)i * 16u, 0, 0);
+  for (int i = tid; i < (int)layer / 16; i += blockDim.x) sts16(sm.zero + (uint32_t)i * 16u, 0, 0);
   if (tid == 0) {
-    for (int s = 0; s < a.fs; ++s) mbar_init(smem_u32(sm.bars + s), 1);
+    for (int s = 0; s < kFrameStages; ++s) {
+      mbar_init(sm.bars + 8u * s, 1);
+      mbar_init(sm.bars + 8u * (kFrameStages + s), a.W);
+    }
+    sm.state[0] = sm.state[1] = 0;
     fence_mbar_init();
   }
   __syncthreads();
   if constexpr (MIX) {
     // warps of four alternate between V and V - 1 vectors
     const int base = v0 + (warp >> 3) * R * 4 * (2 * V - 1), in = (warp & 3) * R + r;
-    if (warp & 4) framed_body<OP, M, V - 1, GT>(a, sm, base + R * 4 * V + in * (V - 1));
-    else framed_body<OP, M, V, GT>(a, sm, base + in * V);
+    if (warp & 4) framed_body<OP, M, V - 1, GT>(a, sm, ch, base + R * 4 * V + in * (V - 1), 4);
+    else framed_body<OP, M, V, GT>(a, sm, ch, base + in * V, 4);
   } else {
-    framed_body<OP, M, V, GT>(a, sm, v0 + (warp * R + r) * V);
+    framed_body<OP, M, V, GT>(a, sm, ch, v0 + (warp * R + r) * V, 0);
   }
+}
+
+template <int OP, int M, int V, int GT, bool MIX>
+__global__ void __launch_bounds__(framed_max_threads(M, V), 1) framed_kernel(const FramedArgs a0) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int G = GT ? GT : a0.G, cap = framed_cta_vectors(a0.W, 32 / G, V, MIX);
+  FramedArgs a = a0;
+  a.v0 = blockIdx.x * cap;
+  a.vend = min(a.B, a.v0 + cap);
+  if (OP == OP_BWD) a.partial = a0.partial + (size_t)blockIdx.x * a.L * ((G * M) >> 1);
+  framed_run<OP, M, V, GT, MIX>(a, smem);
 }
 
 // dp[l][q][k] (= or +=) the sum over the nC per-CTA partials times the frames' weights, in the CTAs' order (as
 // dp_reduce_kernel, whose layout of threads it shares); a float2 holds gradient k of the crossings e and e + M/4
-static __global__ void __launch_bounds__(256) framed_reduce_kernel(const float2* __restrict__ partial, int nC, int L, int np2,
-                                                            int M, int G, int N, float* dp, int ldp, int accumulate,
-                                                            const int* __restrict__ geo, const float2* __restrict__ wts,
-                                                            const int* __restrict__ count, int refuse) {
-  constexpr int kCols = 32, kRows = 8;
-  __shared__ float2 acc[kRows][kCols];
+constexpr int kFReduceCols = 32, kFReduceRows = 8;
+struct FramedReduceArgs {
+  const float2* partial;
+  int nC, L, np2, M, G, N;
+  float* dp;
+  int ldp, accumulate;
+  const int* geo;
+  const float2* wts;
+  const int* count;
+  int refuse;
+};
+// columns [kFReduceCols blk, ..); the caller's threads meet before acc is used again
+__device__ __forceinline__ void framed_reduce_block(const FramedReduceArgs& a, int blk, float2 (&acc)[kFReduceRows][kFReduceCols]) {
+  constexpr int kCols = kFReduceCols, kRows = kFReduceRows;
+  const float2* partial = a.partial;
+  float* dp = a.dp;
+  const int nC = a.nC, L = a.L, np2 = a.np2, M = a.M, G = a.G, N = a.N, ldp = a.ldp, accumulate = a.accumulate;
+  const int* geo = a.geo;
   const int col = threadIdx.x % kCols, row = threadIdx.x / kCols;
-  const int idx = blockIdx.x * kCols + col;
+  const int idx = blk * kCols + col;
   const bool valid = idx < L * np2;
   const size_t stride = (size_t)L * np2;
   float2 s = make_float2(0.f, 0.f);
@@ -610,7 +666,7 @@ static __global__ void __launch_bounds__(256) framed_reduce_kernel(const float2*
   if (row != 0 || !valid) return;
   for (int k = 1; k < kRows; ++k) s = cadd(s, acc[k][col]);
   const int l = idx / np2, rem = idx - l * np2;
-  if (__ldg(count) >= refuse) {   // partials of the unframed body: (dJ/dth, dJ/dph) of one slot
+  if (__ldg(a.count) >= a.refuse) {   // partials of the unframed body: (dJ/dth, dJ/dph) of one slot
     const int q = pos_slot(rem, M, G);
     if (q >= N / 2) return;
     const bool active = q >= geo[2 * l] / 2 && q < geo[2 * l] / 2 + geo[2 * l + 1];
@@ -622,7 +678,7 @@ static __global__ void __launch_bounds__(256) framed_reduce_kernel(const float2*
   const int k = rem & 1, pos = rem >> 1;
   const int j = pos % G, q0 = j * (M / 2) + pos / G;
   const int sh = geo[2 * l] / 2, ln = geo[2 * l + 1];
-  const float2 w = __ldg(wts + idx);
+  const float2 w = __ldg(a.wts + idx);
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
     const int q = q0 + c * (M / 4);
@@ -631,6 +687,11 @@ static __global__ void __launch_bounds__(256) framed_reduce_kernel(const float2*
     float* o = dp + (size_t)l * ldp + 2 * (size_t)q + k;
     *o = accumulate ? *o + v : v;
   }
+}
+
+static __global__ void __launch_bounds__(256) framed_reduce_kernel(const FramedReduceArgs a) {
+  __shared__ float2 acc[kFReduceRows][kFReduceCols];
+  framed_reduce_block(a, blockIdx.x, acc);
 }
 
 }  // namespace mg

@@ -10,11 +10,12 @@ constexpr int kFrameTop = 22, kFrameDue = -8, kFrameNow = -18;
 constexpr int kFrameSeg = 16;              // layers per segment, about
 constexpr int kFrameBatch = 16;            // layers whose frames are held in shared memory at a time
 constexpr int kFrameThreads = 512;
+constexpr int kFrameStages = 3;            // pipeline stages and gradient slots: the chunk at work, the one before, the next
 constexpr int KIND_RESCALE = 1 << 14;      // OR-ed into a layer's kind: the frames start again behind it
 
-// Tile planes of one layer, lane j, pair e < M/4 of the lane's crossings (e, e + M/4), values of the two side by side:
+// Planes of one layer, lane j, pair e < M/4 of the lane's crossings (e, e + M/4), values of the two side by side:
 //   main [(2e + h) G + j] = (re, re', im, im') of alpha (h = 0), beta (h = 1)
-//   gam  [e G + j]          gamma
+//   gam  [e G + j]          gamma, back-propagation only: behind the layer's main plane (framed_layer_bytes)
 //   resc [k G + j], k < M/2 RESCALE layers: the factors of the lane's modes k and k + M/2
 // Gradient partials and their weights: float4 (th, th', ph, ph') at [e G + j].
 struct FrameArgs {
@@ -25,9 +26,8 @@ struct FrameArgs {
   const float* tmag;
   const float2* tcs;
   const int* kinds;              // [L]
-  float4* main;                  // [L][np2]
+  float4* main;                  // [L][np2, bwd: + np2/2 of gamma]
   float4* resc;                  // [L][np2]
-  float4* gam;                   // [L][np2/2]
   float4* wts;                   // [L][np2/2]
   float2* dfin;                  // [modes]: frames after the last layer
   int* fkinds;                   // [L] kinds with KIND_RESCALE
@@ -45,12 +45,11 @@ inline size_t frame_smem_bytes(int modes, int rows) {
 struct FramedArgs : PropArgs {
   const float4* main;
   const float4* resc;
-  const float4* gam;
   const float2* dfin;
   const int* fkinds;
   const int* count;
-  int fcl, fs;                   // layers per stage, stages
-  int xr;                        // rows of resc in a pipeline stage
+  int fcl;                       // layers per stage
+  unsigned flb;                  // bytes of a layer's tile
   int refuse;                    // count from which on the mesh takes the unframed body
 };
 // threads per CTA the kernels are compiled for
@@ -59,20 +58,20 @@ __host__ __device__ constexpr int framed_max_threads(int M, int V) { return M * 
 __host__ __device__ constexpr int framed_cta_vectors(int W, int R, int V, bool mix) {
   return R * (W * V - (mix ? W / 8 * 4 : 0));
 }
-// one pipeline stage: CL layers of the main plane, xr rows of resc, (back-propagation) CL layers of gamma
-__host__ __device__ inline size_t framed_stage_bytes(int op, int np2, int CL, int xr) {
-  return (size_t)np2 * (16 * (size_t)(CL + xr) + (op == OP_BWD ? 8 * (size_t)CL : 0));
+// rows of resc staged with CL layers (few layers have one: each segment's last and those that bound the frames; more are
+// read from global memory)
+__host__ __device__ constexpr int framed_resc_rows(int CL) { return CL / 8 > 1 ? CL / 8 : 1; }
+// one layer's tile (op: that the tiles are built for); one pipeline stage: CL tiles of lb bytes and the rows of resc
+__host__ __device__ constexpr unsigned framed_layer_bytes(int op, int np2) { return (unsigned)np2 * (op == OP_BWD ? 24 : 16); }
+__host__ __device__ constexpr size_t framed_stage_bytes(unsigned lb, int np2, int CL) { return (size_t)CL * lb + (size_t)framed_resc_rows(CL) * np2 * 16; }
+// shared memory of a launch: [stages][a layer of zeros][BWD: per slot the W warps' gradients of CL layers, one layer beyond
+// the last][2 mbarriers per stage][state][step codes][RESCALEs per chunk]
+__host__ __device__ constexpr size_t framed_bars_offset(int op, unsigned lb, int np2, int W, int CL) {
+  return kFrameStages * framed_stage_bytes(lb, np2, CL) + lb +
+         (op == OP_BWD ? ((size_t)kFrameStages * W * CL + 1) * np2 * 8 : 0);
 }
-// rows of resc in a stage of CL layers: few layers have one (each segment's last, and those that bound the frames);
-// the rows beyond are read from global memory
-inline int framed_resc_rows(int CL) { return CL / 8 + 1 < CL ? CL / 8 + 1 : CL; }
-// shared memory of a launch: [S stages][a layer of zeros][BWD: per-warp gradients, one layer beyond the last warp's]
-// [S mbarriers][step codes]
-__host__ __device__ inline size_t framed_bars_offset(int op, int np2, int W, int CL, int S, int xr) {
-  return S * framed_stage_bytes(op, np2, CL, xr) + (size_t)np2 * 16 + (op == OP_BWD ? ((size_t)W * CL + 1) * np2 * 8 : 0);
-}
-inline size_t framed_smem_bytes(int op, int np2, int W, int CL, int S, int L) {
-  return framed_bars_offset(op, np2, W, CL, S, framed_resc_rows(CL)) + 8 * (size_t)(S + (S & 1)) + 4 * (size_t)(L + 8);
+__host__ __device__ constexpr size_t framed_smem_bytes(int op, unsigned lb, int np2, int W, int CL, int L) {
+  return framed_bars_offset(op, lb, np2, W, CL) + 16 * kFrameStages + 16 + 4 * (size_t)(L + 8) + 4 * (size_t)((L + CL) / CL) * framed_resc_rows(CL);
 }
 
 }  // namespace mg
