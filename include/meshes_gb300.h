@@ -261,6 +261,29 @@ int mg_batched_propagate(int op, const mg_batch_mesh* meshes, int n_meshes, cons
 /* Deterministic sum of the back-propagation partials of every mesh into its dp. */
 int mg_batched_reduce(const mg_batch_mesh* meshes, int n_meshes, void* stream);
 
+/* The same for meshes on framed tiles (mg_config{8, 4, 8, .., split 5}): nearest-neighbour MZI meshes of 129 to 256 modes.
+ * mg_batched_framed_desc describes a mesh on the workspace that mg_build_tiles(MG_OP_BWD) filled with that
+ * configuration, for both ops (forward reads back-propagation's tiles); the caller sets the fields, B, ldu, n_items, ldp,
+ * n_p, dp and partial of `mesh` (back-propagation: n_items * L * 128 float2).  *smem_fwd, *smem_bwd: dynamic shared
+ * memory of a launch.  An item is up to 32 vectors. */
+typedef struct mg_batch_framed {
+  mg_batch_mesh mesh;
+  const void* main;
+  const void* resc;
+  const void* wts;
+  const void* dfin;
+  const int* fkinds;
+  const int* count;
+  int fcl, refuse;
+  unsigned flb;
+} mg_batch_framed;
+int mg_batched_framed_desc(int N, int L, int B, int crossing, int geometry, const mg_config* cfg, const void* workspace,
+                           size_t workspace_bytes, mg_batch_framed* fwd, mg_batch_framed* bwd, size_t* smem_fwd,
+                           size_t* smem_bwd);
+int mg_batched_framed(int op, const mg_batch_framed* meshes, int n_meshes, const mg_batch_item* items, int n_items, int* head,
+                      int grid, size_t smem, int* status, void* stream);
+int mg_batched_framed_reduce(const mg_batch_framed* meshes, int n_meshes, void* stream);
+
 /* Back-propagation with the L2 loss to a target fused into the kernel: dJ/dy* = 2 (y - target) is
  * formed on load (J = sum |y - target|^2), then as mg_propagate(MG_OP_BWD) with tiles built earlier.
  * The reference computes this gradient in a separate pass (gpu/mesh.py:176-181, 219-221). */

@@ -48,6 +48,11 @@ class mg_batch_mesh(Structure):
                 ("out0", c_void_p), ("out1", c_void_p), ("dp", c_void_p), ("partial", c_void_p)]
 
 
+class mg_batch_framed(Structure):
+    _fields_ = [("mesh", mg_batch_mesh), ("main", c_void_p), ("resc", c_void_p), ("wts", c_void_p), ("dfin", c_void_p),
+                ("fkinds", c_void_p), ("count", c_void_p), ("fcl", c_int), ("refuse", c_int), ("flb", c_uint)]
+
+
 class mg_server_mesh(Structure):
     _fields_ = [("N", c_int), ("L", c_int), ("cls", c_int), ("G", c_int), ("n_p", c_int), ("cap", c_int),
                 ("fwd_CL", c_int), ("fwd_S", c_int), ("bwd_CL", c_int), ("bwd_S", c_int),
@@ -129,6 +134,11 @@ _SIGS = {
     "mg_batched_propagate": (c_int, [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_size_t, c_void_p,
                                      c_void_p]),
     "mg_batched_reduce": (c_int, [c_void_p, c_int, c_void_p]),
+    "mg_batched_framed_desc": (c_int, [c_int, c_int, c_int, c_int, c_int, POINTER(mg_config), c_void_p, c_size_t,
+                                       POINTER(mg_batch_framed), POINTER(mg_batch_framed), POINTER(c_size_t),
+                                       POINTER(c_size_t)]),
+    "mg_batched_framed": (c_int, [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_size_t, c_void_p, c_void_p]),
+    "mg_batched_framed_reduce": (c_int, [c_void_p, c_int, c_void_p]),
 }
 
 _lock = threading.Lock()

@@ -1,4 +1,4 @@
-"""Batched meshes: many independent meshes of uneven size and depth in one persistent launch.
+"""Batched meshes: many independent meshes of uneven size and depth in a few persistent launches.
 
 ``BatchedMeshes(meshes)`` keeps every mesh's coefficient tiles resident (built once, rebuilt by
 ``update_phases``), owns device buffers for each mesh's batch, and propagates all of them with one
@@ -16,7 +16,8 @@ from typing import List, Optional, Sequence
 import torch
 
 from . import _lib
-from ._lib import BATCH_NN, GEO_NN, OP_BWD, OP_FWD, check, load, mg_batch_item, mg_batch_mesh, mg_plan_info
+from ._lib import (BATCH_NN, GEO_NN, OP_BWD, OP_FWD, check, load, mg_batch_framed, mg_batch_item, mg_batch_mesh,
+                   mg_plan_info)
 from .mesh import MeshNetworkGPU, _stream
 
 BCLS_C8, BCLS_C16, BCLS_R8 = 0, 1, 2
@@ -59,16 +60,21 @@ def _to_device(structs, device) -> torch.Tensor:
 
 
 class _MeshState:
-    def __init__(self, mesh: MeshNetworkGPU, B: int):
+    def __init__(self, mesh: MeshNetworkGPU, B: int, framed: bool = False):
         self.mesh, self.B = mesh, int(B)
         self.cls = kernel_class(mesh)
         M, V = _CLS_MV[self.cls]
         self.M, self.V = M, V
-        self.cfg = {op: _lib.config(M, V, WARPS, 0, 0, 2) for op in (OP_FWD, OP_BWD)}
-        self.info = {op: plan(op, mesh.N, mesh.L, max(self.B, 1), mesh.crossing, mesh.geometry, self.cfg[op])
-                     for op in (OP_FWD, OP_BWD)}
+        # Complex nearest-neighbour meshes of 129 to 256 modes run on framed tiles: half the forward and two thirds of the
+        # back-propagation FMAs (96 uneven meshes, forward and back-propagation: 2606 -> 2194 us on GB300), and one build
+        # for both ops, since forward reads back-propagation's tiles.  Smaller meshes keep the tile they share lanes in.
+        self.framed = framed and self.cls == BCLS_C8 and mesh.geometry == GEO_NN and mesh.N > 128 and self._plan_framed()
+        if not self.framed:
+            self.cfg = {op: _lib.config(M, V, WARPS, 0, 0, 2) for op in (OP_FWD, OP_BWD)}
+            self.info = {op: plan(op, mesh.N, mesh.L, max(self.B, 1), mesh.crossing, mesh.geometry, self.cfg[op])
+                         for op in (OP_FWD, OP_BWD)}
         self.ws = {}
-        for op in (OP_FWD, OP_BWD):
+        for op in ((OP_BWD,) if self.framed else (OP_FWD, OP_BWD)):
             self.ws[op] = torch.empty(self.info[op].total, dtype=torch.uint8, device=mesh.device)
             check(load().mg_workspace_init(self.ws[op].data_ptr(), self.ws[op].numel(), _stream(mesh.device)),
                   "mg_workspace_init")
@@ -86,32 +92,63 @@ class _MeshState:
         self.partial = torch.empty(max(self.n_items, 1) * mesh.L * self.np2 * 2, dtype=torch.float32, device=dev)
         self.build_tiles()
 
+    def _plan_framed(self) -> bool:
+        """Plan the mesh on framed tiles; False where the library has none for it."""
+        m = self.mesh
+        self.cfg = {op: _lib.config(8, 4, WARPS, 0, 0, 5) for op in (OP_FWD, OP_BWD)}
+        try:
+            self.info = {op: plan(op, m.N, m.L, max(self.B, 1), m.crossing, m.geometry, self.cfg[op])
+                         for op in (OP_FWD, OP_BWD)}
+        except _lib.MeshLibraryError:
+            return False
+        return True
+
     def build_tiles(self, p: Optional[torch.Tensor] = None):
         m = self.mesh
         p = m.p_phase if p is None else p
         s = m.p_splitter
         geo = ((None, None, m.strides.data_ptr()) if m.strides is not None else (m.lens.data_ptr(), m.shifts.data_ptr(), None))
-        for op in (OP_FWD, OP_BWD):
+        for op in self.ws:
             check(load().mg_build_tiles(op, m.N, m.L, m.geometry, *geo, m.crossing, p.data_ptr(), m.N // 2 * m.X_np,
                                         s.data_ptr() if s.numel() else None, m.N // 2 * m.X_ns, None, None, None,
                                         max(self.B, 1), _lib.cfg_ptr(self.cfg[op]), self.ws[op].data_ptr(),
                                         self.ws[op].numel(), _stream(m.device)), "mg_build_tiles")
 
     def descriptor(self, op) -> mg_batch_mesh:
-        m, info, ws = self.mesh, self.info[op], self.ws[op]
         d = mg_batch_mesh()
+        if self.framed:                                   # its items and its reduction run on framed_descriptors()
+            return d
+        m, info, ws = self.mesh, self.info[op], self.ws[op]
         d.N, d.L, d.B, d.ldu = m.N, m.L, self.B, m.N
         d.cls, d.G, d.CL, d.S = self.cls, info.G, info.CL, info.S
         d.layer_bytes, d.n_items, d.ldp, d.n_p = info.layer_bytes, self.n_items, m.N // 2 * m.X_np, m.X_np
         d.tiles = ws.data_ptr() + info.off_tiles
         d.kinds = ws.data_ptr() + info.off_kinds
+        self._fields(op, d)
+        return d
+
+    def _fields(self, op, d: mg_batch_mesh):
         if op == OP_FWD:
             d.in0, d.in1, d.out0, d.out1 = self.x.data_ptr(), None, self.y.data_ptr(), None
             d.dp, d.partial = None, None
         else:
             d.in0, d.in1, d.out0, d.out1 = self.y.data_ptr(), self.gy.data_ptr(), None, self.gx.data_ptr()
             d.dp, d.partial = self.dp.data_ptr(), self.partial.data_ptr()
-        return d
+
+    def framed_descriptors(self):
+        """({op: mg_batch_framed}, {op: shared memory}) of a mesh on framed tiles."""
+        m, ds, smem = self.mesh, {}, {}
+        for op in (OP_FWD, OP_BWD):
+            ds[op], smem[op] = mg_batch_framed(), ctypes.c_size_t()
+        check(load().mg_batched_framed_desc(m.N, m.L, max(self.B, 1), m.crossing, m.geometry, _lib.cfg_ptr(self.cfg[OP_BWD]),
+                                            self.ws[OP_BWD].data_ptr(), self.ws[OP_BWD].numel(), ctypes.byref(ds[OP_FWD]),
+                                            ctypes.byref(ds[OP_BWD]), ctypes.byref(smem[OP_FWD]),
+                                            ctypes.byref(smem[OP_BWD])), "mg_batched_framed_desc")
+        for op, d in ds.items():
+            d.mesh.B, d.mesh.ldu, d.mesh.n_items = self.B, m.N, self.n_items
+            d.mesh.ldp, d.mesh.n_p = m.N // 2 * m.X_np, m.X_np
+            self._fields(op, d.mesh)
+        return ds, {op: v.value for op, v in smem.items()}
 
     def cost(self) -> int:
         """Padded work of one full item: layers x slots x vector capacity."""
@@ -126,27 +163,30 @@ class BatchedMeshes:
         if len(meshes) != len(batch_sizes):
             raise ValueError("one batch size per mesh")
         self.device = meshes[0].device
-        self.states: List[_MeshState] = [_MeshState(m, b) for m, b in zip(meshes, batch_sizes)]
+        self.states: List[_MeshState] = [_MeshState(m, b, full_warp) for m, b in zip(meshes, batch_sizes)]
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.grid = grid or sms
-        # launch groups: with full_warp (the default) and every mesh nearest-neighbour (MG_BATCH_NN), the M = 8
-        # meshes whose vector fills the warp (G = 32; complex, and real ones in a second group) run in launches
-        # of their own with a compile-time lane group, issued first; everything else runs in one launch of the
-        # three-class kernel on a side stream, whose CTAs take the SMs as the earlier launches' CTAs finish.  Measured on GB300 on 512 uneven meshes
-        # (N 8..256): fwd+bwd 318 against 301 G MZI-apps/s for a single launch, dJ/dp bitwise the same.  Each
+        # launch groups: with full_warp (the default) the meshes on framed tiles in a launch of their own and, with every
+        # mesh nearest-neighbour (MG_BATCH_NN), the other M = 8 meshes whose vector fills the warp (G = 32; real ones) in
+        # another with a compile-time lane group, issued first; everything else runs in one launch of the three-class
+        # kernel on a side stream, whose CTAs take the SMs as the earlier launches' CTAs finish.  Measured on GB300 on 512
+        # uneven meshes (N 8..256) before framed tiles: fwd+bwd 318 against 301 G MZI-apps/s for a single launch.  Each
         # group is sorted longest-first and drained from its own counter.
         self.nn = BATCH_NN if all(st.mesh.geometry == GEO_NN for st in self.states) else 0
+        framed = [i for i, st in enumerate(self.states) if st.framed]
         groups = {}
         for i, st in enumerate(self.states):
             full = full_warp and bool(self.nn) and st.cls in (BCLS_C8, BCLS_R8) and st.G == 32
-            flags = (MG_BATCH_ONLY(st.cls) | MG_BATCH_FULL_WARP) if full else 0
+            flags = (MG_BATCH_ONLY(st.cls) | MG_BATCH_FULL_WARP) if full or st.framed else 0
+            mesh = framed.index(i) if st.framed else i
             for k in range(st.n_items):
                 v0 = k * st.cap
-                groups.setdefault(flags, []).append((st.cost(), i, v0, min(v0 + st.cap, st.B), k))
+                groups.setdefault((flags, st.framed), []).append((st.cost(), mesh, v0, min(v0 + st.cap, st.B), k))
         self.groups = []
         # the full-warp groups first, the largest total work first; the mixed launch (short items) last
-        order = sorted(groups.items(), key=lambda kv: (kv[0] == 0, -sum(t[0] for t in kv[1])))
-        for flags, items in order:
+        order = sorted(groups.items(), key=lambda kv: (kv[0][0] == 0, -sum(t[0] for t in kv[1])))
+        self.group_framed = [key[1] for key, _ in order]
+        for (flags, _), items in order:
             items.sort(key=lambda t: -t[0])               # longest processing time first
             arr = (mg_batch_item * max(len(items), 1))()
             for n, (_, i, v0, v1, k) in enumerate(items):
@@ -160,7 +200,14 @@ class BatchedMeshes:
             for i, st in enumerate(self.states):
                 ds[i] = st.descriptor(op)
             self.desc[op] = _to_device(ds, self.device)
-            self.smem[op] = max(st.info[op].smem for st in self.states)
+            self.smem[op] = max((st.info[op].smem for st in self.states if not st.framed), default=0)
+        self.n_framed, self.fdesc, self.fsmem = len(framed), {}, {}
+        if framed:
+            pairs = [self.states[i].framed_descriptors() for i in framed]
+            for op in (OP_FWD, OP_BWD):
+                fs = (mg_batch_framed * len(framed))(*[ds[op] for ds, _ in pairs])
+                self.fdesc[op] = _to_device(fs, self.device)
+                self.fsmem[op] = max(smem[op] for _, smem in pairs)
         self.head = torch.zeros(max(len(self.groups), 1), dtype=torch.int32, device=self.device)
         self.side = None
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
@@ -208,6 +255,11 @@ class BatchedMeshes:
                 sd.wait_event(fork)
         for g, (flags, n, items) in enumerate(self.groups):
             s_g = stream if g == 0 else self.side[g - 1].cuda_stream
+            if self.group_framed[g]:
+                check(lib.mg_batched_framed(op, self.fdesc[op].data_ptr(), self.n_framed, items.data_ptr(), n,
+                                            self.head[g:].data_ptr(), self.grid, self.fsmem[op], self.status.data_ptr(),
+                                            s_g), "mg_batched_framed")
+                continue
             # all meshes nearest-neighbour: the kernel bodies without strided layers (MG_BATCH_NN)
             check(lib.mg_batched_propagate(op | self.nn | flags, self.desc[op].data_ptr(), len(self.states),
                                            items.data_ptr(), n, self.head[g:].data_ptr(), self.grid, self.smem[op],
@@ -219,6 +271,9 @@ class BatchedMeshes:
                 main.wait_event(join)
         if op == OP_BWD:
             check(lib.mg_batched_reduce(self.desc[op].data_ptr(), len(self.states), stream), "mg_batched_reduce")
+            if self.n_framed:
+                check(lib.mg_batched_framed_reduce(self.fdesc[op].data_ptr(), self.n_framed, stream),
+                      "mg_batched_framed_reduce")
 
     def forward(self):
         """y[i] = U_i x[i] for every mesh, one launch."""

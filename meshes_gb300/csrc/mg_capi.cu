@@ -882,6 +882,38 @@ int mg_build_tiles(int op, int N, int L, int geometry, const int* lens, const in
                      static_cast<cudaStream_t>(stream));
 }
 
+int mg_batched_framed_desc(int N, int L, int B, int crossing, int geometry, const mg_config* cfg, const void* workspace,
+                           size_t wsb, mg_batch_framed* fwd, mg_batch_framed* bwd, size_t* smem_fwd, size_t* smem_bwd) {
+  g_err.clear();
+  if (!cfg || cfg->split != 5 || cfg->M != 8 || cfg->V != 4 || cfg->W != 8 || crossing != CR_MZI)
+    return fail(MG_E_CONFIG, "batched framed meshes are MZI, M=8 V=4 W=8 split=5");
+  if (!fwd || !bwd || !smem_fwd || !smem_bwd) return fail(MG_E_ARG, "NULL output");
+  Plan Pb, Pf;
+  TRY(make_plan(OP_BWD, N, L, B, crossing, geometry, cfg, &Pb));
+  TRY(check_ws(Pb, const_cast<void*>(workspace), wsb));
+  const mg_config cf = {8, 4, 8, 0, 0, 5};
+  TRY(make_plan(OP_FWD, N, L, B, crossing, geometry, &cf, &Pf));
+  TRY(use_bwd_tiles(Pb, &Pf));
+  const unsigned char* ws = static_cast<const unsigned char*>(workspace);
+  for (const Plan* P : {&Pf, &Pb}) {
+    mg_batch_framed d{};
+    d.mesh.N = N; d.mesh.L = L; d.mesh.cls = MG_BCLS_C8; d.mesh.G = P->G;
+    d.mesh.CL = P->CL; d.mesh.S = P->S; d.mesh.layer_bytes = P->lb;
+    d.mesh.tiles = ws + Pb.off_tiles;
+    d.mesh.kinds = reinterpret_cast<const int*>(ws + Pb.off_kinds);
+    d.main = ws + Pb.off_main;
+    d.resc = ws + Pb.off_resc;
+    d.wts = ws + Pb.off_wts;
+    d.dfin = ws + Pb.off_dfin;
+    d.fkinds = reinterpret_cast<const int*>(ws + Pb.off_fkinds);
+    d.count = reinterpret_cast<const int*>(ws + Pb.off_count);
+    d.fcl = P->fcl; d.flb = P->flb; d.refuse = framed_refuse(L);
+    *(P == &Pf ? fwd : bwd) = d;
+    *(P == &Pf ? smem_fwd : smem_bwd) = P->smem;
+  }
+  return MG_OK;
+}
+
 int mg_propagate(int op, int N, int L, int B, int crossing, int geometry, const void* in0, const void* in1, void* out0,
                  void* out1, int ldu, float* dp, int ldp, int accumulate, const mg_config* cfg, void* ws, size_t wsb,
                  void* stream) {
