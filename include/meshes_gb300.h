@@ -276,6 +276,7 @@ typedef struct mg_batch_framed {
   const int* count;
   int fcl, refuse;
   unsigned flb;
+  int V;                 /* mg_batched_small */
 } mg_batch_framed;
 int mg_batched_framed_desc(int N, int L, int B, int crossing, int geometry, const mg_config* cfg, const void* workspace,
                            size_t workspace_bytes, mg_batch_framed* fwd, mg_batch_framed* bwd, size_t* smem_fwd,
@@ -283,6 +284,13 @@ int mg_batched_framed_desc(int N, int L, int B, int crossing, int geometry, cons
 int mg_batched_framed(int op, const mg_batch_framed* meshes, int n_meshes, const mg_batch_item* items, int n_items, int* head,
                       int grid, size_t smem, int* status, void* stream);
 int mg_batched_framed_reduce(const mg_batch_framed* meshes, int n_meshes, void* stream);
+/* Meshes of every class in one launch with V vectors per lane group, of each mesh's own: on framed tiles (mg_config{4 or 8, 4,
+ * 8, .., split 5}: 65 to 256 modes) 1 or 4, back-propagation 2 too; with main NULL on plain ones as for
+ * mg_batched_propagate, V its class's (4; C16 2), forward 1 too.  Items are up to 8 * 32 / G * V vectors.  A vector's
+ * result does not depend on V, the order of the gradients' sums does.  smem as for the 8-warp plans;
+ * mg_batched_framed_reduce sums the partials. */
+int mg_batched_small(int op, const mg_batch_framed* meshes, int n_meshes, const mg_batch_item* items, int n_items, int* head,
+                     int grid, size_t smem, int* status, void* stream);
 
 /* Back-propagation with the L2 loss to a target fused into the kernel: dJ/dy* = 2 (y - target) is
  * formed on load (J = sum |y - target|^2), then as mg_propagate(MG_OP_BWD) with tiles built earlier.
@@ -312,6 +320,9 @@ typedef struct mg_server mg_server;
  * of the meshes' W = 8 plans per op. */
 mg_server* mg_server_create(const mg_server_mesh* meshes, int n_meshes, size_t arena_bytes, int n_streams,
                             int max_per_tick, int grid, size_t smem_fwd, size_t smem_bwd, int device);
+/* Framed tiles of a mesh as well (mg_batched_framed_desc); before the mesh's first request. */
+int mg_server_frame(mg_server* s, int mesh, const mg_batch_framed* fwd, const mg_batch_framed* bwd, size_t smem_fwd,
+                    size_t smem_bwd);
 /* Device bytes a request needs (admission accounting). */
 int mg_server_request_bytes(const mg_server* s, int mesh, int b, int grad, size_t* out);
 /* Queue a request: x (b, N) complex64 (float32 for orth), y (b, N) receives U x; with gy (b, N) = 2 dJ/dy*,

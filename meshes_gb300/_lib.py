@@ -50,7 +50,7 @@ class mg_batch_mesh(Structure):
 
 class mg_batch_framed(Structure):
     _fields_ = [("mesh", mg_batch_mesh), ("main", c_void_p), ("resc", c_void_p), ("wts", c_void_p), ("dfin", c_void_p),
-                ("fkinds", c_void_p), ("count", c_void_p), ("fcl", c_int), ("refuse", c_int), ("flb", c_uint)]
+                ("fkinds", c_void_p), ("count", c_void_p), ("fcl", c_int), ("refuse", c_int), ("flb", c_uint), ("V", c_int)]
 
 
 class mg_server_mesh(Structure):
@@ -139,6 +139,8 @@ _SIGS = {
                                        POINTER(c_size_t)]),
     "mg_batched_framed": (c_int, [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_size_t, c_void_p, c_void_p]),
     "mg_batched_framed_reduce": (c_int, [c_void_p, c_int, c_void_p]),
+    "mg_batched_small": (c_int, [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_size_t, c_void_p, c_void_p]),
+    "mg_server_frame": (c_int, [c_void_p, c_int, POINTER(mg_batch_framed), POINTER(mg_batch_framed), c_size_t, c_size_t]),
 }
 
 _lock = threading.Lock()

@@ -9,15 +9,13 @@
 // longest-first gets longest-processing-time scheduling.
 #include <cuda_runtime.h>
 
-#include "../../include/meshes_gb300.h"
+#include "mg_batched.cuh"
 #include "mg_launch.h"
 
 namespace mg {
 namespace {
 
 constexpr int kBatchWarps = 8;
-
-__device__ __forceinline__ int cls_M(int cls) { return cls == MG_BCLS_C16 ? 16 : 8; }
 
 // NN: every mesh of the launch is nearest-neighbour (layer kinds 0 and odd-shift), so the bodies without
 // the strided and butterfly layers run (fewer registers; a mesh with another kind is refused per item).
@@ -50,22 +48,12 @@ batched_kernel(const mg_batch_mesh* __restrict__ meshes, int n_meshes, const mg_
       continue;
     }
     const int M = cls_M(md.cls);
-    if (md.G < 1 || md.G > 32 || (md.G & (md.G - 1)) || md.G * M < md.N || it.v0 < 0 || it.vend > md.B) {
+    if (!batch_item_ok(md, it, M)) {
       if (threadIdx.x == 0) set_status(status, ST_BAD_WORK);
       continue;
     }
     PropArgs a{};
-    a.N = md.N; a.L = md.L; a.B = md.B; a.ldu = md.ldu;
-    a.G = md.G; a.logG = 31 - __clz(md.G); a.W = kBatchWarps; a.CL = md.CL; a.S = md.S;
-    a.layer_bytes = md.layer_bytes; a.dlayer_bytes = 0;
-    a.tiles = static_cast<const unsigned char*>(md.tiles); a.dtiles = nullptr;
-    a.kinds = md.kinds;
-    a.in0 = md.in0; a.in1 = md.in1; a.out0 = md.out0; a.out1 = md.out1;
-    a.partial = (OP == OP_BWD) ? static_cast<float2*>(md.partial) + (size_t)it.part * md.L * (md.G * M / 2) : nullptr;
-    a.status = status;
-    a.v0 = it.v0; a.vend = it.vend;
-    a.target = nullptr;
-    a.perm = a.pflags = a.perm_last = a.pflag_last = nullptr;   // batched meshes carry no permutations
+    batch_args<OP>(a, md, it, md.G * M / 2, kBatchWarps, status);
     if constexpr (NN) {
       // the nearest-neighbour bodies know layer kinds 0 and odd-shift only: an item whose mesh has another
       // kind is refused (status, no output)
@@ -108,49 +96,11 @@ batched_kernel(const mg_batch_mesh* __restrict__ meshes, int n_meshes, const mg_
   }
 }
 
-// dp[l][q][k] = sum over the mesh's items (in item order) of the partials.  Grid (meshes, kReduceY): the
-// kReduceY CTAs of a mesh stride over its slot positions, one position per thread at a time, consecutive
-// threads on consecutive positions (coalesced); each thread keeps 8 item loads in flight and adds them in item
-// order, so the sums are those of a plain sequential loop.  (One CTA per mesh, one load in flight per thread,
-// took 3.85 ms on the 512-mesh benchmark - 23% of its forward + backward step.)
 constexpr int kReduceY = 64;
 __global__ void batched_reduce_kernel(const mg_batch_mesh* __restrict__ meshes) {
   const mg_batch_mesh md = meshes[blockIdx.x];
   if (!md.dp || !md.partial || md.n_items <= 0) return;
-  const int M = cls_M(md.cls), G = md.G, np2 = G * M / 2, L = md.L, N = md.N;
-  const int* geo = md.kinds + L;
-  const float2* part = static_cast<const float2*>(md.partial);
-  const size_t stride = (size_t)L * np2;
-  const int n = md.n_items;
-  for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < L * np2; idx += gridDim.y * blockDim.x) {
-    const int l = idx / np2, pos = idx - l * np2;
-    const int q = pos_slot(pos, M, G);
-    if (q >= N / 2) continue;
-    const int sh = geo[2 * l], ln = geo[2 * l + 1];
-    float sx = 0.f, sy = 0.f;
-    if (q >= sh / 2 && q < sh / 2 + ln) {
-      const float2* p = part + (size_t)l * np2 + pos;
-      int k = 0;
-      for (; k + 8 <= n; k += 8) {
-        float2 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = p[(size_t)(k + i) * stride];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          sx += v[i].x;
-          sy += v[i].y;
-        }
-      }
-      for (; k < n; ++k) {
-        const float2 v = p[(size_t)k * stride];
-        sx += v.x;
-        sy += v.y;
-      }
-    }
-    float* o = md.dp + (size_t)l * md.ldp + (size_t)q * md.n_p;
-    o[0] = sx;
-    if (md.n_p > 1) o[1] = sy;
-  }
+  batch_reduce(md, blockIdx.y, gridDim.y);
 }
 
 }  // namespace

@@ -3,43 +3,13 @@
 //
 // What bounds it: as the one-mesh kernel, the FMA pipe's register operands.  An item is 32 vectors (8 warps of 4), what a
 // full wave of the one-mesh kernel gives a CTA; items are drained longest first.
-#include "../../include/meshes_gb300.h"
-#include "mg_framed.cuh"
-#include "mg_launch.h"
+#include "mg_batched_framed.cuh"
+#include "mg_batched_small.h"
 
 namespace mg {
 namespace {
 
 constexpr int kBFWarps = 8, kBFM = 8, kBFV = 4;
-
-// the item's launch arguments; false: a work item outside its mesh or its batch, or a stage that shared memory cannot hold
-template <int OP>
-__device__ bool framed_item(const mg_batch_framed* __restrict__ meshes, int n_meshes, const mg_batch_item& it, int* status,
-                            FramedArgs& a) {
-  if (it.mesh < 0 || it.mesh >= n_meshes) return false;
-  const mg_batch_framed f = meshes[it.mesh];
-  const mg_batch_mesh& md = f.mesh;
-  if (md.G != 32 || md.N < 1 || md.N > 32 * kBFM || it.v0 < 0 || it.vend > md.B || f.fcl < 1) return false;
-  unsigned dynamic;
-  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynamic));
-  if (framed_smem_bytes(OP, f.flb, 16 * kBFM, kBFWarps, f.fcl, md.L) > dynamic) return false;
-  a.N = md.N; a.L = md.L; a.B = md.B; a.ldu = md.ldu;
-  a.G = 32; a.logG = 5; a.W = kBFWarps; a.CL = md.CL; a.S = md.S;
-  a.layer_bytes = md.layer_bytes; a.dlayer_bytes = 0;
-  a.tiles = static_cast<const unsigned char*>(md.tiles); a.dtiles = nullptr;
-  a.kinds = md.kinds;
-  a.in0 = md.in0; a.in1 = md.in1; a.out0 = md.out0; a.out1 = md.out1;
-  a.partial = OP == OP_BWD ? static_cast<float2*>(md.partial) + (size_t)it.part * md.L * (16 * kBFM) : nullptr;
-  a.status = status;
-  a.v0 = it.v0; a.vend = it.vend;
-  a.main = static_cast<const float4*>(f.main);
-  a.resc = static_cast<const float4*>(f.resc);
-  a.dfin = static_cast<const float2*>(f.dfin);
-  a.fkinds = f.fkinds;
-  a.count = f.count;
-  a.fcl = f.fcl; a.flb = f.flb; a.refuse = f.refuse;
-  return true;
-}
 
 template <int OP>
 __global__ void __launch_bounds__(kBFWarps * 32, 1)
@@ -55,8 +25,9 @@ batched_framed_kernel(const mg_batch_framed* __restrict__ meshes, int n_meshes, 
       const int i = atomicAdd(head, 1);
       next = i >= n_items ? -1 : 0;
       if (i < n_items) {
+        const mg_batch_item it = items[i];
         args = FramedArgs{};
-        if (framed_item<OP>(meshes, n_meshes, items[i], status, args)) next = 1;
+        if (it.mesh >= 0 && it.mesh < n_meshes && framed_item<OP>(meshes[it.mesh], it, kBFM, kBFWarps, status, args)) next = 1;
         else set_status(status, ST_BAD_WORK);
       }
     }
@@ -66,14 +37,18 @@ batched_framed_kernel(const mg_batch_framed* __restrict__ meshes, int n_meshes, 
   }
 }
 
-// grid (columns, meshes): a mesh's CTAs stride over the blocks of its columns
+// grid (columns, meshes): a mesh's CTAs stride over the blocks of its columns; meshes on plain tiles have no main
 __global__ void __launch_bounds__(256) batched_framed_reduce_kernel(const mg_batch_framed* __restrict__ meshes) {
   __shared__ float2 acc[kFReduceRows][kFReduceCols];
   const mg_batch_framed f = meshes[blockIdx.y];
   const mg_batch_mesh& md = f.mesh;
   if (!md.dp || !md.partial || md.n_items <= 0) return;
-  const int np2 = 16 * kBFM;
-  const FramedReduceArgs a{static_cast<const float2*>(md.partial), md.n_items, md.L, np2, kBFM, 32, md.N, md.dp, md.ldp, 0,
+  if (!f.main) {
+    batch_reduce(md, blockIdx.x, gridDim.x);
+    return;
+  }
+  const int M = batch_framed_M(md.N), np2 = 16 * M;
+  const FramedReduceArgs a{static_cast<const float2*>(md.partial), md.n_items, md.L, np2, M, 32, md.N, md.dp, md.ldp, 0,
                            md.kinds + md.L, static_cast<const float2*>(f.wts), f.count, f.refuse};
   for (int blk = blockIdx.x; blk * kFReduceCols < md.L * np2; blk += gridDim.x) {
     framed_reduce_block(a, blk, acc);
@@ -111,6 +86,27 @@ extern "C" int mg_batched_framed(int op, const mg_batch_framed* meshes, int n_me
   const cudaError_t e = op == MG_OP_FWD ? launch<OP_FWD>(meshes, n_meshes, items, n_items, head, grid, smem, status, st)
                                         : launch<OP_BWD>(meshes, n_meshes, items, n_items, head, grid, smem, status, st);
   return e == cudaSuccess ? MG_OK : set_last_error(MG_E_CUDA, "batched_framed_kernel: %s", cudaGetErrorString(e));
+}
+
+extern "C" int mg_batched_small(int op, const mg_batch_framed* meshes, int n_meshes, const mg_batch_item* items, int n_items,
+                                int* head, int grid, size_t smem, int* status, void* stream) {
+  if (op != MG_OP_FWD && op != MG_OP_BWD) return set_last_error(MG_E_ARG, "batched op must be fwd or bwd");
+  if (!meshes || n_meshes < 0 || (!items && n_items > 0) || !head || grid < 1)
+    return set_last_error(MG_E_ARG, "batched launch: bad arguments");
+  if (n_items == 0) return MG_OK;
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (smem + 1024 > (size_t)optin) return set_last_error(MG_E_CONFIG, "batched smem %zu above %d", smem, optin);
+  (void)cudaGetLastError();   // start from a clean error state: launch errors below are this call's
+  const BatchedSmall b{meshes, n_meshes, items, n_items, head, status};
+  LaunchCfg lc;
+  lc.grid = dim3(grid);
+  lc.block = dim3(32 * kSmallWarps);
+  lc.smem = smem;
+  lc.stream = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = op == MG_OP_FWD ? batched_small_fwd(lc, b) : batched_small_bwd(lc, b);
+  return e == cudaSuccess ? MG_OK : set_last_error(MG_E_CUDA, "batched_small_kernel: %s", cudaGetErrorString(e));
 }
 
 extern "C" int mg_batched_framed_reduce(const mg_batch_framed* meshes, int n_meshes, void* stream) {

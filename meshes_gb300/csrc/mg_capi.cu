@@ -885,13 +885,13 @@ int mg_build_tiles(int op, int N, int L, int geometry, const int* lens, const in
 int mg_batched_framed_desc(int N, int L, int B, int crossing, int geometry, const mg_config* cfg, const void* workspace,
                            size_t wsb, mg_batch_framed* fwd, mg_batch_framed* bwd, size_t* smem_fwd, size_t* smem_bwd) {
   g_err.clear();
-  if (!cfg || cfg->split != 5 || cfg->M != 8 || cfg->V != 4 || cfg->W != 8 || crossing != CR_MZI)
-    return fail(MG_E_CONFIG, "batched framed meshes are MZI, M=8 V=4 W=8 split=5");
+  if (!cfg || cfg->split != 5 || (cfg->M != 4 && cfg->M != 8) || cfg->V != 4 || cfg->W != 8 || crossing != CR_MZI)
+    return fail(MG_E_CONFIG, "batched framed meshes are MZI, M=4 or 8, V=4 W=8 split=5");
   if (!fwd || !bwd || !smem_fwd || !smem_bwd) return fail(MG_E_ARG, "NULL output");
   Plan Pb, Pf;
   TRY(make_plan(OP_BWD, N, L, B, crossing, geometry, cfg, &Pb));
   TRY(check_ws(Pb, const_cast<void*>(workspace), wsb));
-  const mg_config cf = {8, 4, 8, 0, 0, 5};
+  const mg_config cf = {cfg->M, 4, 8, 0, 0, 5};
   TRY(make_plan(OP_FWD, N, L, B, crossing, geometry, &cf, &Pf));
   TRY(use_bwd_tiles(Pb, &Pf));
   const unsigned char* ws = static_cast<const unsigned char*>(workspace);

@@ -95,6 +95,7 @@ struct Arena {
 
 struct mg_server {
   std::vector<mg_server_mesh> meshes;
+  std::vector<mg_batch_framed> framed_fwd, framed_bwd;   // main NULL: the mesh has plain tiles only
   int device = 0, grid = 0, max_per_tick = 512;
   size_t smem_fwd = 0, smem_bwd = 0;
   unsigned char* arena_dev = nullptr;
@@ -228,25 +229,63 @@ struct mg_server {
     for (size_t i = 0; i < K; ++i)
       if (reqs[i].gy) gidx.push_back(i);
     const size_t KG = gidx.size();
-    std::vector<size_t> fe(K), nit(K), np2(K);
+    // Vectors per lane group, per request and op.  An item goes through all layers of its mesh, at a rate that falls with
+    // its vectors (on GB300, 256 modes forward: 99 us for an item of 32 vectors on plain tiles, 42 us for one of 8 on
+    // framed ones), so forward takes 1 while the tick's items fill the SMs no more than once.  A vector's result does
+    // not depend on that; the order of the gradients' sums does, and a request's results are the same whatever else its
+    // tick holds: back-propagation goes by the request alone, by the fewest vectors that leave it as many items (and
+    // partials) as the mesh's own capacity does.
+    struct Shape {
+      bool framed;
+      int V, cap;
+      size_t n, np2;   // items, slots per layer
+    };
+    auto own_V = [](const mg_server_mesh& m) { return m.cls == MG_BCLS_C16 ? 2 : 4; };
+    auto shape = [&](const Req& r, bool framed, int V) {
+      const mg_server_mesh& m = meshes[r.mesh];
+      const int cap = framed ? 8 * V : V == own_V(m) ? m.cap : std::max(1, m.cap / own_V(m) * V);
+      const size_t np2 = framed ? (m.N > 128 ? 128 : 64) : (size_t)m.G * (m.cls == MG_BCLS_C16 ? 16 : 8) / 2;
+      return Shape{framed, V, cap, (size_t)((r.b + cap - 1) / cap), np2};
+    };
+    bool spread = true;
+    auto forward = [&](const Req& r) {
+      const bool framed = framed_fwd[r.mesh].main != nullptr;
+      const int V = framed ? 4 : own_V(meshes[r.mesh]);
+      const Shape one = shape(r, framed, 1);
+      return spread || one.n == 1 ? one : shape(r, framed, V);
+    };
+    auto backward = [&](const Req& r) {
+      const mg_server_mesh& m = meshes[r.mesh];
+      const Shape own = shape(r, false, own_V(m));
+      if (framed_bwd[r.mesh].main)
+        for (int V : {1, 2, 4}) {
+          const Shape f = shape(r, true, V);
+          if (f.n <= own.n && f.np2 <= own.np2) return f;
+        }
+      return own;
+    };
+    size_t n_one = 0;
+    for (const Req& r : reqs) n_one += forward(r).n;
+    spread = n_one <= (size_t)grid;
+    std::vector<size_t> fe(K);
     size_t n_if = 0, n_ib = 0, n_x = 0, n_gy = 0, n_dp = 0, n_pt = 0;
     for (size_t i = 0; i < K; ++i) {
-      const mg_server_mesh& m = meshes[reqs[i].mesh];
-      fe[i] = al((size_t)reqs[i].b * m.N * (m.cls == MG_BCLS_R8 ? 4 : 8));
-      nit[i] = (size_t)(reqs[i].b + m.cap - 1) / m.cap;
-      np2[i] = (size_t)m.G * (m.cls == MG_BCLS_C16 ? 16 : 8) / 2;
-      n_if += nit[i];
+      const Req& r = reqs[i];
+      const mg_server_mesh& m = meshes[r.mesh];
+      fe[i] = al((size_t)r.b * m.N * (m.cls == MG_BCLS_R8 ? 4 : 8));
+      n_if += forward(r).n;
       n_x += fe[i];
-      if (reqs[i].gy) {
-        n_ib += nit[i];
+      if (r.gy) {
+        const Shape o = backward(r);
+        n_ib += o.n;
         n_gy += fe[i];
         n_dp += al((size_t)m.L * (m.N / 2) * m.n_p * 4);
-        n_pt += al(nit[i] * m.L * np2[i] * 8);
+        n_pt += al(o.n * m.L * o.np2 * 8);
       }
     }
     const size_t off_df = 0;
-    const size_t off_db = off_df + al(K * sizeof(mg_batch_mesh));
-    const size_t off_if = off_db + al(std::max<size_t>(KG, 1) * sizeof(mg_batch_mesh));
+    const size_t off_db = off_df + al(K * sizeof(mg_batch_framed));
+    const size_t off_if = off_db + al(std::max<size_t>(KG, 1) * sizeof(mg_batch_framed));
     const size_t off_ib = off_if + al(std::max<size_t>(n_if, 1) * sizeof(mg_batch_item));
     const size_t off_head = off_ib + al(std::max<size_t>(n_ib, 1) * sizeof(mg_batch_item));
     const size_t off_x = off_head + kAlign;
@@ -266,7 +305,7 @@ struct mg_server {
       return;
     }
     Tick t;
-    t.host = pinned_get(total, &t.host_cap);
+    t.host = pinned_get(out_end, &t.host_cap);   // (the partials stay on the device)
     if (!t.host) {
       arena.release(dev_off, total);
       fail_all("cudaHostAlloc failed");
@@ -274,8 +313,8 @@ struct mg_server {
     }
     unsigned char* h = t.host;
     unsigned char* base = arena_dev + dev_off;
-    auto* df = reinterpret_cast<mg_batch_mesh*>(h + off_df);
-    auto* db = reinterpret_cast<mg_batch_mesh*>(h + off_db);
+    auto* df = reinterpret_cast<mg_batch_framed*>(h + off_df);
+    auto* db = reinterpret_cast<mg_batch_framed*>(h + off_db);
     std::memset(h, 0, off_x);                          // descriptors, items, queue heads
     struct It {
       size_t cost;
@@ -291,32 +330,44 @@ struct mg_server {
       const mg_server_mesh& m = meshes[r.mesh];
       const size_t fb = (size_t)r.b * m.N * (m.cls == MG_BCLS_R8 ? 4 : 8);
       std::memcpy(h + off_x + ox, r.x, fb);
-      mg_batch_mesh& d = df[i];
-      d.N = m.N; d.L = m.L; d.B = r.b; d.ldu = m.N;
-      d.cls = m.cls; d.G = m.G; d.CL = m.fwd_CL; d.S = m.fwd_S;
-      d.layer_bytes = m.fwd_layer_bytes; d.n_items = 0; d.ldp = 0; d.n_p = m.n_p;
-      d.tiles = m.fwd_tiles; d.kinds = m.fwd_kinds;
-      d.in0 = base + off_x + ox; d.out0 = base + off_y + ox;
+      auto describe = [&](const Shape& o, const mg_batch_framed& f, const void* tiles, const int* kinds, int CL, int S,
+                          unsigned layer_bytes) {
+        mg_batch_framed d{};
+        if (o.framed) {
+          d = f;
+        } else {
+          d.mesh.cls = m.cls; d.mesh.G = m.G; d.mesh.CL = CL; d.mesh.S = S;
+          d.mesh.layer_bytes = layer_bytes;
+          d.mesh.tiles = tiles; d.mesh.kinds = kinds;
+        }
+        d.V = o.V;
+        d.mesh.N = m.N; d.mesh.L = m.L; d.mesh.B = r.b; d.mesh.ldu = m.N; d.mesh.n_p = m.n_p;
+        return d;
+      };
+      auto add = [&](std::vector<It>& to, const Shape& o, size_t at) {
+        const size_t cost = (size_t)m.L * o.np2 * o.cap;
+        for (size_t k = 0; k < o.n; ++k)
+          to.push_back({cost, (int)at, (int)(k * o.cap), (int)std::min<size_t>((k + 1) * o.cap, r.b), (int)k});
+      };
+      const Shape of = forward(r);
+      df[i] = describe(of, framed_fwd[r.mesh], m.fwd_tiles, m.fwd_kinds, m.fwd_CL, m.fwd_S, m.fwd_layer_bytes);
+      df[i].mesh.in0 = base + off_x + ox; df[i].mesh.out0 = base + off_y + ox;
       t.o_y[i] = off_y + ox;
-      const size_t cost = (size_t)m.L * np2[i] * m.cap;
-      for (size_t k = 0; k < nit[i]; ++k)
-        itf.push_back({cost, (int)i, (int)(k * m.cap), (int)std::min<size_t>((k + 1) * m.cap, r.b), (int)k});
+      add(itf, of, i);
       if (r.gy) {
         std::memcpy(h + off_gy + og, r.gy, fb);
-        mg_batch_mesh& e = db[j];
-        e = d;
-        e.CL = m.bwd_CL; e.S = m.bwd_S; e.layer_bytes = m.bwd_layer_bytes;
-        e.tiles = m.bwd_tiles; e.kinds = m.bwd_kinds;
-        e.n_items = (int)nit[i]; e.ldp = m.N / 2 * m.n_p;
+        const Shape ob = backward(r);
+        db[j] = describe(ob, framed_bwd[r.mesh], m.bwd_tiles, m.bwd_kinds, m.bwd_CL, m.bwd_S, m.bwd_layer_bytes);
+        mg_batch_mesh& e = db[j].mesh;
+        e.n_items = (int)ob.n; e.ldp = m.N / 2 * m.n_p;
         e.in0 = base + off_y + ox; e.in1 = base + off_gy + og; e.out0 = nullptr; e.out1 = base + off_gx + og;
         e.dp = reinterpret_cast<float*>(base + off_dp + odp); e.partial = base + off_pt + opt;
         t.o_gx.push_back(off_gx + og);
         t.o_dp.push_back(off_dp + odp);
-        for (size_t k = 0; k < nit[i]; ++k)
-          itb.push_back({cost, (int)j, (int)(k * m.cap), (int)std::min<size_t>((k + 1) * m.cap, r.b), (int)k});
+        add(itb, ob, j);
         og += fe[i];
         odp += al((size_t)m.L * (m.N / 2) * m.n_p * 4);
-        opt += al(nit[i] * m.L * np2[i] * 8);
+        opt += al(ob.n * m.L * ob.np2 * 8);
         ++j;
       }
       ox += fe[i];
@@ -334,16 +385,15 @@ struct mg_server {
     cudaError_t e = cudaMemcpyAsync(base, h, in_bytes, cudaMemcpyHostToDevice, st);
     int head_rc = MG_OK;
     int* head = reinterpret_cast<int*>(base + off_head);
+    const auto* dfd = reinterpret_cast<const mg_batch_framed*>(base + off_df);
+    const auto* dbd = reinterpret_cast<const mg_batch_framed*>(base + off_db);
     if (e == cudaSuccess)
-      head_rc = mg_batched_propagate(MG_OP_FWD, reinterpret_cast<const mg_batch_mesh*>(base + off_df), (int)K,
-                                     reinterpret_cast<const mg_batch_item*>(base + off_if), (int)n_if, head, grid,
-                                     smem_fwd, status, st);
+      head_rc = mg_batched_small(MG_OP_FWD, dfd, (int)K, reinterpret_cast<const mg_batch_item*>(base + off_if), (int)n_if, head,
+                                 (int)std::min<size_t>(grid, n_if), smem_fwd, status, st);
     if (e == cudaSuccess && head_rc == MG_OK && KG) {
-      head_rc = mg_batched_propagate(MG_OP_BWD, reinterpret_cast<const mg_batch_mesh*>(base + off_db), (int)KG,
-                                     reinterpret_cast<const mg_batch_item*>(base + off_ib), (int)n_ib, head + 1, grid,
-                                     smem_bwd, status, st);
-      if (head_rc == MG_OK)
-        head_rc = mg_batched_reduce(reinterpret_cast<const mg_batch_mesh*>(base + off_db), (int)KG, st);
+      head_rc = mg_batched_small(MG_OP_BWD, dbd, (int)KG, reinterpret_cast<const mg_batch_item*>(base + off_ib), (int)n_ib,
+                                 head + 1, (int)std::min<size_t>(grid, n_ib), smem_bwd, status, st);
+      if (head_rc == MG_OK) head_rc = mg_batched_framed_reduce(dbd, (int)KG, st);
     }
     if (e == cudaSuccess && head_rc == MG_OK)
       e = cudaMemcpyAsync(h + off_y, base + off_y, out_end - off_y, cudaMemcpyDeviceToHost, st);
@@ -397,6 +447,8 @@ mg_server* mg_server_create(const mg_server_mesh* meshes, int n_meshes, size_t a
   }
   auto* s = new mg_server();
   s->meshes.assign(meshes, meshes + n_meshes);
+  s->framed_fwd.assign(n_meshes, mg_batch_framed{});
+  s->framed_bwd.assign(n_meshes, mg_batch_framed{});
   s->device = device;
   s->grid = grid;
   s->max_per_tick = max_per_tick;
@@ -422,6 +474,18 @@ mg_server* mg_server_create(const mg_server_mesh* meshes, int n_meshes, size_t a
   s->arena.init(arena_bytes);
   s->worker = std::thread([s] { s->loop(); });
   return s;
+}
+
+int mg_server_frame(mg_server* s, int mesh, const mg_batch_framed* fwd, const mg_batch_framed* bwd, size_t smem_fwd,
+                    size_t smem_bwd) {
+  if (!s || mesh < 0 || mesh >= (int)s->meshes.size() || !fwd || !bwd)
+    return mg::set_last_error(MG_E_ARG, "mg_server_frame: bad arguments");
+  std::lock_guard<std::mutex> lk(s->qmu);   // the scheduler reads them for requests it takes from the queue
+  s->framed_fwd[mesh] = *fwd;
+  s->framed_bwd[mesh] = *bwd;
+  s->smem_fwd = std::max(s->smem_fwd, smem_fwd);
+  s->smem_bwd = std::max(s->smem_bwd, smem_bwd);
+  return MG_OK;
 }
 
 int mg_server_request_bytes(const mg_server* s, int mesh, int b, int grad, size_t* out) {

@@ -30,8 +30,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import OP_BWD, OP_FWD, check, load, mg_server_mesh
-from .batched import WARPS, _CLS_MV, kernel_class, plan
+from ._lib import GEO_NN, OP_BWD, OP_FWD, check, load, mg_batch_framed, mg_server_mesh
+from .batched import BCLS_C8, WARPS, _CLS_MV, kernel_class, plan
 from .mesh import MeshNetworkGPU
 
 
@@ -51,6 +51,7 @@ class _Resident:
     info: dict
     ws: dict
     n_mzi: int
+    framed: Optional[tuple] = None   # (configuration, workspace) of framed tiles
 
 
 class MeshServer:
@@ -96,7 +97,38 @@ class MeshServer:
                                           ws[op].numel(), st), "mg_build_tiles")
         G = info[OP_FWD].G
         n_mzi = sum(m.lens_h) if m.strides is None else m.L * (m.N // 2)
-        return _Resident(m, cls, M, V, G, WARPS * (32 // G) * V, G * M // 2, info, ws, n_mzi)
+        return _Resident(m, cls, M, V, G, WARPS * (32 // G) * V, G * M // 2, info, ws, n_mzi, self._frame(m, cls, geo))
+
+    def _frame(self, m: MeshNetworkGPU, cls: int, geo):
+        """The mesh on framed tiles too (mg_server_frame): (configuration, workspace), or None."""
+        if cls != BCLS_C8 or m.geometry != GEO_NN or m.N <= 64:
+            return None
+        cfg = _lib.config(8 if m.N > 128 else 4, 4, WARPS, 0, 0, 5)
+        try:
+            for op in (OP_FWD, OP_BWD):
+                info = plan(op, m.N, m.L, 1, m.crossing, m.geometry, cfg)
+        except _lib.MeshLibraryError:                     # no framed tiles for it
+            return None
+        ws = torch.empty(info.total, dtype=torch.uint8, device=m.device)
+        st = torch.cuda.current_stream(m.device).cuda_stream
+        s = m.p_splitter
+        check(self.lib.mg_workspace_init(ws.data_ptr(), ws.numel(), st), "mg_workspace_init")
+        check(self.lib.mg_build_tiles(OP_BWD, m.N, m.L, m.geometry, *geo, m.crossing, m.p_phase.data_ptr(),
+                                      m.N // 2 * m.X_np, s.data_ptr() if s.numel() else None, m.N // 2 * m.X_ns, None, None,
+                                      None, 1, _lib.cfg_ptr(cfg), ws.data_ptr(), ws.numel(), st), "mg_build_tiles")
+        return cfg, ws
+
+    def _describe_framed(self, handle):
+        for i, r in enumerate(self.res):
+            if r.framed is None:
+                continue
+            cfg, ws = r.framed
+            m, ds = r.mesh, [mg_batch_framed(), mg_batch_framed()]
+            smem = [ctypes.c_size_t(), ctypes.c_size_t()]
+            check(self.lib.mg_batched_framed_desc(m.N, m.L, 1, m.crossing, m.geometry, _lib.cfg_ptr(cfg), ws.data_ptr(),
+                                                  ws.numel(), *map(ctypes.byref, ds), *map(ctypes.byref, smem)),
+                  "mg_batched_framed_desc")
+            check(self.lib.mg_server_frame(handle, i, *map(ctypes.byref, ds), *[v.value for v in smem]), "mg_server_frame")
 
     def _descriptors(self):
         arr = (mg_server_mesh * len(self.res))()
@@ -119,6 +151,11 @@ class MeshServer:
                                       self.device.index or 0)
         if not h:
             raise ServerError(_lib.last_error())
+        try:
+            self._describe_framed(h)
+        except Exception:
+            self.lib.mg_server_destroy(h, 0)
+            raise
         self.handle = h
         self.waiter = threading.Thread(target=self._wait_loop, args=(h,), name="mesh-server-completions",
                                        daemon=True)
