@@ -52,9 +52,6 @@ __host__ __device__ inline int crossing_np(int c) { return c == CR_ORTH ? 1 : 2;
 __host__ __device__ inline int crossing_ns(int c) { return c == CR_MZI ? 2 : (c == CR_SYM ? 1 : 0); }
 
 // csb (MZI crossings): receives (cos, sin)(pi/4 + beta) of an active slot
-// QUAD: the four lanes of a quad compute the same slot together (mzi_T_ff_quad); only for MZI crossings
-// without derivative tiles, which the host guarantees when it launches the quad form.
-template <bool QUAD = false>
 __device__ __forceinline__ void slot_T(const CoefArgs& a, int l, int q, bool active, C2x2& T, C2x2& D0, C2x2& D1,
                                        float2* csb, Tff& F) {
   if (!active) {
@@ -90,7 +87,7 @@ __device__ __forceinline__ void slot_T(const CoefArgs& a, int l, int q, bool act
     // tiles, or angles beyond the float-float range, the double-precision form
     const float al = ss ? ss[0] : 0.f, be = ss ? ss[1] : 0.f;
     if (need_d ||
-        !(QUAD ? mzi_T_ff_quad(pp[0], pp[1], al, be, ss == nullptr, &F, csb) : mzi_T_ff(pp[0], pp[1], al, be, &F, csb))) {
+        !mzi_T_ff(pp[0], pp[1], al, be, &F, csb)) {
       mzi_T(pp[0], pp[1], al, be, &T, need_d ? &D0 : nullptr, need_d ? &D1 : nullptr, csb);
       tff_from(T, &F);
     } else {
@@ -130,68 +127,113 @@ __device__ __forceinline__ int layer_kind(const CoefArgs& a, int l, int q, bool*
   return (2 * st <= a.M) ? (ok ? e : 0) : KIND_XL + e;
 }
 
-// The frame pass's inputs of slot q (layer kinds 0 and odd-shift): in the quad form lane k of the quad writes entry k.
-template <bool QUAD>
-__device__ __forceinline__ void frame_inputs(const CoefArgs& a, int l, int q, int t, int sh, const Tff& F, float2 cs) {
-  const int modes = a.G * a.M, m0 = sh + 2 * q;
-  const size_t o = (size_t)l * modes;
-  // the framed gradient divides by cos(pi/4 + beta): NaN marks a slot that all but lacks it
-  const bool flat = a.tcs && !(fabsf(cs.x) >= 0x1p-6f * fabsf(cs.y));
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (QUAD && (t & 3) != k) continue;
-    ffz z = F.t[k];
-    const int m = m0 + (k >> 1);             // row of the entry
-    if (m >= modes) continue;                // (the last odd-shift slot has no second mode)
-    if (k == 0 || k == 3) {
-      float w = z.x.h * z.x.h + z.y.h * z.y.h;
-      if (w < 0x1p-60f) {                    // a diagonal entry below 2^-30 counts as 2^-30
-        z = {ff{0x1p-30f, 0.f}, ff{0.f, 0.f}};
-        w = 0x1p-60f;
-      }
-      a.tdiag[o + m] = make_float4(z.x.h, z.x.l, z.y.h, z.y.l);
-      a.tmag[o + m] = flat ? __int_as_float(0x7fc00000) : w;
-    } else {
-      a.toff[o + m] = make_float4(z.x.h, z.x.l, z.y.h, z.y.l);
+// The frame pass's input for entry k of slot q (layer kinds 0 and odd-shift)
+__device__ __forceinline__ void frame_entry(const CoefArgs& a, int l, int q, int k, int sh, ffz z, float2 cs) {
+  const int modes = a.G * a.M, m = sh + 2 * q + (k >> 1);   // row of the entry
+  if (m >= modes) return;                                   // (the last odd-shift slot has no second mode)
+  const size_t o = (size_t)l * modes + m;
+  if (k == 0 || k == 3) {
+    // the framed gradient divides by cos(pi/4 + beta): NaN marks a slot that all but lacks it
+    const bool flat = a.tcs && !(fabsf(cs.x) >= 0x1p-6f * fabsf(cs.y));
+    float w = z.x.h * z.x.h + z.y.h * z.y.h;
+    if (w < 0x1p-60f) {                    // a diagonal entry below 2^-30 counts as 2^-30
+      z = {ff{0x1p-30f, 0.f}, ff{0.f, 0.f}};
+      w = 0x1p-60f;
     }
+    a.tdiag[o] = make_float4(z.x.h, z.x.l, z.y.h, z.y.l);
+    a.tmag[o] = flat ? __int_as_float(0x7fc00000) : w;
+  } else {
+    a.toff[o] = make_float4(z.x.h, z.x.l, z.y.h, z.y.l);
   }
+}
+// and what a slot has once
+__device__ __forceinline__ void frame_slot(const CoefArgs& a, int l, int q, int t, int sh, float2 cs) {
+  const int modes = a.G * a.M;
   if (t == 0) *a.fcount = 0;
-  if (QUAD ? (t & 3) == 0 : true) {
-    if (a.tcs) a.tcs[(size_t)l * (modes / 2) + q] = cs;
-    if (sh && q == 0) {                      // mode 0 lies in no slot
-      a.tdiag[o] = make_float4(1.f, 0.f, 0.f, 0.f);
-      a.toff[o] = make_float4(0.f, 0.f, 0.f, 0.f);
-      a.tmag[o] = 1.f;
-    }
+  if (a.tcs) a.tcs[(size_t)l * (modes / 2) + q] = cs;
+  if (sh && q == 0) {                      // mode 0 lies in no slot
+    const size_t o = (size_t)l * modes;
+    a.tdiag[o] = make_float4(1.f, 0.f, 0.f, 0.f);
+    a.toff[o] = make_float4(0.f, 0.f, 0.f, 0.f);
+    a.tmag[o] = 1.f;
   }
 }
 
-// Thread t of the coefficient pass: one thread per slot, or (QUAD) one quad of lanes per slot - a quad shares its
-// slot, so quads leave at the bounds check whole, and its first lane writes.
-template <bool QUAD, bool FRAME>
-__device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
-  const int np2 = a.G * a.M / 2;
-  const int idx = QUAD ? (t >> 2) : t;
-  const bool writer = !QUAD || (t & 3) == 0;
+// The layer's kind and its active range (shift, len), once per layer
+__device__ __forceinline__ void write_layer(const CoefArgs& a, int l, int kind) {
+  a.kinds[l] = kind;
+  int sh = 0, ln = 0;
+  if (a.geometry == GEO_NN) {
+    sh = __ldg(a.shifts + l);
+    ln = __ldg(a.lens + l);
+    if (sh < 0 || ln < 0 || sh + 2 * ln > a.N) sh = ln = 0;
+  } else {
+    bool any = false;
+    layer_kind(a, l, 0, &any);
+    ln = any ? a.N / 2 : 0;
+  }
+  a.kinds[a.L + 2 * l] = sh;
+  a.kinds[a.L + 2 * l + 1] = ln;
+}
+
+// Lane t & 3 of the quad of lanes that does slot t / 4: MZI crossings without derivative tiles.  Quads leave at the bounds
+// check whole; lane k computes and writes entry k.
+template <bool FRAME>
+__device__ __forceinline__ void coef_quad(const CoefArgs& a, int t) {
+  const int np2 = a.G * a.M / 2, idx = t >> 2, k = t & 3;
   if (idx >= a.L * np2) return;
   const int l = idx / np2, q = idx - l * np2;
   bool active = false;
   const int kind = layer_kind(a, l, q, &active);
-  if (q == 0 && writer) {
-    a.kinds[l] = kind;
-    int sh = 0, ln = 0;
-    if (a.geometry == GEO_NN) {
-      sh = __ldg(a.shifts + l);
-      ln = __ldg(a.lens + l);
-      if (sh < 0 || ln < 0 || sh + 2 * ln > a.N) sh = ln = 0;
-    } else {
-      bool any = false;
-      layer_kind(a, l, 0, &any);
-      ln = any ? a.N / 2 : 0;
+  if (q == 0 && k == 0) write_layer(a, l, kind);
+  const bool bwd = a.op == OP_BWD;   // (direct gradients)
+  float2 cs = make_float2(0.f, 0.f);   // (cos, sin)(pi/4 + beta) for the direct gradient; 0 if inactive
+  ffz z = {ff{k == 0 || k == 3 ? 1.f : 0.f, 0.f}, ff{0.f, 0.f}};
+  float2 v = make_float2(z.x.h, 0.f);
+  if (active) {
+    const float* pp = a.p + (size_t)l * a.ldp + 2 * (size_t)q;
+    const float* ss = a.s ? a.s + (size_t)l * a.lds + 2 * (size_t)q : nullptr;
+    const float al = ss ? ss[0] : 0.f, be = ss ? ss[1] : 0.f;
+    if (mzi_T_ff_quad(pp[0], pp[1], al, be, ss == nullptr, &z, bwd ? &cs : nullptr)) {
+      v = ffz_round(z);
+    } else {   // angles beyond the float-float range
+      C2x2 T;
+      mzi_T(pp[0], pp[1], al, be, &T, nullptr, nullptr, bwd ? &cs : nullptr);
+      v = k == 0 ? T.t00 : k == 1 ? T.t01 : k == 2 ? T.t10 : T.t11;
+      z = {ff{v.x, 0.f}, ff{v.y, 0.f}};
     }
-    a.kinds[a.L + 2 * l] = sh;
-    a.kinds[a.L + 2 * l + 1] = ln;
   }
+  if constexpr (FRAME) {
+    const int sh = kind == KIND_MIS ? 1 : 0;
+    frame_entry(a, l, q, k, sh, z, cs);
+    if (k == 0) frame_slot(a, l, q, t, sh, cs);
+  }
+  const int M = a.M, G = a.G;
+  float2* tl = reinterpret_cast<float2*>(a.tiles + (size_t)l * a.layer_bytes);   // two entries of a row side by side
+  if (kind < KIND_XL) {
+    const int j = q / (M / 2), e = q % (M / 2);
+    if (bwd && k == 0) tl[2 * M * G + e * G + j] = cs;
+    tl[2 * ((2 * e + (k >> 1)) * G + j) + (k & 1)] = v;
+  } else {
+    // butterfly over lanes: own rows of T, a -> (t00, t01), b -> (t11, t10); back-propagation: of T^H, a -> (conj t00,
+    // conj t10), b -> (conj t11, conj t01)
+    const int st = 1 << (kind - KIND_XL);
+    const int A = 2 * st * (q / st) + (q % st), row = bwd ? k & 1 : k >> 1, m = row ? A + st : A;
+    const int la = A / M, ma = A % M;
+    if (bwd && k == 0) tl[2 * M * G + ma * (G / 2) + a_lane_index(la, st / M)] = cs;
+    tl[2 * ((m % M) * G + m / M) + (k == 0 || k == 3 ? 0 : 1)] = bwd ? make_float2(v.x, -v.y) : v;
+  }
+}
+
+// Thread t of the coefficient pass, one per slot: every other crossing and tile
+template <bool FRAME>
+__device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
+  const int np2 = a.G * a.M / 2, idx = t;
+  if (idx >= a.L * np2) return;
+  const int l = idx / np2, q = idx - l * np2;
+  bool active = false;
+  const int kind = layer_kind(a, l, q, &active);
+  if (q == 0) write_layer(a, l, kind);
   const int M = a.M, G = a.G;
   const bool real = a.crossing == CR_ORTH;
   float4* tl = reinterpret_cast<float4*>(a.tiles + (size_t)l * a.layer_bytes);
@@ -207,9 +249,13 @@ __device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
     C2x2 T, D0, D1;
     float2 csv = make_float2(0.f, 0.f);   // (cos, sin)(pi/4 + beta) for the direct MZI gradient; 0 if inactive
     Tff F;
-    slot_T<QUAD>(a, l, q, active, T, D0, D1, (a.op == OP_BWD && a.gr == 1) ? &csv : nullptr, F);
-    if constexpr (FRAME) frame_inputs<QUAD>(a, l, q, t, kind == KIND_MIS ? 1 : 0, F, csv);
-    if (!writer) return;
+    slot_T(a, l, q, active, T, D0, D1, (a.op == OP_BWD && a.gr == 1) ? &csv : nullptr, F);
+    if constexpr (FRAME) {
+      const int sh = kind == KIND_MIS ? 1 : 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) frame_entry(a, l, q, k, sh, F.t[k], csv);
+      frame_slot(a, l, q, t, sh, csv);
+    }
     if (a.op == OP_BWD && a.gr == 1) {
       float2* cs = reinterpret_cast<float2*>(tl + M * G);
       if (!xl) cs[e * G + j] = csv;
@@ -257,7 +303,6 @@ __device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
   } else {
     R2x2 T, D0;
     slot_R(a, l, q, active, T, D0);
-    if (!writer) return;
     if (a.op == OP_BWD && a.gr == 0) {
       float4* D = reinterpret_cast<float4*>(a.dtiles + (size_t)l * a.dlayer_bytes) + slot_pos(q, M, G);
       D[0] = make_float4(D0.t00, D0.t01, D0.t10, D0.t11);
@@ -294,7 +339,9 @@ __device__ __forceinline__ void coef_body(const CoefArgs& a, int t) {
 
 template <bool QUAD, bool FRAME>
 __global__ void coef_kernel(const CoefArgs a) {
-  coef_body<QUAD, FRAME>(a, blockIdx.x * blockDim.x + threadIdx.x);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if constexpr (QUAD) coef_quad<FRAME>(a, t);
+  else coef_body<FRAME>(a, t);
 }
 
 }  // namespace mg
