@@ -64,11 +64,13 @@ extern "C" {
 typedef struct mg_config {
   int M, V, W, CL, S;
   int split;   /* 0: automatic, 1: two CTA kinds per SM (V and V-1 vectors per lane group), 2: uniform CTAs,
-                * 3: warp pairs, 4: two CTAs per SM, 5: framed (crossings with a unit diagonal; CL and S are those of
-                * its pipeline), 6: framed, the warps of a CTA holding V and V-1 vectors in turn.  Without a
+                * 3: warp pairs, 4: two CTAs per SM, 5: framed (crossings with a unit diagonal; CL is that of its
+                * pipeline, of 3 stages), 6: framed, the warps of a CTA holding V and V-1 vectors in turn.  Without a
                 * configuration a nearest-neighbour MZI mesh of 64 < N takes a framed launch where that is faster; it
                 * computes with fields scaled by up to 2^22 either way, so magnitudes beyond about 1e30 (1e25 for a
-                * product of field and gradient) overflow in it */
+                * product of field and gradient) overflow in it.  7: butterfly kernels for FFT meshes of 2^k modes (64 to 256;
+                * forward also 512; the other fields then describe the general launch), taken without a configuration
+                * where faster, the general launch where there is none */
 } mg_config;
 
 /* ---- library ---------------------------------------------------------------------------- */

@@ -47,6 +47,17 @@ extern "C" int mg_autotune(int op, int N, int L, int B, int crossing, int geomet
     for (int V : {1, 2})
       for (int W : {2, 4, 8}) cands.push_back(mg_config{mg::kWideM, V, W, 0, 0, 2});
 
+  // the launches that the library would take by itself: framed (with the vectors and warps it picks), butterfly
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int lanes = N > 512 ? 32 * mg::kWideM : Np;
+  mg_config fc;
+  if (geometry == MG_GEO_NN && !real && N > 64 && mg::framed_pays(op, lanes / 32, L, lanes / 2, B, sms) &&
+      mg::framed_pick(op, lanes / 32, B, sms, &fc))
+    cands.push_back(fc);
+  if (geometry == MG_GEO_FFT) cands.push_back(mg_config{0, 0, 0, 0, 0, 7});
+
   // scratch (stream-ordered, freed before returning): fields x, dx / g, y, dy / g_in, dJ/dp, an L2 flush
   // buffer and the workspace of the largest candidate so far
   const size_t field = (size_t)B * N * el;

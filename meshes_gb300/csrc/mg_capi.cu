@@ -21,6 +21,7 @@
 #include "mg_reduce.cuh"
 #include "mg_inst_table.h"
 #include "mg_launch.h"
+#include "mg_fft_args.cuh"
 #include "mg_framed_args.cuh"
 
 using namespace mg;
@@ -119,6 +120,9 @@ struct Plan {
   size_t off_main, off_resc, off_wts, off_dfin, off_fkinds, off_tdiag, off_toff, off_tmag, off_tcs, off_count;
   unsigned flb;     // bytes of a layer's framed tile
   int fcl;          // layers per stage of the framed pipeline (CL, S: of the unframed body in the same kernel)
+  bool fft;         // butterfly kernels (mg_fft.cuh) on this plan's tiles
+  int fft_grid;
+  size_t fft_smem;
   bool perm;        // MG_GEO_PERM: permutation tables at off_perm, gather scratch after the smem layout
   size_t off_perm;
 };
@@ -141,6 +145,26 @@ int default_warps(int B, int per_warp, int sms) {
   long w = std::max<long>((warps + sms - 1) / sms, 1);
   if (w > 2) w = (w + 3) / 4 * 4;
   return (int)std::min<long>(w, 8);
+}
+
+// CTAs of a butterfly launch (mg_fft.cuh), 0: none.  Meshes of 2^k modes whose layers all fit shared memory take it, for
+// any batch in back-propagation, in forward from 8 warps' batches per SM on (N = 64: 1), below which laying out the tiles
+// takes longer than the general kernel's shuffles.  Measured on GB300 with launch and reduction, general -> butterfly
+// kernel: forward N = 256 B = 4000 15 -> 19 us, B = 6000 25 -> 21; N = 128 B = 6000 15 -> 15, B = 10000 23 -> 17; N = 64
+// B = 1500 11 -> 9, B = 20000 22 -> 15; N = 512 B = 4000 29 -> 29, B = 20000 109 -> 80; back-propagation N = 64 B = 1 26 -> 17,
+// B = 20000 60 -> 35; N = 256 B = 1 29 -> 26, B = 1000 32 -> 30, B = 6000 62 -> 48, B = 20000 145 -> 95.
+// asked: by the configuration, whatever the batch
+int fft_ctas(int op, int gr, bool real, int N, int L, int B, bool asked, const DevInfo& di, size_t* smem) {
+  const int M = fft_modes(op, N);
+  if (M == 0 || real || L < 1 || !(op == OP_FWD || (op == OP_BWD && gr == 1))) return 0;
+  const int G = N / M, per_sm = fft_ctas_per_sm(op, M);
+  if (L > 64) return 0;
+  *smem = fft_layout(op, M, G, L).total;
+  if (*smem > (per_sm == 1 ? (size_t)di.smem_optin - 1024 : (size_t)di.smem_per_sm / per_sm - 1024)) return 0;
+  const long batch = 32 / G * kFftVectors, batches = (B + batch - 1) / batch;
+  if (!asked && op == OP_FWD && batches < (M == 8 ? 1 : 8) * (long)di.sms) return 0;
+  if (B < 1) return 0;
+  return (int)std::min<long>(per_sm * di.sms, batches);
 }
 
 // Layers without their partner from which on a mesh takes the unframed body: each costs the framed one a layer of zeros
@@ -207,6 +231,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   // back-propagation with direct gradients
   const bool may_frame = !stored && !perm && geometry == GEO_NN && N > 64 && L > 0 && L <= kMaxSmemKinds &&
                          (crossing == CR_MZI ? op != OP_FWDDIFF : crossing == CR_SYM && op == OP_FWD);
+  const bool chosen = cfg != nullptr;   // a configuration given or tuned
   mg_config fc;
   if (!cfg && may_frame && framed_pays(op, Np / 32, L, Np / 2, B, di.sms) && framed_pick(op, Np / 32, B, di.sms, &fc)) cfg = &fc;
   int small_v = 0;
@@ -352,7 +377,11 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   p.off_dtiles = p.off_tiles + align256((size_t)L * p.lb);
   p.off_perm = p.off_dtiles + align256((size_t)L * p.dlb);
   p.off_partial = p.off_perm + (perm ? align256(perm_table_bytes(N, L)) : 0);
-  p.total = p.off_partial + ((op == OP_BWD) ? align256((size_t)p.grid * L * p.np2 * (p.gr == 4 ? 32 : 8)) : 0);
+  p.fft_smem = 0;
+  p.fft_grid = (!chosen || split_mode == 7) && !perm && !stored && geometry == GEO_FFT
+                   ? fft_ctas(op, p.gr, p.real, N, L, B, split_mode == 7, di, &p.fft_smem) : 0;
+  p.fft = p.fft_grid > 0;
+  p.total = p.off_partial + ((op == OP_BWD) ? align256((size_t)std::max(p.grid, p.fft_grid) * L * p.np2 * (p.gr == 4 ? 32 : 8)) : 0);
   if (p.framed) {
     const size_t n = (size_t)L * p.np2;
     const bool bwd = op == OP_BWD;
@@ -549,7 +578,17 @@ int run_prop(const Plan& P, const void* in0, const void* in1, void* out0, void* 
   lc.smem = P.smem;
   lc.stream = st;
   cudaError_t e;
-  if (P.framed) {
+  const bool fft = P.fft && !ckpt;
+  const int nC = fft ? P.fft_grid : P.grid;   // CTAs, with a set of partials each
+  if (fft) {
+    FftArgs f;
+    static_cast<PropArgs&>(f) = a;
+    f.M = P.M;
+    lc.grid = dim3(nC);
+    lc.block = dim3(kFftThreads);
+    lc.smem = P.fft_smem;
+    e = P.op == OP_FWD ? launch_fft_fwd(lc, f) : launch_fft_bwd(lc, f);
+  } else if (P.framed) {
     FramedArgs f;
     static_cast<PropArgs&>(f) = a;
     f.main = reinterpret_cast<const float4*>(ws + P.off_main);
@@ -583,7 +622,7 @@ int run_prop(const Plan& P, const void* in0, const void* in1, void* out0, void* 
       return e == cudaSuccess ? MG_OK : cuda_fail(e, "framed_reduce_kernel launch");
     }
     dp_reduce_kernel<<<(n + kReduceCols - 1) / kReduceCols, kReduceCols * kReduceRows, 0, st>>>(
-        a.partial, P.grid, P.L, P.np2, P.M, P.G, P.N, dp, ldp, crossing_np(P.crossing), accumulate, geo);
+        a.partial, nC, P.L, P.np2, P.M, P.G, P.N, dp, ldp, crossing_np(P.crossing), accumulate, geo);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "dp_reduce_kernel launch");
   }

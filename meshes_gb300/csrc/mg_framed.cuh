@@ -34,6 +34,11 @@ __device__ __forceinline__ ulonglong2 lds16(uint32_t addr) {
   asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ unsigned long long lds8(uint32_t addr) {
+  unsigned long long v;
+  asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ int lds4(uint32_t addr) {
   int v;
   asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(addr));

@@ -90,6 +90,10 @@ bool nn_fwddiff_instantiated(int op, bool real, int M, int V, int gr, bool full)
 cudaError_t launch_prop_nn_fwddiff(bool real, int M, int V, const LaunchCfg& lc, const PropArgs& a);
 cudaError_t launch_prop_nn(int op, bool real, int M, int V, int gr, bool full, bool split, const LaunchCfg& lc,
                            const PropArgs& a);
+// butterfly meshes (mg_fft.cuh): one unit per op
+struct FftArgs;
+cudaError_t launch_fft_fwd(const LaunchCfg& lc, const FftArgs& a);
+cudaError_t launch_fft_bwd(const LaunchCfg& lc, const FftArgs& a);
 // wide nearest-neighbour meshes (512 < N <= 640): kWideM modes in each of 32 lanes (mg_prop_wide.cu)
 constexpr int kWideM = 20;
 bool wide_instantiated(int op, bool real, int V, int gr);
