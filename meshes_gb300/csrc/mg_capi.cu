@@ -1103,11 +1103,20 @@ int range_impl(int op, int N, int L, int l0, int l1, int B, int crossing, int ge
   if (op != OP_FWD && op != MG_OP_BWD_STORED) return fail(MG_E_ARG, "op %d not in {MG_OP_FWD, MG_OP_BWD_STORED}", op);
   if (l0 < 0 || l1 < l0 || l1 > L) return fail(MG_E_ARG, "layer range [%d, %d) outside [0, %d)", l0, l1, L);
   // layer ranges run uniform CTAs (the stored-activation kernels have no split form)
+  const mg_config* given = cfg;
   mg_config cu = cfg ? *cfg : mg_config{0, 0, 0, 0, 0, 0};
   cu.split = 2;
   cfg = &cu;
   Plan P;
   TRY(make_plan(op, N, L, B, crossing, geometry, cfg, &P));
+  {   // the tiles' modes per lane, where the whole-mesh launch takes others
+    Plan built;
+    if (make_plan(op, N, L, B, crossing, geometry, given, &built) == MG_OK && built.M != P.M) {
+      cu.M = built.M;
+      TRY(make_plan(op, N, L, B, crossing, geometry, cfg, &P));
+    }
+    g_err.clear();
+  }
   if (P.perm) return fail(MG_E_ARG, "layer ranges take no permutations");
   TRY(check_ws(P, ws, wsb));
   TRY(check_ldu(P, ldu));

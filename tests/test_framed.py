@@ -187,3 +187,20 @@ def test_framed_plans_on_the_host():
         assert plan(kw["op"], kw["N"], 16, 64, kw["crossing"], kw["geo"], (8, 4, 8, 0, 0, 5)) is None
     assert plan(0, 256, 256, 64, cfg=(8, 4, 4, 0, 0, 6)) is None               # mixed warps come in eights
     assert plan(2, 600, 600, 2048).total > 0 and plan(2, 2, 1, 1).total > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,B", [(100, 3000), (128, 9000), (200, 700)])
+def test_layer_ranges_of_framed_tiles(N, B):
+    """Tiles built for a whole-mesh launch that is framed (other modes per lane than the range's own choice at N <= 128)
+    serve mg_propagate_range."""
+    rng = np.random.default_rng(N)
+    om = _mesh(rng, N, "clements")
+    run = _Run(om, 0, B, None)
+    x = O.unit_columns(rng, N, B)
+    xd = torch.tensor(x, dtype=torch.complex64, device="cuda")
+    mid, y = torch.zeros_like(xd), torch.zeros_like(xd)
+    for l0, l1, src, dst in ((0, 20, xd, mid), (20, om.L, mid, y)):
+        run.check(run.lib.mg_propagate_range(0, N, om.L, l0, l1, B, 0, 0, src.data_ptr(), None, dst.data_ptr(), None, N, None,
+                                             None, 0, None, run.ws.data_ptr(), run.nb, run.st), "range")
+    assert O.rel_err(y.cpu().numpy(), O.propagate(om, x)) < TOL
