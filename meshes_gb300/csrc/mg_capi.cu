@@ -186,12 +186,32 @@ int stored_default_v(int op, int M) { return op == OP_FWD ? (M <= 4 ? 8 : (M == 
 // Tile of a nearest-neighbour complex mesh whose batch would leave schedulers without a warp at the default tile (8 modes
 // and 4 vectors per lane: at N = 100 and B = 777, 98 warps for 608 schedulers): a vector over all 32 lanes, and as few
 // vectors per lane as fill the schedulers.  Measured on GB300 at B = 608: N = 128 forward 31 -> 13 us, back-propagation
-// 132 -> 35 us; N = 100 (Reck), B = 777 forward 52 -> 21 us.  From n vectors per scheduler on the default tile's reuse of
-// coefficients wins.  0: the default.
+// 132 -> 35 us; N = 100 (Reck), B = 777 forward 52 -> 21 us.  N = 256, B = 300 forward 64 -> 38 us, B = 1000 64 -> 46
+// us.  From n vectors per scheduler on the default tile's reuse of coefficients wins.  0: the default.
 int small_batch_v(int op, int M, int B, int sms) {
   const long n = ((long)B + 4 * sms - 1) / (4 * sms);
-  if (op == OP_FWD) return M == 2 ? (n <= 1 ? 1 : n <= 4 ? 2 : n <= 8 ? 4 : 0) : M == 4 ? (n <= 2 ? 1 : n <= 8 ? 2 : 0) : 0;
+  if (op == OP_FWD) return M == 2 ? (n <= 1 ? 1 : n <= 4 ? 2 : n <= 8 ? 4 : 0) : M == 4 ? (n <= 2 ? 1 : n <= 8 ? 2 : 0) : M == 8 ? (n <= 1 ? 1 : n <= 2 ? 2 : 0) : 0;
   return M > 4 ? 0 : n <= 2 ? 1 : n <= 8 ? 2 : 0;
+}
+
+// Forward derivatives, M modes per lane: vectors per lane and warps such that waves x (vectors per scheduler + 1.8) is
+// least.  Measured on GB300, N = 256: 76 us at n = 1, 99 at 2 (V = 2, W = 4; 113 as V = 1, W = 8), 154 at 4, 267 at 8.
+// Against the lane groups of 8 or 16 modes that every op takes: N = 64, B = 300 31 -> 13 us; N = 100, B = 300 54 -> 23; N =
+// 130, B = 1000 54 -> 46; N = 128, B = 20000 412 -> 367; N = 300, B = 1000 259 -> 154; N = 256, B = 5000 517 -> 451.
+mg_config fwddiff_pick(int M, int B, int sms) {
+  mg_config best{};
+  double least = 0;
+  for (int V : {1, 2, 4})
+    for (int W : {4, 8}) {
+      if (M > 8 && V > 2) continue;
+      const long cap = (long)W * V, ctas = (B + cap - 1) / cap, waves = (ctas + sms - 1) / sms;
+      const double cost = waves * (cap / 4 + (V == 1 && W == 8 ? 2.2 : 1.8));
+      if (least == 0 || cost < least) {
+        least = cost;
+        best = mg_config{M, V, W, M == 8 ? 8 : 0, 0, 2};
+      }
+    }
+  return best;
 }
 
 // op MG_OP_BWD_STORED plans the back-propagation kernel in its stored-activation mode (GR 4): T tiles
@@ -226,12 +246,24 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   p.real = crossing == CR_ORTH;
   p.gr = stored ? 4 : (op != OP_BWD) ? 0 : (crossing == CR_MZI ? 1 : (crossing == CR_ORTH ? 2 : 0));
   const bool wide = N > 512;
-  const int Np = wide ? 32 * kWideM : pow2ceil(N);
+  // forward derivatives of a nearest-neighbour complex mesh: a vector over the whole warp, in 6 or 12 modes per lane where
+  // that holds it
+  const bool diff = op == OP_FWDDIFF && geometry == GEO_NN && !perm && crossing != CR_ORTH && !wide && N > 32;
+  int diff_m = 0;
+  if (diff && (!cfg || cfg->M == 6 || cfg->M == 12))
+    diff_m = N > 256 ? (N <= 384 ? 12 : 16) : N > 128 ? (N <= 192 ? 6 : 8) : pow2ceil(N) / 32;
+  if (diff && cfg && diff_m != cfg->M) diff_m = 0;
+  const int Np = wide ? 32 * kWideM : diff_m ? 32 * diff_m : pow2ceil(N);
+  mg_config dc;
+  if (!cfg && diff_m) {
+    dc = fwddiff_pick(diff_m, B, di.sms);
+    cfg = &dc;
+  }
+  const bool chosen = cfg != nullptr;   // a configuration given or tuned
   // framed launch: nearest-neighbour complex meshes whose vector fills the warp at M >= 4, forward and MZI
   // back-propagation with direct gradients
   const bool may_frame = !stored && !perm && geometry == GEO_NN && N > 64 && L > 0 && L <= kMaxSmemKinds &&
                          (crossing == CR_MZI ? op != OP_FWDDIFF : crossing == CR_SYM && op == OP_FWD);
-  const bool chosen = cfg != nullptr;   // a configuration given or tuned
   mg_config fc;
   if (!cfg && may_frame && framed_pays(op, Np / 32, L, Np / 2, B, di.sms) && framed_pick(op, Np / 32, B, di.sms, &fc)) cfg = &fc;
   int small_v = 0;
@@ -251,7 +283,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
     }
   }
   int M = (cfg && cfg->M) ? cfg->M : small_v ? Np / 32 : (wide ? kWideM : std::max(std::min(8, Np), Np / 32));
-  if (wide ? M != kWideM : (M < 2 || M > 16 || (M & (M - 1))))
+  if (wide ? M != kWideM : (M < 2 || M > 16 || (M != diff_m && (M & (M - 1)))))
     return fail(MG_E_CONFIG, "modes per lane M=%d not in %s", M, wide ? "{20} for N > 512" : "{2,4,8,16}");
   if (M > Np) M = Np;
   const int G = Np / M;
@@ -284,7 +316,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   } else if (wide ? (perm || stored || !wide_instantiated(op, crossing == CR_ORTH, V, p.gr))
            : perm ? !perm_instantiated(op, crossing == CR_ORTH, M, V, p.gr)
                   : (stored ? !instantiated_stored(OP_BWD, M, V, geometry == GEO_NN && G == 32)
-                            : !(instantiated(op, M, V) ||
+                            : !((diff_m ? nn_instantiated(op, false, M, V, p.gr, true, false) : instantiated(op, M, V)) ||
                                 (geometry == GEO_NN && nn_small_instantiated(op, p.real, M, V, p.gr, G == 32)))))
     return fail(MG_E_CONFIG, "no %skernel instantiated for op=%d M=%d V=%d",
                 wide ? "wide-mesh " : perm ? "permuted-mesh " : "", stored ? MG_OP_BWD_STORED : op, M, V);

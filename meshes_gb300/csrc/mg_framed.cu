@@ -25,19 +25,24 @@ bool framed_instantiated(int op, int M, int V, bool full, bool mix) {
 // The launch of a batch: warps per CTA and vectors per lane such that waves x (vectors per scheduler + 4) is least.
 // Measured on GB300 over one-wave batches, a launch takes time proportional to n + 4 for n vectors per scheduler: the
 // layers' latency is worth about four vectors (M = 8, L = 256, back-propagation: 87 us at n = 1, 160 at 4, 236 at 8;
-// forward 36, 53, 79).
+// forward 36, 53, 79).  Two vectors per scheduler go as V = 2 in 4 warps rather than V = 1 in 8 where that is faster (each
+// coefficient serves two vectors): forward at N = 256 44 -> 40 us, N = 400 97 -> 86, N = 600 171 -> 148; back-propagation at
+// N = 400 314 -> 267, but at N = 256 101 -> 105 and at N = 600 531 -> 580 (it spills).
 bool framed_pick(int op, int M, int B, int sms, mg_config* out) {
   long best = 0;
   auto consider = [&](int V, bool mix, int W) {
     const int cap = framed_cta_vectors(W, 1, V, mix);
-    const long ctas = std::max(1, (B + cap - 1) / cap), waves = (ctas + sms - 1) / sms, cost = waves * (cap / 4 + 4);
+    const long ctas = std::max(1, (B + cap - 1) / cap), waves = (ctas + sms - 1) / sms;
+    const bool pairs = op == OP_FWD || M == 16;   // V = 2 in 4 warps before V = 1 in 8
+    const long cost = 2 * waves * (cap / 4 + 4) + (W == 8 && V == 1 && pairs ? 1 : 0);
+    if (W == 4 && V > 1 && !(V == 2 && !mix && pairs)) return;
     if (best != 0 && cost >= best) return;
     best = cost;
     *out = mg_config{M, V, W, 0, 0, mix ? 6 : 5};
   };
 #define MG_X(M_, V_, MIX_)                            \
   if (M == M_) {                                      \
-    if (V_ == 1) consider(V_, MIX_, 4);               \
+    if (!MIX_) consider(V_, MIX_, 4);                 \
     consider(V_, MIX_, 8);                            \
     if (M_ == 4 && V_ > 1) consider(V_, MIX_, 16);    \
   }
@@ -47,14 +52,15 @@ bool framed_pick(int op, int M, int B, int sms, mg_config* out) {
   return best != 0;
 }
 
-// Whether the framed launch repays the frame pass.  The pass takes about 8 us and 1e-4 us per slot (N = 256, L = 256: 10
-// us; N = 600, L = 600: 28 us).  A framed layer saves, per M modes of a lane and with n vectors per scheduler, about
-// 0.006 (1 + (n-1)/4) us forward and 0.018 (1 + (n-1)/8) us in back-propagation (N = 256: forward 48 -> 36 us at n = 1,
-// 105 -> 72 at 7; back-propagation 122 -> 81 and 265 -> 216; N = 128: forward 19 -> 17 at n = 1, 60 -> 44 at 16).
+// Whether the framed launch repays the frame pass.  The pass takes about 8 us and 6e-5 us per slot (tiles with it and without:
+// N = 128 17 and 9 us, N = 256 19 and 11, N = 600 42 and 22).  With n vectors per scheduler a framed layer saves, per M modes
+// of a lane, forward 0.0018 n us up to M = 8, where the general kernel has a tile for every n (N = 256: 46 -> 40 us at n = 2,
+// 64 -> 50 at 4, 99 -> 72 at 7; N = 128: 60 -> 44 at 16), and 0.006 (1 + (n-1)/4) us beyond; in back-propagation about
+// 0.018 (1 + (n-1)/8) us (N = 256: 122 -> 75 us at n = 1, 265 -> 199 at 7).
 bool framed_pays(int op, int M, int L, int np2, int B, int sms) {
   const double n = std::max(1.0, (double)B / (4.0 * sms));
-  const double saved = L * M * (op == OP_BWD ? 0.018 * (1 + (n - 1) / 8) : 0.006 * (1 + (n - 1) / 4));
-  return saved > 1.1 * (8.0 + 1e-4 * L * np2);
+  const double layer = op == OP_BWD ? 0.018 * (1 + (n - 1) / 8) : M <= 8 ? 0.0018 * n : 0.006 * (1 + (n - 1) / 4);
+  return L * M * layer > 8.0 + 6e-5 * L * np2;
 }
 
 cudaError_t launch_prop_framed(int op, int M, int V, bool mix, const LaunchCfg& lc, const FramedArgs& a) {

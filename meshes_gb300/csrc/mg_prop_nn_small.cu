@@ -10,7 +10,7 @@ namespace mg {
 namespace {
 // (op, gr, M, V)
 constexpr int kSmall[][4] = {{OP_FWD, 0, 2, 1}, {OP_FWD, 0, 2, 2}, {OP_FWD, 0, 2, 4}, {OP_FWD, 0, 4, 1},
-                             {OP_FWD, 0, 4, 2}, {OP_BWD, 1, 4, 1}, {OP_BWD, 1, 4, 2}, {OP_BWD, 1, 2, 1},
+                             {OP_FWD, 0, 4, 2}, {OP_FWD, 0, 8, 1}, {OP_FWD, 0, 8, 2}, {OP_BWD, 1, 4, 1}, {OP_BWD, 1, 4, 2}, {OP_BWD, 1, 2, 1},
                              {OP_BWD, 1, 2, 2}};
 }  // namespace
 
@@ -27,6 +27,8 @@ cudaError_t launch_prop_nn_small(int op, int M, int V, const LaunchCfg& lc, cons
     case 22: return launch_one<OP_FWD, 2, 2, false, 32, 0, false, true>(lc, a);
     case 24: return launch_one<OP_FWD, 2, 4, false, 32, 0, false, true>(lc, a);
     case 41: return launch_one<OP_FWD, 4, 1, false, 32, 0, false, true>(lc, a);
+    case 81: return launch_one<OP_FWD, 8, 1, false, 32, 0, false, true>(lc, a);
+    case 82: return launch_one<OP_FWD, 8, 2, false, 32, 0, false, true>(lc, a);
     case 42: return launch_one<OP_FWD, 4, 2, false, 32, 0, false, true>(lc, a);
     case OP_BWD * 10000 + 41: return launch_one<OP_BWD, 4, 1, false, 32, 1, false, true>(lc, a);
     case OP_BWD * 10000 + 21: return launch_one<OP_BWD, 2, 1, false, 32, 1, false, true>(lc, a);
