@@ -190,15 +190,17 @@ int stored_default_v(int op, int M) { return op == OP_FWD ? (M <= 4 ? 8 : (M == 
 // us.  From n vectors per scheduler on the default tile's reuse of coefficients wins.  0: the default.
 int small_batch_v(int op, int M, int B, int sms) {
   const long n = ((long)B + 4 * sms - 1) / (4 * sms);
-  if (op == OP_FWD) return M == 2 ? (n <= 1 ? 1 : n <= 4 ? 2 : n <= 8 ? 4 : 0) : M == 4 ? (n <= 2 ? 1 : n <= 8 ? 2 : 0) : M == 8 ? (n <= 1 ? 1 : n <= 2 ? 2 : 0) : 0;
+  if (op == OP_FWD)
+    return M == 2 ? (n <= 1 ? 1 : n <= 4 ? 2 : n <= 8 ? 4 : 0) : M == 4 ? (n <= 2 ? 1 : n <= 8 ? 2 : 0)
+         : M == 8 ? (n <= 1 ? 1 : n <= 2 ? 2 : 0) : M == 16 ? (n <= 1 ? 1 : 0) : 0;
   return M > 4 ? 0 : n <= 2 ? 1 : n <= 8 ? 2 : 0;
 }
 
-// Forward derivatives, M modes per lane: vectors per lane and warps such that waves x (vectors per scheduler + 1.8) is
+// Forward derivatives and back-propagation through dJ/dT, M modes per lane: vectors per lane and warps such that waves x (vectors per scheduler + 1.8) is
 // least.  Measured on GB300, N = 256: 76 us at n = 1, 99 at 2 (V = 2, W = 4; 113 as V = 1, W = 8), 154 at 4, 267 at 8.
 // Against the lane groups of 8 or 16 modes that every op takes: N = 64, B = 300 31 -> 13 us; N = 100, B = 300 54 -> 23; N =
 // 130, B = 1000 54 -> 46; N = 128, B = 20000 412 -> 367; N = 300, B = 1000 259 -> 154; N = 256, B = 5000 517 -> 451.
-mg_config fwddiff_pick(int M, int B, int sms) {
+mg_config vectors_pick(int M, int B, int sms) {
   mg_config best{};
   double least = 0;
   for (int V : {1, 2, 4})
@@ -256,7 +258,13 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   const int Np = wide ? 32 * kWideM : diff_m ? 32 * diff_m : pow2ceil(N);
   mg_config dc;
   if (!cfg && diff_m) {
-    dc = fwddiff_pick(diff_m, B, di.sms);
+    dc = vectors_pick(diff_m, B, di.sms);
+    cfg = &dc;
+  }
+  // back-propagation through dJ/dT: a vector over the whole warp as well
+  if (!cfg && op == OP_BWD && p.gr == 0 && !stored && !perm && !wide && geometry == GEO_NN && N > 32) {
+    dc = vectors_pick(Np / 32, B, di.sms);
+    dc.CL = 0;
     cfg = &dc;
   }
   const bool chosen = cfg != nullptr;   // a configuration given or tuned
@@ -1002,6 +1010,7 @@ int mg_propagate(int op, int N, int L, int B, int crossing, int geometry, const 
     if (!cfg && !Pb.perm && lookup_tuned(OP_FWD, crossing, Pb.geometry, N, B, &tf) && tf.M == Pb.M) cf = tf;
     if (Pb.framed) framed_pick(OP_FWD, Pb.M, B, dev_info().sms, &cf);
     else if (cf.split >= 5) cf = {Pb.M, 0, 0, 0, 0, 2};
+    else if (!cfg && cf.V == 0 && Pb.G == 32 && !Pb.real && !Pb.perm) cf.V = small_batch_v(OP_FWD, Pb.M, B, dev_info().sms);
     TRY(make_plan(OP_FWD, N, L, B, crossing, geometry, &cf, &Pf));
     TRY(use_bwd_tiles(Pb, &Pf));
     TRY(check_ldu(Pf, ldu));

@@ -80,7 +80,9 @@ bool nn_instantiated(int op, bool real, int M, int V, int gr, bool full, bool sp
 // the small-mesh tiles among them (complex, full warp, few modes and vectors per lane, so that a small batch
 // spreads over more schedulers; forward, and back-propagation at 4 x 2; mg_prop_nn_small.cu)
 bool nn_small_instantiated(int op, bool real, int M, int V, int gr, bool full);
-cudaError_t launch_prop_nn_small(int op, int M, int V, const LaunchCfg& lc, const PropArgs& a);
+cudaError_t launch_prop_nn_small(int op, int gr, int M, int V, const LaunchCfg& lc, const PropArgs& a);
+bool nn_raw_instantiated(int M, int V);
+cudaError_t launch_prop_nn_raw(int M, int V, const LaunchCfg& lc, const PropArgs& a);
 // stored-activation kernels (GR 4) of nearest-neighbour meshes with a vector over the whole warp, N <= 128
 // (mg_prop_stored_nn.cu)
 bool stored_nn_instantiated(int op, int M, int V);
