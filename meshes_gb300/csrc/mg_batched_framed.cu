@@ -39,7 +39,7 @@ batched_framed_kernel(const mg_batch_framed* __restrict__ meshes, int n_meshes, 
 
 // grid (columns, meshes): a mesh's CTAs stride over the blocks of its columns; meshes on plain tiles have no main
 __global__ void __launch_bounds__(256) batched_framed_reduce_kernel(const mg_batch_framed* __restrict__ meshes) {
-  __shared__ float2 acc[kFReduceRows][kFReduceCols];
+  __shared__ float4 acc[kFReduceRows][kFReduceCols];
   const mg_batch_framed f = meshes[blockIdx.y];
   const mg_batch_mesh& md = f.mesh;
   if (!md.dp || !md.partial || md.n_items <= 0) return;
@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) batched_framed_reduce_kernel(const mg_bat
   const int M = batch_framed_M(md.N), np2 = 16 * M;
   const FramedReduceArgs a{static_cast<const float2*>(md.partial), md.n_items, md.L, np2, M, 32, md.N, md.dp, md.ldp, 0,
                            md.kinds + md.L, static_cast<const float2*>(f.wts), f.count, f.refuse};
-  for (int blk = blockIdx.x; blk * kFReduceCols < md.L * np2; blk += gridDim.x) {
+  for (int blk = blockIdx.x; 2 * blk * kFReduceCols < md.L * np2; blk += gridDim.x) {
     framed_reduce_block(a, blk, acc);
     __syncthreads();
   }

@@ -359,7 +359,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   if (p.tree > 1) W = p.tree * default_warps(B, p.tree * 4, di.sms);
   if (!W) {
     W = std::min(default_warps(B, p.R * V, di.sms), maxw);
-    if (small_v && op == OP_BWD && W < 4) W = 4;   // fewer CTAs leave fewer partials
+    if (small_v) W = std::max(W, op == OP_BWD ? 4 : 2);   // fewer CTAs fetch tiles and leave partials
   }
   if (W < 1 || W > maxw) return fail(MG_E_CONFIG, "W=%d warps outside [1, %d]", W, maxw);
   int S = (cfg && cfg->S) ? cfg->S : ((op == OP_FWD || p.split) ? 2 : 3);

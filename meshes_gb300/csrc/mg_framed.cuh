@@ -15,7 +15,7 @@
 // B = 4096 back-propagation's 458 per layer and scheduler are 1050 to 1370 of its 1500 cycles.  Three or four warps per
 // scheduler with fewer vectors each do not raise that (257 us for 12 warps of 3, 201 for 8 of 4).  Measured on GB300 at
 // N = 256, L = 256, B = 4096 against the unframed kernels: forward 94 -> 63 us, back-propagation 249 -> 197 us; N = 600,
-// L = 600, B = 2048: forward 314 -> 200 us, back-propagation 1412 -> 717 us.
+// L = 600, B = 2048: forward 314 -> 200 us, back-propagation 1412 -> 684 us.
 //
 // Work decomposition, pipeline, bounded waits and the gradient partials are those of mg_prop.cuh; a stage holds
 // its layers' tiles and the factors of their first RESCALEs.
@@ -410,10 +410,13 @@ __device__ __forceinline__ ulonglong2 frame_pair(const float2* __restrict__ d, i
 __device__ __forceinline__ void cta_sync() { asm volatile("barrier.cta.sync.aligned 0;" ::: "memory"); }
 
 // Sum of the W warps' staged gradients of a chunk (W a multiple of 4), in warp order, into this CTA's partials of the
-// layers from lo on: n float4 of consecutive layers
-__device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int W, int n, ulonglong2* out) {
+// layers from lo on: n float4 of consecutive layers.  turn: the chunk; the warps that the last round of a chunk leaves over
+// change with it (the same two of eight at M = 20: back-propagation at N = 600, B = 2048 727 us, in turns 684)
+__device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int W, int n, int turn, ulonglong2* out) {
+  int first = threadIdx.x + (64 * turn) % (int)blockDim.x;
+  if (first >= (int)blockDim.x) first -= blockDim.x;
 #pragma unroll 1
-  for (int idx = threadIdx.x; idx < n; idx += blockDim.x) {
+  for (int idx = first; idx < n; idx += blockDim.x) {
     uint32_t p = gst + (uint32_t)idx * 16u;
     ulonglong2 t = make_ulonglong2(0, 0);
 #pragma unroll 1
@@ -434,8 +437,8 @@ __device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int 
 // finished that earlier chunk, so the warps of a scheduler may drift apart by up to a chunk and keep each other's
 // latency covered.  The copies are issued by one thread, of another warp for every chunk (those of V - 1 vectors where
 // there are some): what a warp does beyond its layers holds all the others up.  Measured on GB300 against two CTA barriers
-// and the sum at every chunk's end, copies issued by warp 0: N = 600, L = 600, B = 2048 803 -> 717 us, N = 400, B = 2432
-// 432 -> 368 us, N = 128, B = 4000 68 -> 63 us.
+// and the sum at every chunk's end, copies issued by warp 0: N = 600, L = 600, B = 2048 803 -> 684 us, N = 400, B = 2432
+// 432 -> 368 us, N = 128, B = 4000 68 -> 60 us.
 struct FramedSmem {
   unsigned char* base;
   uint32_t zero, gst;
@@ -505,7 +508,7 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
   // chunk c: stage and gradient slot s = c % S, of whose barriers it is phase ph = (c / S) & 1
   auto reduce = [&](int c, int s) {
     const int lo = ch.lo(c);
-    f_reduce(sm.gst + (uint32_t)s * slot_bytes, warp_bytes, a.W, (ch.hi(c) - lo) * (np2 / 2),
+    f_reduce(sm.gst + (uint32_t)s * slot_bytes, warp_bytes, a.W, (ch.hi(c) - lo) * (np2 / 2), c,
              reinterpret_cast<ulonglong2*>(a.partial + (size_t)lo * np2));
   };
   const FTile none{sm.zero + j16, sm.gst + (uint32_t)S * slot_bytes + j16};
@@ -644,58 +647,59 @@ struct FramedReduceArgs {
   const int* count;
   int refuse;
 };
-// columns [kFReduceCols blk, ..); the caller's threads meet before acc is used again
-__device__ __forceinline__ void framed_reduce_block(const FramedReduceArgs& a, int blk, float2 (&acc)[kFReduceRows][kFReduceCols]) {
+// columns [2 kFReduceCols blk, ..), two a thread (16-byte loads: with 8-byte ones a batch's 134 MB took 82 us, 20 at the
+// measured copy rate); the caller's threads meet before acc is used again
+__device__ __forceinline__ void framed_reduce_block(const FramedReduceArgs& a, int blk, float4 (&acc)[kFReduceRows][kFReduceCols]) {
   constexpr int kCols = kFReduceCols, kRows = kFReduceRows;
-  const float2* partial = a.partial;
-  float* dp = a.dp;
-  const int nC = a.nC, L = a.L, np2 = a.np2, M = a.M, G = a.G, N = a.N, ldp = a.ldp, accumulate = a.accumulate;
+  const int nC = a.nC, L = a.L, np2 = a.np2, M = a.M, G = a.G, N = a.N;
   const int* geo = a.geo;
   const int col = threadIdx.x % kCols, row = threadIdx.x / kCols;
-  const int idx = blk * kCols + col;
-  const bool valid = idx < L * np2;
-  const size_t stride = (size_t)L * np2;
-  float2 s = make_float2(0.f, 0.f);
+  const int idx0 = 2 * (blk * kCols + col);
+  const bool valid = idx0 < L * np2;
+  const size_t stride = (size_t)L * np2 / 2;
+  auto add = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
+  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
   if (valid) {
-    const float2* p = partial + idx;
+    const float4* p = reinterpret_cast<const float4*>(a.partial) + idx0 / 2;
     int c = row;
     for (; c + 3 * kRows < nC; c += 4 * kRows) {
-      const float2 a0 = __ldg(p + (size_t)c * stride), a1 = __ldg(p + (size_t)(c + kRows) * stride);
-      const float2 a2 = __ldg(p + (size_t)(c + 2 * kRows) * stride), a3 = __ldg(p + (size_t)(c + 3 * kRows) * stride);
-      s = cadd(cadd(cadd(cadd(s, a0), a1), a2), a3);
+      const float4 a0 = __ldg(p + (size_t)c * stride), a1 = __ldg(p + (size_t)(c + kRows) * stride);
+      const float4 a2 = __ldg(p + (size_t)(c + 2 * kRows) * stride), a3 = __ldg(p + (size_t)(c + 3 * kRows) * stride);
+      t = add(add(add(add(t, a0), a1), a2), a3);
     }
-    for (; c < nC; c += kRows) s = cadd(s, __ldg(p + (size_t)c * stride));
+    for (; c < nC; c += kRows) t = add(t, __ldg(p + (size_t)c * stride));
   }
-  acc[row][col] = s;
+  acc[row][col] = t;
   __syncthreads();
   if (row != 0 || !valid) return;
-  for (int k = 1; k < kRows; ++k) s = cadd(s, acc[k][col]);
-  const int l = idx / np2, rem = idx - l * np2;
-  if (__ldg(a.count) >= a.refuse) {   // partials of the unframed body: (dJ/dth, dJ/dph) of one slot
-    const int q = pos_slot(rem, M, G);
+  for (int k = 1; k < kRows; ++k) t = add(t, acc[k][col]);
+  const int l = idx0 / np2, sh = geo[2 * l] / 2, ln = geo[2 * l + 1];
+  auto put = [&](int q, int k, float v) {
     if (q >= N / 2) return;
-    const bool active = q >= geo[2 * l] / 2 && q < geo[2 * l] / 2 + geo[2 * l + 1];
-    float* o = dp + (size_t)l * ldp + 2 * (size_t)q;
-    o[0] = (accumulate ? o[0] : 0.f) + (active ? s.x : 0.f);
-    o[1] = (accumulate ? o[1] : 0.f) + (active ? s.y : 0.f);
+    float* o = a.dp + (size_t)l * a.ldp + 2 * (size_t)q + k;
+    v = q >= sh && q < sh + ln ? v : 0.f;
+    *o = a.accumulate ? *o + v : v;
+  };
+  const int rem = idx0 - l * np2;
+  if (__ldg(a.count) >= a.refuse) {   // partials of the unframed body: (dJ/dth, dJ/dph) of one slot each
+    const int q0 = pos_slot(rem, M, G), q1 = pos_slot(rem + 1, M, G);
+    put(q0, 0, t.x);
+    put(q0, 1, t.y);
+    put(q1, 0, t.z);
+    put(q1, 1, t.w);
     return;
   }
-  const int k = rem & 1, pos = rem >> 1;
-  const int j = pos % G, q0 = j * (M / 2) + pos / G;
-  const int sh = geo[2 * l] / 2, ln = geo[2 * l + 1];
-  const float2 w = __ldg(a.wts + idx);
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    const int q = q0 + c * (M / 4);
-    if (q >= N / 2) continue;
-    const float v = q >= sh && q < sh + ln ? (c ? s.y * w.y : s.x * w.x) : 0.f;
-    float* o = dp + (size_t)l * ldp + 2 * (size_t)q + k;
-    *o = accumulate ? *o + v : v;
-  }
+  // (th, th'), (ph, ph') of one pair of crossings
+  const int pos = rem >> 1, j = pos % G, q = j * (M / 2) + pos / G;
+  const float4 w = __ldg(reinterpret_cast<const float4*>(a.wts) + idx0 / 2);
+  put(q, 0, t.x * w.x);
+  put(q + M / 4, 0, t.y * w.y);
+  put(q, 1, t.z * w.z);
+  put(q + M / 4, 1, t.w * w.w);
 }
 
 static __global__ void __launch_bounds__(256) framed_reduce_kernel(const FramedReduceArgs a) {
-  __shared__ float2 acc[kFReduceRows][kFReduceCols];
+  __shared__ float4 acc[kFReduceRows][kFReduceCols];
   framed_reduce_block(a, blockIdx.x, acc);
 }
 
