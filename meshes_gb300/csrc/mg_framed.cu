@@ -56,11 +56,12 @@ bool framed_pick(int op, int M, int B, int sms, mg_config* out) {
 // N = 128 17 and 9 us, N = 256 19 and 11, N = 600 42 and 22).  With n vectors per scheduler a framed layer saves, per M modes
 // of a lane, forward 0.0018 n us up to M = 8, where the general kernel has a tile for every n (N = 256: 46 -> 40 us at n = 2,
 // 64 -> 50 at 4, 99 -> 72 at 7; N = 128: 60 -> 44 at 16), and 0.006 (1 + (n-1)/4) us beyond; in back-propagation about
-// 0.018 (1 + (n-1)/8) us (N = 256: 122 -> 75 us at n = 1, 265 -> 199 at 7).
+// 0.018 (1 + (n-1)/8) us (N = 256: 122 -> 75 us at n = 1, 265 -> 199 at 7), of which a forward launch on the same tiles can lose
+// some at n = 1 (N = 128, B = 128: 38.6 -> 30.4 us, forward 19.1 -> 21.2, tiles 8.9 -> 17.1: not framed).
 bool framed_pays(int op, int M, int L, int np2, int B, int sms) {
   const double n = std::max(1.0, (double)B / (4.0 * sms));
   const double layer = op == OP_BWD ? 0.018 * (1 + (n - 1) / 8) : M <= 8 ? 0.0018 * n : 0.006 * (1 + (n - 1) / 4);
-  return L * M * layer > 8.0 + 6e-5 * L * np2;
+  return L * M * layer > (op == OP_BWD ? 1.15 : 1.0) * (8.0 + 6e-5 * L * np2);
 }
 
 cudaError_t launch_prop_framed(int op, int M, int V, bool mix, const LaunchCfg& lc, const FramedArgs& a) {
