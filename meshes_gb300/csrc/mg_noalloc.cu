@@ -52,7 +52,14 @@ cudaError_t scratch_address(void** out) {
 extern "C" int mg_fwdprop_noalloc(int N, int L, int B, const int* lens, const int* shifts, const float* p, int ldp,
                                   const float* s, int lds, const void* u_in, void* u_out, int ldu, int crossing,
                                   void* stream) {
-  const size_t need = mg_workspace_bytes(MG_OP_FWD, N, L, B, crossing, MG_GEO_NN, nullptr);
+  size_t need = mg_workspace_bytes(MG_OP_FWD, N, L, B, crossing, MG_GEO_NN, nullptr);
+  // a framed launch's workspace is four times the plain one's (N = L = 600: 27 and 6 MB): the plain launch where it alone fits
+  const mg_config plain = {0, 0, 0, 0, 0, 0};
+  const mg_config* cfg = nullptr;
+  if (need > kNoAllocScratchBytes) {
+    cfg = &plain;
+    need = mg_workspace_bytes(MG_OP_FWD, N, L, B, crossing, MG_GEO_NN, cfg);
+  }
   if (need == 0) return MG_E_ARG;   // the argument error is already in mg_last_error()
   if (need > kNoAllocScratchBytes)
     return mg::set_last_error(MG_E_WORKSPACE,
@@ -67,6 +74,11 @@ extern "C" int mg_fwdprop_noalloc(int N, int L, int B, const int* lens, const in
   e = cudaMemsetAsync(scratch, 0, 256, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess)
     return mg::set_last_error(MG_E_CUDA, "mg_fwdprop_noalloc: clearing status: %s", cudaGetErrorString(e));
-  return mg_fwdprop(N, L, B, lens, shifts, p, ldp, s, lds, u_in, u_out, ldu, crossing, scratch, kNoAllocScratchBytes,
-                    stream);
+  if (!cfg)
+    return mg_fwdprop(N, L, B, lens, shifts, p, ldp, s, lds, u_in, u_out, ldu, crossing, scratch, kNoAllocScratchBytes,
+                      stream);
+  const int rc = mg_build_tiles(MG_OP_FWD, N, L, MG_GEO_NN, lens, shifts, nullptr, crossing, p, ldp, s, lds, nullptr, nullptr,
+                                nullptr, B, cfg, scratch, kNoAllocScratchBytes, stream);
+  return rc != MG_OK ? rc : mg_propagate(MG_OP_FWD, N, L, B, crossing, MG_GEO_NN, u_in, nullptr, u_out, nullptr, ldu, nullptr,
+                                         0, 0, cfg, scratch, kNoAllocScratchBytes, stream);
 }
