@@ -301,6 +301,10 @@ int mg_propagate_l2(int N, int L, int B, int crossing, int geometry, const void*
                     void* g_out, int ldu, float* dp, int ldp, int accumulate, const mg_config* cfg, void* workspace,
                     size_t workspace_bytes, void* stream);
 
+/* J = sum |y - t|^2 over n floats (the parts of complex fields) into the device float *out; scratch: up to scratch_doubles
+ * device doubles, one per CTA (none: one cluster of CTAs). */
+int mg_l2_loss(const float* y, const float* t, size_t n, float* out, double* scratch, int scratch_doubles, void* stream);
+
 /* ---- serving: native continuous-batching scheduler over resident meshes ------------------------
  * The meshes' tiles are built beforehand (mg_build_tiles, W = 8 persistent configuration of their kernel
  * class, both ops) and stay resident.  A scheduler thread owned by the server packs queued requests

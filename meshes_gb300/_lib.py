@@ -133,6 +133,7 @@ _SIGS = {
     # mesh and item arrays live in device memory: passed as raw addresses
     "mg_batched_propagate": (c_int, [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_size_t, c_void_p,
                                      c_void_p]),
+    "mg_l2_loss": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p, c_void_p, c_int, c_void_p]),
     "mg_batched_reduce": (c_int, [c_void_p, c_int, c_void_p]),
     "mg_batched_framed_desc": (c_int, [c_int, c_int, c_int, c_int, c_int, POINTER(mg_config), c_void_p, c_size_t,
                                        POINTER(mg_batch_framed), POINTER(mg_batch_framed), POINTER(c_size_t),

@@ -117,6 +117,9 @@ def _forward_y(mesh: MeshNetworkGPU, x: torch.Tensor, p: torch.Tensor):
     return y, (ver if shared else None)
 
 
+LOSS_CTAS = 304                # partial sums of mg_l2_loss: two CTAs per SM
+
+
 class MeshL2Function(torch.autograd.Function):
     """J = sum_b ||U(p) x_b - t_b||^2 for a lossless mesh.  The backward pass forms dJ/dy* = 2 (y - t)
     inside the back-propagation kernel (mg_propagate_l2) instead of in separate elementwise passes, the
@@ -129,8 +132,11 @@ class MeshL2Function(torch.autograd.Function):
         p = p.detach().to(torch.float32).contiguous()
         assert t.shape == x.shape, "target must have the shape of x"
         y, ver = _forward_y(mesh, x, p)
-        d = y - t
-        J = (torch.view_as_real(d) if d.is_complex() else d).square().sum()
+        J = torch.empty((), dtype=torch.float32, device=y.device)
+        n = y.numel() * (2 if y.is_complex() else 1)
+        scratch = torch.empty(LOSS_CTAS, dtype=torch.float64, device=y.device)
+        check(load().mg_l2_loss(y.data_ptr(), t.data_ptr(), n, J.data_ptr(), scratch.data_ptr(), LOSS_CTAS,
+                                _stream(y.device)), "mg_l2_loss")
         ctx.mesh, ctx.tiles_version = mesh, ver
         ctx.save_for_backward(y, p, t)
         return J
