@@ -735,7 +735,7 @@ def run_step(args, rank, world, local_rank):
         print(json.dumps({"profile_bwd_config": args.bwd_config, "status": lib.mg_read_status(ws_c.data_ptr(), 0, st)}))
         return None
     if args.profile:
-        # one warm-up step and one profiled step, no timing (for ncu captures: -s 2 -c 2 on prop_kernel)
+        # one warm-up step and one profiled step, no timing (for ncu captures: -s 2 -c 2 on framed_kernel)
         step(x, yt)
         step(x, yt)
         torch.cuda.synchronize(dev)
@@ -876,14 +876,14 @@ def run_step(args, rank, world, local_rank):
     units = n_mzi * B * world
     value = units / t_max
     bwd_flops = n_mzi * B * FLOP_BWD
-    traffic = traffic_from_profiles("prop_bwd_clements_N256_L256_B4096.md")
+    traffic = traffic_from_profiles("framed_clements_N256_L256_B4096.md")
     bwd_bytes = B * N * 3 * 8 + n_mzi * 4 * (2 + 2) + n_mzi * 4 * 2
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             hbm_peak, hbm_src = float(json.load(f)["hbm_gbs"]), "measured (copy bandwidth)"
     except (OSError, KeyError, ValueError):
         hbm_peak, hbm_src = 6800.0, "fallback"
-    roof = roofline_fp32(bwd_flops / t_bwd, peak, "prop_kernel<BWD> (back-propagation)")
+    roof = roofline_fp32(bwd_flops / t_bwd, peak, "framed_kernel<BWD> (back-propagation)")
     roof.update(traffic=traffic, algorithmic_flops_per_launch=bwd_flops)
     step_flops = value / world * (FLOP_FWD + FLOP_BWD)
     line = {
@@ -907,7 +907,7 @@ def run_step(args, rank, world, local_rank):
         "roofline": roof,
         # the same kernel against the HBM roofline (algorithmic bytes: read y and g, write g_in, the
         # parameters and dJ/dp), showing how far it is from being memory-bound
-        "roofline_hbm": {"kernel": "prop_kernel<BWD> (back-propagation)", "bound": "hbm",
+        "roofline_hbm": {"kernel": "framed_kernel<BWD> (back-propagation)", "bound": "hbm",
                          "achieved": bwd_bytes / t_bwd / 1e9, "peak": hbm_peak, "unit": "GB/s",
                          "frac": bwd_bytes / t_bwd / 1e9 / hbm_peak, "traffic": traffic,
                          "peak_source": hbm_src, "algorithmic_bytes_per_launch": bwd_bytes},
