@@ -496,8 +496,8 @@ CoefArgs coef_args(const Plan& P, const int* lens, const int* shifts, const int*
   return a;
 }
 
-// MZI crossings without derivative tiles take the float-float quad form of the coefficient pass
-bool quad_coef(const Plan& P) { return P.crossing == CR_MZI && (P.op == OP_FWD || (P.op == OP_BWD && P.gr == 1)); }
+// MZI crossings take the float-float quad form of the coefficient pass
+bool quad_coef(const Plan& P) { return P.crossing == CR_MZI && (P.op != OP_BWD || P.gr == 1); }
 
 int build_tiles(const Plan& P, const int* lens, const int* shifts, const int* strides, const float* p, int ldp,
                 const float* s, int lds, const float* dp, const void* Tgen, const void* Dgen, unsigned char* ws,
@@ -506,7 +506,7 @@ int build_tiles(const Plan& P, const int* lens, const int* shifts, const int* st
   if (P.geometry == GEO_NN && (!lens || !shifts)) return fail(MG_E_ARG, "lens/shifts are NULL");
   if (P.geometry == GEO_FFT && !strides) return fail(MG_E_ARG, "strides is NULL");
   const CoefArgs a = coef_args(P, lens, shifts, strides, p, ldp, s, lds, dp, Tgen, Dgen, ws);
-  // MZI crossings without derivative tiles (forward, and back-propagation with direct gradients) take the
+  // MZI crossings (without dT/dp tiles) take the
   // float-float path with a quad of lanes per slot: the four sin/cos chains of a slot run side by side.  Measured
   // on GB300 (ncu, N=64, L=64) one thread per slot spent ~8500 cycles per warp on a 1550-instruction chain; the
   // pass is latency-bound for small meshes, so it is spread over every SM in blocks of 32 to 256 threads.

@@ -83,12 +83,11 @@ __device__ __forceinline__ void slot_T(const CoefArgs& a, int l, int q, bool act
     D1 = c2x2_zero();
   }
   if (a.crossing == CR_MZI) {
-    // T alone (and the splitter pair of the direct gradient) in float-float on the FP32 pipe; with derivative
-    // tiles, or angles beyond the float-float range, the double-precision form
+    // (stored activations; every other MZI tile takes the quad form) T in float-float on the FP32 pipe; for angles beyond its
+    // range the double-precision form
     const float al = ss ? ss[0] : 0.f, be = ss ? ss[1] : 0.f;
-    if (need_d ||
-        !mzi_T_ff(pp[0], pp[1], al, be, &F, csb)) {
-      mzi_T(pp[0], pp[1], al, be, &T, need_d ? &D0 : nullptr, need_d ? &D1 : nullptr, csb);
+    if (!mzi_T_ff(pp[0], pp[1], al, be, &F, csb)) {
+      mzi_T(pp[0], pp[1], al, be, &T, nullptr, nullptr, csb);
       tff_from(T, &F);
     } else {
       tff_round(F, &T);
@@ -176,7 +175,7 @@ __device__ __forceinline__ void write_layer(const CoefArgs& a, int l, int kind) 
   a.kinds[a.L + 2 * l + 1] = ln;
 }
 
-// Lane t & 3 of the quad of lanes that does slot t / 4: MZI crossings without derivative tiles.  Quads leave at the bounds
+// Lane t & 3 of the quad of lanes that does slot t / 4: MZI crossings.  Quads leave at the bounds
 // check whole; lane k computes and writes entry k.
 template <bool FRAME>
 __device__ __forceinline__ void coef_quad(const CoefArgs& a, int t) {
@@ -186,21 +185,30 @@ __device__ __forceinline__ void coef_quad(const CoefArgs& a, int t) {
   bool active = false;
   const int kind = layer_kind(a, l, q, &active);
   if (q == 0 && k == 0) write_layer(a, l, kind);
-  const bool bwd = a.op == OP_BWD;   // (direct gradients)
+  const bool bwd = a.op == OP_BWD, diff = a.op == OP_FWDDIFF;   // bwd: direct gradients
   float2 cs = make_float2(0.f, 0.f);   // (cos, sin)(pi/4 + beta) for the direct gradient; 0 if inactive
   ffz z = {ff{k == 0 || k == 3 ? 1.f : 0.f, 0.f}, ff{0.f, 0.f}};
-  float2 v = make_float2(z.x.h, 0.f);
+  float2 v = make_float2(z.x.h, 0.f), dv = make_float2(0.f, 0.f);
   if (active) {
     const float* pp = a.p + (size_t)l * a.ldp + 2 * (size_t)q;
     const float* ss = a.s ? a.s + (size_t)l * a.lds + 2 * (size_t)q : nullptr;
     const float al = ss ? ss[0] : 0.f, be = ss ? ss[1] : 0.f;
-    if (mzi_T_ff_quad(pp[0], pp[1], al, be, ss == nullptr, &z, bwd ? &cs : nullptr)) {
+    float2 d0 = make_float2(0.f, 0.f);   // the entry of dT/dth; that of dT/dph is i times T's first column
+    ffz dth;
+    if (mzi_T_ff_quad(pp[0], pp[1], al, be, ss == nullptr, &z, bwd ? &cs : nullptr, diff ? &dth : nullptr)) {
       v = ffz_round(z);
+      if (diff) d0 = ffz_round(dth);
     } else {   // angles beyond the float-float range
-      C2x2 T;
-      mzi_T(pp[0], pp[1], al, be, &T, nullptr, nullptr, bwd ? &cs : nullptr);
-      v = k == 0 ? T.t00 : k == 1 ? T.t01 : k == 2 ? T.t10 : T.t11;
+      C2x2 T, D0, D1;
+      mzi_T(pp[0], pp[1], al, be, &T, diff ? &D0 : nullptr, diff ? &D1 : nullptr, bwd ? &cs : nullptr);
+      auto entry = [&](const C2x2& c) { return k == 0 ? c.t00 : k == 1 ? c.t01 : k == 2 ? c.t10 : c.t11; };
+      v = entry(T);
+      if (diff) d0 = entry(D0);
       z = {ff{v.x, 0.f}, ff{v.y, 0.f}};
+    }
+    if (diff && a.dp) {
+      const float* d = a.dp + (size_t)l * a.ldp + 2 * (size_t)q;
+      dv = cadd(cscale(d[0], d0), cscale(d[1], k & 1 ? make_float2(0.f, 0.f) : make_float2(-v.y, v.x)));
     }
   }
   if constexpr (FRAME) {
@@ -213,7 +221,9 @@ __device__ __forceinline__ void coef_quad(const CoefArgs& a, int t) {
   if (kind < KIND_XL) {
     const int j = q / (M / 2), e = q % (M / 2);
     if (bwd && k == 0) tl[2 * M * G + e * G + j] = cs;
-    tl[2 * ((2 * e + (k >> 1)) * G + j) + (k & 1)] = v;
+    const int at = 2 * ((2 * e + (k >> 1)) * G + j) + (k & 1);
+    tl[at] = v;
+    if (diff) tl[2 * M * G + at] = dv;
   } else {
     // butterfly over lanes: own rows of T, a -> (t00, t01), b -> (t11, t10); back-propagation: of T^H, a -> (conj t00,
     // conj t10), b -> (conj t11, conj t01)
@@ -221,7 +231,9 @@ __device__ __forceinline__ void coef_quad(const CoefArgs& a, int t) {
     const int A = 2 * st * (q / st) + (q % st), row = bwd ? k & 1 : k >> 1, m = row ? A + st : A;
     const int la = A / M, ma = A % M;
     if (bwd && k == 0) tl[2 * M * G + ma * (G / 2) + a_lane_index(la, st / M)] = cs;
-    tl[2 * ((m % M) * G + m / M) + (k == 0 || k == 3 ? 0 : 1)] = bwd ? make_float2(v.x, -v.y) : v;
+    const int at = 2 * ((m % M) * G + m / M) + (k == 0 || k == 3 ? 0 : 1);
+    tl[at] = bwd ? make_float2(v.x, -v.y) : v;
+    if (diff) tl[2 * M * G + at] = dv;
   }
 }
 

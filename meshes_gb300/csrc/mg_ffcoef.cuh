@@ -138,23 +138,6 @@ __device__ __forceinline__ void mzi_T_ff_from(ff S, ff C, ff Sph, ff Cph, ff sa,
   T->t[3] = ffz_mul(E0, A11);
 }
 
-// The same for ideal splitters (alpha = beta = 0: cos = 1, sin = 0), without the splitter products.  Each entry is
-// the value mzi_T_ff_from computes for those angles, its operations reduced to the ones that are not exact
-// multiplications by 1 or additions of 0.
-__device__ __forceinline__ void mzi_T_ff_ideal(ff S, ff C, ff Sph, ff Cph, Tff* T, float2* csb) {
-  if (csb) {
-    const float r = 0.707106769f;   // (1/sqrt 2)(cos 0 -+ sin 0), rounded
-    *csb = make_float2(r, r);
-  }
-  const ffz E1 = ffz_mul(ffz{C, S}, ffz{Cph, Sph});        // e^{i(th/2 + ph)}
-  const ff E1yS = ff_mul(E1.y, S), E1xS = ff_mul(E1.x, S), E1yC = ff_mul(E1.y, C), E1xC = ff_mul(E1.x, C);
-  const ff SC = ff_mul(S, C), CC = ff_mul(C, C), SS = ff_mul(S, S), CS = ff_mul(C, S);
-  T->t[0] = {ff_neg(E1yS), E1xS};   // e^{i(th/2+ph)} (i S)
-  T->t[1] = {ff_neg(SC), CC};       // e^{i th/2} (i C)
-  T->t[2] = {ff_neg(E1yC), E1xC};   // e^{i(th/2+ph)} (i C)
-  T->t[3] = {SS, ff_neg(CS)};       // e^{i th/2} (-i S)
-}
-
 // mzi_T_ff_from on the angles of one thread; false (nothing written) when an angle is outside the float-float
 // range, and the caller takes the double path.
 __device__ __forceinline__ bool mzi_T_ff(float th, float ph, float al, float be, Tff* T, float2* csb) {
@@ -168,12 +151,17 @@ __device__ __forceinline__ bool mzi_T_ff(float th, float ph, float al, float be,
 
 // The same over the four lanes of a quad (lanes 4k..4k+3 of a warp, all given the same angles and all calling it): lane k
 // takes the sin/cos of angle k (th/2, ph, alpha, beta), the quad exchanges them by shuffles, and lane k combines them into
-// entry k (00, 01, 10, 11) of T, which it returns; csb on every lane.  The entries are those of mzi_T_ff_from and
-// mzi_T_ff_ideal, operation by operation.  (All four entries on every lane: 45.6 us for a 600-mode, 600-layer mesh, 11.8 us
-// for 256; one each: 20.0 and 5.9 us, GB300.)  false on every lane of the quad when any angle is out of range.
-// ideal (uniform over the launch): no splitter array, alpha = beta = 0, and the lanes 2 and 3 of the quad idle.
+// entry k (00, 01, 10, 11) of T, which it returns; csb on every lane.  The entries are those of mzi_T_ff_from,
+// operation by operation.  (All four entries on every lane: 45.6 us for a 600-mode, 600-layer mesh, 11.8 us for 256; one each:
+// 20.0 and 5.9 us, GB300; with the derivatives, for 130 modes and layers, 4.0 us, in double precision by one thread
+// per slot 8.1.)  false on every lane of the quad when any angle is out of range.
+// ideal (uniform over the launch): no splitter array, alpha = beta = 0 (cos = 1, sin = 0) without the splitter products; each entry
+// is the value of the general form, its operations reduced to those that are not exact.
+// dth: receives the entry of dT/dth.  With e = e^{i th/2}, E = e or e e^{i ph} (entries 01, 11 and 00, 10), a sum behind each:
+//   00: i/2 (cos(alpha-beta) - sin(alpha+beta)) E e     01: -1/2 (cos(alpha+beta) + sin(alpha-beta)) E e
+//   10: 1/2 (sin(alpha-beta) - cos(alpha+beta)) E e     11: -i/2 (cos(alpha-beta) + sin(alpha+beta)) E e
 __device__ __forceinline__ ff ff_sel(bool p, ff a, ff b) { return ff{p ? a.h : b.h, p ? a.l : b.l}; }
-__device__ __forceinline__ bool mzi_T_ff_quad(float th, float ph, float al, float be, bool ideal, ffz* entry, float2* csb) {
+__device__ __forceinline__ bool mzi_T_ff_quad(float th, float ph, float al, float be, bool ideal, ffz* entry, float2* csb, ffz* dth) {
   const int lane = threadIdx.x & 31, base = lane & ~3, sub = lane & 3;
   const unsigned qmask = 0xFu << base;
   const float x = sub == 0 ? 0.5f * th : (sub == 1 ? ph : (sub == 2 ? al : be));
@@ -187,7 +175,17 @@ __device__ __forceinline__ bool mzi_T_ff_quad(float th, float ph, float al, floa
   const bool diag = sub == 0 || sub == 3;                  // entries 00, 11
   const ffz E0 = {C, S}, E1 = ffz_mul(E0, ffz{Cph, Sph});  // e^{i th/2} (entries 01, 11), e^{i(th/2 + ph)} (00, 10)
   const ffz E = {ff_sel(sub & 1, E0.x, E1.x), ff_sel(sub & 1, E0.y, E1.y)};
+  // g (p sine, q cosine of the splitters' sum or difference) times E e, for dT/dth
+  auto derivative = [&](ff p, ff q) {
+    const ff a = ff_sel(sub == 2, p, q), b = ff_sel(sub == 2, q, p);
+    const ff g = ff_add(a, ff_sel(sub == 0 || sub == 2, ff_neg(b), b));
+    const float h = sub == 1 ? -0.5f : 0.5f;
+    const ffz w = ffz_mul(E, E0);
+    const ff x = ff_mul(ff{h * g.h, h * g.l}, w.x), y = ff_mul(ff{h * g.h, h * g.l}, w.y);
+    *dth = sub == 0 ? ffz{ff_neg(y), x} : sub == 3 ? ffz{y, ff_neg(x)} : ffz{x, y};
+  };
   if (ideal) {
+    if (dth) derivative(ff{0.f, 0.f}, ff{1.f, 0.f});
     if (csb) {
       const float r = 0.707106769f;   // (1/sqrt 2)(cos 0 -+ sin 0), rounded
       *csb = make_float2(r, r);
@@ -206,6 +204,7 @@ __device__ __forceinline__ bool mzi_T_ff_quad(float th, float ph, float al, floa
   const ff casb = ff_mul(ca, sb), sasb = ff_mul(sa, sb);
   const ff p = ff_add(ff_mul(sa, cb), ff_sel(diag, casb, ff_neg(casb)));
   const ff q = ff_add(ff_mul(ca, cb), ff_sel(diag, sasb, ff_neg(sasb)));
+  if (dth) derivative(p, q);
   const ff u = ff_mul(ff_sel(diag, C, S), p), v = ff_mul(ff_sel(diag, S, C), q);
   const ffz A = {sub == 2 ? u : ff_neg(u), sub == 3 ? ff_neg(v) : v};
   *entry = ffz_mul(E, A);
