@@ -44,6 +44,11 @@ extern "C" {
 /* OR-ed into a geometry: the mesh has permutations between layers (mg_build_perms).  Plans made with
  * it reserve the permutation tables in the workspace and a gather scratch in shared memory. */
 #define MG_GEO_PERM 4
+/* OR-ed into a geometry, in every call on a workspace alike: its tiles serve calls of exactly this B.  Without it, and
+ * without a configuration, mg_build_tiles writes the tiles of every launch that some batch takes (nearest-neighbour complex
+ * meshes of 33 to 128 modes: two sets; MZI meshes above 64 modes: framed tiles too); with it only those of the
+ * launch of B, which is what a caller wants that builds for each batch. */
+#define MG_GEO_ONE_BATCH 8
 
 /* return codes */
 #define MG_OK 0
@@ -167,8 +172,10 @@ int mg_fwdprop_noalloc(int N, int L, int B, const int* lens, const int* shifts, 
 /* ---- programmed-mesh entry points (coefficients kept resident between calls) -----------------
  * mg_build_tiles runs only the coefficient precompute of `op` into the workspace; mg_propagate runs
  * only the propagation kernel on tiles built earlier with the same (op, N, L, crossing, geometry,
- * cfg).  Used by the autograd function, the batched engine and the server, which re-use one set of
- * tiles across many batches.  Tgen/Dgen (crossing MG_GENERIC) give T per slot as 4 complex64
+ * cfg), for any B whose mg_workspace_bytes the workspace holds: B enters neither what a build writes nor where (with
+ * MG_GEO_ONE_BATCH it does, and B has to be the same too).  The batched engine and the server re-use one set of
+ * tiles across many batches.  Tuned entries (mg_set_tuned) apply to such calls where their tiles are among those
+ * built.  Tgen/Dgen (crossing MG_GENERIC) give T per slot as 4 complex64
  * (t00, t01, t10, t11) and, for op MG_OP_BWD, dT/dp0 and dT/dp1 (8 complex64). */
 int mg_build_tiles(int op, int N, int L, int geometry, const int* lens, const int* shifts, const int* strides,
                    int crossing, const float* p, int ldp, const float* s, int lds, const float* dp, const void* Tgen,
@@ -350,8 +357,8 @@ void mg_server_destroy(mg_server* s, int drain);
  * which is exact only for unitary crossings; for lossy ones (crossing.py:444-508, gains g_ij) that
  * gradient is wrong.  These calls back-propagate from stored layer inputs instead, for checkpointed
  * adjoints that keep one input every ~sqrt(L) layers and recompute the rest segment by segment.
- * Both run layers [l0, l1) of tiles built earlier by mg_build_tiles for the same (N, L, B, crossing,
- * geometry, cfg): op MG_OP_FWD with tiles of MG_OP_FWD, op MG_OP_BWD_STORED with tiles of
+ * Both run layers [l0, l1) of tiles built earlier by mg_build_tiles for the same (N, L, crossing,
+ * geometry, cfg; B as for mg_propagate): op MG_OP_FWD with tiles of MG_OP_FWD, op MG_OP_BWD_STORED with tiles of
  * MG_OP_BWD_STORED (complex crossings only; MG_GENERIC takes T per slot from Tgen and needs no Dgen).
  *   MG_OP_FWD:        in0 = input of layer l0, out0 = output of layer l1-1 (may be NULL); when act is
  *                     not NULL the input of every layer l of the range is also written to

@@ -20,7 +20,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import GEO_NN, OP_BWD, OP_FWD, OP_FWD_BWDTILES, check, load
+from ._lib import GEO_NN, GEO_ONE_BATCH, OP_BWD, OP_FWD, OP_FWD_BWDTILES, check, load
 from .mesh import MeshNetworkGPU, Workspace, _stream
 
 
@@ -33,8 +33,13 @@ class _Plan(Workspace):
 
     def size(self, B: int):
         m = self.mesh
-        return lambda: load().mg_workspace_bytes(self.op, m.N, m.L, B, m.crossing, m.geo_code,
+        return lambda: load().mg_workspace_bytes(self.op, m.N, m.L, B, m.crossing, _geo(m),
                                                  _lib.cfg_ptr(m.config.get(self.op)))
+
+
+def _geo(mesh: MeshNetworkGPU) -> int:
+    """Geometry code: every forward pass builds its tiles, for its own batch."""
+    return mesh.geo_code | GEO_ONE_BATCH
 
 
 def _plans(mesh: MeshNetworkGPU):
@@ -55,12 +60,12 @@ def _build(mesh: MeshNetworkGPU, op: int, p: torch.Tensor, B: int):
     cfg, stream = _lib.cfg_ptr(mesh.config.get(op)), _stream(mesh.device)
     plan_.version += 1                       # whatever happens below, the tiles of earlier calls are gone
     check(plan_.call(plan_.size(B), lambda ws, nb: lib.mg_build_tiles(
-        op, mesh.N, mesh.L, mesh.geo_code, *geo, mesh.crossing, p.data_ptr(), mesh.N // 2 * mesh.X_np,
+        op, mesh.N, mesh.L, _geo(mesh), *geo, mesh.crossing, p.data_ptr(), mesh.N // 2 * mesh.X_np,
         s.data_ptr() if s.numel() else None, mesh.N // 2 * mesh.X_ns, None, None, None, B, cfg, ws, nb, stream)),
         "mg_build_tiles")
     ws, nb = plan_.buf.data_ptr(), plan_.buf.numel()
     if mesh.perm_table is not None:
-        check(lib.mg_build_perms(op, mesh.N, mesh.L, B, mesh.crossing, mesh.geo_code, mesh.perm_table.data_ptr(), cfg, ws,
+        check(lib.mg_build_perms(op, mesh.N, mesh.L, B, mesh.crossing, _geo(mesh), mesh.perm_table.data_ptr(), cfg, ws,
                                  nb, stream), "mg_build_perms")
     return ws, nb, plan_.version
 
@@ -93,7 +98,7 @@ class MeshFunction(torch.autograd.Function):
             ws, nb, _ = _build(mesh, OP_BWD, p, B)
         gx = torch.empty_like(gy)
         dp = torch.empty(p.numel(), dtype=torch.float32, device=y.device)
-        check(lib.mg_propagate(OP_BWD, N, mesh.L, B, mesh.crossing, mesh.geo_code, y.data_ptr(), gy.data_ptr(), None,
+        check(lib.mg_propagate(OP_BWD, N, mesh.L, B, mesh.crossing, _geo(mesh), y.data_ptr(), gy.data_ptr(), None,
                                gx.data_ptr(), N, dp.data_ptr(), N // 2 * mesh.X_np, 0,
                                _lib.cfg_ptr(mesh.config.get(OP_BWD)), ws, nb, _stream(mesh.device)), "mg_propagate")
         return gx, dp.view_as(p), None
@@ -112,7 +117,7 @@ def _forward_y(mesh: MeshNetworkGPU, x: torch.Tensor, p: torch.Tensor):
     else:
         ws, nb, ver = _build(mesh, OP_FWD, p, B)
         op, cfg = OP_FWD, mesh.config.get(OP_FWD)
-    check(lib.mg_propagate(op, N, mesh.L, B, mesh.crossing, mesh.geo_code, x.data_ptr(), None, y.data_ptr(),
+    check(lib.mg_propagate(op, N, mesh.L, B, mesh.crossing, _geo(mesh), x.data_ptr(), None, y.data_ptr(),
                            None, N, None, 0, 0, _lib.cfg_ptr(cfg), ws, nb, _stream(mesh.device)), "mg_propagate")
     return y, (ver if shared else None)
 
@@ -154,7 +159,7 @@ class MeshL2Function(torch.autograd.Function):
             ws, nb, _ = _build(mesh, OP_BWD, p, B)
         gx = torch.empty_like(y)
         dp = torch.empty(p.numel(), dtype=torch.float32, device=y.device)
-        check(lib.mg_propagate_l2(N, mesh.L, B, mesh.crossing, mesh.geo_code, y.data_ptr(), t.data_ptr(), None,
+        check(lib.mg_propagate_l2(N, mesh.L, B, mesh.crossing, _geo(mesh), y.data_ptr(), t.data_ptr(), None,
                                   gx.data_ptr(), N, dp.data_ptr(), N // 2 * mesh.X_np, 0,
                                   _lib.cfg_ptr(mesh.config.get(OP_BWD)), ws, nb, _stream(mesh.device)),
               "mg_propagate_l2")

@@ -125,6 +125,12 @@ struct Plan {
   size_t fft_smem;
   bool perm;        // MG_GEO_PERM: permutation tables at off_perm, gather scratch after the smem layout
   size_t off_perm;
+  bool may_frame;   // the mesh has framed tiles where they are asked for
+  bool tuned;       // from the tuning table
+  bool resident;    // the build serves every batch: all tiles that the launch of some batch reads (place)
+  int n_lay;        // tiles of the build: modes per lane and place of each
+  int lay_M[2];
+  size_t lay_tiles[2];
 };
 
 // Permutation tables in the workspace: forward rows [L+1][N], back-propagation rows [L+1][N], forward
@@ -216,9 +222,13 @@ mg_config vectors_pick(int M, int B, int sms) {
   return best;
 }
 
+constexpr int kNoTuned = 1;   // how a launch without a configuration is planned: by the heuristic alone,
+constexpr int kUniform = 2;   // uniform CTAs on plain tiles (layer ranges)
+
+// The launch of a plan, without its places in the workspace.
 // op MG_OP_BWD_STORED plans the back-propagation kernel in its stored-activation mode (GR 4): T tiles
 // only, 32-byte dJ/dT staging per slot, raw partials of 4 complex per slot.
-int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_config* cfg, Plan* P) {
+int plan_launch(int op, int N, int L, int B, int crossing, int geometry, const mg_config* cfg, int how, Plan* P) {
   const bool stored = op == MG_OP_BWD_STORED;
   if (stored) {
     if (crossing == CR_ORTH) return fail(MG_E_ARG, "stored-activation back-propagation needs a complex crossing");
@@ -241,8 +251,9 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   const DevInfo di = dev_info();
   mg_config tuned;
   // tuned entries were measured without the permutation scratch: permuted meshes take the defaults
-  if (!cfg && !perm && lookup_tuned(op, crossing, geometry, N, B, &tuned)) cfg = &tuned;
   Plan& p = *P;
+  p.tuned = !cfg && !perm && !stored && !how && lookup_tuned(op, crossing, geometry, N, B, &tuned);
+  if (p.tuned) cfg = &tuned;
   p.op = op; p.N = N; p.L = L; p.B = B; p.crossing = crossing; p.geometry = geometry;
   p.perm = perm;
   p.real = crossing == CR_ORTH;
@@ -272,10 +283,12 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   // back-propagation with direct gradients
   const bool may_frame = !stored && !perm && geometry == GEO_NN && N > 64 && L > 0 && L <= kMaxSmemKinds &&
                          (crossing == CR_MZI ? op != OP_FWDDIFF : crossing == CR_SYM && op == OP_FWD);
+  p.may_frame = may_frame;
   mg_config fc;
-  if (!cfg && may_frame && framed_pays(op, Np / 32, L, Np / 2, B, di.sms) && framed_pick(op, Np / 32, B, di.sms, &fc)) cfg = &fc;
+  if (!cfg && !(how & kUniform) && may_frame && framed_pays(op, Np / 32, L, Np / 2, B, di.sms) && framed_pick(op, Np / 32, B, di.sms, &fc)) cfg = &fc;
+  // (a configuration without modes per lane leaves them where they were, whatever the batch)
   int small_v = 0;
-  if (!(cfg && (cfg->M || cfg->V)) && geometry == GEO_NN && !perm && !wide && N > 32 && crossing != CR_ORTH &&
+  if (!(cfg && (cfg->M || cfg->V || N <= 128)) && geometry == GEO_NN && !perm && !wide && N > 32 && crossing != CR_ORTH &&
       (op == OP_FWD || (op == OP_BWD && p.gr == 1)))
     small_v = small_batch_v(op, Np / 32, B, di.sms);
   // stored activations, N <= 128: the default tile's lane groups (R = 32 / G per warp) as a warp each, a vector over all
@@ -283,7 +296,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   // adds the R warps of a former warp pairwise first), so dJ/dT keeps its bits.  Measured on GB300 at N = 128, B = 1024:
   // the stored kernels of a step 352 -> 144 us, with one segment instead of eleven.
   p.tree = 1;
-  if (stored && !(cfg && (cfg->M || cfg->V || cfg->W)) && geometry == GEO_NN && !wide && N > 32 && N <= 128) {
+  if (stored && !cfg && geometry == GEO_NN && !wide && N > 32 && N <= 128) {
     const int R = 256 / Np, w = default_warps(B, R * 4, di.sms);
     if (R * w <= 8) {
       small_v = 4;
@@ -305,7 +318,7 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
   }
   if (perm && stored) return fail(MG_E_ARG, "stored-activation back-propagation takes no permutations");
   // warp-pair launch (split 3): back-propagation of a nearest-neighbour complex mesh with a full-warp M = 8 plan
-  const int split_mode = cfg ? cfg->split : 0;
+  const int split_mode = cfg ? cfg->split : how & kUniform ? 2 : 0;
   p.framed = split_mode == 5 || split_mode == 6;
   if (p.framed && !(may_frame && framed_instantiated(op, M, V, G == 32, split_mode == 6)))
     return fail(MG_E_CONFIG, "no framed kernel for op=%d crossing=%d geometry=%d M=%d G=%d V=%d", op, crossing, geometry,
@@ -412,31 +425,81 @@ int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_
     p.nA = (int)nA;
     p.grid = (int)(nA + (rem + capB - 1) / capB);
   }
-  p.off_kinds = 256;
-  p.off_tiles = p.off_kinds + align256((size_t)std::max(L, 1) * 12);   // kinds + (shift, len)
-  p.off_dtiles = p.off_tiles + align256((size_t)L * p.lb);
-  p.off_perm = p.off_dtiles + align256((size_t)L * p.dlb);
-  p.off_partial = p.off_perm + (perm ? align256(perm_table_bytes(N, L)) : 0);
   p.fft_smem = 0;
   p.fft_grid = (!chosen || split_mode == 7) && !perm && !stored && geometry == GEO_FFT
                    ? fft_ctas(op, p.gr, p.real, N, L, B, split_mode == 7, di, &p.fft_smem) : 0;
   p.fft = p.fft_grid > 0;
-  p.total = p.off_partial + ((op == OP_BWD) ? align256((size_t)std::max(p.grid, p.fft_grid) * L * p.np2 * (p.gr == 4 ? 32 : 8)) : 0);
-  if (p.framed) {
-    const size_t n = (size_t)L * p.np2;
-    const bool bwd = op == OP_BWD;
-    p.off_main = p.total;
-    p.off_resc = p.off_main + align256(n * (bwd ? 24 : 16));
-    p.off_wts = p.off_resc + align256(16 * n);
-    p.off_dfin = p.off_wts + (bwd ? align256(8 * n) : 0);
-    p.off_fkinds = p.off_dfin + align256(16 * (size_t)p.np2);
-    p.off_tdiag = p.off_fkinds + align256(4 * (size_t)L);
-    p.off_toff = p.off_tdiag + align256(32 * n);
-    p.off_tmag = p.off_toff + align256(32 * n);
-    p.off_tcs = p.off_tmag + align256(8 * n);
-    p.off_count = p.off_tcs + (bwd ? align256(8 * n) : 0);
-    p.total = p.off_count + 256;
+  return MG_OK;
+}
+
+// The places of the frame pass's tiles from `at` on; returns their end
+size_t place_frames(Plan* P, size_t at) {
+  Plan& p = *P;
+  const size_t n = (size_t)p.L * p.np2;
+  const bool bwd = p.op == OP_BWD;
+  p.off_main = at;
+  p.off_resc = p.off_main + align256(n * (bwd ? 24 : 16));
+  p.off_wts = p.off_resc + align256(16 * n);
+  p.off_dfin = p.off_wts + (bwd ? align256(8 * n) : 0);
+  p.off_fkinds = p.off_dfin + align256(16 * (size_t)p.np2);
+  p.off_tdiag = p.off_fkinds + align256(4 * (size_t)p.L);
+  p.off_toff = p.off_tdiag + align256(32 * n);
+  p.off_tmag = p.off_toff + align256(32 * n);
+  p.off_tcs = p.off_tmag + align256(8 * n);
+  p.off_count = p.off_tcs + (bwd ? align256(8 * n) : 0);
+  return p.off_count + 256;
+}
+
+// Nearest-neighbour complex meshes of 33 to 128 modes: modes per lane go by the batch (small_batch_v, framed_pays), the
+// whole warp's (2, 4) or 8
+bool two_layouts(const Plan& p) {
+  return p.geometry == GEO_NN && !p.perm && !p.real && p.N > 32 && p.N <= 128 &&
+         (p.op == OP_FWD || (p.op == OP_BWD && (p.gr == 1 || p.gr == 4)));
+}
+
+// The workspace: status, kinds, tiles (and frames), permutation tables, partials.  Tiles of a resident plan are those of
+// every launch that some batch takes, at places that the batch does not enter, so that one build serves them all: the
+// whole warp's modes per lane, with frames where the mesh may have them, and 8 modes per lane where small meshes take
+// those.
+void place(Plan* P) {
+  Plan& p = *P;
+  p.n_lay = 1;
+  p.lay_M[0] = p.M;
+  if (p.resident && two_layouts(p)) {
+    p.n_lay = 2;
+    p.lay_M[0] = pow2ceil(p.N) / 32;
+    p.lay_M[1] = 8;
   }
+  p.off_kinds = 256;
+  size_t at = p.off_kinds + align256((size_t)std::max(p.L, 1) * 12);   // kinds + (shift, len)
+  for (int k = 0; k < p.n_lay; ++k) {
+    p.lay_tiles[k] = at;
+    if (p.lay_M[k] == p.M) p.off_tiles = at;
+    at += align256((size_t)p.L * p.lb);
+    p.off_dtiles = at;
+    at += align256((size_t)p.L * p.dlb);
+    if (k == 0 && (p.resident ? p.may_frame : p.framed)) at = place_frames(&p, at);
+  }
+  p.off_perm = at;
+  p.off_partial = p.off_perm + (p.perm ? align256(perm_table_bytes(p.N, p.L)) : 0);
+  p.total = p.off_partial + ((p.op == OP_BWD) ? align256((size_t)std::max(p.grid, p.fft_grid) * p.L * p.np2 * (p.gr == 4 ? 32 : 8)) : 0);
+}
+
+// geometry | MG_GEO_ONE_BATCH: the tiles that the launch of B reads, and no others
+int make_plan(int op, int N, int L, int B, int crossing, int geometry, const mg_config* cfg, Plan* P, int how = 0) {
+  const bool once = geometry >= 0 && (geometry & MG_GEO_ONE_BATCH) != 0;
+  if (once) geometry &= ~MG_GEO_ONE_BATCH;
+  const int rc = plan_launch(op, N, L, B, crossing, geometry, cfg, how, P);
+  if (rc != MG_OK) return rc;
+  P->resident = !cfg && !once && !P->perm;
+  if (P->resident && P->tuned && !(two_layouts(*P) && (P->M == 8 || P->M == pow2ceil(N) / 32))) {
+    Plan h;   // a tuned launch whose tiles other batches do not take gives way to the heuristic's
+    const int rh = plan_launch(op, N, L, B, crossing, geometry, cfg, kNoTuned, &h);
+    if (rh != MG_OK) return rh;
+    if (h.M != P->M) *P = h;
+    P->resident = true;
+  }
+  place(P);
   return MG_OK;
 }
 
@@ -537,6 +600,21 @@ int build_tiles(const Plan& P, const int* lens, const int* shifts, const int* st
     e = launch_frames(f, sms, st);
   }
   return e == cudaSuccess ? MG_OK : cuda_fail(e, "coef_kernel launch");
+}
+
+// All tiles of the plan's build
+int build_all(const Plan& P, const int* lens, const int* shifts, const int* strides, const float* p, int ldp, const float* s,
+              int lds, const float* dp, const void* Tgen, const void* Dgen, unsigned char* ws, cudaStream_t st) {
+  for (int k = 0; k < P.n_lay; ++k) {
+    Plan q = P;
+    q.M = P.lay_M[k];
+    q.G = P.G * P.M / q.M;
+    q.off_tiles = P.lay_tiles[k];
+    q.framed = k == 0 && (P.resident ? P.may_frame : P.framed);
+    const int rc = build_tiles(q, lens, shifts, strides, p, ldp, s, lds, dp, Tgen, Dgen, ws, st);
+    if (rc != MG_OK) return rc;
+  }
+  return MG_OK;
 }
 
 // Forward plan Pf reads the tiles in back-propagation plan Pb's workspace: their layer strides, a stage that still fits
@@ -685,7 +763,7 @@ int fwdprop_impl(int geo, int N, int L, int B, const int* lens, const int* shift
                  size_t wsb, void* stream) {
   g_err.clear();
   Plan P;
-  TRY(make_plan(OP_FWD, N, L, B, crossing, geo, nullptr, &P));
+  TRY(make_plan(OP_FWD, N, L, B, crossing, geo | MG_GEO_ONE_BATCH, nullptr, &P));
   if (crossing == CR_GENERIC) return fail(MG_E_ARG, "use mg_build_tiles for generic crossings");
   TRY(check_ws(P, ws, wsb));
   TRY(check_ldu(P, ldu));
@@ -703,7 +781,7 @@ int fwddiff_impl(int geo, int N, int L, int B, const int* lens, const int* shift
                  void* du_out, int ldu, int crossing, void* ws, size_t wsb, void* stream) {
   g_err.clear();
   Plan P;
-  TRY(make_plan(OP_FWDDIFF, N, L, B, crossing, geo, nullptr, &P));
+  TRY(make_plan(OP_FWDDIFF, N, L, B, crossing, geo | MG_GEO_ONE_BATCH, nullptr, &P));
   if (crossing == CR_GENERIC) return fail(MG_E_ARG, "use mg_build_tiles for generic crossings");
   TRY(check_ws(P, ws, wsb));
   TRY(check_ldu(P, ldu));
@@ -723,7 +801,7 @@ int backdiff_impl(int geo, int N, int L, int B, const int* lens, const int* shif
                   void* dJdu_in, int ldu, int crossing, int accumulate, void* ws, size_t wsb, void* stream) {
   g_err.clear();
   Plan P;
-  TRY(make_plan(OP_BWD, N, L, B, crossing, geo, nullptr, &P));
+  TRY(make_plan(OP_BWD, N, L, B, crossing, geo | MG_GEO_ONE_BATCH, nullptr, &P));
   if (crossing == CR_GENERIC) return fail(MG_E_ARG, "use mg_build_tiles for generic crossings");
   TRY(check_ws(P, ws, wsb));
   TRY(check_ldu(P, ldu));
@@ -872,7 +950,10 @@ const char* mg_version(void) { return "meshes_gb300 0.1 (sm_103a)"; }
 size_t mg_workspace_bytes(int op, int N, int L, int B, int crossing, int geometry, const mg_config* cfg) {
   Plan P;
   if (make_plan(op, N, L, B, crossing, geometry, cfg, &P) != MG_OK) return 0;
-  return P.total;
+  if (!P.resident) return P.total;
+  Plan one;   // the reference-shaped entry points' calls, which build what they run
+  if (make_plan(op, N, L, B, crossing, geometry | MG_GEO_ONE_BATCH, cfg, &one) != MG_OK) return 0;
+  return std::max(P.total, one.total);
 }
 
 int mg_workspace_init(void* ws, size_t bytes, void* stream) {
@@ -900,7 +981,7 @@ int mg_read_status(void* ws, int clear, void* stream) {
 int mg_default_config(int op, int N, int B, int crossing, mg_config* out) {
   g_err.clear();
   Plan P;
-  TRY(make_plan(op, N, 1, B, crossing, GEO_NN, nullptr, &P));
+  TRY(make_plan(op, N, 1, B, crossing, GEO_NN | MG_GEO_ONE_BATCH, nullptr, &P));
   if (out) {
     out->M = P.M; out->V = P.V; out->W = P.W; out->CL = P.CL; out->S = P.S;
   }
@@ -957,7 +1038,7 @@ int mg_build_tiles(int op, int N, int L, int geometry, const int* lens, const in
                                     8 * (size_t)(L + 1), static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(permutation flags)");
   }
-  return build_tiles(P, lens, shifts, strides, p, ldp, s, lds, dp, Tgen, Dgen, static_cast<unsigned char*>(ws),
+  return build_all(P, lens, shifts, strides, p, ldp, s, lds, dp, Tgen, Dgen, static_cast<unsigned char*>(ws),
                      static_cast<cudaStream_t>(stream));
 }
 
@@ -1000,7 +1081,7 @@ int mg_propagate(int op, int N, int L, int B, int crossing, int geometry, const 
   if (op == MG_OP_FWD_BWDTILES) {
     // forward propagation reading the tiles mg_build_tiles(MG_OP_BWD) wrote: the layer stride and the
     // workspace layout are the back-propagation plan's, the kernel is the forward one
-    if ((geometry & ~MG_GEO_PERM) != GEO_NN)
+    if ((geometry & ~(MG_GEO_PERM | MG_GEO_ONE_BATCH)) != GEO_NN)
       return fail(MG_E_ARG, "forward from back-propagation tiles needs nearest-neighbour geometry");
     Plan Pb, Pf;
     TRY(make_plan(OP_BWD, N, L, B, crossing, geometry, cfg, &Pb));
@@ -1147,17 +1228,19 @@ int range_impl(int op, int N, int L, int l0, int l1, int B, int crossing, int ge
   const mg_config* given = cfg;
   mg_config cu = cfg ? *cfg : mg_config{0, 0, 0, 0, 0, 0};
   cu.split = 2;
-  cfg = &cu;
+  if (cfg) cfg = &cu;
   Plan P;
-  TRY(make_plan(op, N, L, B, crossing, geometry, cfg, &P));
-  {   // the tiles' modes per lane, where the whole-mesh launch takes others
+  TRY(make_plan(op, N, L, B, crossing, geometry, cfg, &P, kUniform));
+  if (!P.resident) {   // the tiles' modes per lane, where the whole-mesh launch takes others
     Plan built;
     if (make_plan(op, N, L, B, crossing, geometry, given, &built) == MG_OK && built.M != P.M) {
       cu.M = built.M;
+      cfg = &cu;
       TRY(make_plan(op, N, L, B, crossing, geometry, cfg, &P));
     }
     g_err.clear();
   }
+  geometry &= ~MG_GEO_ONE_BATCH;
   if (P.perm) return fail(MG_E_ARG, "layer ranges take no permutations");
   TRY(check_ws(P, ws, wsb));
   TRY(check_ldu(P, ldu));
@@ -1249,8 +1332,7 @@ int range_impl(int op, int N, int L, int l0, int l1, int B, int crossing, int ge
 // back-propagation left at its layers' places (range_impl with keep_partials): one reduction over all layers
 int reduce_raw(int N, int L, int B, int geometry, void* dT, int accumulate, void* ws, size_t wsb, void* stream) {
   Plan P;
-  mg_config cu{0, 0, 0, 0, 0, 2};
-  TRY(make_plan(MG_OP_BWD_STORED, N, L, B, CR_GENERIC, geometry, &cu, &P));
+  TRY(make_plan(MG_OP_BWD_STORED, N, L, B, CR_GENERIC, geometry, nullptr, &P, kUniform));
   TRY(check_ws(P, ws, wsb));
   if (!dT) return fail(MG_E_ARG, "dT is NULL");
   if (reinterpret_cast<uintptr_t>(dT) & 7) return fail(MG_E_ARG, "dT not 8-byte aligned");

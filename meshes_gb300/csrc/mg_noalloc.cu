@@ -52,7 +52,7 @@ cudaError_t scratch_address(void** out) {
 extern "C" int mg_fwdprop_noalloc(int N, int L, int B, const int* lens, const int* shifts, const float* p, int ldp,
                                   const float* s, int lds, const void* u_in, void* u_out, int ldu, int crossing,
                                   void* stream) {
-  size_t need = mg_workspace_bytes(MG_OP_FWD, N, L, B, crossing, MG_GEO_NN, nullptr);
+  size_t need = mg_workspace_bytes(MG_OP_FWD, N, L, B, crossing, MG_GEO_NN | MG_GEO_ONE_BATCH, nullptr);
   // a framed launch's workspace is four times the plain one's (N = L = 600: 27 and 6 MB): the plain launch where it alone fits
   const mg_config plain = {0, 0, 0, 0, 0, 0};
   const mg_config* cfg = nullptr;

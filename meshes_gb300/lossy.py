@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from . import geometry as geom
-from ._lib import GENERIC, GEO_FFT, GEO_NN, OP_BWD_STORED, OP_FWD, check, load
+from ._lib import GENERIC, GEO_FFT, GEO_NN, GEO_ONE_BATCH, OP_BWD_STORED, OP_FWD, check, load
 from .mesh import Workspace, _stream
 
 
@@ -119,6 +119,7 @@ class LossyMesh:
             active = np.zeros((self.L, N // 2), dtype=bool)
             for l, (ln, sh) in enumerate(zip(self.lens_h, self.shifts_h)):
                 active[l, sh // 2: sh // 2 + ln] = True
+        self._geometry = self.geometry | GEO_ONE_BATCH   # every pass builds its tiles, for its own batch
         self.active = torch.as_tensor(active, device=self.device)
         self._segment = int(segment) if segment else None
         self._ws = {}
@@ -153,15 +154,15 @@ class LossyMesh:
         if w is None:
             w = self._ws[op] = Workspace(self.device)
         stream = _stream(self.device)
-        check(w.call(lambda: load().mg_workspace_bytes(op, self.N, self.L, B, GENERIC, self.geometry, None),
-                     lambda ws, nb: load().mg_build_tiles(op, self.N, self.L, self.geometry, *self._geo(), GENERIC, None, 0,
+        check(w.call(lambda: load().mg_workspace_bytes(op, self.N, self.L, B, GENERIC, self._geometry, None),
+                     lambda ws, nb: load().mg_build_tiles(op, self.N, self.L, self._geometry, *self._geo(), GENERIC, None, 0,
                                                           None, 0, None, Tc.data_ptr(), None, B, None, ws, nb, stream)),
               "mg_build_tiles")
         return w.buf.data_ptr(), w.buf.numel()
 
     def _range(self, op, l0, l1, B, in0, in1, out0, out1, act, dT, ws, nb):
         ptr = (lambda t: None if t is None else t.data_ptr())
-        check(load().mg_propagate_range(op, self.N, self.L, l0, l1, B, GENERIC, self.geometry, ptr(in0), ptr(in1),
+        check(load().mg_propagate_range(op, self.N, self.L, l0, l1, B, GENERIC, self._geometry, ptr(in0), ptr(in1),
                                         ptr(out0), ptr(out1), self.N, ptr(act), ptr(dT), 0, None, ws, nb,
                                         _stream(self.device)), "mg_propagate_range")
 
@@ -201,7 +202,7 @@ class LossyMeshFunction(torch.autograd.Function):
         y = torch.empty_like(x)
         if B > 0:
             ws, nb = mesh._build(OP_FWD, Tc, B) if L > 0 else (None, 0)
-            check(load().mg_lossy_forward(mesh.N, L, B, mesh.geometry, seg, x.data_ptr(), y.data_ptr(),
+            check(load().mg_lossy_forward(mesh.N, L, B, mesh._geometry, seg, x.data_ptr(), y.data_ptr(),
                                           ckpt.data_ptr() if ckpt.numel() else None, mesh.N, ws, nb,
                                           _stream(mesh.device)), "mg_lossy_forward")
         ctx.mesh = mesh
@@ -223,7 +224,7 @@ class LossyMeshFunction(torch.autograd.Function):
             wsb, nbb = mesh._build(OP_BWD_STORED, Tc, B) if L > 0 else (None, 0)
             act = torch.empty((min(seg, max(L, 1)), B, N), dtype=torch.complex64, device=mesh.device)
             gtmp = torch.empty_like(gy)
-            check(load().mg_lossy_backward(N, L, B, mesh.geometry, seg, x.data_ptr(),
+            check(load().mg_lossy_backward(N, L, B, mesh._geometry, seg, x.data_ptr(),
                                            ckpt.data_ptr() if ckpt.numel() else None, gy.data_ptr(), g.data_ptr(),
                                            gtmp.data_ptr(), act.data_ptr(), dT.data_ptr(), N, wsf, nbf, wsb, nbb,
                                            _stream(mesh.device)), "mg_lossy_backward")

@@ -20,7 +20,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import GEO_FFT, GEO_NN, GEO_PERM, OP_BWD, OP_FWD, OP_FWDDIFF, check, load
+from ._lib import GEO_FFT, GEO_NN, GEO_ONE_BATCH, GEO_PERM, OP_BWD, OP_FWD, OP_FWDDIFF, check, load
 from . import geometry as geom
 
 _NP_NS = {"mzi": (2, 2), "sym": (2, 1), "orth": (1, 0)}   # gpu/mesh.py:72-73
@@ -199,7 +199,7 @@ class MeshNetworkGPU:
         return p.data_ptr(), ldp, sp, lds
 
     def _ws_bytes(self, op, B):
-        return lambda: load().mg_workspace_bytes(op, self._N, self._L, B, self.crossing, self.geometry, None)
+        return lambda: load().mg_workspace_bytes(op, self._N, self._L, B, self.crossing, self.geometry | GEO_ONE_BATCH, None)
 
     def _programmed(self, op, p, s, B, dp=None) -> Tuple[int, int]:
         """Tiles of op for phases p (and direction dp) plus the permutation tables, in op's workspace."""
