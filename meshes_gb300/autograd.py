@@ -132,6 +132,8 @@ class MeshL2Function(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x: torch.Tensor, p: torch.Tensor, t: torch.Tensor, mesh: MeshNetworkGPU):
+        if t.device != x.device:                 # the loss kernel takes its address
+            raise RuntimeError("mesh_l2_loss: target is on %s, the fields are on %s" % (t.device, x.device))
         x = x.resolve_conj().resolve_neg().contiguous()
         t = t.resolve_conj().resolve_neg().to(x.dtype).contiguous()
         p = p.detach().to(torch.float32).contiguous()
