@@ -69,8 +69,8 @@ extern "C" {
 typedef struct mg_config {
   int M, V, W, CL, S;
   int split;   /* 0: automatic, 1: two CTA kinds per SM (V and V-1 vectors per lane group), 2: uniform CTAs,
-                * 3: warp pairs, 4: two CTAs per SM, 5: framed (crossings with a unit diagonal; CL is that of its
-                * pipeline, of 3 stages), 6: framed, the warps of a CTA holding V and V-1 vectors in turn.  Without a
+                * 3: warp pairs, 4: two CTAs per SM, 5: framed (crossings with a unit diagonal; W a multiple of 4; CL is
+                * that of its pipeline, of 3 stages), 6: framed, the warps of a CTA holding V and V-1 vectors in turn.  Without a
                 * configuration a nearest-neighbour MZI mesh of 64 < N takes a framed launch where that is faster; it
                 * computes with fields scaled by up to 2^22 either way, so magnitudes beyond about 1e30 (1e25 for a
                 * product of field and gradient) overflow in it.  7: butterfly kernels for FFT meshes of 2^k modes (64 to 256;

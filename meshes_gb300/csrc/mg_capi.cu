@@ -368,6 +368,8 @@ int plan_launch(int op, int N, int L, int B, int crossing, int geometry, const m
   const int maxw = p.framed ? framed_max_threads(M, V) / 32 : p.occ2 ? 8 : prop_max_threads(op, M, V) / 32;
   int W = (cfg && cfg->W) ? cfg->W : p.framed ? 8 : (p.split ? 4 : (p.pair || p.occ2) ? 8 : 0);
   if (p.framed && p.split && W % 8) return fail(MG_E_CONFIG, "mixed warps need W a multiple of 8, got %d", W);
+  // (the gradients' sum adds warps in fours, and four warps issue the copies in turn)
+  if (p.framed && W % 4) return fail(MG_E_CONFIG, "framed launches need W a multiple of 4, got %d", W);
   if (p.pair && (W & 1)) return fail(MG_E_CONFIG, "a warp-pair launch needs an even W, got %d", W);
   if (p.tree > 1) W = p.tree * default_warps(B, p.tree * 4, di.sms);
   if (!W) {

@@ -1,6 +1,15 @@
 """What the host refuses, or plans otherwise, before anything is launched; runs without a GPU."""
+import ctypes
+
 import pytest
 import torch
+
+
+def _plan(op, N, L, B, crossing=0, geo=0, cfg=None):
+    from meshes_gb300 import _lib
+    i = _lib.mg_plan_info()
+    c = None if cfg is None else _lib.cfg_ptr(_lib.config(*cfg))
+    return i if _lib.load().mg_plan(op, N, L, B, crossing, geo, c, ctypes.byref(i)) == 0 else None
 
 
 def test_l2_target_on_another_device_is_refused():
@@ -8,3 +17,10 @@ def test_l2_target_on_another_device_is_refused():
     x = torch.zeros(3, 8, dtype=torch.complex64)
     with pytest.raises(RuntimeError, match="target is on meta"):
         MeshL2Function.apply(x, torch.zeros(8, 4, 2), torch.zeros(3, 8, dtype=torch.complex64, device="meta"), None)
+
+
+@pytest.mark.parametrize("op", [0, 2])
+def test_framed_warps_come_in_fours(op):
+    for M, V, N in ((4, 1, 100), (8, 4, 256), (16, 1, 400), (20, 2, 600)):
+        for W in range(1, 9):
+            assert (_plan(op, N, 64, 300, cfg=(M, V, W, 0, 0, 5)) is not None) == (W % 4 == 0), (M, W)
