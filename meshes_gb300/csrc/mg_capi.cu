@@ -1385,8 +1385,10 @@ int mg_lossy_forward(int N, int L, int B, int geometry, int seg, const void* x, 
   if (L > seg) {
     int cl = std::min(P.CL, seg);
     while (seg % cl) --cl;
-    if (cl < P.CL && P.S == 1) P.S = 2;   // (one stage was to hold every layer)
+    const bool one = P.S == 1;   // one stage was to hold every layer: two hold a chunk each where they fit
+    if (cl < P.CL && one) P.S = 2;
     P.CL = cl;
+    if (one && launch_smem(P, OP_FWD, 0, L) > (size_t)dev_info().smem_optin - 1024) P.S = 1;
   }
   P.smem = launch_smem(P, OP_FWD, 0, L);
   return run_prop(P, x, nullptr, y, nullptr, ldu, nullptr, 0, 0, static_cast<unsigned char*>(ws),
