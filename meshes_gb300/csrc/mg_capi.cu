@@ -249,10 +249,18 @@ int plan_launch(int op, int N, int L, int B, int crossing, int geometry, const m
   // the permutation flags travel in the shared-memory copy of the layer kinds
   if (perm && L > kMaxSmemKinds) return fail(MG_E_ARG, "permuted meshes take at most %d layers", kMaxSmemKinds);
   const DevInfo di = dev_info();
+  // framed launch: nearest-neighbour complex meshes whose vector fills the warp at M >= 4, forward and MZI
+  // back-propagation with direct gradients
+  const bool may_frame = !stored && !perm && geometry == GEO_NN && N > 64 && L > 0 && L <= kMaxSmemKinds &&
+                         (crossing == CR_MZI ? op != OP_FWDDIFF : crossing == CR_SYM && op == OP_FWD);
+  const int full_m = N > 512 ? kWideM : pow2ceil(N) / 32;   // modes per lane of the whole warp
+  const bool pays = may_frame && framed_pays(op, full_m, L, 16 * full_m, B, di.sms);
   mg_config tuned;
   // tuned entries were measured without the permutation scratch: permuted meshes take the defaults
   Plan& p = *P;
   p.tuned = !cfg && !perm && !stored && !how && lookup_tuned(op, crossing, geometry, N, B, &tuned);
+  // (an entry holds for every depth; one that was measured framed, where this depth may be and gains by it)
+  if (p.tuned && (tuned.split == 5 || tuned.split == 6)) p.tuned = pays;
   if (p.tuned) cfg = &tuned;
   p.op = op; p.N = N; p.L = L; p.B = B; p.crossing = crossing; p.geometry = geometry;
   p.perm = perm;
@@ -279,13 +287,9 @@ int plan_launch(int op, int N, int L, int B, int crossing, int geometry, const m
     cfg = &dc;
   }
   const bool chosen = cfg != nullptr;   // a configuration given or tuned
-  // framed launch: nearest-neighbour complex meshes whose vector fills the warp at M >= 4, forward and MZI
-  // back-propagation with direct gradients
-  const bool may_frame = !stored && !perm && geometry == GEO_NN && N > 64 && L > 0 && L <= kMaxSmemKinds &&
-                         (crossing == CR_MZI ? op != OP_FWDDIFF : crossing == CR_SYM && op == OP_FWD);
   p.may_frame = may_frame;
   mg_config fc;
-  if (!cfg && !(how & kUniform) && may_frame && framed_pays(op, Np / 32, L, Np / 2, B, di.sms) && framed_pick(op, Np / 32, B, di.sms, &fc)) cfg = &fc;
+  if (!cfg && !(how & kUniform) && pays && framed_pick(op, full_m, B, di.sms, &fc)) cfg = &fc;
   // (a configuration without modes per lane leaves them where they were, whatever the batch)
   int small_v = 0;
   if (!(cfg && (cfg->M || cfg->V || N <= 128)) && geometry == GEO_NN && !perm && !wide && N > 32 && crossing != CR_ORTH &&

@@ -24,3 +24,24 @@ def test_framed_warps_come_in_fours(op):
     for M, V, N in ((4, 1, 100), (8, 4, 256), (16, 1, 400), (20, 2, 600)):
         for W in range(1, 9):
             assert (_plan(op, N, 64, 300, cfg=(M, V, W, 0, 0, 5)) is not None) == (W % 4 == 0), (M, W)
+
+
+def test_tuned_framed_entry_at_other_depths():
+    """A recorded framed launch holds for depths that may be framed and gain by it; the others keep the launch they had."""
+    from meshes_gb300 import _lib
+    lib = _lib.load()
+    shapes = [(op, L) for op in (0, 2) for L in (0, 1, 8, 300, 4096, 4097, 5000)]
+    before = [_plan(op, 300, L, 50) for op, L in shapes]
+    try:
+        for op in (0, 2):
+            _lib.check(lib.mg_set_tuned(op, 0, 0, 300, 1, 100, ctypes.byref(_lib.config(16, 2, 4, 0, 0, 5))), "mg_set_tuned")
+        after = [_plan(op, 300, L, 50) for op, L in shapes]
+    finally:
+        for op in (0, 2):
+            lib.mg_set_tuned(op, 0, 0, 300, 0, 0, None)
+    for (op, L), a, b in zip(shapes, before, after):
+        assert b is not None, (op, L)
+        if L in (300, 4096):
+            assert (b.V, b.W) == (2, 4)
+        else:
+            assert all(getattr(a, f) == getattr(b, f) for f, _ in a._fields_), (op, L)
