@@ -16,6 +16,8 @@ __device__ __forceinline__ bool framed_item(const mg_batch_framed& f, const mg_b
   const mg_batch_mesh& md = f.mesh;
   const int np2 = 16 * M;
   if (md.G != 32 || !batch_item_ok(md, it, M) || f.fcl < 1) return false;
+  // the mesh's tiles are those of M modes per lane, with gamma (both ops read back-propagation's)
+  if (M != batch_framed_M(md.N) || f.flb != framed_layer_bytes(OP_BWD, np2)) return false;
   unsigned dynamic;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynamic));
   if (framed_smem_bytes(OP, f.flb, np2, W, f.fcl, md.L) > dynamic) return false;

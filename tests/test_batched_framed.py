@@ -68,3 +68,33 @@ def test_items_outside_the_batch_are_refused():
     y = bm.states[0].y.cpu().numpy()
     assert O.rel_err(y[:32], O.propagate(om, x)[:32]) < TOL
     assert float(np.abs(y[32:]).max()) == 0.0
+
+
+@pytest.mark.parametrize("op", [0, 2])
+def test_tiles_of_four_modes_per_lane_are_refused(op):
+    """mg_batched_framed runs 8 modes per lane; a mesh of 65 to 128 modes, whose framed tiles have 4, is not its item."""
+    import ctypes
+    from meshes_gb300 import _lib
+    from meshes_gb300.batched import _to_device
+    from meshes_gb300.serve import MeshServer
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    om = _mesh(np.random.default_rng(73), 128, "clements", 24)
+    cfg, ws = MeshServer([gpu_mesh(om)]).res[0].framed
+    ds, smem = [_lib.mg_batch_framed(), _lib.mg_batch_framed()], [ctypes.c_size_t(), ctypes.c_size_t()]
+    _lib.check(lib.mg_batched_framed_desc(128, om.L, 1, 0, 0, _lib.cfg_ptr(cfg), ws.data_ptr(), ws.numel(),
+                                          *map(ctypes.byref, ds), *map(ctypes.byref, smem)), "mg_batched_framed_desc")
+    u, g, out = (torch.zeros((32, 128), dtype=torch.complex64, device="cuda") for _ in range(3))
+    u += 1
+    dp = torch.zeros(om.p.shape, device="cuda")
+    partial = torch.zeros((om.L, 128, 2), device="cuda")     # of 8 modes per lane
+    d = ds[0 if op == 0 else 1]
+    d.mesh.B, d.mesh.ldu, d.mesh.n_items, d.mesh.ldp, d.mesh.n_p = 32, 128, 1, 128, 2
+    d.mesh.in0, d.mesh.in1 = u.data_ptr(), g.data_ptr()
+    d.mesh.out0, d.mesh.out1 = (out.data_ptr(), None) if op == 0 else (None, out.data_ptr())
+    d.mesh.dp, d.mesh.partial = dp.data_ptr(), partial.data_ptr()
+    dev, item = _to_device((_lib.mg_batch_framed * 1)(d), u.device), _to_device((_lib.mg_batch_item * 1)((0, 0, 32, 0)), u.device)
+    head, status = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+    _lib.check(lib.mg_batched_framed(op, dev.data_ptr(), 1, item.data_ptr(), 1, head.data_ptr(), 1, 200000, status.data_ptr(),
+                                     st), "mg_batched_framed")
+    assert int(status) == 3
+    assert not out.any() and not partial.any()
