@@ -88,7 +88,9 @@ const char* mg_version(void);
 
 /* Bytes of workspace an entry point needs for (op, N, L, B, crossing, geometry) with config cfg
  * (NULL = heuristic).  The workspace is caller-allocated device memory, 256-byte aligned; its first
- * 256 bytes hold the status word. */
+ * 256 bytes hold the status word.  Without a configuration (and without MG_GEO_ONE_BATCH) a workspace of that size holds
+ * every smaller batch as well; back-propagation of a batch whose own launch leaves more partials than fit takes the
+ * launch that leaves fewest. */
 size_t mg_workspace_bytes(int op, int N, int L, int B, int crossing, int geometry, const mg_config* cfg);
 
 /* Zero the status word of a freshly allocated workspace. */

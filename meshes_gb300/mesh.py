@@ -39,10 +39,20 @@ class Workspace:
     def __init__(self, device):
         self.device = device
         self.buf: Optional[torch.Tensor] = None
+        self.sized = set()
 
-    def call(self, size, fn) -> int:
+    def call(self, size, fn, key=None) -> int:
         """rc of fn(ws, ws_bytes) on the buffer as it is; grown to size() bytes first where the library says it is too small
-        (which it does before anything else happens), so that a call does not ask for the size each time."""
+        (which it does before anything else happens), so that a call does not ask for the size each time.  key: of calls
+        that the library would also run, another way, on less than size() bytes: the size is asked for once per key."""
+        if key is not None and key not in self.sized:
+            nb = size()
+            if nb == 0:
+                check(-1, "mg_workspace_bytes")
+            self.get(nb)
+            if len(self.sized) >= 256:
+                self.sized.clear()
+            self.sized.add(key)
         rc = _lib.E_WORKSPACE
         if self.buf is not None:
             rc = fn(self.buf.data_ptr(), self.buf.numel())
@@ -369,7 +379,7 @@ class MeshNetworkGPU:
         check(self._ws[OP_BWD].call(self._ws_bytes(OP_BWD, B), lambda ws, wsn: fn(
             self._N, self._L, B, *self._geo_args(), pptr, out_dp.data_ptr(), ldp, sptr, lds, v2.data_ptr(),
             g.data_ptr(), None if out_vin is None else out_vin.data_ptr(), out_dJdv.data_ptr(), ldu,
-            self.crossing, accumulate, ws, wsn, stream)), fn.__name__)
+            self.crossing, accumulate, ws, wsn, stream), B), fn.__name__)
         return out_dp, out_dJdv
 
     # ---- phase screen: is_phase with phi_pos 'in' (y = U D v) or 'out' (y = D U v), D = diag(exp(i ph)),

@@ -51,6 +51,27 @@ def _lib_bytes(op, N, L, B, X):
     return _lib.load().mg_workspace_bytes(op, N, L, B, X, 0, None)
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="calls on addresses that nothing may be launched on")
+@pytest.mark.parametrize("X", [0, 1])
+def test_a_workspace_holds_every_smaller_batch(X):
+    """Back-propagation of no batch is refused for want of space (MG_E_WORKSPACE, before the launch that fails here for want of
+    a device) in a workspace of a larger one's size."""
+    from meshes_gb300 import _lib
+    lib = _lib.load()
+    Bs = (1, 7, 600, 1216, 2500, 4096, 4864, 4900, 6000, 9000, 19000, 30000, 99000, 100000)
+    a = 1 << 20                                          # an aligned address that is not looked at
+    for N in (8, 32, 34, 64, 100, 128, 130, 256, 400, 512, 600, 640):
+        for L in (1, 20, N):
+            sizes = [_lib_bytes(BWD, N, L, B, X) for B in Bs]
+            for n, nb in enumerate(sizes):
+                for B in Bs[:n + 1]:
+                    rcs = [lib.mg_propagate(BWD, N, L, B, X, 0, a, a, None, a, N, a, N, 0, None, a, nb, None),
+                           lib.mg_propagate(FWD_BWDTILES, N, L, B, X, 0, a, None, a, None, N, None, 0, 0, None, a, nb, None),
+                           lib.mg_propagate_l2(N, L, B, X, 0, a, a, None, a, N, a, N, 0, None, a, nb, None),
+                           lib.mg_backdiff(N, L, B, a, a, a, a, N, a, N, a, a, None, a, N, X, 0, a, nb, None)]
+                    assert rcs == [-3] * 4, (N, L, Bs[n], B, _lib.last_error())
+
+
 class _Tiles:
     """op's tiles of om in a workspace for all of Bs, built with B_build."""
 
@@ -171,3 +192,37 @@ def test_layer_ranges(N):
             G, _, gin = O.vjp_unitary(om, y[:B], g[:B])
             assert O.rel_err(gx.cpu().numpy(), gin) < TOL, (b, B)
             assert O.rel_err(dT.cpu().numpy(), np.conj(G)) < TOL, (b, B)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("crossing", ["mzi", "sym"])
+@pytest.mark.parametrize("N,L,Bmax,called", [(100, 20, 6000, (6000, 4864, 1, 1216)), (256, 128, 4096, (1216, 3000)),
+                                             (256, 40, 10000, (9900, 5000)), (64, 20, 6000, (2600, 600)),
+                                             (600, 10, 3000, (1900, 100)), (20, 20, 9000, (2500,))])
+def test_smaller_batches_in_one_workspace(N, L, Bmax, called, crossing):
+    """A workspace of the largest batch's size serves smaller ones, whose launches of their own may leave more partials:
+    mg_propagate on resident tiles and the entry points that build for each call."""
+    rng = np.random.default_rng(N + L)
+    om = _mesh(rng, N, L, crossing)
+    x, g = O.unit_columns(rng, N, Bmax), O.unit_columns(rng, N, Bmax)
+    y = O.propagate(om, x)
+    xd, yd, gd = _c64(x), _c64(y), _c64(g)
+    t = _Tiles(om, BWD, Bmax, ())
+    n_s = 2 if crossing == "mzi" else 1
+    d = [torch.tensor(np.asarray(a), device="cuda") for a in (np.int32(om.lens), np.int32(om.shifts), om.p, om.s)]
+    for one in (False, True):
+        for B in called:
+            out, xo, gx = (torch.zeros_like(yd[:B]) for _ in range(3))
+            dp = torch.zeros(om.p.shape, device="cuda")
+            if one:
+                t.check(t.lib.mg_backdiff(N, om.L, B, d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), dp.data_ptr(), N,
+                                          d[3].data_ptr(), n_s * N // 2, yd.data_ptr(), gd.data_ptr(), xo.data_ptr(),
+                                          gx.data_ptr(), N, t.X, 0, t.ws.data_ptr(), t.nb, t.st), "mg_backdiff")
+                t.ok()
+            else:
+                t.run(FWD_BWDTILES, B, xd.data_ptr(), None, out.data_ptr(), None, N, None, 0, 0)
+                assert O.rel_err(out.cpu().numpy(), y[:B]) < TOL, B
+                t.run(BWD, B, yd.data_ptr(), gd.data_ptr(), xo.data_ptr(), gx.data_ptr(), N, dp.data_ptr(), N, 0)
+            G, _, gin = O.vjp_unitary(om, y[:B], g[:B])
+            assert O.rel_err(xo.cpu().numpy(), x[:B]) < TOL and O.rel_err(gx.cpu().numpy(), gin) < TOL, B
+            assert O.rel_err(dp.cpu().numpy(), O.contract_dp(om, G)) < TOL, B
