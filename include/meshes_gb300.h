@@ -71,11 +71,9 @@ typedef struct mg_config {
   int split;   /* 0: automatic, 1: two CTA kinds per SM (V and V-1 vectors per lane group), 2: uniform CTAs,
                 * 3: warp pairs, 4: two CTAs per SM, 5: framed (crossings with a unit diagonal; W a multiple of 4; CL is
                 * that of its pipeline, of 3 stages), 6: framed, the warps of a CTA holding V and V-1 vectors in turn.  Without a
-                * configuration a nearest-neighbour MZI mesh of 64 < N takes a framed launch where that is faster; it
-                * computes with fields scaled by up to 2^22 either way, so magnitudes beyond about 1e30 (1e25 for a
-                * product of field and gradient) overflow in it.  7: butterfly kernels for FFT meshes of 2^k modes (64 to 256;
-                * forward also 512; the other fields then describe the general launch), taken without a configuration
-                * where faster, the general launch where there is none */
+                * configuration a nearest-neighbour MZI mesh of 64 < N takes a framed launch where that is faster.  7:
+                * butterfly kernels for FFT meshes of 2^k modes (64 to 256; forward also 512; the other fields then describe
+                * the general launch), taken without a configuration where faster, the general launch where there is none */
 } mg_config;
 
 /* ---- library ---------------------------------------------------------------------------- */
@@ -275,7 +273,7 @@ int mg_batched_reduce(const mg_batch_mesh* meshes, int n_meshes, void* stream);
 /* The same for meshes on framed tiles (mg_config{8, 4, 8, .., split 5}): nearest-neighbour MZI meshes of 129 to 256 modes.
  * mg_batched_framed_desc describes a mesh on the workspace that mg_build_tiles(MG_OP_BWD) filled with that
  * configuration, for both ops (forward reads back-propagation's tiles); the caller sets the fields, B, ldu, n_items, ldp,
- * n_p, dp and partial of `mesh` (back-propagation: n_items * L * 128 float2).  *smem_fwd, *smem_bwd: dynamic shared
+ * n_p, dp and partial of `mesh` (back-propagation: n_items * L * 128 float2) and `scales`.  *smem_fwd, *smem_bwd: dynamic shared
  * memory of a launch.  An item is up to 32 vectors. */
 typedef struct mg_batch_framed {
   mg_batch_mesh mesh;
@@ -288,6 +286,9 @@ typedef struct mg_batch_framed {
   int fcl, refuse;
   unsigned flb;
   int V;                 /* mg_batched_small */
+  int* scales;           /* back-propagation, the caller's: n_items ints of device memory, in which partials of fields and
+                          * gradients of any size keep their scale (NULL: products of a field and a gradient beyond about
+                          * 1e25, or below 1e-9 behind a cross state, leave the range of a float) */
 } mg_batch_framed;
 int mg_batched_framed_desc(int N, int L, int B, int crossing, int geometry, const mg_config* cfg, const void* workspace,
                            size_t workspace_bytes, mg_batch_framed* fwd, mg_batch_framed* bwd, size_t* smem_fwd,

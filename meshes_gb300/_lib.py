@@ -51,7 +51,7 @@ class mg_batch_mesh(Structure):
 
 class mg_batch_framed(Structure):
     _fields_ = [("mesh", mg_batch_mesh), ("main", c_void_p), ("resc", c_void_p), ("wts", c_void_p), ("dfin", c_void_p),
-                ("fkinds", c_void_p), ("count", c_void_p), ("fcl", c_int), ("refuse", c_int), ("flb", c_uint), ("V", c_int)]
+                ("fkinds", c_void_p), ("count", c_void_p), ("fcl", c_int), ("refuse", c_int), ("flb", c_uint), ("V", c_int), ("scales", c_void_p)]
 
 
 class mg_server_mesh(Structure):

@@ -148,6 +148,8 @@ class _MeshState:
             d.mesh.B, d.mesh.ldu, d.mesh.n_items = self.B, m.N, self.n_items
             d.mesh.ldp, d.mesh.n_p = m.N // 2 * m.X_np, m.X_np
             self._fields(op, d.mesh)
+        self.scales = torch.zeros(max(self.n_items, 1), dtype=torch.int32, device=m.device)
+        ds[OP_BWD].scales = self.scales.data_ptr()
         return ds, {op: v.value for op, v in smem.items()}
 
     def cost(self) -> int:

@@ -49,7 +49,8 @@ __global__ void __launch_bounds__(256) batched_framed_reduce_kernel(const mg_bat
   }
   const int M = batch_framed_M(md.N), np2 = 16 * M;
   const FramedReduceArgs a{static_cast<const float2*>(md.partial), md.n_items, md.L, np2, M, 32, md.N, md.dp, md.ldp, 0,
-                           md.kinds + md.L, static_cast<const float2*>(f.wts), f.count, f.refuse};
+                           md.kinds + md.L, static_cast<const float2*>(f.wts), f.count, f.refuse,
+                           f.scales};
   for (int blk = blockIdx.x; 2 * blk * kFReduceCols < md.L * np2; blk += gridDim.x) {
     framed_reduce_block(a, blk, acc);
     __syncthreads();

@@ -27,6 +27,7 @@ __device__ __forceinline__ bool framed_item(const mg_batch_framed& f, const mg_b
   a.dfin = static_cast<const float2*>(f.dfin);
   a.fkinds = f.fkinds;
   a.count = f.count;
+  a.scales = OP == OP_BWD && f.scales ? f.scales + it.part : nullptr;
   a.fcl = f.fcl; a.flb = f.flb; a.refuse = f.refuse;
   return true;
 }

@@ -117,7 +117,7 @@ struct Plan {
   size_t off_kinds, off_tiles, off_dtiles, off_partial, total;
   int tree;         // stored activations: warps whose gradients are added pairwise before the others (1: none)
   bool framed;      // unit-diagonal crossings on the frame pass's tiles (mg_framed.cuh)
-  size_t off_main, off_resc, off_wts, off_dfin, off_fkinds, off_tdiag, off_toff, off_tmag, off_tcs, off_count;
+  size_t off_main, off_resc, off_wts, off_dfin, off_fkinds, off_tdiag, off_toff, off_tmag, off_tcs, off_count, off_scales;
   unsigned flb;     // bytes of a layer's framed tile
   int fcl;          // layers per stage of the framed pipeline (CL, S: of the unframed body in the same kernel)
   bool fft;         // butterfly kernels (mg_fft.cuh) on this plan's tiles
@@ -489,6 +489,8 @@ void place(Plan* P) {
   p.off_perm = at;
   p.off_partial = p.off_perm + (p.perm ? align256(perm_table_bytes(p.N, p.L)) : 0);
   p.total = p.off_partial + ((p.op == OP_BWD) ? align256((size_t)std::max(p.grid, p.fft_grid) * p.L * p.np2 * (p.gr == 4 ? 32 : 8)) : 0);
+  p.off_scales = p.total;
+  if (p.framed && p.op == OP_BWD) p.total += align256(4 * (size_t)p.grid);
 }
 
 // geometry | MG_GEO_ONE_BATCH: the tiles that the launch of B reads, and no others
@@ -742,6 +744,7 @@ int run_prop(const Plan& P, const void* in0, const void* in1, void* out0, void* 
     f.dfin = reinterpret_cast<const float2*>(ws + P.off_dfin);
     f.fkinds = reinterpret_cast<const int*>(ws + P.off_fkinds);
     f.count = reinterpret_cast<const int*>(ws + P.off_count);
+    f.scales = P.op == OP_BWD ? reinterpret_cast<int*>(ws + P.off_scales) : nullptr;
     f.fcl = P.fcl;
     f.flb = P.flb;
     f.refuse = framed_refuse(P.L);
@@ -764,7 +767,8 @@ int run_prop(const Plan& P, const void* in0, const void* in1, void* out0, void* 
     if (P.framed) {
       e = launch_framed_reduce(a.partial, P.grid, P.L, P.np2, P.M, P.G, P.N, dp, ldp, accumulate, geo,
                                reinterpret_cast<const float2*>(ws + P.off_wts),
-                               reinterpret_cast<const int*>(ws + P.off_count), framed_refuse(P.L), st);
+                               reinterpret_cast<const int*>(ws + P.off_count), framed_refuse(P.L),
+                               reinterpret_cast<const int*>(ws + P.off_scales), st);
       return e == cudaSuccess ? MG_OK : cuda_fail(e, "framed_reduce_kernel launch");
     }
     dp_reduce_kernel<<<(n + kReduceCols - 1) / kReduceCols, kReduceCols * kReduceRows, 0, st>>>(

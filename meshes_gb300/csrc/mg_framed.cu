@@ -101,9 +101,9 @@ cudaError_t launch_frames(const FrameArgs& a, int sms, cudaStream_t stream) {
 
 cudaError_t launch_framed_reduce(const float2* partial, int nC, int L, int np2, int M, int G, int N, float* dp, int ldp,
                                  int accumulate, const int* geo, const float2* wts, const int* count, int refuse,
-                                 cudaStream_t stream) {
+                                 const int* scales, cudaStream_t stream) {
   framed_reduce_kernel<<<(L * np2 / 2 + kFReduceCols - 1) / kFReduceCols, 256, 0, stream>>>(
-      FramedReduceArgs{partial, nC, L, np2, M, G, N, dp, ldp, accumulate, geo, wts, count, refuse});
+      FramedReduceArgs{partial, nC, L, np2, M, G, N, dp, ldp, accumulate, geo, wts, count, refuse, scales});
   return cudaGetLastError();
 }
 

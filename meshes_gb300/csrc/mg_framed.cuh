@@ -19,6 +19,12 @@
 //
 // Work decomposition, pipeline, bounded waits and the gradient partials are those of mg_prop.cuh; a stage holds
 // its layers' tiles and the factors of their first RESCALEs.
+//
+// Framed fields are 2^-22 to 2^48 of the fields' own (forward) or 2^-48 to 2^22 (back-propagation, the products of two of them
+// 2^-96 to 2^44), so every vector comes in times a power of two that brings its largest part to 2^kFieldTop and leaves by
+// its inverse: nothing overflows, or falls below the normal range, that does not without frames (but for products 2^35
+// times smaller than the largest of their warp's).  The factors are exact; results do not depend on them.  They cost 2 us of
+// a back-propagation launch (N = 256, B = 4096: 197 -> 199 us).
 #pragma once
 #include "mg_frame.cuh"
 
@@ -285,9 +291,57 @@ __device__ __forceinline__ void f_each(Fields<M, V>& u, Fields<M, V>& w, F f) {
 #pragma unroll
     for (int k = 0; k < M / 2; ++k) f(u.m[0][k], w.m[0][k]);
 }
+// 2^k, -126 <= k <= 127
+__device__ __forceinline__ float pow2f(int k) { return __int_as_float((k + 127) << 23); }
+// vector v of the lane times 2^k(v), |k| <= 252, in two steps
+template <int M, int V, typename K>
+__device__ __forceinline__ void f_scale(K k, Fields<M, V>& u) {
+  auto times = [](p64 a, p64 b, P2& x) { x = P2{pmul(pmul(x.r, a), b), pmul(pmul(x.i, a), b)}; };
+#pragma unroll
+  for (int p = 0; p < V / 2; ++p) {
+    const int k0 = k(2 * p), k1 = k(2 * p + 1);
+    const p64 a = p_pack(pow2f(k0 >> 1), pow2f(k1 >> 1)), b = p_pack(pow2f(k0 - (k0 >> 1)), pow2f(k1 - (k1 >> 1)));
+#pragma unroll
+    for (int m = 0; m < M; ++m) times(a, b, u.v[p][m]);
+  }
+  if constexpr (V & 1) {
+    const int k0 = k(V - 1);
+    const float a = pow2f(k0 >> 1), b = pow2f(k0 - (k0 >> 1));
+#pragma unroll
+    for (int m = 0; m < M / 2; ++m) times(p_pack(a, a), p_pack(b, b), u.m[0][m]);
+  }
+}
+// The k that brings the largest part of each of the warp's vectors to [2^kFieldTop, 2^(kFieldTop + 1)); kNoScale for one that is
+// 0 or holds infinity
+constexpr int kNoScale = 1 << 20;
 template <int M, int V>
-__device__ __forceinline__ void f_scale(float s, Fields<M, V>& u) {
-  f_each<M, V>(u, u, [&](P2& a, P2&) { a = P2{pmul(p_pack(s, s), a.r), pmul(p_pack(s, s), a.i)}; });
+__device__ __forceinline__ void f_wanted(const Fields<M, V>& u, int (&k)[V]) {
+  auto of = [](float m) {   // (fmaxf passes NaN by)
+    const unsigned b = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if (b == 0 || b >= 0x7f800000u) return kNoScale;
+    return kFieldTop - (b >= 0x00800000u ? (int)(b >> 23) - 127 : -118 - __clz(b));
+  };
+#pragma unroll
+  for (int p = 0; p < V / 2; ++p) {
+    float a = 0.f, b = 0.f;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const float2 re = p_split(u.v[p][m].r), im = p_split(u.v[p][m].i);
+      a = fmaxf(a, fmaxf(fabsf(re.x), fabsf(im.x)));
+      b = fmaxf(b, fmaxf(fabsf(re.y), fabsf(im.y)));
+    }
+    k[2 * p] = of(a);
+    k[2 * p + 1] = of(b);
+  }
+  if constexpr (V & 1) {
+    float a = 0.f;
+#pragma unroll
+    for (int m = 0; m < M / 2; ++m) {
+      const float2 re = p_split(u.m[0][m].r), im = p_split(u.m[0][m].i);
+      a = fmaxf(a, fmaxf(fmaxf(fabsf(re.x), fabsf(re.y)), fmaxf(fabsf(im.x), fabsf(im.y))));
+    }
+    k[V - 1] = of(a);
+  }
 }
 
 // Steps: the walk goes by pairs of layers, (aligned, odd-shift) forward and (odd-shift, aligned) in back-propagation, as
@@ -409,10 +463,13 @@ __device__ __forceinline__ ulonglong2 frame_pair(const float2* __restrict__ d, i
 // CTA barrier by number: with MIX, warps of both kinds meet at it from their own copies of the body
 __device__ __forceinline__ void cta_sync() { asm volatile("barrier.cta.sync.aligned 0;" ::: "memory"); }
 
-// Sum of the W warps' staged gradients of a chunk (W a multiple of 4), in warp order, into this CTA's partials of the
+// Sum of the W warps' staged gradients of a chunk (W a multiple of 4), in warp order, at the least of their scales, into this CTA's partials of the
 // layers from lo on: n float4 of consecutive layers.  turn: the chunk; the warps that the last round of a chunk leaves over
 // change with it (the same two of eight at M = 20: back-propagation at N = 600, B = 2048 727 us, in turns 684)
-__device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int W, int n, int turn, ulonglong2* out) {
+__device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int W, int n, int turn, const int* scales,
+                                         const int* scale, ulonglong2* out) {
+  const int least = scales[0];
+  const bool one = least >= scales[1];
   int first = threadIdx.x + (64 * turn) % (int)blockDim.x;
   if (first >= (int)blockDim.x) first -= blockDim.x;
 #pragma unroll 1
@@ -421,7 +478,17 @@ __device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int 
     ulonglong2 t = make_ulonglong2(0, 0);
 #pragma unroll 1
     for (int w = 0; w < W; w += 4, p += 4 * warp_bytes) {
-      const ulonglong2 a = lds16(p), b = lds16(p + warp_bytes), c = lds16(p + 2 * warp_bytes), d = lds16(p + 3 * warp_bytes);
+      ulonglong2 a = lds16(p), b = lds16(p + warp_bytes), c = lds16(p + 2 * warp_bytes), d = lds16(p + 3 * warp_bytes);
+      if (!one) {
+        auto at = [&](ulonglong2& x, int i) {
+          const float f = pow2f(max(least - scale[kWarpScales * (w + i) + 8], -126));
+          x = make_ulonglong2(pmul(p_pack(f, f), x.x), pmul(p_pack(f, f), x.y));
+        };
+        at(a, 0);
+        at(b, 1);
+        at(c, 2);
+        at(d, 3);
+      }
       t.x = padd(padd(padd(padd(t.x, a.x), b.x), c.x), d.x);
       t.y = padd(padd(padd(padd(t.y, a.y), b.y), c.y), d.y);
     }
@@ -446,6 +513,8 @@ struct FramedSmem {
   uint32_t codes;       // of layer 0
   uint32_t resc;        // per chunk: the layers of its first framed_resc_rows RESCALE, -1 behind the last
   volatile int* state;  // [0] a wait ran out, [1] chunks whose copies were issued
+  int* scales;          // least and largest of the warps' scales (gradients' products)
+  int* scale;           // kWarpScales per warp: its vectors' exponents (4 of u, 4 of w), its scale
 };
 // Layers of the walk in chunks of CL; the first chunk is one shorter where that keeps pairs of layers whole
 template <int OP>
@@ -493,14 +562,58 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
   };
   if (tid == 0)
     for (int c = 0; c < min(S, nch); ++c) issue(c, c);
+  int* const scale = sm.scale + kWarpScales * warp;
   if constexpr (OP == OP_FWD) {
-    f_scale<M, V>(1.f / (1ull << kFrameTop), u);
+    int ku[V];
+    f_wanted<M, V>(u, ku);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      if (ku[v] == kNoScale) ku[v] = 0;
+      if (lane == 0) scale[v] = ku[v];
+    }
+    f_scale<M, V>([&](int v) { return ku[v] - kFrameTop; }, u);
   } else {
     if (a.target)   // fused L2 loss to a target: g = 2 (y - t)
       f_each<M, V>(u, w, [](P2& y, P2& t) {
         const p64 two = p_pack(2.f, 2.f);
         t = P2{pmul(two, psub(y.r, t.r)), pmul(two, psub(y.i, t.i))};
       });
+    // one scale for all products of the warp, since its vectors' are added: that of the largest, in the range where a float
+    // holds it, a multiple of 16 (most launches then have one scale).  What a vector's own product is short of that, u and
+    // w bear half each, up to 2^80, within which neither loses bits (a product below 2^-160 of the largest counts as up to that).
+    int ku[V], kw[V], all = kNoScale;
+#pragma unroll
+    for (int v = 0; v < V; ++v) ku[v] = kw[v] = 0;
+    if (a.scales) {
+      f_wanted<M, V>(u, ku);
+      f_wanted<M, V>(w, kw);
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (ku[v] != kNoScale && kw[v] != kNoScale) all = min(all, ku[v] + kw[v]);
+      if (all != kNoScale) all = max(all, -80) & ~15;
+      if (lane == 0) {
+        scale[8] = all;
+        if (all != kNoScale) {
+          atomicMin(sm.scales, all);
+          atomicMax(sm.scales + 1, all);
+        }
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {   // (a product with 0 or infinity has no scale)
+      if (a.scales && ku[v] != kNoScale && kw[v] != kNoScale) {
+        kw[v] -= min(max((ku[v] + kw[v] - all) >> 1, 0), 80);
+        ku[v] = max(all - kw[v], ku[v] - 80);
+      }
+      if (ku[v] == kNoScale) ku[v] = 0;
+      if (kw[v] == kNoScale) kw[v] = 0;
+      if (lane == 0) {
+        scale[v] = ku[v];
+        scale[4 + v] = kw[v];
+      }
+    }
+    f_scale<M, V>([&](int v) { return ku[v]; }, u);
+    f_scale<M, V>([&](int v) { return kw[v]; }, w);
     f_diag<M, V, true>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, u);
     f_diag<M, V, true>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, w);
   }
@@ -508,7 +621,7 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
   // chunk c: stage and gradient slot s = c % S, of whose barriers it is phase ph = (c / S) & 1
   auto reduce = [&](int c, int s) {
     const int lo = ch.lo(c);
-    f_reduce(sm.gst + (uint32_t)s * slot_bytes, warp_bytes, a.W, (ch.hi(c) - lo) * (np2 / 2), c,
+    f_reduce(sm.gst + (uint32_t)s * slot_bytes, warp_bytes, a.W, (ch.hi(c) - lo) * (np2 / 2), c, sm.scales, sm.scale,
              reinterpret_cast<ulonglong2*>(a.partial + (size_t)lo * np2));
   };
   const FTile none{sm.zero + j16, sm.gst + (uint32_t)S * slot_bytes + j16};
@@ -554,17 +667,20 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
   }
   if (tid == 0)
     for (int k = 0; k < 2 * S; ++k) mbar_inval(sm.bars + 8u * k);
-  if constexpr (OP == OP_BWD)
+  if constexpr (OP == OP_BWD) {
     if (nch > 0) reduce(nch - 1, (nch - 1) % S);
+    if (tid == 0 && a.scales) *a.scales = sm.scales[0];
+  }
   if constexpr (OP == OP_FWD) {
     f_diag<M, V, false>([&](int k) { return frame_pair<M>(a.dfin, j, k); }, u);
+    f_scale<M, V>([&](int v) { return -scale[v]; }, u);
     f_store<M, V>(u, a.out0, vb0, a.vend, a.N, a.ldu, j);
   } else {
     if (a.out0 != nullptr) {
-      f_scale<M, V>(1.f / (1ull << kFrameTop), u);
+      f_scale<M, V>([&](int v) { return -scale[v] - kFrameTop; }, u);
       f_store<M, V>(u, a.out0, vb0, a.vend, a.N, a.ldu, j);
     }
-    f_scale<M, V>(1.f / (1ull << kFrameTop), w);
+    f_scale<M, V>([&](int v) { return -scale[4 + v] - kFrameTop; }, w);
     f_store<M, V>(w, a.out1, vb0, a.vend, a.N, a.ldu, j);
   }
 }
@@ -589,7 +705,9 @@ __device__ __forceinline__ void framed_run(const FramedArgs& a, unsigned char* s
   sm.gst = sm.zero + layer;
   sm.bars = smem_u32(smem + bars);
   sm.state = reinterpret_cast<volatile int*>(smem + bars + 16 * kFrameStages);
-  int* codes = reinterpret_cast<int*>(smem + bars + 16 * kFrameStages + 16) + kCodePad;
+  sm.scales = reinterpret_cast<int*>(smem + bars + 16 * kFrameStages + 8);
+  sm.scale = reinterpret_cast<int*>(smem + bars + 16 * kFrameStages + 16);
+  int* codes = sm.scale + kWarpScales * a.W + kCodePad;
   int* resc = codes + a.L + kCodePad;
   sm.codes = smem_u32(codes);
   sm.resc = smem_u32(resc);
@@ -610,6 +728,8 @@ __device__ __forceinline__ void framed_run(const FramedArgs& a, unsigned char* s
       mbar_init(sm.bars + 8u * (kFrameStages + s), a.W);
     }
     sm.state[0] = sm.state[1] = 0;
+    sm.scales[0] = kNoScale;
+    sm.scales[1] = -kNoScale;
     fence_mbar_init();
   }
   __syncthreads();
@@ -630,11 +750,14 @@ __global__ void __launch_bounds__(framed_max_threads(M, V), 1) framed_kernel(con
   FramedArgs a = a0;
   a.v0 = blockIdx.x * cap;
   a.vend = min(a.B, a.v0 + cap);
-  if (OP == OP_BWD) a.partial = a0.partial + (size_t)blockIdx.x * a.L * ((G * M) >> 1);
+  if (OP == OP_BWD) {
+    a.partial = a0.partial + (size_t)blockIdx.x * a.L * ((G * M) >> 1);
+    a.scales = a0.scales + blockIdx.x;
+  }
   framed_run<OP, M, V, GT, MIX>(a, smem);
 }
 
-// dp[l][q][k] (= or +=) the sum over the nC per-CTA partials times the frames' weights, in the CTAs' order (as
+// dp[l][q][k] (= or +=) the sum over the nC per-CTA partials, each 2^scales[c] of its own size, times the frames' weights, in the CTAs' order (as
 // dp_reduce_kernel, whose layout of threads it shares); a float2 holds gradient k of the crossings e and e + M/4
 constexpr int kFReduceCols = 32, kFReduceRows = 8;
 struct FramedReduceArgs {
@@ -646,6 +769,7 @@ struct FramedReduceArgs {
   const float2* wts;
   const int* count;
   int refuse;
+  const int* scales;   // null: 0
 };
 // columns [2 kFReduceCols blk, ..), two a thread (16-byte loads: with 8-byte ones a batch's 134 MB took 82 us, 20 at the
 // measured copy rate); the caller's threads meet before acc is used again
@@ -659,20 +783,42 @@ __device__ __forceinline__ void framed_reduce_block(const FramedReduceArgs& a, i
   const size_t stride = (size_t)L * np2 / 2;
   auto add = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
   float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+  // t is at the least scale of what it holds
+  const bool framed = __ldg(a.count) < a.refuse;
+  const int* sc = framed ? a.scales : nullptr;
+  int scale = kNoScale;
+  auto scale_of = [&](int c) { return sc ? __ldg(sc + c) : 0; };
+  auto take = [&](float4 x, int s) {
+    if (s != scale) {
+      const int to = min(s, scale);
+      const float fx = pow2f(max(to - s, -126)), ft = pow2f(max(to - scale, -126));
+      x = make_float4(x.x * fx, x.y * fx, x.z * fx, x.w * fx);
+      t = make_float4(t.x * ft, t.y * ft, t.z * ft, t.w * ft);
+      scale = to;
+    }
+    t = add(t, x);
+  };
+  __shared__ int row_scale[kRows];
   if (valid) {
     const float4* p = reinterpret_cast<const float4*>(a.partial) + idx0 / 2;
     int c = row;
     for (; c + 3 * kRows < nC; c += 4 * kRows) {
       const float4 a0 = __ldg(p + (size_t)c * stride), a1 = __ldg(p + (size_t)(c + kRows) * stride);
       const float4 a2 = __ldg(p + (size_t)(c + 2 * kRows) * stride), a3 = __ldg(p + (size_t)(c + 3 * kRows) * stride);
-      t = add(add(add(add(t, a0), a1), a2), a3);
+      const int s0 = scale_of(c), s1 = scale_of(c + kRows), s2 = scale_of(c + 2 * kRows), s3 = scale_of(c + 3 * kRows);
+      take(a0, s0);
+      take(a1, s1);
+      take(a2, s2);
+      take(a3, s3);
     }
-    for (; c < nC; c += kRows) t = add(t, __ldg(p + (size_t)c * stride));
+    for (; c < nC; c += kRows) take(__ldg(p + (size_t)c * stride), scale_of(c));
   }
   acc[row][col] = t;
+  if (col == 0) row_scale[row] = scale;   // (the block's first column is always valid, and a row's scale is that of all)
   __syncthreads();
   if (row != 0 || !valid) return;
-  for (int k = 1; k < kRows; ++k) t = add(t, acc[k][col]);
+  for (int k = 1; k < kRows; ++k) take(acc[k][col], row_scale[k]);
+  if (scale == kNoScale) scale = 0;
   const int l = idx0 / np2, sh = geo[2 * l] / 2, ln = geo[2 * l + 1];
   auto put = [&](int q, int k, float v) {
     if (q >= N / 2) return;
@@ -681,7 +827,7 @@ __device__ __forceinline__ void framed_reduce_block(const FramedReduceArgs& a, i
     *o = a.accumulate ? *o + v : v;
   };
   const int rem = idx0 - l * np2;
-  if (__ldg(a.count) >= a.refuse) {   // partials of the unframed body: (dJ/dth, dJ/dph) of one slot each
+  if (!framed) {   // partials of the unframed body: (dJ/dth, dJ/dph) of one slot each
     const int q0 = pos_slot(rem, M, G), q1 = pos_slot(rem + 1, M, G);
     put(q0, 0, t.x);
     put(q0, 1, t.y);
@@ -692,10 +838,12 @@ __device__ __forceinline__ void framed_reduce_block(const FramedReduceArgs& a, i
   // (th, th'), (ph, ph') of one pair of crossings
   const int pos = rem >> 1, j = pos % G, q = j * (M / 2) + pos / G;
   const float4 w = __ldg(reinterpret_cast<const float4*>(a.wts) + idx0 / 2);
-  put(q, 0, t.x * w.x);
-  put(q + M / 4, 0, t.y * w.y);
-  put(q, 1, t.z * w.z);
-  put(q + M / 4, 1, t.w * w.w);
+  const int k0 = min(scale, 120), k1 = min(scale - k0, 120);   // (beyond 2^-240 nothing is left)
+  const float s0 = pow2f(-k0), s1 = pow2f(-k1);
+  put(q, 0, t.x * w.x * s0 * s1);
+  put(q + M / 4, 0, t.y * w.y * s0 * s1);
+  put(q, 1, t.z * w.z * s0 * s1);
+  put(q + M / 4, 1, t.w * w.w * s0 * s1);
 }
 
 static __global__ void __launch_bounds__(256) framed_reduce_kernel(const FramedReduceArgs a) {

@@ -4,9 +4,13 @@
 
 namespace mg {
 
-// Frames start at 2^22, are due to start again below 2^-8 and do so at once below 2^-18: the products of two framed
-// fields stay within 2^44 and 2^-16 of the fields' own, the middle of the float range (2^-76 behind a cross state)
+// Frames start at 2^22, are due to start again below 2^-8 and do so at once below 2^-18; a layer may take one down by 2^-30
+// (a cross state), so they stay within 2^-48 and 2^22.
 constexpr int kFrameTop = 22, kFrameDue = -8, kFrameNow = -18;
+// Largest part of a vector as it enters, 2^22: with its 640 modes' energy in one (2^28) the products of two framed fields stay
+// below 2^102 and the sum of 2^20 vectors' below 2^122; behind a cross state a product 2^-35 of the largest keeps its bits
+constexpr int kFieldTop = 22;
+constexpr int kWarpScales = 12;            // ints of shared memory per warp (16-byte steps)
 constexpr int kFrameSeg = 16;              // layers per segment, about
 constexpr int kFrameBatch = 16;            // layers whose frames are held in shared memory at a time
 constexpr int kFrameThreads = 512;
@@ -48,6 +52,7 @@ struct FramedArgs : PropArgs {
   const float2* dfin;
   const int* fkinds;
   const int* count;
+  int* scales;                   // back-propagation: the CTA's partials are 2^this of their own size (null: fields as they are)
   int fcl;                       // layers per stage
   unsigned flb;                  // bytes of a layer's tile
   int refuse;                    // count from which on the mesh takes the unframed body
@@ -65,13 +70,13 @@ __host__ __device__ constexpr int framed_resc_rows(int CL) { return CL / 8 > 1 ?
 __host__ __device__ constexpr unsigned framed_layer_bytes(int op, int np2) { return (unsigned)np2 * (op == OP_BWD ? 24 : 16); }
 __host__ __device__ constexpr size_t framed_stage_bytes(unsigned lb, int np2, int CL) { return (size_t)CL * lb + (size_t)framed_resc_rows(CL) * np2 * 16; }
 // shared memory of a launch: [stages][a layer of zeros][BWD: per slot the W warps' gradients of CL layers, one layer beyond
-// the last][2 mbarriers per stage][state][step codes][RESCALEs per chunk]
+// the last][2 mbarriers per stage][state][warps' scales][step codes][RESCALEs per chunk]
 __host__ __device__ constexpr size_t framed_bars_offset(int op, unsigned lb, int np2, int W, int CL) {
   return kFrameStages * framed_stage_bytes(lb, np2, CL) + lb +
          (op == OP_BWD ? ((size_t)kFrameStages * W * CL + 1) * np2 * 8 : 0);
 }
 __host__ __device__ constexpr size_t framed_smem_bytes(int op, unsigned lb, int np2, int W, int CL, int L) {
-  return framed_bars_offset(op, lb, np2, W, CL) + 16 * kFrameStages + 16 + 4 * (size_t)(L + 8) + 4 * (size_t)((L + CL) / CL) * framed_resc_rows(CL);
+  return framed_bars_offset(op, lb, np2, W, CL) + 16 * kFrameStages + 16 + 4 * (size_t)kWarpScales * W + 4 * (size_t)(L + 8) + 4 * (size_t)((L + CL) / CL) * framed_resc_rows(CL);
 }
 
 }  // namespace mg

@@ -119,7 +119,7 @@ cudaError_t launch_prop_framed(int op, int M, int V, bool mix, const LaunchCfg& 
 cudaError_t launch_frames(const FrameArgs& a, int sms, cudaStream_t stream);
 cudaError_t launch_framed_reduce(const float2* partial, int nC, int L, int np2, int M, int G, int N, float* dp, int ldp,
                                  int accumulate, const int* geo, const float2* wts, const int* count, int refuse,
-                                 cudaStream_t stream);
+                                 const int* scales, cudaStream_t stream);
 // split launches (two CTA kinds per SM); instantiated only for the full-warp configurations in
 // split_instantiated()
 bool split_instantiated(int op, bool real, int M, int V, bool full, int gr);

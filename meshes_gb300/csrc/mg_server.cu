@@ -323,7 +323,7 @@ struct mg_server {
     std::vector<It> itf, itb;
     itf.reserve(n_if);
     itb.reserve(n_ib);
-    size_t ox = 0, og = 0, odp = 0, opt = 0;
+    size_t ox = 0, og = 0, odp = 0, opt = 0, osc = 0;
     t.o_y.resize(K);
     for (size_t i = 0, j = 0; i < K; ++i) {
       const Req& r = reqs[i];
@@ -362,6 +362,9 @@ struct mg_server {
         e.n_items = (int)ob.n; e.ldp = m.N / 2 * m.n_p;
         e.in0 = base + off_y + ox; e.in1 = base + off_gy + og; e.out0 = nullptr; e.out1 = base + off_gx + og;
         e.dp = reinterpret_cast<float*>(base + off_dp + odp); e.partial = base + off_pt + opt;
+        // (where the forward launch's items were: a request has no more of them in back-propagation, 4 bytes for 16)
+        db[j].scales = reinterpret_cast<int*>(base + off_if) + osc;
+        osc += ob.n;
         t.o_gx.push_back(off_gx + og);
         t.o_dp.push_back(off_dp + odp);
         add(itb, ob, j);
