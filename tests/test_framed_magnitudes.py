@@ -98,3 +98,36 @@ def test_vectors_without_a_scale():
     keep = (np.arange(28) != 7) & (np.arange(28) != 8)
     assert np.array_equal(x[keep], x0[keep]) and np.array_equal(gx[keep], gx0[keep])
     assert np.array_equal(x[8], x0[8]) and np.array_equal(gx[7], gx0[7])
+
+
+def test_batched_and_served():
+    """The persistent launches keep their items' scales as well: gradients 2^-100 of their size."""
+    from meshes_gb300.batched import BatchedMeshes
+    from meshes_gb300.serve import MeshServer
+    from test_batched import gpu_mesh
+    rng = np.random.default_rng(4)
+    oms = [_mesh(rng, 130, "cross", 40), _mesh(rng, 256, "few_cross", 40)]
+    xs, gs = [_fields(rng, om.N, 70) for om in oms], [_fields(rng, om.N, 70) for om in oms]
+    k = np.full(70, -100)
+    bm = BatchedMeshes([gpu_mesh(om) for om in oms], [70, 70])
+    assert bm.n_framed == 2
+    srv = MeshServer([gpu_mesh(om) for om in oms], mem_budget=256 << 20)
+    srv.start()
+    got = []
+    try:
+        for size in (0 * k, k):
+            for st, x, g in zip(bm.states, xs, gs):
+                st.x.copy_(torch.tensor(x))
+                st.gy.copy_(torch.tensor(_times(g, size)))
+            bm.forward()
+            bm.backward()
+            assert bm.check_status() == 0
+            got.append([(st.dp.cpu().numpy(), st.gx.cpu().numpy()) for st in bm.states])
+            fs = [srv.submit(i, x, _times(g, size)) for i, (x, g) in enumerate(zip(xs, gs))]
+            got[-1] += [f.result(timeout=60)[1:] for f in fs]
+    finally:
+        srv.stop()
+    for (dp0, gx0), (dp, gx) in zip(*got):
+        small = np.abs(dp0) < 2.0 ** -20
+        assert np.array_equal(gx, _times(gx0, k)) and np.array_equal(dp[~small], (dp0 * np.float32(2.0 ** -100))[~small])
+        assert not small.all() and np.all(np.abs(dp[small]) <= 2.0 ** -120)
