@@ -8,7 +8,8 @@ the segments in reverse, recomputes each segment's layer inputs from its checkpo
 to a (segment, B, N) buffer) and back-propagates through the segment from those stored inputs (one launch plus a
 deterministic reduction).  Each direction is one library call (mg_lossy_forward / mg_lossy_backward) that runs all its
 segments.  A segment is at least ceil(sqrt(L)) layers (about 2 sqrt(L) fields of memory instead of L) and as long as its
-stored inputs stay within SEGMENT_BYTES; work is one extra forward pass.
+stored inputs stay within SEGMENT_BYTES; work is one extra forward pass.  Where there is no memory for them, back-propagation
+takes segments of ceil(sqrt(L)) layers, for another forward pass.
 
 The crossing is given as its transfer matrices ``T`` (L, N/2, 2, 2), complex, in the reference's slot
 grid (gpu/mesh.py:77-81); ``mzi_generic_T`` builds them from (theta, phi) and the 14 error parameters
@@ -141,6 +142,8 @@ class LossyMesh:
 
     @property
     def segment(self) -> int:
+        """The shortest checkpoint spacing: the given one, or ceil(sqrt(L)), which a batch takes whose stored inputs would go
+        beyond ``SEGMENT_BYTES`` or, in back-propagation, find no memory (``segment_for``: what it takes otherwise)."""
         return self._segment or max(1, math.ceil(math.sqrt(max(self.L, 1))))
 
     # ---- plumbing
@@ -186,6 +189,10 @@ class LossyMesh:
         return LossyMeshFunction.apply(x, T, self)
 
 
+def _stored_inputs(layers: int, B: int, N: int, device) -> torch.Tensor:
+    return torch.empty((layers, B, N), dtype=torch.complex64, device=device)
+
+
 class LossyMeshFunction(torch.autograd.Function):
     """y = U(T) x for x (B, N) complex, T (L, N/2, 2, 2) complex; gradients to x and T."""
 
@@ -222,7 +229,18 @@ class LossyMeshFunction(torch.autograd.Function):
         if B > 0:
             wsf, nbf = mesh._build(OP_FWD, Tc, B) if L > 0 else (None, 0)
             wsb, nbb = mesh._build(OP_BWD_STORED, Tc, B) if L > 0 else (None, 0)
-            act = torch.empty((min(seg, max(L, 1)), B, N), dtype=torch.complex64, device=mesh.device)
+            try:
+                act = _stored_inputs(min(seg, max(L, 1)), B, N, mesh.device)
+            except torch.OutOfMemoryError:
+                # as many layers at a time as the shortest spacing has, from checkpoints of its own
+                if mesh.segment >= min(seg, L):
+                    raise
+                seg = mesh.segment
+                ckpt = torch.empty((-(-L // seg) - 1, B, N), dtype=torch.complex64, device=mesh.device)
+                check(load().mg_lossy_forward(N, L, B, mesh._geometry, seg, x.data_ptr(), g.data_ptr(),
+                                              ckpt.data_ptr() if ckpt.numel() else None, N, wsf, nbf,
+                                              _stream(mesh.device)), "mg_lossy_forward")
+                act = _stored_inputs(seg, B, N, mesh.device)
             gtmp = torch.empty_like(gy)
             check(load().mg_lossy_backward(N, L, B, mesh._geometry, seg, x.data_ptr(),
                                            ckpt.data_ptr() if ckpt.numel() else None, gy.data_ptr(), g.data_ptr(),

@@ -40,3 +40,27 @@ def test_shallow_meshes_with_long_segments(N, L, segment):
     from meshes_gb300.lossy import LossyMesh
     om, T, x, g = _case(N, L, 5)
     _check(om, T, x, g, LossyMesh(N, om.lens, om.shifts, segment=segment))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,segment", [(5, None), (300, 24)])
+def test_without_memory_for_the_stored_inputs(B, segment, monkeypatch):
+    """Back-propagation then runs by the shortest spacing; a spacing that the caller fixed stays (and the error with it)."""
+    from meshes_gb300 import lossy
+    om, T, x, g = _case(64, 40, B)
+    mesh = lossy.LossyMesh(64, om.lens, om.shifts, segment=segment)
+    stored, asked = lossy._stored_inputs, []
+
+    def scarce(layers, *args):
+        asked.append(layers)
+        if layers > 7:
+            raise torch.OutOfMemoryError("scarce")
+        return stored(layers, *args)
+    monkeypatch.setattr(lossy, "_stored_inputs", scarce)
+    if segment:
+        with pytest.raises(torch.OutOfMemoryError):
+            _check(om, T, x, g, mesh)
+        assert asked == [24]
+    else:
+        _check(om, T, x, g, mesh)
+        assert asked == [40, 7] and mesh.segment == 7 and mesh.segment_for(B) == 40
