@@ -56,6 +56,13 @@ extern "C" int mg_autotune(int op, int N, int L, int B, int crossing, int geomet
   if (geometry == MG_GEO_NN && !real && N > 64 && mg::framed_pays(op, lanes / 32, L, lanes / 2, B, sms) &&
       mg::framed_pick(op, lanes / 32, B, sms, &fc))
     cands.push_back(fc);
+  // (forward derivatives: also those of 6 and 12 modes per lane, 129 to 192 and 257 to 384 modes)
+  if (op == MG_OP_FWDDIFF && geometry == MG_GEO_NN && !real)
+    for (int M : {6, 12}) {
+      if (N <= 32 * (M == 6 ? 4 : 8) || N > 32 * M) continue;
+      for (int V : {1, 2, 4})
+        for (int W : {2, 4, 8}) cands.push_back(mg_config{M, V, W, 0, 0, 2});
+    }
   if (geometry == MG_GEO_FFT) cands.push_back(mg_config{0, 0, 0, 0, 0, 7});
 
   // scratch (stream-ordered, freed before returning): fields x, dx / g, y, dy / g_in, dJ/dp, an L2 flush

@@ -61,3 +61,12 @@ def test_autotune_argument_errors():
     assert lib.mg_autotune(0, 8, 2, 4, 0, 0, None, None, None, p.data_ptr(), 8, None, 0, 0, 0, ctypes.byref(best),
                            None, None, None, 0, None, st) == -1
     assert "mg_autotune" in _lib.last_error()
+
+
+@pytest.mark.parametrize("N,M", [(130, 6), (192, 6), (258, 12), (384, 12)])
+def test_derivative_tiles_of_the_heuristic_are_candidates(N, M):
+    """Forward derivatives run 6 or 12 modes per lane without a configuration; a recorded winner replaces that, so the tuner
+    has to have timed them."""
+    from meshes_gb300.autotune import tune
+    _, results = tune(1, N, 8, 64, crossing=0, reps=1)
+    assert {c[1] for c in results if c[0] == M} == ({1, 2, 4} if M == 6 else {1, 2})
