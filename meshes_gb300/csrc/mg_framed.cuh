@@ -23,8 +23,8 @@
 // Framed fields are 2^-22 to 2^48 of the fields' own (forward) or 2^-48 to 2^22 (back-propagation, the products of two of them
 // 2^-96 to 2^44), so every vector comes in times a power of two that brings its largest part to 2^kFieldTop and leaves by
 // its inverse: nothing overflows, or falls below the normal range, that does not without frames (but for products 2^35
-// times smaller than the largest of their warp's).  The factors are exact; results do not depend on them.  They cost 2 us of
-// a back-propagation launch (N = 256, B = 4096: 197 -> 199 us).
+// times smaller than the largest of their warp's).  The factors are exact; results do not depend on them.  They cost
+// a launch and its reduction up to 2 us (N = 256, B = 4096 back-propagation 205.8 -> 207.3 us, forward 69.3 -> 67.7).
 #pragma once
 #include "mg_frame.cuh"
 
@@ -463,34 +463,40 @@ __device__ __forceinline__ ulonglong2 frame_pair(const float2* __restrict__ d, i
 // CTA barrier by number: with MIX, warps of both kinds meet at it from their own copies of the body
 __device__ __forceinline__ void cta_sync() { asm volatile("barrier.cta.sync.aligned 0;" ::: "memory"); }
 
-// Sum of the W warps' staged gradients of a chunk (W a multiple of 4), in warp order, at the least of their scales, into this CTA's partials of the
-// layers from lo on: n float4 of consecutive layers.  turn: the chunk; the warps that the last round of a chunk leaves over
+// Sum of the W warps' staged gradients of a chunk (W a multiple of 4), in warp order, at the least of their scales, into this
+// CTA's partials of the layers from lo on: n float4 of consecutive layers.  Equal scales, nearly always, have a loop of their
+// own: with the factors in one loop for both, N = 400, B = 2432 took 393 us instead of 383.  turn: the chunk; the warps that the last round of a chunk leaves over
 // change with it (the same two of eight at M = 20: back-propagation at N = 600, B = 2048 727 us, in turns 684)
 __device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int W, int n, int turn, const int* scales,
                                          const int* scale, ulonglong2* out) {
   const int least = scales[0];
-  const bool one = least >= scales[1];
   int first = threadIdx.x + (64 * turn) % (int)blockDim.x;
   if (first >= (int)blockDim.x) first -= blockDim.x;
+  if (least >= scales[1]) {
+#pragma unroll 1
+    for (int idx = first; idx < n; idx += blockDim.x) {
+      uint32_t p = gst + (uint32_t)idx * 16u;
+      ulonglong2 t = make_ulonglong2(0, 0);
+#pragma unroll 1
+      for (int w = 0; w < W; w += 4, p += 4 * warp_bytes) {
+        const ulonglong2 a = lds16(p), b = lds16(p + warp_bytes), c = lds16(p + 2 * warp_bytes), d = lds16(p + 3 * warp_bytes);
+        t.x = padd(padd(padd(padd(t.x, a.x), b.x), c.x), d.x);
+        t.y = padd(padd(padd(padd(t.y, a.y), b.y), c.y), d.y);
+      }
+      out[idx] = t;
+    }
+    return;
+  }
 #pragma unroll 1
   for (int idx = first; idx < n; idx += blockDim.x) {
     uint32_t p = gst + (uint32_t)idx * 16u;
     ulonglong2 t = make_ulonglong2(0, 0);
 #pragma unroll 1
-    for (int w = 0; w < W; w += 4, p += 4 * warp_bytes) {
-      ulonglong2 a = lds16(p), b = lds16(p + warp_bytes), c = lds16(p + 2 * warp_bytes), d = lds16(p + 3 * warp_bytes);
-      if (!one) {
-        auto at = [&](ulonglong2& x, int i) {
-          const float f = pow2f(max(least - scale[kWarpScales * (w + i) + 8], -126));
-          x = make_ulonglong2(pmul(p_pack(f, f), x.x), pmul(p_pack(f, f), x.y));
-        };
-        at(a, 0);
-        at(b, 1);
-        at(c, 2);
-        at(d, 3);
-      }
-      t.x = padd(padd(padd(padd(t.x, a.x), b.x), c.x), d.x);
-      t.y = padd(padd(padd(padd(t.y, a.y), b.y), c.y), d.y);
+    for (int w = 0; w < W; ++w, p += warp_bytes) {
+      const ulonglong2 a = lds16(p);
+      const float f = pow2f(max(least - scale[kWarpScales * w + 8], -126));
+      t.x = padd(t.x, pmul(p_pack(f, f), a.x));
+      t.y = padd(t.y, pmul(p_pack(f, f), a.y));
     }
     out[idx] = t;
   }
@@ -783,41 +789,48 @@ __device__ __forceinline__ void framed_reduce_block(const FramedReduceArgs& a, i
   const size_t stride = (size_t)L * np2 / 2;
   auto add = [](float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); };
   float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-  // t is at the least scale of what it holds
+  // t is at the least scale of the row's partials
   const bool framed = __ldg(a.count) < a.refuse;
-  const int* sc = framed ? a.scales : nullptr;
-  int scale = kNoScale;
-  auto scale_of = [&](int c) { return sc ? __ldg(sc + c) : 0; };
-  auto take = [&](float4 x, int s) {
-    if (s != scale) {
-      const int to = min(s, scale);
-      const float fx = pow2f(max(to - s, -126)), ft = pow2f(max(to - scale, -126));
-      x = make_float4(x.x * fx, x.y * fx, x.z * fx, x.w * fx);
-      t = make_float4(t.x * ft, t.y * ft, t.z * ft, t.w * ft);
-      scale = to;
+  int scale = framed && a.scales ? kNoScale : 0, most = scale == 0 ? 0 : -kNoScale;
+  if (scale != 0) {
+    for (int c = row + kRows * (threadIdx.x & 31); c < nC; c += 32 * kRows) {
+      const int s = __ldg(a.scales + c);
+      scale = min(scale, s);
+      most = max(most, s);
     }
-    t = add(t, x);
+    scale = __reduce_min_sync(0xffffffffu, scale);
+    most = __reduce_max_sync(0xffffffffu, most);
+  }
+  auto times = [](float4 x, int k) {
+    const float f = pow2f(max(k, -126));
+    return make_float4(x.x * f, x.y * f, x.z * f, x.w * f);
   };
   __shared__ int row_scale[kRows];
   if (valid) {
     const float4* p = reinterpret_cast<const float4*>(a.partial) + idx0 / 2;
     int c = row;
+    if (scale < most)   // (seldom)
+      for (; c < nC; c += kRows) t = add(t, times(__ldg(p + (size_t)c * stride), scale - __ldg(a.scales + c)));
     for (; c + 3 * kRows < nC; c += 4 * kRows) {
       const float4 a0 = __ldg(p + (size_t)c * stride), a1 = __ldg(p + (size_t)(c + kRows) * stride);
       const float4 a2 = __ldg(p + (size_t)(c + 2 * kRows) * stride), a3 = __ldg(p + (size_t)(c + 3 * kRows) * stride);
-      const int s0 = scale_of(c), s1 = scale_of(c + kRows), s2 = scale_of(c + 2 * kRows), s3 = scale_of(c + 3 * kRows);
-      take(a0, s0);
-      take(a1, s1);
-      take(a2, s2);
-      take(a3, s3);
+      t = add(add(add(add(t, a0), a1), a2), a3);
     }
-    for (; c < nC; c += kRows) take(__ldg(p + (size_t)c * stride), scale_of(c));
+    for (; c < nC; c += kRows) t = add(t, __ldg(p + (size_t)c * stride));
   }
   acc[row][col] = t;
-  if (col == 0) row_scale[row] = scale;   // (the block's first column is always valid, and a row's scale is that of all)
+  if (col == 0) row_scale[row] = scale;
   __syncthreads();
   if (row != 0 || !valid) return;
-  for (int k = 1; k < kRows; ++k) take(acc[k][col], row_scale[k]);
+  for (int k = 1; k < kRows; ++k) {
+    const int s = row_scale[k], to = min(s, scale);
+    if (s == scale) {
+      t = add(t, acc[k][col]);
+    } else {
+      t = add(times(t, to - scale), times(acc[k][col], to - s));
+      scale = to;
+    }
+  }
   if (scale == kNoScale) scale = 0;
   const int l = idx0 / np2, sh = geo[2 * l] / 2, ln = geo[2 * l + 1];
   auto put = [&](int q, int k, float v) {
