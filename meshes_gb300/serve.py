@@ -100,7 +100,8 @@ class MeshServer:
         return _Resident(m, cls, M, V, G, WARPS * (32 // G) * V, G * M // 2, info, ws, n_mzi, self._frame(m, cls, geo))
 
     def _frame(self, m: MeshNetworkGPU, cls: int, geo):
-        """The mesh on framed tiles too (mg_server_frame): (configuration, workspace), or None."""
+        """The mesh on framed tiles too (mg_server_frame): (configuration, workspace), or None (no such tiles, or no memory
+        for them)."""
         if cls != BCLS_C8 or m.geometry != GEO_NN or m.N <= 64:
             return None
         cfg = _lib.config(8 if m.N > 128 else 4, 4, WARPS, 0, 0, 5)
@@ -109,7 +110,10 @@ class MeshServer:
                 info = plan(op, m.N, m.L, 1, m.crossing, m.geometry, cfg)
         except _lib.MeshLibraryError:                     # no framed tiles for it
             return None
-        ws = torch.empty(info.total, dtype=torch.uint8, device=m.device)
+        try:
+            ws = torch.empty(info.total, dtype=torch.uint8, device=m.device)
+        except torch.OutOfMemoryError:
+            return None
         st = torch.cuda.current_stream(m.device).cuda_stream
         s = m.p_splitter
         check(self.lib.mg_workspace_init(ws.data_ptr(), ws.numel(), st), "mg_workspace_init")
@@ -146,9 +150,15 @@ class MeshServer:
     # ---- lifecycle
     def start(self):
         torch.cuda.synchronize(self.device)               # tiles built before the scheduler reads them
-        h = self.lib.mg_server_create(self._descriptors(), len(self.res), self.mem_budget, self.n_streams,
-                                      self.max_per_tick, self.sms, self.smem[OP_FWD], self.smem[OP_BWD],
-                                      self.device.index or 0)
+        create = (lambda: self.lib.mg_server_create(
+            self._descriptors(), len(self.res), self.mem_budget, self.n_streams, self.max_per_tick, self.sms,
+            self.smem[OP_FWD], self.smem[OP_BWD], self.device.index or 0))
+        h = create()
+        if not h and any(r.framed is not None for r in self.res):
+            for r in self.res:                            # their memory may be what the arena lacks
+                r.framed = None
+            torch.cuda.empty_cache()
+            h = create()
         if not h:
             raise ServerError(_lib.last_error())
         try:

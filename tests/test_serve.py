@@ -7,6 +7,7 @@ import threading
 
 import numpy as np
 import pytest
+import torch
 
 from oracle import meshes_oracle as O
 
@@ -123,3 +124,45 @@ def test_client_thread_dying_midway_leaves_the_loop_draining():
     assert len(futs) == 31
     assert all(f.done() and not f.cancelled() and f.exception() is None for f in futs)
     assert srv.error is None
+
+
+def test_framed_tiles_give_way_to_memory(monkeypatch):
+    """A server whose framed tiles, or whose arena beside them, find no memory runs on the plain ones."""
+    from meshes_gb300.serve import MeshServer
+    rng = np.random.default_rng(91)
+    om = O.random_mesh(rng, 200, "clements", "mzi", 0.01)
+    mesh, x = gpu_mesh(om), O.unit_columns(rng, 200, 20).astype(np.complex64)
+    y_ref = O.propagate(om, x)
+
+    def result(srv):
+        srv.start()
+        try:
+            return srv.submit(0, x).result(timeout=60)
+        finally:
+            srv.stop()
+    empty, plain = torch.empty, MeshServer([mesh]).res[0].info[2].total
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: _refuse() if a and isinstance(a[0], int) and a[0] > plain else empty(*a, **k))
+    srv = MeshServer([mesh], mem_budget=64 << 20)
+    monkeypatch.undo()
+    assert srv.res[0].framed is None and O.rel_err(result(srv), y_ref) < 1e-5
+
+    class Scarce:
+        """The library, whose first server finds no memory."""
+        def __init__(self, lib):
+            self.lib, self.created = lib, 0
+
+        def __getattr__(self, name):
+            return getattr(self.lib, name)
+
+        def mg_server_create(self, *args):
+            self.created += 1
+            return self.lib.mg_server_create(*args) if self.created > 1 else None
+    srv = MeshServer([mesh], mem_budget=64 << 20)
+    assert srv.res[0].framed is not None
+    srv.lib = Scarce(srv.lib)
+    assert O.rel_err(result(srv), y_ref) < 1e-5
+    assert srv.res[0].framed is None and srv.lib.created == 2
+
+
+def _refuse():
+    raise torch.OutOfMemoryError("scarce")
