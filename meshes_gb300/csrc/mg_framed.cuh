@@ -492,11 +492,19 @@ __device__ __forceinline__ void f_reduce(uint32_t gst, uint32_t warp_bytes, int 
     uint32_t p = gst + (uint32_t)idx * 16u;
     ulonglong2 t = make_ulonglong2(0, 0);
 #pragma unroll 1
-    for (int w = 0; w < W; ++w, p += warp_bytes) {
-      const ulonglong2 a = lds16(p);
-      const float f = pow2f(max(least - scale[kWarpScales * w + 8], -126));
-      t.x = padd(t.x, pmul(p_pack(f, f), a.x));
-      t.y = padd(t.y, pmul(p_pack(f, f), a.y));
+    for (int w = 0; w < W; w += 4, p += 4 * warp_bytes) {
+      ulonglong2 x[4];
+      float f[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[i] = lds16(p + i * warp_bytes);
+        f[i] = pow2f(max(least - scale[kWarpScales * (w + i) + 8], -126));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        t.x = padd(t.x, pmul(p_pack(f[i], f[i]), x[i].x));
+        t.y = padd(t.y, pmul(p_pack(f[i], f[i]), x[i].y));
+      }
     }
     out[idx] = t;
   }
@@ -585,7 +593,8 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
         t = P2{pmul(two, psub(y.r, t.r)), pmul(two, psub(y.i, t.i))};
       });
     // one scale for all products of the warp, since its vectors' are added: that of the largest, in the range where a float
-    // holds it, a multiple of 16 (most launches then have one scale).  What a vector's own product is short of that, u and
+    // holds it, in steps of 16 (most launches then have one scale; unit vectors of 64 to 640 modes and gradients of their size
+    // want 46 to 54, the middle of a step).  What a vector's own product is short of that, u and
     // w bear half each, up to 2^80, within which neither loses bits (a product below 2^-160 of the largest counts as up to that).
     int ku[V], kw[V], all = kNoScale;
 #pragma unroll
@@ -596,7 +605,7 @@ __device__ __forceinline__ void framed_body(const FramedArgs& a, const FramedSme
 #pragma unroll
       for (int v = 0; v < V; ++v)
         if (ku[v] != kNoScale && kw[v] != kNoScale) all = min(all, ku[v] + kw[v]);
-      if (all != kNoScale) all = max(all, -80) & ~15;
+      if (all != kNoScale) all = ((max(all, -80) + 8) & ~15) - 8;
       if (lane == 0) {
         scale[8] = all;
         if (all != kNoScale) {
