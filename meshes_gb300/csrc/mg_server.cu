@@ -223,7 +223,8 @@ struct mg_server {
     return true;
   }
 
-  void pack(std::vector<Req> reqs) {
+  // plain: forward items of the meshes' own capacity on plain tiles, never more of them than request_bytes counts on
+  void pack(std::vector<Req> reqs, bool plain = false) {
     const size_t K = reqs.size();
     std::vector<size_t> gidx;
     for (size_t i = 0; i < K; ++i)
@@ -249,6 +250,7 @@ struct mg_server {
     };
     bool spread = true;
     auto forward = [&](const Req& r) {
+      if (plain) return shape(r, false, own_V(meshes[r.mesh]));
       const bool framed = framed_fwd[r.mesh].main != nullptr;
       const int V = framed ? 4 : own_V(meshes[r.mesh]);
       const Shape one = shape(r, framed, 1);
@@ -298,7 +300,20 @@ struct mg_server {
     const size_t off_pt = out_end;
     const size_t total = off_pt + n_pt;
     size_t dev_off = 0;
-    if (!arena.alloc(total, &dev_off)) {   // fragmentation: put the requests back in front
+    if (!arena.alloc(total, &dev_off)) {
+      if (inflight.empty() && !plain) {
+        // Nothing will be given back.  Framed items of 65 to 128 modes hold half as many vectors, and a list of them beyond what
+        // admission leaves for lists (100000 vectors: 75 of 66 KB) may be what an arena of just the request's size lacks.
+        // One request by itself first: whether it takes plain tiles then does not depend on the others.
+        if (K > 1) {
+          std::lock_guard<std::mutex> lk(qmu);
+          for (size_t i = K; --i > 0;) queue.push_front(reqs[i]);
+          queued += (long long)K - 1;
+        }
+        reqs.erase(reqs.begin() + 1, reqs.end());
+        return pack(std::move(reqs), K == 1);
+      }
+      // fragmentation: put the requests back in front
       std::lock_guard<std::mutex> lk(qmu);
       for (size_t i = K; i-- > 0;) queue.push_front(reqs[i]);
       queued += (long long)K;

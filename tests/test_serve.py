@@ -3,6 +3,7 @@
 Failures are made on the host (bad requests, an over-budget request, a cancelled request, a client
 thread that dies mid-stream); nothing here faults or hangs the GPU.
 """
+import ctypes
 import threading
 
 import numpy as np
@@ -162,6 +163,44 @@ def test_framed_tiles_give_way_to_memory(monkeypatch):
     srv.lib = Scarce(srv.lib)
     assert O.rel_err(result(srv), y_ref) < 1e-5
     assert srv.res[0].framed is None and srv.lib.created == 2
+
+
+def test_an_arena_of_just_the_requests_size():
+    """100000 vectors of 66 modes: the framed forward items' list is 24 KB longer than the plain ones', which the arena has no
+    room for beside the request's fields; it is served all the same, after a small one that came with it."""
+    from meshes_gb300.serve import MeshServer
+    rng = np.random.default_rng(92)
+    lens, shifts = O.clements_geometry(66)
+    om = O.OracleMesh(N=66, L=2, crossing="mzi", lens=list(lens[:2]), shifts=list(shifts[:2]),
+                      p=rng.uniform(0, 2 * np.pi, (2, 33, 2)).astype(np.float32),
+                      s=rng.normal(0, 0.02, (2, 33, 2)).astype(np.float32))
+    mask = om.active_mask()
+    om.p[~mask] = 0
+    om.s[~mask] = 0
+    b = 100000
+    x = O.unit_columns(rng, 66, b).astype(np.complex64)
+    gy = O.unit_columns(rng, 66, b).astype(np.complex64)
+    mesh, need = gpu_mesh(om), ctypes.c_size_t()
+    srv = MeshServer([mesh], mem_budget=16 << 20)
+    assert srv.res[0].framed is not None
+    srv.start()
+    try:
+        assert srv.lib.mg_server_request_bytes(srv.handle, 0, b, 1, ctypes.byref(need)) == 0
+    finally:
+        srv.stop()
+    srv = MeshServer([mesh], mem_budget=need.value + 65536 + 2048)
+    srv.start()
+    try:
+        small = srv.submit(0, x[:5])
+        big = srv.submit(0, x, gy)
+        y, dp, gx = big.result(timeout=60)
+        assert O.rel_err(small.result(timeout=60), O.propagate(om, x[:5])) < 1e-5
+    finally:
+        srv.stop(drain=False)
+    y_ref = O.propagate(om, x)
+    G, _, gx_ref = O.vjp_unitary(om, y_ref, gy)
+    assert O.rel_err(y, y_ref) < 1e-5 and O.rel_err(gx, gx_ref) < 1e-5
+    assert O.rel_err(dp.reshape(om.p.shape), O.contract_dp(om, G)) < 1e-5
 
 
 def _refuse():
