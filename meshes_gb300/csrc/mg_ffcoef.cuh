@@ -68,8 +68,10 @@ __device__ __forceinline__ ffz ffz_mul(ffz a, ffz b) {
 }
 __device__ __forceinline__ float2 ffz_round(ffz a) { return make_float2(ff_round(a.x), ff_round(a.y)); }
 
-// sin and cos of a float x with |x| < 400 in float-float; returns false (nothing written) beyond
-__device__ __forceinline__ bool ff_sincos(float x, ff* s, ff* c) {
+// sin and cos of a float x with |x| < 400 in float-float; returns false (nothing written) beyond.  The cosine's tail in float
+// is good to 2e-13; fine (uniform over the launch): one more of its terms in float-float, to 2e-15, which the derivative tiles take,
+// whose former form in double precision was good to 2e-14 (N = 130, 130 layers: no time that can be measured).
+__device__ __forceinline__ bool ff_sincos(float x, ff* s, ff* c, bool fine = false) {
   if (!(fabsf(x) < 400.f)) return false;
   // Cody-Waite: pi/2 = P1 + P2 + P3 (residual 1.2e-18); k * P1, k * P2 exact for |k| < 256
   constexpr float P1 = 1.57080078125f, P2 = -4.4543994590640068e-06f, P3 = -5.5644315544167711e-11f;
@@ -86,9 +88,11 @@ __device__ __forceinline__ bool ff_sincos(float x, ff* s, ff* c) {
   ps = ff_add(ff{-0.166666672f, 4.96705388e-09f}, ff_mul(r2, ps));                     // -1/3!
   const ff sr = ff_add(r, ff_mul(ff_mul(r, r2), ps));
   // cos r = 1 + r^2 (-1/2 + r^2 (1/4! + r^2 (-1/6! + r^2 q)))
-  const float qc = __fmaf_rn(t, __fmaf_rn(t, __fmaf_rn(t, -1.14707454e-11f, 2.08767559e-09f), -2.755732e-07f),
-                             2.48015876e-05f);
-  ff pc = ff_add(ff{-0.00138888892f, 3.36310944e-11f}, ff_mulf(r2, qc));                // -1/6! + r^2 q
+  const float q10 = __fmaf_rn(t, __fmaf_rn(t, -1.14707454e-11f, 2.08767559e-09f), -2.755732e-07f);
+  ff pc;
+  if (fine) pc = ff_mul(r2, ff_add(ff{2.48015876e-05f, -3.406996e-13f}, ff_mulf(r2, q10)));   // r^2 (1/8! + r^2 q)
+  else pc = ff_mulf(r2, __fmaf_rn(t, q10, 2.48015876e-05f));
+  pc = ff_add(ff{-0.00138888892f, 3.36310944e-11f}, pc);                               // -1/6! + r^2 q
   pc = ff_add(ff{0.0416666679f, -1.24176347e-09f}, ff_mul(r2, pc));                    // 1/4!
   pc = ff_add(ff{-0.5f, 0.f}, ff_mul(r2, pc));                                         // -1/2!
   const ff cr = ff_add(ff{1.f, 0.f}, ff_mul(r2, pc));
@@ -166,7 +170,7 @@ __device__ __forceinline__ bool mzi_T_ff_quad(float th, float ph, float al, floa
   const unsigned qmask = 0xFu << base;
   const float x = sub == 0 ? 0.5f * th : (sub == 1 ? ph : (sub == 2 ? al : be));
   ff s = {0.f, 0.f}, c = {1.f, 0.f};
-  int ok = ff_sincos(x, &s, &c) ? 1 : 0;
+  int ok = ff_sincos(x, &s, &c, dth != nullptr) ? 1 : 0;
   ok &= __shfl_xor_sync(qmask, ok, 1);
   ok &= __shfl_xor_sync(qmask, ok, 2);
   if (!ok) return false;

@@ -2,6 +2,8 @@
 the oracle's complex128 derivatives - phases at their extremes and beyond the float-float range (400), splitters and
 none, pairs within a lane, across lanes and odd-shift.  Tolerance: two float32 products and their sum of entries rounded once,
 3 x 2^-24 of the direction's size, and 1e-9."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -59,3 +61,43 @@ def test_one_layer(N, shift, stride, splitters):
     assert lib.mg_read_status(ws.data_ptr(), 1, st) == 0
     size = np.abs(d).sum(axis=2).max()
     assert np.abs(dy.cpu().numpy() - want).max() <= 3 * 2.0 ** -24 * size + 1e-9
+
+
+def test_float_float_is_no_further_off_than_double():
+    """dT/dth and T of 131072 slots, alone and rounded once to float32.  Where that is not the nearest float, the value before the
+    rounding lay on the wrong side of the middle between two, by as much as the error goes beyond the nearest float's.  Bound:
+    two sines or cosines of the product off by 2e-14 (where the double-precision form stops its series, and the float tail of the
+    float-float sine ends) and ten operations of 2^-48."""
+    from meshes_gb300 import _lib
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    N = L = 256
+    h, cfg, info = N // 2, _lib.config(8, 2, 4, 8, 0, 2), _lib.mg_plan_info()
+    assert lib.mg_plan(1, N, L, 64, 0, 0, _lib.cfg_ptr(cfg), ctypes.byref(info)) == 0, _lib.last_error()
+    M, G = info.M, info.G
+    lens, shifts = (torch.full((L,), v, dtype=torch.int32, device="cuda") for v in (h, 0))
+    beyond = 0.0
+    for seed in (8, 9, 10, 11):
+        rng = np.random.default_rng(seed)
+        p, s = rng.uniform(-7, 7, (L, h, 2)).astype(np.float32), rng.normal(0, 0.3, (L, h, 2)).astype(np.float32)
+        d = np.zeros_like(p)
+        d[..., 0] = 1
+        pd, sd, dd = (torch.tensor(a.reshape(-1), device="cuda") for a in (p, s, d))
+        ws = torch.zeros(info.total, dtype=torch.uint8, device="cuda")
+        _lib.check(lib.mg_build_tiles(1, N, L, 0, lens.data_ptr(), shifts.data_ptr(), None, 0, pd.data_ptr(), N, sd.data_ptr(), N,
+                                      dd.data_ptr(), None, None, 64, _lib.cfg_ptr(cfg), ws.data_ptr(), info.total, st), "tiles")
+        raw = ws.cpu().numpy()[info.off_tiles:info.off_tiles + L * info.layer_bytes]
+        tile = raw.copy().view(np.float32).reshape(L, 2, M // 2, 2, G, 2, 2)     # (T or dT), e, row, lane, column
+        got = tile.transpose(0, 1, 4, 2, 3, 5, 6).reshape(L, 2, h, 2, 2, 2)
+        th, ph, al, be = (a.astype(np.float64) for a in (p[..., 0], p[..., 1], s[..., 0], s[..., 1]))
+
+        def T(th):
+            e, f, S, C = np.exp(0.5j * th), np.exp(1j * ph), np.sin(th / 2), np.cos(th / 2)
+            Sp, Cp, Sm, Cm = np.sin(al + be), np.cos(al + be), np.sin(al - be), np.cos(al - be)
+            return np.stack([e * f * (-C * Sp + 1j * S * Cm), e * (-S * Sm + 1j * C * Cp),
+                             e * f * (S * Sm + 1j * C * Cp), e * (-C * Sp - 1j * S * Cm)], -1).reshape(L, h, 2, 2)
+        for k, want in enumerate((T(th), 0.5j * (T(th) - T(th + np.pi)))):
+            want = np.stack([want.real, want.imag], -1)
+            err = np.abs(got[:, k] - want)
+            assert err.max() < 1e-6
+            beyond = max(beyond, float((err - np.abs(want.astype(np.float32) - want)).max()))
+    assert beyond <= 2 * 2e-14 + 10 * 2.0 ** -48
