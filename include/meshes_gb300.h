@@ -359,7 +359,7 @@ void mg_server_destroy(mg_server* s, int drain);
  * The reference back-propagates by inverting each layer with T^H (c/dot.cpp:75-80, gpu/backprop.cu),
  * which is exact only for unitary crossings; for lossy ones (crossing.py:444-508, gains g_ij) that
  * gradient is wrong.  These calls back-propagate from stored layer inputs instead, for checkpointed
- * adjoints that keep one input every ~sqrt(L) layers and recompute the rest segment by segment.
+ * adjoints that keep one input per segment of layers and recompute the rest segment by segment.
  * Both run layers [l0, l1) of tiles built earlier by mg_build_tiles for the same (N, L, crossing,
  * geometry, cfg; B as for mg_propagate): op MG_OP_FWD with tiles of MG_OP_FWD, op MG_OP_BWD_STORED with tiles of
  * MG_OP_BWD_STORED (complex crossings only; MG_GENERIC takes T per slot from Tgen and needs no Dgen).

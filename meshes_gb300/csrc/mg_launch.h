@@ -78,12 +78,12 @@ cudaError_t launch_prop_perm(int op, bool real, int M, int V, int gr, const Laun
 // nn_instantiated(), uniform or split (mg_prop_nn.cu)
 bool nn_instantiated(int op, bool real, int M, int V, int gr, bool full, bool split);
 // the small-mesh tiles among them (complex, full warp, few modes and vectors per lane, so that a small batch
-// spreads over more schedulers; forward, and back-propagation at 4 x 2; mg_prop_nn_small.cu)
+// spreads over more schedulers; forward and back-propagation; mg_prop_nn_small.cu)
 bool nn_small_instantiated(int op, bool real, int M, int V, int gr, bool full);
 cudaError_t launch_prop_nn_small(int op, int gr, int M, int V, const LaunchCfg& lc, const PropArgs& a);
 bool nn_raw_instantiated(int M, int V);
 cudaError_t launch_prop_nn_raw(int M, int V, const LaunchCfg& lc, const PropArgs& a);
-// stored-activation kernels (GR 4) of nearest-neighbour meshes with a vector over the whole warp, N <= 128
+// stored-activation kernels (GR 4) of nearest-neighbour meshes with a vector over the whole warp, N <= 256
 // (mg_prop_stored_nn.cu)
 bool stored_nn_instantiated(int op, int M, int V);
 cudaError_t launch_prop_stored_nn(int op, int M, int V, const LaunchCfg& lc, const PropArgs& a);

@@ -1,5 +1,5 @@
 // Nearest-neighbour instantiations for small meshes and batches (Clements or Reck, complex, a vector over the 32
-// lanes of a warp): forward with 2, 4 or 8 modes and 1 to 4 vectors per lane, and back-propagation with 2 or 4 modes
+// lanes of a warp): forward with 2 to 16 modes and 1 to 4 vectors per lane, and back-propagation with 2 or 4 modes
 // and 1 or 2 vectors per lane (through dJ/dT: mg_prop_nn_raw.cu).  A call on a small mesh is latency-bound - at
 // N=64, B=1024 the default 2-mode x 4-vector forward tile gives 256 warps for 608 schedulers, one warp per busy
 // scheduler - so fewer vectors per lane put more warps on more schedulers.
