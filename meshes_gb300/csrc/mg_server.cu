@@ -8,9 +8,9 @@
 //     a fixed device arena (admission by free device memory) and the tick has slots left;
 //   * packs them: one pinned staging buffer holds the per-request descriptors and work items (items
 //     sorted longest first), the queue heads and the inputs; one host->device copy, one persistent
-//     forward launch over all admitted requests (mg_batched_propagate), one persistent back-propagation
-//     launch and a deterministic gradient reduction for the gradient requests, one device->host copy of
-//     every result, one event;
+//     forward launch over all admitted requests (mg_batched_small), one persistent back-propagation
+//     launch (mg_batched_propagate where no request is framed) and a deterministic gradient reduction
+//     for the gradient requests, one device->host copy of every result, one event;
 //   * rotates over several streams, so a tick starts while earlier ones are still on the GPU; at most
 //     one tick per stream is in flight, so under load the queue gathers requests into larger ticks.
 // Each request's work items cover only its own vectors, so its result does not depend on the mix.
